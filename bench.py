@@ -356,11 +356,9 @@ def grad_report(fb, si, MOc, nocc, fp64_peak, reps=3):
     n, naux = si.n, si.naux
     npad = st["npad"]
     noccp = (nocc + 15) // 16 * 16
-    te = st["ntile"] * 4096
-    chunked = st["grad_qchunk"] < naux
-    flops = {"x_recompute": 2.0 * noccp * npad * npad * naux if chunked else 0.0,
-             "y_t": 4.0 * noccp * noccp * npad * naux, "gamma": 2.0 * te * noccp * naux,
-             "d3c_M_gamma": 2.0 * te * naux * naux, "g_gamma_B": 2.0 * te * naux * naux, "dV_MtGM": 4.0 * naux ** 3}
+    pairs = nocc * (nocc + 1) // 2 + 1  # packed (i, j), and the row of w
+    flops = {"y_t": 2.0 * noccp * nocc * npad * naux, "gamma": 2.0 * pairs * naux * naux + 2.0 * n * nocc * nocc * naux,
+             "d3c_M_gamma": 1.0 * n * (n + 1) * nocc * naux, "dV_MtGM": 2.0 * pairs * naux * naux}
     stages = {}
     for k, ms in st["grad_stages"].items():
         e = {"ms": ms}
@@ -370,17 +368,16 @@ def grad_report(fb, si, MOc, nocc, fp64_peak, reps=3):
         stages[k] = e
     top = max((k for k in stages if k in flops), key=lambda k: stages[k]["ms"])
     return {"wall_ms": 1e3 * wall, "device_ms": st["ms_grad_total"], "aux_chunk": st["grad_qchunk"],
-            "recompute_path": bool(chunked), "stages": stages, "top_stage": top,
+            "stages": stages, "top_stage": top,
             "flops": sum(flops.values()), "fp64_peak_tflops": fp64_peak,
             "what": "rijk_grad through the C ABI: E, dE/dC, dE/d(P|mu nu) (packed) and dE/d(P|Q) to host memory; "
-                    "device_ms = its kernels before the host copies (stage events), wall_ms includes the copies "
-                    "(%.2f GB, into pageable arrays reused between calls) and the call's device buffer allocation"
+                    "device_ms = its stages (events; d3c_M_gamma includes its blocks' copies to the host), wall_ms includes "
+                    "every copy (%.2f GB, into pageable arrays reused between calls)"
                     % ((n * (n + 1) // 2 * naux + naux * naux) * 8 / 1e9)}
 
 
 def c40h82_grad(seed, dev, fp64_peak, chunk=1200):
-    """The C40H82 cc-pVDZ adjoint case: mixed -> FP64 SCF, then rijk_grad with Gamma in aux chunks and
-    X^Q recomputed in tiles (the path taken when HBM cannot hold Gamma for every aux function)."""
+    """The C40H82 cc-pVDZ adjoint case: mixed -> FP64 SCF, then rijk_grad with Y^Q in aux chunks."""
     from nopt_b200 import rijk
     si, _, _ = build_system("c40h82_dz", seed, ri_integrals=False)
     with rijk.FockBuilder(dev.index) as fb:

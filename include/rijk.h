@@ -92,9 +92,9 @@ typedef struct {
   int kernels_setup_ints; /* integral kernels it launched                                    */
   long q0, nq;            /* aux functions [q0, q0 + nq) held (all of them unless sliced)      */
   long grad_qchunk;       /* aux functions per chunk of the last rijk_grad (naux: one chunk)    */
-  /* Device time of the stages of the last rijk_grad, summed over its aux chunks (with profiling
-   * on): [0] the FP64 Fock build, energy and dE/dC, [1] X^Q recomputed in tiles (0 unless chunked),
-   * [2] Y^Q and T^Q, [3] Gamma, [4] dE/d(P|mu nu) = M^T Gamma, [5] G = Gamma B, [6] -M^T G M.      */
+  /* Device time of the stages of the last rijk_grad (with profiling on): [0] the FP64 Fock build,
+   * energy and dE/dC, [1] 0, [2] Y^Q = X^Q C^T, [3] Z^P = sum_Q M_QP Y^Q and C^T Z^P,
+   * [4] dE/d(P|mu nu) with its copies to the host, [5] 0, [6] dE/d(P|Q) from Z.                     */
   double ms_grad_stage[7];
   double ms_grad_total;   /* device time of rijk_grad before its host copies (profiling on)     */
 } rijk_stats_t;
@@ -362,9 +362,8 @@ int rijk_mo_ints_aaag(rijk_ctx* ctx, double* MO_INTS, const double* MO_VEC, long
 int rijk_soscf_hess_ints(rijk_ctx* ctx, double* aa_J, double* aa_K, const double* MO_VEC, long n_c, long n_a,
                          long n_mo);
 
-/* Aux functions per chunk of rijk_grad's Gamma stage (0, the default: all of them when HBM holds
- * Gamma for every aux function, else as many as it holds).  Below naux, each chunk's
- * half-transformed tensor is recomputed in tiles instead of read from the stored one. */
+/* Aux functions per chunk of rijk_grad's Y^Q stage (0, the default: all of them at once); the
+ * derivatives do not depend on it beyond rounding. */
 int rijk_set_grad_chunk(rijk_ctx* ctx, long q_per_chunk);
 
 /* Adjoint of the Fock build (no reference counterpart; the reference differentiates by finite

@@ -14,14 +14,19 @@
 //     dE/d(P|Q)    = -(M^T G M)_PQ,  G_QR = (1/2) sum_{mu nu} Gamma^Q_{mu nu} B^R_{mu nu}
 // (E depends on the metric only through V^-1 = M^T M, for either metric form).
 //
-// Device work, FP64 throughout, every contraction on hand-written DMMA kernels: one FP64 Fock build
-// (which leaves w and the half-transformed XT in the context), then, over chunks of aux functions,
-// the products Y^Q = X^Q C^T and T^Q = Y^Q C for every Q of the chunk at once (k_gemm_f64), k_gamma_f64
-// forming the packed Gamma tiles Gamma^Q_tile = 4 w_Q D_tile - 2 T^Q_rows Ct_cols^T, and two contractions of
-// the chunk of Gamma: with M, written straight into the packed pair layout of dE/d(P|mu nu)
-// (accumulated over chunks), and with B, the chunk's rows of G (diagonal tiles weighted 1/2).  When
-// HBM cannot hold Gamma for every aux function at once, each chunk's X^Q is recomputed in tiles
-// from B instead of read from the stored tensor.
+// Gamma^Q depends on Q only through w_Q and the n_c x n_c matrix Y^Q, so neither derivative needs Gamma
+// itself.  With the metric factor applied to those, u_P = sum_Q M_QP w_Q and Z^P = sum_Q M_QP Y^Q,
+//     dE/d(P|mu nu) = 4 u_P D_{mu nu} - 2 (C^T Z^P C)_{mu nu}
+//     dE/d(P|Q)     = sum_ij Z^P_ij Z^Q_ij - 2 u_P u_Q
+// (from G_QR = 2 w_Q w_R - sum_ij Y^Q_ij Y^R_ij, as <D, B^R> = w_R and C B^R C^T = Y^R).  The contractions with
+// the metric then run over n_c (n_c + 1) / 2 values per aux function instead of the n (n + 1) / 2 of Gamma.
+//
+// Device work, FP64 throughout, every contraction on the hand-written DMMA GEMM: one FP64 Fock build
+// (which leaves w and the half-transformed XT in the context), Y^Q = X^Q C^T over chunks of aux functions,
+// Z and u by one GEMM with M (the pairs i >= j packed, u as one more row), dE/d(P|Q) by one GEMM over the
+// packed pairs, the first index of C^T Z C by one GEMM, and the second by one GEMM per orbital row mu, whose
+// epilogue writes the packed pair rows.  Those rows leave in blocks: the copy of one block to the host runs
+// while the next is formed, so the device never holds the whole derivative.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -34,80 +39,35 @@
 namespace rijk {
 namespace {
 
-constexpr int G_THREADS = 128;
-
-// Gamma[Q][t][r][c] = 4 w_Q D[mu][nu] - 2 sum_i T^Q[mu][i] Ct[nu][i], tile t = (I, J), I >= J.
-// Tt: [(Q, i)][npad] = T^Q transposed (row (Q, i), mu contiguous); Ct: [npad][noccp]; D: n x n.
-constexpr int G_ASTAGE = (64 * LDK > KC * LDM) ? 64 * LDK : KC * LDM;
-__global__ void __launch_bounds__(G_THREADS)
-    k_gamma_f64(const double* __restrict__ Tt, const double* __restrict__ Ct, const double* __restrict__ D,
-                const double* __restrict__ w, long n, long npad, long noccp, long tile_elems,
-                double* __restrict__ Gamma) {
-  extern __shared__ __align__(16) double smem_g[];
-  double* sA[2] = {smem_g, smem_g + G_ASTAGE};
-  double* sB[2] = {smem_g + 2 * G_ASTAGE, smem_g + 2 * G_ASTAGE + 64 * LDK};
-  const long t = blockIdx.x, Q = blockIdx.y;
-  long I, J;
-  tri_decode(t, I, J);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  const double* Ar = Tt + Q * noccp * npad + I * TILE;  // A(mu, i) = Ar[i * npad + mu]: staged [i][mu]
-  const double* Br = Ct + J * TILE * noccp;
-  auto load = [&](int stage, long k0) {
-#pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      int idx = tid + it * G_THREADS;
-      int ka = idx >> 5, pa = idx & 31;  // A: k row (i) 0..31, mu pair 0..31
-      bool oka = k0 + ka < noccp;
-      cp_async16(&sA[stage][ka * LDM + pa * 2], oka ? Ar + (k0 + ka) * npad + pa * 2 : Tt, oka);
-      int row = idx >> 4, seg = idx & 15;  // B: row nu 0..63, i pair 0..15
-      long k = k0 + seg * 2;
-      bool ok = k < noccp;
-      cp_async16(&sB[stage][row * LDK + seg * 2], ok ? Br + row * noccp + k : Ct, ok);
-    }
-  };
-  double acc[4][4][2];
-  zero_acc(acc);
-  const long nk = (noccp + KC - 1) / KC;
-  load(0, 0);
-  cp_async_commit();
-  for (long kc = 0; kc < nk; ++kc) {
-    if (kc + 1 < nk) {
-      load(static_cast<int>((kc + 1) & 1), (kc + 1) * KC);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    warp_mma_chunk<4, 4, false>(acc, sA[kc & 1], sB[kc & 1], wm * 32, wn * 32, lane);
-    __syncthreads();
-  }
-  const int g = lane >> 2, tq = lane & 3;
-  const double wq4 = 4.0 * w[Q];
-  double* out = Gamma + Q * tile_elems + t * TILE2;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = wm * 32 + i * 8 + g;
-    const long mu = I * TILE + r;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = wn * 32 + j * 8 + 2 * tq;
-      const long nu = J * TILE + c;
-      double d0 = (mu < n && nu < n) ? D[mu * n + nu] : 0.0;
-      double d1 = (mu < n && nu + 1 < n) ? D[mu * n + nu + 1] : 0.0;
-      *reinterpret_cast<double2*>(out + r * TILE + c) =
-          make_double2(wq4 * d0 - 2.0 * acc[i][j][0], wq4 * d1 - 2.0 * acc[i][j][1]);
-    }
+// Yp[Q][p] = Y[(Q, i)][j] for the pairs p = (i, j), i >= j, of aux functions q0 .. q0 + nq; Yp[Q][np] = w_Q.
+__global__ void k_pack_pairs(const double* __restrict__ Y, const double* __restrict__ w, long q0, long nq, long nocc,
+                             long noccp, long np, long ldp, double* __restrict__ Yp) {
+  for (long p = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; p < ldp;
+       p += static_cast<long>(gridDim.x) * blockDim.x) {
+    long i, j;
+    tri_decode(p, i, j);
+    for (long q = blockIdx.y; q < nq; q += gridDim.y)
+      Yp[(q0 + q) * ldp + p] = p < np ? Y[(q * noccp + i) * nocc + j] : p == np ? w[q0 + q] : 0.0;
   }
 }
 
-// Ct[nu][i] = C_{i nu} from the padded MOp[i][nu]
-__global__ void k_transpose_mo(const double* __restrict__ MOp, long noccp, long npad, double* __restrict__ Ct) {
-  long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  for (; idx < noccp * npad; idx += static_cast<long>(gridDim.x) * blockDim.x) {
-    long nu = idx / noccp, i = idx % noccp;
-    Ct[idx] = MOp[i * npad + nu];
+// From Z[p][P] (rows p = (i, j), i >= j, then u): the weighted rows Zw (1 on the diagonal i = j, 2 off it, -2 for
+// u), and the full square Zf[j][i][P] with zeros from naux to the even pitch ldP.
+__global__ void k_expand_pairs(const double* __restrict__ Z, long nocc, long np, long naux, long ldP,
+                               double* __restrict__ Zw, double* __restrict__ Zf) {
+  for (long p = blockIdx.y; p <= np; p += gridDim.y) {
+    long i, j;
+    tri_decode(p, i, j);
+    const double f = p == np ? -2.0 : i == j ? 1.0 : 2.0;
+    for (long P = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; P < ldP;
+         P += static_cast<long>(gridDim.x) * blockDim.x) {
+      const double z = P < naux ? Z[p * ldP + P] : 0.0;
+      if (Zw) Zw[p * ldP + P] = f * z;
+      if (Zf && p < np) {
+        Zf[(j * nocc + i) * ldP + P] = z;
+        if (i != j) Zf[(i * nocc + j) * ldP + P] = z;
+      }
+    }
   }
 }
 
@@ -201,12 +161,12 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
     return set_err(ctx, RIJK_ERR_STATE, "rijk_grad needs all aux functions in one context (no aux range)");
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
-  const long n = ctx->n, naux = ctx->naux, npad = ctx->npad, nt = ctx->nt, ntile = ctx->ntile;
-  const long nn = n * n, te = ntile * TILE2, noccp = round_up(nocc, 16), nauxp = round_up(naux, KC);
+  const long n = ctx->n, naux = ctx->naux, npad = ctx->npad;
+  const long nn = n * n, noccp = round_up(nocc, 16), nauxp = round_up(naux, KC);
   const size_t b_nn = nn * sizeof(double);
-  DeviceBuf dMO, dH, dD, dJ, dK, dF, dG, red, Y, Tb, Ct, Gam, Gm, T1, out;
+  DeviceBuf dMO, dH, dD, dJ, dK, dF, dG, red, Y, Yp, Z, Zw, Zf, dV, out[2];
   auto cleanup = [&]() {
-    DeviceBuf* all[] = {&dMO, &dH, &dD, &dJ, &dK, &dF, &dG, &red, &Y, &Tb, &Ct, &Gam, &Gm, &T1, &out};
+    DeviceBuf* all[] = {&dMO, &dH, &dD, &dJ, &dK, &dF, &dG, &red, &Y, &Yp, &Z, &Zw, &Zf, &dV, &out[0], &out[1]};
     for (DeviceBuf* b : all) release(*b);
   };
   auto chk = [&](int r) {
@@ -270,134 +230,118 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
     cleanup();
     return RIJK_OK;
   }
-  // Gamma and its contractions over chunks of aux functions [q0, q0 + qc).  X^Q comes from the
-  // tensor the FP64 build left in HBM when every chunk fits at once; otherwise (HBM short, or a
-  // chunk size set by rijk_set_grad_chunk) each chunk's X^Q is recomputed in tiles by the
-  // half-transform kernel, and only one chunk of X, Y, T and Gamma exists at a time.
+  // Y^Q over chunks of aux functions (rijk_set_grad_chunk; all at once by default), from the X the FP64 build
+  // left in XT.
   const long kdim = naux * noccp;
-  const long npair = n * (n + 1) / 2;
+  const long np = nocc * (nocc + 1) / 2, ldp = round_up(np + 1, 2), ldP = round_up(naux, 2);
   const double* MOp = static_cast<const double*>(ctx->MOp.p);
   const double* pM = static_cast<const double*>(ctx->M.p);  // row-major [Q][P], ld nauxp
-  if (dEdI3 && (rc = chk(ensure(ctx, out, static_cast<size_t>(npair) * naux * sizeof(double), "grad dI3"))))
+  const long qc = ctx->grad_qchunk > 0 ? std::min(ctx->grad_qchunk, naux) : naux;
+  const size_t b_pairs = static_cast<size_t>(np + 1) * ldP * sizeof(double);
+  // blocks of orbital rows of dE/d(P|mu nu), about 64 MB each and at least one row
+  const long blk = std::max<long>(n * naux, (64L << 20) / 8);
+  if ((rc = chk(ensure(ctx, Y, static_cast<size_t>(qc) * noccp * nocc * sizeof(double), "grad Y"))) ||
+      (rc = chk(ensure(ctx, Yp, static_cast<size_t>(naux) * ldp * sizeof(double), "grad Y pairs"))) ||
+      (rc = chk(ensure(ctx, Z, b_pairs, "grad Z"))))
     return rc;
-  if (dEdPQ && ((rc = chk(ensure(ctx, Gm, static_cast<size_t>(naux) * naux * sizeof(double), "grad G"))) ||
-                (rc = chk(ensure(ctx, T1, static_cast<size_t>(naux) * naux * sizeof(double), "grad T1")))))
+  if (dEdPQ && ((rc = chk(ensure(ctx, Zw, b_pairs, "grad weighted Z"))) ||
+                (rc = chk(ensure(ctx, dV, static_cast<size_t>(naux) * naux * sizeof(double), "grad dPQ")))))
     return rc;
-  if ((rc = chk(ensure(ctx, Ct, static_cast<size_t>(npad) * noccp * sizeof(double), "grad Ct")))) return rc;
-  k_transpose_mo<<<grid_of(noccp * npad), 256, 0, s>>>(MOp, noccp, npad, static_cast<double*>(Ct.p));
-  // bytes per aux function of one chunk: Y, T, Gamma (and X when recomputed)
-  const double per_q = 8.0 * (static_cast<double>(noccp) * noccp + static_cast<double>(npad) * noccp + te);
-  const double per_q_x = per_q + 8.0 * npad * noccp;
-  size_t free_b = 0, total_b = 0;
-  cudaMemGetInfo(&free_b, &total_b);
-  const double room = 0.85 * static_cast<double>(free_b) - 64.0 * 1024 * 1024;
-  long qc = ctx->grad_qchunk > 0 ? std::min(ctx->grad_qchunk, naux) : naux;
-  if (ctx->grad_qchunk <= 0 && per_q * naux > room)
-    qc = std::max<long>(1, std::min<long>(naux, static_cast<long>(room / per_q_x)));
-  const bool recompute = qc < naux;
-  if ((rc = chk(ensure(ctx, Y, static_cast<size_t>(qc) * noccp * noccp * sizeof(double), "grad Y"))) ||
-      (rc = chk(ensure(ctx, Tb, static_cast<size_t>(qc) * npad * noccp * sizeof(double), "grad T"))) ||
-      (rc = chk(ensure(ctx, Gam, static_cast<size_t>(qc) * te * sizeof(double), "grad Gamma"))))
+  if (dEdI3 && ((rc = chk(ensure(ctx, Zf, static_cast<size_t>(nocc) * nocc * ldP * sizeof(double), "grad Z square"))) ||
+                (rc = chk(ensure(ctx, out[0], blk * sizeof(double), "grad dI3 block"))) ||
+                (rc = chk(ensure(ctx, out[1], blk * sizeof(double), "grad dI3 block")))))
     return rc;
-  DeviceBuf Xc;
-  if (recompute && (rc = chk(ensure(ctx, Xc, static_cast<size_t>(npad) * qc * noccp * sizeof(double), "grad X chunk")))) {
-    release(Xc);
-    return rc;
-  }
-  double* pGam = static_cast<double*>(Gam.p);
   double* pY = static_cast<double*>(Y.p);
-  double* pT = static_cast<double*>(Tb.p);
-  const size_t gsmem = (2 * G_ASTAGE + 2 * 64 * LDK) * sizeof(double);
-  ensure_smem_limit(reinterpret_cast<const void*>(k_gamma_f64), gsmem);
+  double* pZ = static_cast<double*>(Z.p);
   for (long q0 = 0; q0 < naux; q0 += qc) {
     const long nq = std::min(qc, naux - q0);
-    const double* X;  // X^Q_{i nu} at X[nu * ldx + (Q - q0) * noccp + i]
-    long ldx;
-    if (recompute) {
-      launch_xform_f64(static_cast<const double*>(ctx->B.p) + q0 * te, MOp, nq, nt, noccp, static_cast<double*>(Xc.p), s);
-      X = static_cast<const double*>(Xc.p);
-      ldx = nq * noccp;
-      tm.mark(1);
-    } else {
-      X = static_cast<const double*>(ctx->XT.p) + q0 * noccp;
-      ldx = kdim;
-    }
-    {  // Y^Q[i][j] = sum_nu X^Q_{i nu} C_{j nu} (= C B^Q C^T), every Q of the chunk in one product:
-       // rows (Q, i) of X^T's columns are contiguous, so Y[(Q, i)][j] is one GEMM over nu
-      GemmF64Args g;
-      g.M = nq * noccp, g.N = noccp, g.K = npad;
-      g.A = X, g.lda = ldx, g.a_kmajor = false;
-      g.B = MOp, g.ldb = npad, g.b_kmajor = true;
-      g.C = pY, g.ldc = noccp;
-      gemm_f64(g, 1, s);
-    }
-    {  // T^Q transposed, Tt[(Q, i)][mu] = sum_j Y^Q[i][j] C_{j mu}: again one GEMM for the chunk
-      GemmF64Args g;
-      g.M = nq * noccp, g.N = npad, g.K = noccp;
-      g.A = pY, g.lda = noccp, g.a_kmajor = true;
-      g.B = MOp, g.ldb = npad, g.b_kmajor = false;
-      g.C = pT, g.ldc = npad;
-      gemm_f64(g, 1, s);
-    }
-    tm.mark(2);
-    dim3 grid(static_cast<unsigned>(ntile), static_cast<unsigned>(nq));
-    k_gamma_f64<<<grid, G_THREADS, gsmem, s>>>(pT, static_cast<const double*>(Ct.p), pD,
-                                               static_cast<const double*>(ctx->w.p) + q0, n, npad, noccp, te, pGam);
+    // Y^Q[i][j] = sum_nu X^Q_{i nu} C_{j nu} (= C B^Q C^T), every Q of the chunk in one product: rows (Q, i)
+    // of X^T's columns are contiguous
+    GemmF64Args g;
+    g.M = nq * noccp, g.N = nocc, g.K = npad;
+    g.A = static_cast<const double*>(ctx->XT.p) + q0 * noccp, g.lda = kdim, g.a_kmajor = false;
+    g.B = MOp, g.ldb = npad, g.b_kmajor = true;
+    g.C = pY, g.ldc = nocc;
+    gemm_f64(g, 1, s);
+    dim3 grid(static_cast<unsigned>((ldp + 255) / 256), static_cast<unsigned>(std::min<long>(nq, 1024)));
+    k_pack_pairs<<<grid, 256, 0, s>>>(pY, static_cast<const double*>(ctx->w.p), q0, nq, nocc, noccp, np, ldp,
+                                      static_cast<double*>(Yp.p));
+  }
+  tm.mark(2);
+  {  // Z[p][P] = sum_Q Y[Q][p] M_QP, the last row u_P = sum_Q w_Q M_QP
+    GemmF64Args g;
+    g.M = np + 1, g.N = naux, g.K = naux;
+    g.A = static_cast<const double*>(Yp.p), g.lda = ldp, g.a_kmajor = false;
+    g.B = pM, g.ldb = nauxp, g.b_kmajor = false;
+    g.C = pZ, g.ldc = ldP;
+    gemm_f64(g, 1, s);
+    k_expand_pairs<<<dim3(static_cast<unsigned>(std::min<long>((ldP + 255) / 256, 64)), static_cast<unsigned>(std::min<long>(np + 1, 32768))),
+                     256, 0, s>>>(pZ, nocc, np, naux, ldP, static_cast<double*>(Zw.p), static_cast<double*>(Zf.p));
+  }
+  tm.mark(3);
+  if (dEdPQ) {  // dE/d(P|Q) = sum_p Zw[p][P] Z[p][Q]
+    GemmF64Args g;
+    g.M = naux, g.N = naux, g.K = np + 1;
+    g.A = static_cast<const double*>(Zw.p), g.lda = ldP, g.a_kmajor = false;
+    g.B = pZ, g.ldb = ldP, g.b_kmajor = false;
+    g.C = static_cast<double*>(dV.p), g.ldc = naux;
+    gemm_f64(g, 1, s);
+    tm.mark(6);
+  }
+  if (dEdI3) {
+    // T[mu][i][P] = sum_j C_{j mu} Z[j][i][P], in XT's memory (X is not needed any more)
+    const long row = nocc * ldP;
+    if ((rc = chk(ensure(ctx, ctx->XT, static_cast<size_t>(n) * row * sizeof(double), "grad T")))) return rc;
+    double* pT = static_cast<double*>(ctx->XT.p);
+    GemmF64Args g;
+    g.M = n, g.N = row, g.K = nocc;
+    g.A = MOp, g.lda = npad, g.a_kmajor = false;
+    g.B = static_cast<const double*>(Zf.p), g.ldb = row, g.b_kmajor = false;
+    g.C = pT, g.ldc = row;
+    gemm_f64(g, 1, s);
     tm.mark(3);
-    if (dEdI3) {
-      // dE/d(P|mu nu) += sum_{Q in chunk} Gamma^Q_{mu nu} M_QP, straight into the packed pair rows
-      GemmF64Args g;
-      g.M = te, g.N = naux, g.K = nq;
-      g.A = pGam, g.lda = te, g.a_kmajor = false;
-      g.B = pM + q0 * nauxp, g.ldb = nauxp, g.b_kmajor = false;
-      g.C = static_cast<double*>(out.p), g.ldc = naux;
-      g.beta = q0 == 0 ? 0.0 : 1.0;
-      g.mode = GEMM_PAIRS;
-      g.n_ao = n;
-      gemm_f64(g, 1, s);
+    // rows mu of dE/d(P|mu nu) in blocks, each on its way to the host while the next one is formed
+    const double* pu = pZ + np * ldP;
+    auto tri = [](long m) { return m * (m + 1) / 2; };
+    long prev0 = -1, prev1 = -1;
+    int slot = 0;
+    auto copy_out = [&](long m0, long m1, int b) -> int {
+      cudaStreamWaitEvent(ctx->copy_stream, ctx->ev_blk[b], 0);
+      const int r = cuda_check(ctx, cudaMemcpyAsync(dEdI3 + tri(m0) * naux, out[b].p,
+                                                    static_cast<size_t>(tri(m1) - tri(m0)) * naux * sizeof(double),
+                                                    cudaMemcpyDeviceToHost, ctx->copy_stream), "D2H dI3 block");
+      cudaEventRecord(ctx->ev_out[b], ctx->copy_stream);
+      return r;
+    };
+    for (long m0 = 0; m0 < n && !rc; slot ^= 1) {
+      long m1 = m0 + 1;
+      while (m1 < n && (tri(m1 + 1) - tri(m0)) * naux <= blk) ++m1;
+      if (prev0 >= 0) cudaStreamWaitEvent(s, ctx->ev_out[slot], 0);  // the copy of the block before the last
+      GemmF64Args h;
+      h.M = m1, h.N = naux, h.K = nocc;
+      h.A = MOp, h.lda = npad, h.a_kmajor = false;
+      h.B = pT + m0 * row, h.ldb = ldP, h.sB = row, h.b_kmajor = false;
+      h.C = static_cast<double*>(out[slot].p), h.ldc = naux;
+      h.mode = GEMM_DPAIRS;
+      h.mu0 = m0, h.n_ao = n, h.D = pD, h.u = pu;
+      gemm_f64(h, m1 - m0, s);
+      cudaEventRecord(ctx->ev_blk[slot], s);
+      if (prev0 >= 0) rc = copy_out(prev0, prev1, slot ^ 1);
+      prev0 = m0;
+      prev1 = m1;
+      m0 = m1;
     }
     tm.mark(4);
-    if (dEdPQ) {
-      // rows q0.. of G_QR = 1/2 sum_{mu nu} Gamma^Q B^R over the full squares: each stored element
-      // of an off-diagonal tile once, of a diagonal tile one half
-      GemmF64Args g;
-      g.M = nq, g.N = naux, g.K = te;
-      g.A = pGam, g.lda = te, g.a_kmajor = true;
-      g.B = static_cast<const double*>(ctx->B.p), g.ldb = te, g.b_kmajor = true;
-      g.C = static_cast<double*>(Gm.p) + q0 * naux, g.ldc = naux;
-      g.kdiag = 1;
-      gemm_f64(g, 1, s);
-    }
-    tm.mark(5);
+    if (!rc) rc = copy_out(prev0, prev1, slot ^ 1);
   }
-  release(Xc);
-  release(Y);
-  release(Tb);
-  tm.mark(-1);  // the frees above wait on the host: that gap is not a stage
-  if (dEdPQ) {
-    // dE/dV = -M^T G M:  T1[Q][P'] = sum_R G[Q][R] M[R][P'];  out[P][P'] = -sum_Q M[Q][P] T1[Q][P']
-    GemmF64Args g;
-    g.M = naux, g.N = naux, g.K = naux;
-    g.A = static_cast<const double*>(Gm.p), g.lda = naux, g.a_kmajor = true;
-    g.B = pM, g.ldb = nauxp, g.b_kmajor = false;
-    g.C = static_cast<double*>(T1.p), g.ldc = naux;
-    gemm_f64(g, 1, s);
-    GemmF64Args h;
-    h.M = naux, h.N = naux, h.K = naux;
-    h.A = pM, h.lda = nauxp, h.a_kmajor = false;
-    h.B = static_cast<const double*>(T1.p), h.ldb = naux, h.b_kmajor = false;
-    h.C = static_cast<double*>(Gm.p), h.ldc = naux;
-    h.alpha = -1.0;
-    gemm_f64(h, 1, s);
-    tm.mark(6);
-    cudaMemcpyAsync(dEdPQ, Gm.p, static_cast<size_t>(naux) * naux * sizeof(double), cudaMemcpyDeviceToHost, s);
-  }
-  if (dEdI3)
-    cudaMemcpyAsync(dEdI3, out.p, static_cast<size_t>(npair) * naux * sizeof(double), cudaMemcpyDeviceToHost, s);
+  if (dEdPQ && !rc)
+    rc = cuda_check(ctx, cudaMemcpyAsync(dEdPQ, dV.p, static_cast<size_t>(naux) * naux * sizeof(double),
+                                         cudaMemcpyDeviceToHost, s), "D2H dPQ");
   ctx->stats.grad_qchunk = qc;
-  rc = cuda_check(ctx, cudaStreamSynchronize(s), "rijk_grad");
+  const int rc_s = cuda_check(ctx, cudaStreamSynchronize(s), "rijk_grad");
+  const int rc_c = cuda_check(ctx, cudaStreamSynchronize(ctx->copy_stream), "rijk_grad copies");
+  if (!rc) rc = rc_s ? rc_s : rc_c;
   if (!rc) tm.collect(ctx->stats);
   cleanup();
-  (void)nt;
   return rc;
 }

@@ -11,13 +11,10 @@
 //
 // Epilogues:
 //   GEMM_STORE  C[m ldc + n] = alpha acc (+ beta C when beta != 0)
-//   GEMM_PAIRS  the rows m are the elements of the packed lower block triangle (tile t = m / 4096,
-//               row r and column c inside it, (mu, nu) = (64 I + r, 64 J + c)); each element with
-//               mu >= nu, both below n_ao, goes to C[(mu (mu + 1) / 2 + nu) ldc + n] with weight 1 on
-//               the diagonal and 2 off it (a stored pair stands for (mu nu) and (nu mu)).
-// kdiag: the contraction index k runs over the packed triangle's elements, and products from a
-// diagonal tile get weight 1/2 (each off-diagonal stored element then counts once, each element of
-// a full-square sum over a diagonal tile once).
+//   GEMM_DPAIRS batch b stands for the orbital row mu = mu0 + b and the rows m for nu <= mu (others are left
+//               out): the packed pair row (mu nu), mu (mu + 1) / 2 + nu less that of (mu0 0), gets
+//               f (4 D[mu][nu] u[n] - 2 acc) with f = 1 on the diagonal and 2 off it (a stored pair stands
+//               for (mu nu) and (nu mu))
 #include <algorithm>
 
 #include "gemm_f64.cuh"
@@ -87,17 +84,13 @@ __device__ __forceinline__ void load_tile(double* sm, const double* __restrict__
 
 template <bool AK, bool BK>
 __device__ __forceinline__ void warp_mma_chunk_ab(double (&acc)[4][4][2], const double* __restrict__ sA,
-                                                  const double* __restrict__ sB, int m0, int n0, int lane, double sc) {
+                                                  const double* __restrict__ sB, int m0, int n0, int lane) {
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int k = 0; k < KC; k += 4) {
     double a[4], b[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) a[i] = AK ? sA[(m0 + i * 8 + g) * LDK + k + t] : sA[(k + t) * LDM + m0 + i * 8 + g];
-    if (sc != 1.0) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] *= sc;
-    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) b[j] = BK ? sB[(n0 + j * 8 + g) * LDK + k + t] : sB[(k + t) * LDM + n0 + j * 8 + g];
 #pragma unroll
@@ -117,6 +110,7 @@ __global__ void __launch_bounds__(GM_THREADS) k_gemm_f64(GemmF64Args p, long ntn
   const long tile = blockIdx.x;
   const long m0 = (tile / ntn) * 64, n0 = (tile % ntn) * 64;
   const long bz = blockIdx.y;
+  if (p.mode == GEMM_DPAIRS && m0 > p.mu0 + bz) return;  // a block of rows nu > mu
   const double* A = p.A + bz * p.sA;
   const double* B = p.B + bz * p.sB;
   double* C = p.C + bz * p.sC;
@@ -136,8 +130,6 @@ __global__ void __launch_bounds__(GM_THREADS) k_gemm_f64(GemmF64Args p, long ntn
     load(0, 0);
     cp_async_commit();
   }
-  long diag_t = -1;  // kdiag: the packed tile of the current chunk and its weight
-  double sc = 1.0;
   for (long kc = 0; kc < nk; ++kc) {
     if (kc + 1 < nk) {
       load(static_cast<int>((kc + 1) & 1), (kc + 1) * KC);
@@ -146,40 +138,28 @@ __global__ void __launch_bounds__(GM_THREADS) k_gemm_f64(GemmF64Args p, long ntn
     } else {
       cp_async_wait<0>();
     }
-    if (p.kdiag && (kc * KC) / TILE2 != diag_t) {  // a 32-chunk lies inside one 64 x 64 tile
-      diag_t = (kc * KC) / TILE2;
-      long I, J;
-      tri_decode(diag_t, I, J);
-      sc = I == J ? 0.5 : 1.0;
-    }
     __syncthreads();
-    warp_mma_chunk_ab<AK, BK>(acc, sA[kc & 1], sB[kc & 1], wm * 32, wn * 32, lane, sc);
+    warp_mma_chunk_ab<AK, BK>(acc, sA[kc & 1], sB[kc & 1], wm * 32, wn * 32, lane);
     __syncthreads();
   }
 
   const int g = lane >> 2, tq = lane & 3;
-  if (p.mode == GEMM_PAIRS) {
-    // the CTA's 64 rows are one row r of one stored tile t: (mu, nu) = (64 I + r, 64 J + c)
-    long I, J;
-    tri_decode(m0 / TILE2, I, J);
-    const long r = (m0 % TILE2) / TILE;
-    const long mu = I * TILE + r;
+  if (p.mode == GEMM_DPAIRS) {
+    const long mu = p.mu0 + bz;
+    const long first = mu * (mu + 1) / 2 - p.mu0 * (p.mu0 + 1) / 2;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const long c = wm * 32 + i * 8 + g;
-      const long nu = J * TILE + c;
-      if (m0 + c >= p.M || mu >= p.n_ao || nu >= p.n_ao || (I == J && c > r)) continue;
-      const double f = (mu == nu ? 1.0 : 2.0) * p.alpha;
-      double* row = C + (mu * (mu + 1) / 2 + nu) * p.ldc;
+      const long m = m0 + wm * 32 + i * 8 + g;
+      if (m > mu) continue;
+      const double f = m == mu ? 1.0 : 2.0;
+      const double d = 4.0 * p.D[mu * p.n_ao + m];
+      double* row = p.C + (first + m) * p.ldc;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const long n = n0 + wn * 32 + j * 8 + 2 * tq + h;
-          if (n >= p.N) continue;
-          double v = f * acc[i][j][h];
-          if (p.beta != 0.0) v += p.beta * row[n];
-          row[n] = v;
+          if (n < p.N) row[n] = f * (d * p.u[n] - 2.0 * acc[i][j][h]);
         }
       }
     }

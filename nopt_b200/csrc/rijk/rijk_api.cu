@@ -363,6 +363,10 @@ RIJK_API int rijk_create(rijk_ctx** out, int device) {
   }
   cudaEventCreateWithFlags(&ctx->ev_mo, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&ctx->ev_j, cudaEventDisableTiming);
+  for (int b = 0; b < 2; ++b) {
+    cudaEventCreateWithFlags(&ctx->ev_blk[b], cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&ctx->ev_out[b], cudaEventDisableTiming);
+  }
   {
     int least = 0, greatest = 0;
     cudaDeviceGetStreamPriorityRange(&least, &greatest);
@@ -418,7 +422,8 @@ RIJK_API int rijk_destroy(rijk_ctx* ctx) {
     cudaStreamDestroy(ctx->copy_stream);
   }
   if (ctx->j_stream) cudaStreamDestroy(ctx->j_stream);
-  cudaEvent_t evs[] = {ctx->ev0, ctx->ev1, ctx->ev2, ctx->ev3, ctx->ev_mo, ctx->ev_j, ctx->ev_pk, ctx->ev_jside};
+  cudaEvent_t evs[] = {ctx->ev0, ctx->ev1, ctx->ev2, ctx->ev3, ctx->ev_mo, ctx->ev_j, ctx->ev_pk, ctx->ev_jside,
+                       ctx->ev_blk[0], ctx->ev_blk[1], ctx->ev_out[0], ctx->ev_out[1]};
   for (cudaEvent_t ev : evs)
     if (ev) cudaEventDestroy(ev);
   for (cudaEvent_t ev : ctx->pev)

@@ -64,6 +64,8 @@ struct rijk_ctx {
   // the Coulomb and exchange kernels run
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t ev_mo = nullptr, ev_j = nullptr;
+  // rijk_grad's output blocks: formed (on the build's stream), copied out (on the copy stream)
+  cudaEvent_t ev_blk[2] = {}, ev_out[2] = {};
   // FP64 builds: the Coulomb pair runs on a high-priority stream beside the half-transform, in the
   // registers and shared memory its CTAs leave free on every SM (joined before the build ends)
   cudaStream_t j_stream = nullptr;
@@ -176,9 +178,9 @@ int noalloc_resolve(rijk_ctx* ctx);
 
 // ---- k_gemm.cu
 // C_b = alpha op(A_b) op(B_b) + beta C_b for b < batch (FP64 DMMA, 64 x 64 tiles); see k_gemm.cu for
-// the layouts and the GEMM_PAIRS epilogue.  K may be 0 (C = beta C).
+// the layouts and the GEMM_DPAIRS epilogue.  K may be 0 (C = beta C).
 constexpr int GEMM_STORE = 0;
-constexpr int GEMM_PAIRS = 1;
+constexpr int GEMM_DPAIRS = 1;
 struct GemmF64Args {
   long M = 0, N = 0, K = 0;
   const double* A = nullptr;
@@ -191,8 +193,10 @@ struct GemmF64Args {
   long ldc = 0, sC = 0;
   double alpha = 1.0, beta = 0.0;
   int mode = GEMM_STORE;
-  long n_ao = 0;       // GEMM_PAIRS: orbital functions
-  int kdiag = 0;       // 1: k runs over packed-triangle elements, diagonal tiles weighted 1/2
+  // GEMM_DPAIRS: the first orbital row, the orbital functions, the density (n_ao x n_ao), u_P
+  long mu0 = 0, n_ao = 0;
+  const double* D = nullptr;
+  const double* u = nullptr;
 };
 void gemm_f64(const GemmF64Args& p, long batch, cudaStream_t s);
 
