@@ -173,11 +173,11 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
     if (r) cleanup();
     return r;
   };
-  if ((rc = chk(ensure(ctx, dMO, nocc * n * sizeof(double), "grad MO"))) || (rc = chk(ensure(ctx, dH, b_nn, "grad H"))) ||
-      (rc = chk(ensure(ctx, dD, b_nn, "grad D"))) || (rc = chk(ensure(ctx, dJ, b_nn, "grad J"))) ||
-      (rc = chk(ensure(ctx, dK, b_nn, "grad K"))) || (rc = chk(ensure(ctx, dF, b_nn, "grad F"))) ||
-      (rc = chk(ensure(ctx, dG, nocc * n * sizeof(double), "grad dEdC"))) ||
-      (rc = chk(ensure(ctx, red, 1024 * sizeof(double), "grad reduce"))))
+  if ((rc = chk(ensure_tmp(ctx, dMO, nocc * n * sizeof(double), "grad MO"))) || (rc = chk(ensure_tmp(ctx, dH, b_nn, "grad H"))) ||
+      (rc = chk(ensure_tmp(ctx, dD, b_nn, "grad D"))) || (rc = chk(ensure_tmp(ctx, dJ, b_nn, "grad J"))) ||
+      (rc = chk(ensure_tmp(ctx, dK, b_nn, "grad K"))) || (rc = chk(ensure_tmp(ctx, dF, b_nn, "grad F"))) ||
+      (rc = chk(ensure_tmp(ctx, dG, nocc * n * sizeof(double), "grad dEdC"))) ||
+      (rc = chk(ensure_tmp(ctx, red, 1024 * sizeof(double), "grad reduce"))))
     return rc;
   double* pMO = static_cast<double*>(dMO.p);
   double* pD = static_cast<double*>(dD.p);
@@ -240,16 +240,16 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
   const size_t b_pairs = static_cast<size_t>(np + 1) * ldP * sizeof(double);
   // blocks of orbital rows of dE/d(P|mu nu), about 64 MB each and at least one row
   const long blk = std::max<long>(n * naux, (64L << 20) / 8);
-  if ((rc = chk(ensure(ctx, Y, static_cast<size_t>(qc) * noccp * nocc * sizeof(double), "grad Y"))) ||
-      (rc = chk(ensure(ctx, Yp, static_cast<size_t>(naux) * ldp * sizeof(double), "grad Y pairs"))) ||
-      (rc = chk(ensure(ctx, Z, b_pairs, "grad Z"))))
+  if ((rc = chk(ensure_tmp(ctx, Y, static_cast<size_t>(qc) * noccp * nocc * sizeof(double), "grad Y"))) ||
+      (rc = chk(ensure_tmp(ctx, Yp, static_cast<size_t>(naux) * ldp * sizeof(double), "grad Y pairs"))) ||
+      (rc = chk(ensure_tmp(ctx, Z, b_pairs, "grad Z"))))
     return rc;
-  if (dEdPQ && ((rc = chk(ensure(ctx, Zw, b_pairs, "grad weighted Z"))) ||
-                (rc = chk(ensure(ctx, dV, static_cast<size_t>(naux) * naux * sizeof(double), "grad dPQ")))))
+  if (dEdPQ && ((rc = chk(ensure_tmp(ctx, Zw, b_pairs, "grad weighted Z"))) ||
+                (rc = chk(ensure_tmp(ctx, dV, static_cast<size_t>(naux) * naux * sizeof(double), "grad dPQ")))))
     return rc;
-  if (dEdI3 && ((rc = chk(ensure(ctx, Zf, static_cast<size_t>(nocc) * nocc * ldP * sizeof(double), "grad Z square"))) ||
-                (rc = chk(ensure(ctx, out[0], blk * sizeof(double), "grad dI3 block"))) ||
-                (rc = chk(ensure(ctx, out[1], blk * sizeof(double), "grad dI3 block")))))
+  if (dEdI3 && ((rc = chk(ensure_tmp(ctx, Zf, static_cast<size_t>(nocc) * nocc * ldP * sizeof(double), "grad Z square"))) ||
+                (rc = chk(ensure_tmp(ctx, out[0], blk * sizeof(double), "grad dI3 block"))) ||
+                (rc = chk(ensure_tmp(ctx, out[1], blk * sizeof(double), "grad dI3 block")))))
     return rc;
   double* pY = static_cast<double*>(Y.p);
   double* pZ = static_cast<double*>(Z.p);

@@ -383,7 +383,7 @@ int upload_basis(rijk_ctx* ctx, const HostBasis& h, DevBasis& d) {
             blob.data() + b0);
   std::copy(reinterpret_cast<const char*>(h.coefs.data()), reinterpret_cast<const char*>(h.coefs.data()) + b1,
             blob.data() + b0 + b1);
-  int rc = ensure(ctx, d.buf, blob.size(), "basis");
+  int rc = ensure_tmp(ctx, d.buf, blob.size(), "basis");
   if (rc) return rc;
   rc = cuda_check(ctx, cudaMemcpyAsync(d.buf.p, blob.data(), blob.size(), cudaMemcpyHostToDevice, ctx->stream),
                   "H2D basis");
@@ -651,7 +651,7 @@ int make_plan(rijk_ctx* ctx, const rijk_basis_t* orb, const rijk_basis_t* aux, E
   if ((rc = upload_basis(ctx, au, p.dauxu))) return rc;
   if (orb && (rc = upload_basis(ctx, p.orb, p.dorb))) return rc;
   p.kets = ket_lists(p.aux);
-  if ((rc = ensure(ctx, p.kets_dev, p.kets.idx.size() * sizeof(int), "ket list"))) return rc;
+  if ((rc = ensure_tmp(ctx, p.kets_dev, p.kets.idx.size() * sizeof(int), "ket list"))) return rc;
   if ((rc = cuda_check(ctx, cudaMemcpyAsync(p.kets_dev.p, p.kets.idx.data(), p.kets.idx.size() * sizeof(int),
                                             cudaMemcpyHostToDevice, ctx->stream), "H2D ket list")))
     return rc;
@@ -660,7 +660,7 @@ int make_plan(rijk_ctx* ctx, const rijk_basis_t* orb, const rijk_basis_t* aux, E
     p.orb_pairs.reserve(static_cast<size_t>(ns) * (ns + 1) / 2);
     for (int a = 0; a < ns; ++a)
       for (int b = 0; b <= a; ++b) p.orb_pairs.push_back(make_int2(a, b));
-    if ((rc = ensure(ctx, p.pairs_dev, p.orb_pairs.size() * sizeof(int2), "pair list"))) return rc;
+    if ((rc = ensure_tmp(ctx, p.pairs_dev, p.orb_pairs.size() * sizeof(int2), "pair list"))) return rc;
   }
   return RIJK_OK;
 }
@@ -676,7 +676,7 @@ int eri2c_device(rijk_ctx* ctx, EriPlan& p, double* dV, long ld, int* launches) 
   bra.push_back(u);
   pair_lists(bra, cand, [](const int2&) { return true; }, pl);
   DeviceBuf dp;
-  int rc = ensure(ctx, dp, pl.pairs.size() * sizeof(int2), "2c pair list");
+  int rc = ensure_tmp(ctx, dp, pl.pairs.size() * sizeof(int2), "2c pair list");
   if (rc) return rc;
   rc = cuda_check(ctx, cudaMemcpyAsync(dp.p, pl.pairs.data(), pl.pairs.size() * sizeof(int2), cudaMemcpyHostToDevice,
                                        ctx->stream), "H2D 2c pairs");
@@ -748,7 +748,7 @@ RIJK_API int rijk_eri2c(rijk_ctx* ctx, const rijk_basis_t* aux, double* PQ) {
   const long na = p.aux.nbf;
   DeviceBuf V;
   int launches = 0;
-  if (!rc) rc = ensure(ctx, V, static_cast<size_t>(na) * na * sizeof(double), "(P|Q)");
+  if (!rc) rc = ensure_tmp(ctx, V, static_cast<size_t>(na) * na * sizeof(double), "(P|Q)");
   if (!rc) rc = eri2c_device(ctx, p, static_cast<double*>(V.p), na, &launches);
   if (!rc)
     rc = cuda_check(ctx, cudaMemcpy(PQ, V.p, static_cast<size_t>(na) * na * sizeof(double), cudaMemcpyDeviceToHost),
@@ -778,7 +778,7 @@ RIJK_API int rijk_eri3c(rijk_ctx* ctx, const rijk_basis_t* orb, const rijk_basis
     const long mu1 = std::min(n, mu0 + rows);
     const long r0 = first_row(mu0), cnt = first_row(mu1) - r0;
     const size_t bytes = static_cast<size_t>(cnt) * naux * sizeof(double);
-    if ((rc = ensure(ctx, out, bytes, "3c block"))) break;
+    if ((rc = ensure_tmp(ctx, out, bytes, "3c block"))) break;
     cudaMemsetAsync(out.p, 0, bytes, ctx->stream);
     rc = eri3c_rows(ctx, p, layout, mu0, mu1, r0, static_cast<double*>(out.p), naux, &launches);
     if (!rc) rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "three-centre integrals");
@@ -805,7 +805,7 @@ RIJK_API int rijk_set_basis(rijk_ctx* ctx, const rijk_basis_t* orb, const rijk_b
   cudaEventCreate(&e1);
   DeviceBuf V;
   float ms_ints = 0.f;
-  rc = ensure(ctx, V, static_cast<size_t>(naux) * naux * sizeof(double), "(P|Q)");
+  rc = ensure_tmp(ctx, V, static_cast<size_t>(naux) * naux * sizeof(double), "(P|Q)");
   if (!rc) {
     cudaEventRecord(e0, ctx->stream);
     rc = eri2c_device(ctx, p, static_cast<double*>(V.p), naux, &launches);

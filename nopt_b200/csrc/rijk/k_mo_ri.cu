@@ -69,7 +69,7 @@ struct Scratch {
   }
   double* get(rijk_ctx* ctx, size_t doubles, const char* what, int* rc) {
     bufs.emplace_back();
-    *rc = ensure(ctx, bufs.back(), std::max<size_t>(doubles, 1) * sizeof(double), what);
+    *rc = ensure_tmp(ctx, bufs.back(), std::max<size_t>(doubles, 1) * sizeof(double), what);
     return static_cast<double*>(bufs.back().p);
   }
 };

@@ -84,13 +84,13 @@ RIJK_API int rijk_mo_ints(rijk_ctx* ctx, const double* DM_D, double* J, double* 
     if (r) cleanup();
     return r;
   };
-  if ((rc = chk(ensure(ctx, dC1, cbytes, "mo_ints C1"))) || (rc = chk(ensure(ctx, dC2, cbytes, "mo_ints C2"))) ||
-      (rc = chk(ensure(ctx, R1, p * npad * sizeof(double), "mo_ints rows1"))) ||
-      (rc = chk(ensure(ctx, R2, p * npad * sizeof(double), "mo_ints rows2"))) ||
-      (rc = chk(ensure(ctx, XTa, static_cast<size_t>(npad) * kdim * sizeof(double), "mo_ints XT"))) ||
-      (rc = chk(ensure(ctx, Y, static_cast<size_t>(naux) * p2 * sizeof(double), "mo_ints Y"))) ||
-      (rc = chk(ensure(ctx, G, static_cast<size_t>(p2) * p2 * sizeof(double), "mo_ints G"))) ||
-      (rc = chk(ensure(ctx, out, static_cast<size_t>(n_a * n_a) * n_a * n_a * sizeof(double), "mo_ints out"))))
+  if ((rc = chk(ensure_tmp(ctx, dC1, cbytes, "mo_ints C1"))) || (rc = chk(ensure_tmp(ctx, dC2, cbytes, "mo_ints C2"))) ||
+      (rc = chk(ensure_tmp(ctx, R1, p * npad * sizeof(double), "mo_ints rows1"))) ||
+      (rc = chk(ensure_tmp(ctx, R2, p * npad * sizeof(double), "mo_ints rows2"))) ||
+      (rc = chk(ensure_tmp(ctx, XTa, static_cast<size_t>(npad) * kdim * sizeof(double), "mo_ints XT"))) ||
+      (rc = chk(ensure_tmp(ctx, Y, static_cast<size_t>(naux) * p2 * sizeof(double), "mo_ints Y"))) ||
+      (rc = chk(ensure_tmp(ctx, G, static_cast<size_t>(p2) * p2 * sizeof(double), "mo_ints G"))) ||
+      (rc = chk(ensure_tmp(ctx, out, static_cast<size_t>(n_a * n_a) * n_a * n_a * sizeof(double), "mo_ints out"))))
     return rc;
   cudaMemcpyAsync(dC1.p, MO_VEC1, cbytes, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dC2.p, MO_VEC2, cbytes, cudaMemcpyHostToDevice, s);

@@ -59,8 +59,42 @@ int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
   b.bytes = 0;
   if (bytes == 0) return RIJK_OK;
   cudaError_t e = cudaMalloc(&b.p, bytes);
-  if (e != cudaSuccess) return cuda_check(ctx, e, what);
+  if (e == cudaErrorMemoryAllocation && ctx->pool) {  // once more without what the scratch pool keeps
+    cudaGetLastError();
+    cudaStreamSynchronize(ctx->stream);
+    cudaMemPoolTrimTo(ctx->pool, 0);
+    e = cudaMalloc(&b.p, bytes);
+  }
+  if (e != cudaSuccess) {
+    b.p = nullptr;
+    return cuda_check(ctx, e, what);
+  }
   b.bytes = bytes;
+  return RIJK_OK;
+}
+
+// The largest single scratch buffer is a 2 GiB block of raw integrals (rows_per_chunk), beside a few
+// matrices of n_aux x n_aux.  With cudaMalloc and cudaFree in every call, a call's 15 to 28 pairs of them
+// took 5 to 8 ms on a B200, each free waiting for the device: more than its kernels for up to some 250
+// orbitals (rijk_mo_calc at 144 orbitals 8 ms, of which 6.4 ms were these).
+constexpr uint64_t kPoolKeep = 3ull << 30;
+
+int ensure_tmp(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
+  if (!ctx->pool) return ensure(ctx, b, bytes, what);
+  if (b.bytes >= bytes && b.p) return RIJK_OK;
+  if (bytes > 0 && ctx->fail_alloc_after >= 0) {  // rijk_selftest_alloc_failure
+    if (ctx->fail_alloc_after == 0) return set_err(ctx, RIJK_ERR_ALLOC, "%s: out of device memory (injected)", what);
+    --ctx->fail_alloc_after;
+  }
+  release(b);
+  if (bytes == 0) return RIJK_OK;
+  const cudaError_t e = cudaMallocFromPoolAsync(&b.p, bytes, ctx->pool, ctx->stream);
+  if (e != cudaSuccess) {
+    b.p = nullptr;
+    return cuda_check(ctx, e, what);
+  }
+  b.bytes = bytes;
+  b.pool = ctx;
   return RIJK_OK;
 }
 
@@ -93,9 +127,11 @@ void prefer_max_shared(const void* fn) {
 }
 
 void release(DeviceBuf& b) {
-  if (b.p) cudaFree(b.p);
-  b.p = nullptr;
-  b.bytes = 0;
+  if (b.p && b.pool)
+    cudaFreeAsync(b.p, b.pool->stream);
+  else if (b.p)
+    cudaFree(b.p);
+  b = DeviceBuf();
 }
 
 __global__ void k_pad_from_colmajor(const double* __restrict__ src, long naux, double* __restrict__ dst, long nauxp) {
@@ -379,6 +415,16 @@ RIJK_API int rijk_create(rijk_ctx** out, int device) {
   cudaEventCreateWithFlags(&ctx->ev_jside, cudaEventDisableTiming);
   cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device);
   if (ctx->sms <= 0) ctx->sms = 148;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  uint64_t keep = kPoolKeep;
+  if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    rijk_destroy(ctx);
+    return RIJK_ERR_CUDA;
+  }
   cudaEventCreate(&ctx->ev0);
   cudaEventCreate(&ctx->ev1);
   cudaEventCreate(&ctx->ev2);
@@ -428,6 +474,7 @@ RIJK_API int rijk_destroy(rijk_ctx* ctx) {
     if (ev) cudaEventDestroy(ev);
   for (cudaEvent_t ev : ctx->pev)
     if (ev) cudaEventDestroy(ev);
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return RIJK_OK;
@@ -509,9 +556,9 @@ int set_metric_impl(rijk_ctx* ctx, const double* PQ, cudaMemcpyKind kind, long n
     release(work);
     release(info);
   };
-  if ((rc = ensure(ctx, V, naux * naux * sizeof(double), "metric V")) ||
-      (rc = ensure(ctx, X, naux * naux * sizeof(double), "metric X")) ||
-      (rc = ensure(ctx, W, naux * sizeof(double), "metric w")) || (rc = ensure(ctx, info, 2 * sizeof(int), "info")) ||
+  if ((rc = ensure_tmp(ctx, V, naux * naux * sizeof(double), "metric V")) ||
+      (rc = ensure_tmp(ctx, X, naux * naux * sizeof(double), "metric X")) ||
+      (rc = ensure_tmp(ctx, W, naux * sizeof(double), "metric w")) || (rc = ensure_tmp(ctx, info, 2 * sizeof(int), "info")) ||
       (rc = ensure(ctx, ctx->M, nauxp * nauxp * sizeof(double), "metric M"))) {
     cleanup();
     return rc;
@@ -531,7 +578,7 @@ int set_metric_impl(rijk_ctx* ctx, const double* PQ, cudaMemcpyKind kind, long n
       cleanup();
       return set_err(ctx, RIJK_ERR_SOLVER, "syevd buffer query failed");
     }
-    if ((rc = ensure(ctx, work, static_cast<size_t>(lwork) * sizeof(double), "syevd work"))) { cleanup(); return rc; }
+    if ((rc = ensure_tmp(ctx, work, static_cast<size_t>(lwork) * sizeof(double), "syevd work"))) { cleanup(); return rc; }
     if (cusolverDnDsyevd(ctx->cusolver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, na, dV, na,
                          static_cast<double*>(W.p), static_cast<double*>(work.p), lwork, dinfo) != CUSOLVER_STATUS_SUCCESS) {
       cleanup();
@@ -542,7 +589,7 @@ int set_metric_impl(rijk_ctx* ctx, const double* PQ, cudaMemcpyKind kind, long n
     k_scale_eigvecs<<<grid1d(naux * naux), 256, 0, s>>>(dX, static_cast<const double*>(W.p), naux, dinfo + 1);
     const double one = 1.0, zero = 0.0;
     DeviceBuf Mt;
-    if ((rc = ensure(ctx, Mt, naux * naux * sizeof(double), "metric tmp"))) { cleanup(); return rc; }
+    if ((rc = ensure_tmp(ctx, Mt, naux * naux * sizeof(double), "metric tmp"))) { cleanup(); return rc; }
     cublasStatus_t st = cublasDgemm(ctx->cublas, CUBLAS_OP_N, CUBLAS_OP_T, na, na, na, &one, dX, na, dV, na, &zero,
                                     static_cast<double*>(Mt.p), na);
     if (st != CUBLAS_STATUS_SUCCESS) {
@@ -561,7 +608,7 @@ int set_metric_impl(rijk_ctx* ctx, const double* PQ, cudaMemcpyKind kind, long n
       cleanup();
       return set_err(ctx, RIJK_ERR_SOLVER, "potrf buffer query failed");
     }
-    if ((rc = ensure(ctx, work, static_cast<size_t>(lwork) * sizeof(double), "potrf work"))) { cleanup(); return rc; }
+    if ((rc = ensure_tmp(ctx, work, static_cast<size_t>(lwork) * sizeof(double), "potrf work"))) { cleanup(); return rc; }
     if (cusolverDnDpotrf(ctx->cusolver, CUBLAS_FILL_MODE_LOWER, na, dV, na, static_cast<double*>(work.p), lwork,
                          dinfo) != CUSOLVER_STATUS_SUCCESS) {
       cleanup();
@@ -664,7 +711,7 @@ int set_3c_impl(rijk_ctx* ctx, long n, long naux, int layout, const ChunkFill& f
     maxcount = std::max(maxcount, c);
   }
   DeviceBuf raw;
-  if ((rc = ensure(ctx, raw, static_cast<size_t>(std::max<long>(maxcount, 1)) * nauxp * sizeof(double), "raw 3c block")))
+  if ((rc = ensure_tmp(ctx, raw, static_cast<size_t>(std::max<long>(maxcount, 1)) * nauxp * sizeof(double), "raw 3c block")))
     return rc;
   cudaMemsetAsync(raw.p, 0, raw.bytes, s);
   cudaMemsetAsync(ctx->B.p, 0, static_cast<size_t>(nq) * ntile * TILE2 * sizeof(double), s);
@@ -820,8 +867,8 @@ RIJK_API int rijk_fock_energy(rijk_ctx* ctx, const double* H, const double* DM, 
   int rc;
   DeviceBuf dH, dJ, dK, dF;
   auto cleanup = [&]() { release(dH); release(dJ); release(dK); release(dF); };
-  if ((rc = ensure(ctx, dH, nn, "H")) || (rc = ensure(ctx, dJ, nn, "J")) || (rc = ensure(ctx, dK, nn, "K")) ||
-      (rc = ensure(ctx, dF, nn, "F"))) {
+  if ((rc = ensure_tmp(ctx, dH, nn, "H")) || (rc = ensure_tmp(ctx, dJ, nn, "J")) || (rc = ensure_tmp(ctx, dK, nn, "K")) ||
+      (rc = ensure_tmp(ctx, dF, nn, "F"))) {
     cleanup();
     return rc;
   }

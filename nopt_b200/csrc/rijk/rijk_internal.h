@@ -26,6 +26,8 @@
 
 #include "rijk.h"
 
+struct rijk_ctx;
+
 namespace rijk {
 
 constexpr int TILE = 64;
@@ -41,6 +43,7 @@ constexpr int DEVERR_BOUNDS = 4;
 struct DeviceBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  rijk_ctx* pool = nullptr;  // from this context's pool (ensure_tmp); null: cudaMalloc
 };
 
 // An NVTX range around one C-ABI call, for timeline tools (Nsight Systems); free when no tool is attached.
@@ -71,6 +74,10 @@ struct rijk_ctx {
   cudaStream_t j_stream = nullptr;
   cudaEvent_t ev_pk = nullptr, ev_jside = nullptr;
   int sms = 148;
+  // Scratch of single calls (set-up, derivatives, MO tensors), allocated and freed in stream order.  The pool
+  // keeps at most kPoolKeep bytes between calls and gives everything back in rijk_destroy, or before a
+  // device allocation of the context fails.
+  cudaMemPool_t pool = nullptr;
 
   long n = 0, naux = 0, npad = 0, nt = 0, ntile = 0;
   long q0 = 0, nq = 0;  // aux functions [q0, q0 + nq) held in B (all of them unless rijk_set_aux_range)
@@ -133,6 +140,9 @@ void prof_mark(rijk_ctx* ctx, const char* name);
 int set_err(rijk_ctx* ctx, int code, const char* fmt, ...);
 int cuda_check(rijk_ctx* ctx, cudaError_t e, const char* what);
 int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);
+// Scratch that one call needs: from the context's pool, in the order of ctx->stream (a buffer that another
+// stream uses is released only once that stream has been waited for).
+int ensure_tmp(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);
 void release(DeviceBuf& b);
 float elapsed(cudaEvent_t a, cudaEvent_t b);
 int check_device_error(rijk_ctx* ctx);
