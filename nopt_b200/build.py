@@ -30,6 +30,11 @@ CUDA_SOURCES = [
     "rijk/k_moints.cu",
     "rijk/rijk_noalloc.cu",
     "rijk/k_eri.cu",
+    "rijk/k_eri_s.cu",
+    "rijk/k_eri_p.cu",
+    "rijk/k_eri_d.cu",
+    "rijk/k_eri_f.cu",
+    "rijk/k_eri_g.cu",
     "rijk/k_mo_ri.cu",
     "rijk/rijk_cache.cu",
     "rijk/rijk_selftest.cu",

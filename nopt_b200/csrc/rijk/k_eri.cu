@@ -7,6 +7,9 @@
 // (gto_ints.cpp): bra primitive pairs expanded in Hermite Gaussians (E coefficients), Hermite
 // Coulomb integrals R_tuv from the Boys function, aux functions as one-centre Hermite sums.
 //
+// Spherical aux shells with la + lb <= 6, all of the usual bases, take k_eri_thread (eri_thread.cuh), one launch
+// per (la + lb, lc).  The rest of this comment is about k_eri here, which takes the others.
+//
 // Work decomposition.  One launch per angular class (l_A, l_B, l_C); a task is one shell triple
 // (A B | C) and runs on a group of G lanes (G = 1 .. 32, chosen per class so that small classes
 // keep the lanes busy).  Per bra primitive pair the group builds the three 1-D E tables, then per
@@ -24,73 +27,17 @@
 #include <cmath>
 #include <vector>
 
-#include "gto_tables.h"
-#include "rijk_internal.h"
+#include "eri_device.cuh"
+#include "eri_thread.cuh"
 
 #define RIJK_API extern "C" __attribute__((visibility("default")))
 
 namespace rijk {
 namespace {
 
-using gto_tab::LMAX;
-constexpr int LTOT = 3 * LMAX;
-constexpr int TET_MAX = (LTOT + 1) * (LTOT + 2) * (LTOT + 3) / 6;  // 455 entries with t+u+v <= 12
-constexpr int NSPH = 245;            // sum over l <= 4 of (2l+1) ncart(l)
-constexpr int TERM_KEYS = 2 * (LMAX + 1);
-constexpr int TERM_STRIDE = 16;      // per key: offsets of m = 0 .. 15 (ncart(4) = 15) and the end
-constexpr int GROUP_F = 24;          // per group: F_0 .. F_15 and the aux power table pw[0..7]
+using namespace eri;
+constexpr int GROUP_F = 24;  // per group: F_0 .. F_15 and the aux power table pw[0..7]
 constexpr int ERI_THREADS = 128;
-
-struct EriShell {
-  double x, y, z;
-  int l, nprim, prim0, off;
-  int nfunc, pure, pad0, pad1;
-};
-
-struct EriTerm {
-  short t, u, v, j;  // Hermite index of the term and the power j of (2 gamma)^-1
-  int pad;
-  double d;
-};
-
-struct EriLaunch {
-  const EriShell* bra;
-  const double* bexp;
-  const double* bcoef;
-  const int2* pairs;
-  long npair;
-  const EriShell* ket;
-  const double* kexp;
-  const double* kcoef;
-  const int* kets;
-  long nket;
-  int la, lb, lc, G;
-  int gsize;        // doubles of shared memory per group
-  int mode;         // 0 packed rows (hi(hi+1)/2 + lo), 1 full rows (mu n + nu), 2 square (P, Q)
-  long mu0, mu1;    // rows written (modes 0, 1)
-  long rowbase;     // row index subtracted before storing
-  long n;           // orbital functions (mode 1 row pitch in pairs)
-  long ld;          // element pitch between stored rows
-  double* out;
-  const double* boys;
-  const double* sph;
-  const EriTerm* terms;
-  const int* term_off;
-  const int* tuv;
-  const int* cart;
-};
-
-__host__ __device__ inline int tet(int L) { return (L + 1) * (L + 2) * (L + 3) / 6; }
-__host__ __device__ inline int ncart_d(int l) { return (l + 1) * (l + 2) / 2; }
-__device__ __forceinline__ int tet_index(int t, int u, int v) {
-  const int s = t + u + v, w = u + v;
-  return s * (s + 1) * (s + 2) / 6 + w * (w + 1) / 2 + v;
-}
-__host__ __device__ inline int sph_off(int l) {
-  int o = 0;
-  for (int k = 0; k < l; ++k) o += (2 * k + 1) * ncart_d(k);
-  return o;
-}
 
 // F_m(T), m = 0 .. L, exactly as the host engine evaluates it (Taylor about the nearest grid
 // point, downward recursion; F_0 and upward recursion past the grid).
@@ -398,7 +345,7 @@ int upload_basis(rijk_ctx* ctx, const HostBasis& h, DevBasis& d) {
 // Device tables shared by all launches: Boys grid, spherical transforms, aux term lists,
 // Hermite index decode and Cartesian exponents.  Built once per context.
 struct TabLayout {
-  size_t boys, sph, terms, term_off, tuv, cart, total;
+  size_t boys, sph, terms, term_off, tuv, cart, rows, norm, total;
 };
 
 TabLayout tab_layout(size_t nterms) {
@@ -415,6 +362,8 @@ TabLayout tab_layout(size_t nterms) {
   t.term_off = take(sizeof(int) * TERM_KEYS * (TERM_STRIDE + 1));
   t.tuv = take(sizeof(int) * TET_MAX);
   t.cart = take(sizeof(int) * (LMAX + 1) * 16);
+  t.rows = take(sizeof(SphRow) * 2 * SPH_ROWS);
+  t.norm = take(sizeof(double) * (LMAX + 1) * 9);
   t.total = o;
   return t;
 }
@@ -426,6 +375,8 @@ struct DevTables {
   const int* term_off;
   const int* tuv;
   const int* cart;
+  const SphRow* rows;
+  const double* norm;
 };
 
 int ensure_tables(rijk_ctx* ctx, DevTables& dt) {
@@ -487,6 +438,29 @@ int ensure_tables(rijk_ctx* ctx, DevTables& dt) {
       for (int lx = l; lx >= 0; --lx)
         for (int ly = l - lx; ly >= 0; --ly)
           cart[l * 16 + gto_tab::cart_index(l, lx, ly)] = lx | (ly << 4) | ((l - lx - ly) << 8);
+    SphRow* rows = reinterpret_cast<SphRow*>(blob.data() + lay.rows);
+    double* norm = reinterpret_cast<double*>(blob.data() + lay.norm);
+    for (int l = 0; l <= LMAX; ++l) {
+      const int nc = ncart_d(l);
+      for (int m = 0; m < 2 * l + 1; ++m)
+        for (int lx = l; lx >= 0; --lx)
+          for (int ly = l - lx; ly >= 0; --ly) {
+            const int lz = l - lx - ly;
+            const double c = S.c[l][static_cast<size_t>(m) * nc + gto_tab::cart_index(l, lx, ly)];
+            const int q = harm(l, m, lx, ly, lz);
+            if (q == 0) continue;  // the table's own value is zero there, or rounding of a cancelled sum
+            SphRow& r = rows[l * 15 + m];
+            r.cart[r.n] = lx | (ly << 4) | (lz << 8);
+            r.c[r.n++] = c;
+            norm[l * 9 + m] = c / q;
+          }
+      for (int c = 0; c < nc; ++c) {
+        SphRow& r = rows[SPH_ROWS + l * 15 + c];
+        r.n = 1;
+        r.cart[0] = cart[l * 16 + c];
+        r.c[0] = 1.0;
+      }
+    }
     int rc = ensure(ctx, ctx->eri_tab, lay.total, "integral tables");
     if (rc) return rc;
     rc = cuda_check(ctx, cudaMemcpyAsync(ctx->eri_tab.p, blob.data(), lay.total, cudaMemcpyHostToDevice, ctx->stream),
@@ -500,6 +474,8 @@ int ensure_tables(rijk_ctx* ctx, DevTables& dt) {
   dt.term_off = reinterpret_cast<const int*>(p + lay.term_off);
   dt.tuv = reinterpret_cast<const int*>(p + lay.tuv);
   dt.cart = reinterpret_cast<const int*>(p + lay.cart);
+  dt.rows = reinterpret_cast<const SphRow*>(p + lay.rows);
+  dt.norm = reinterpret_cast<const double*>(p + lay.norm);
   return RIJK_OK;
 }
 
@@ -519,86 +495,128 @@ int group_doubles(int la, int lb, int lc) {
   return (d + 1) & ~1;
 }
 
-// Ket shells grouped by angular momentum, each group sorted by primitive count (tasks next to
-// each other in a warp then share their loop trip counts).
+// Ket shells grouped by angular momentum, spherical ones before Cartesian ones, each group sorted by
+// primitive count (tasks next to each other then share their loop trip counts).
 struct KetLists {
   std::vector<int> idx;
-  long start[LMAX + 2] = {};
+  long start[2 * (LMAX + 1) + 1] = {};  // group 2 l: spherical, 2 l + 1: Cartesian
+  int nprim[2 * (LMAX + 1)] = {};       // largest primitive count of the group
 };
 
 KetLists ket_lists(const HostBasis& k) {
   KetLists out;
-  for (int l = 0; l <= LMAX; ++l) {
-    out.start[l] = static_cast<long>(out.idx.size());
+  for (int g = 0; g < 2 * (LMAX + 1); ++g) {
+    out.start[g] = static_cast<long>(out.idx.size());
     std::vector<int> v;
     for (int s = 0; s < static_cast<int>(k.sh.size()); ++s)
-      if (k.sh[s].l == l) v.push_back(s);
+      if (2 * k.sh[s].l + (k.sh[s].pure ? 0 : 1) == g) v.push_back(s);
     std::stable_sort(v.begin(), v.end(), [&](int x, int y) { return k.sh[x].nprim < k.sh[y].nprim; });
+    if (!v.empty()) out.nprim[g] = k.sh[v.back()].nprim;
     out.idx.insert(out.idx.end(), v.begin(), v.end());
   }
-  out.start[LMAX + 1] = static_cast<long>(out.idx.size());
+  out.start[2 * (LMAX + 1)] = static_cast<long>(out.idx.size());
   return out;
 }
 
-// Bra pair lists by class (l_A, l_B), concatenated, with class offsets.
+// Bra pair lists by class (l_A, l_B), concatenated in the order of l_A + l_B, with class offsets; for each
+// l_A + l_B the widest pair and the widest contracted one.
+constexpr int NCLASS = (LMAX + 1) * (LMAX + 1);
 struct PairLists {
   std::vector<int2> pairs;
-  long start[(LMAX + 1) * (LMAX + 1) + 1] = {};
+  long start[NCLASS] = {}, count[NCLASS] = {};
+  long lab_start[2 * LMAX + 2] = {};
+  int wide[2 * LMAX + 1] = {}, wide_contracted[2 * LMAX + 1] = {};
 };
 
 template <typename Keep>
 void pair_lists(const std::vector<EriShell>& bra, const std::vector<int2>& cand, Keep keep, PairLists& out) {
-  std::vector<int2> by[(LMAX + 1) * (LMAX + 1)];
-  for (const int2& pr : cand)
-    if (keep(pr)) by[bra[pr.x].l * (LMAX + 1) + bra[pr.y].l].push_back(pr);
-  out.pairs.clear();
-  for (int c = 0; c < (LMAX + 1) * (LMAX + 1); ++c) {
-    out.start[c] = static_cast<long>(out.pairs.size());
-    out.pairs.insert(out.pairs.end(), by[c].begin(), by[c].end());
+  std::vector<int2> by[NCLASS];
+  out = PairLists();
+  for (const int2& pr : cand) {
+    if (!keep(pr)) continue;
+    const EriShell &A = bra[pr.x], &B = bra[pr.y];
+    by[A.l * (LMAX + 1) + B.l].push_back(pr);
+    const int lab = A.l + B.l, nab = A.nfunc * B.nfunc;
+    out.wide[lab] = std::max(out.wide[lab], nab);
+    if (A.nprim * B.nprim > 1) out.wide_contracted[lab] = std::max(out.wide_contracted[lab], nab);
   }
-  out.start[(LMAX + 1) * (LMAX + 1)] = static_cast<long>(out.pairs.size());
+  for (int lab = 0; lab <= 2 * LMAX; ++lab) {
+    out.lab_start[lab] = static_cast<long>(out.pairs.size());
+    for (int la = std::max(0, lab - LMAX); la <= std::min(lab, LMAX); ++la) {
+      const int c = la * (LMAX + 1) + lab - la;
+      out.start[c] = static_cast<long>(out.pairs.size());
+      out.count[c] = static_cast<long>(by[c].size());
+      out.pairs.insert(out.pairs.end(), by[c].begin(), by[c].end());
+    }
+  }
+  out.lab_start[2 * LMAX + 1] = static_cast<long>(out.pairs.size());
+}
+
+using LaunchThread = cudaError_t (*)(int, const EriLaunch&, size_t, cudaStream_t);
+const LaunchThread kLaunchThread[LMAX + 1] = {launch_lc<0>, launch_lc<1>, launch_lc<2>, launch_lc<3>, launch_lc<4>};
+
+// The class (la, lb | group g of the kets) on k_eri.
+int launch_group(rijk_ctx* ctx, EriLaunch P, const PairLists& pl, const int2* pairs_dev, int la, int lb, int lc,
+                 int maxsm) {
+  const int c = la * (LMAX + 1) + lb;
+  if (pl.count[c] == 0) return RIJK_OK;
+  P.la = la;
+  P.lb = lb;
+  P.lc = lc;
+  P.G = group_lanes(la, lb, lc);
+  P.gsize = group_doubles(la, lb, lc);
+  P.pairs = pairs_dev + pl.start[c];
+  P.npair = pl.count[c];
+  const size_t per_warp = static_cast<size_t>(32 / P.G) * P.gsize * sizeof(double);
+  const int warps = static_cast<int>(std::min<size_t>(ERI_THREADS / 32, static_cast<size_t>(maxsm) / per_warp));
+  if (warps < 1) return set_err(ctx, RIJK_ERR_ARG, "integral class (%d %d|%d) needs too much shared memory", la, lb, lc);
+  const size_t smem = per_warp * warps;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = ensure_smem_limit(reinterpret_cast<const void*>(k_eri), smem);
+    if (e != cudaSuccess) return cuda_check(ctx, e, "integral kernel shared memory");
+  }
+  const long gpb = static_cast<long>(warps) * 32 / P.G;
+  const long blocks = std::min<long>((P.npair * P.nket + gpb - 1) / gpb, 148L * 32);
+  k_eri<<<static_cast<unsigned>(blocks), warps * 32, smem, ctx->stream>>>(P);
+  return RIJK_OK;
 }
 
 // Launches every class of one output block.  pairs_dev holds PairLists::pairs on the device.
 int launch_classes(rijk_ctx* ctx, const EriLaunch& base, const PairLists& pl, const int2* pairs_dev,
                    const KetLists& kl, const int* kets_dev, int* launches) {
-  cudaStream_t s = ctx->stream;
   int maxsm = 0;
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-  for (int la = 0; la <= LMAX; ++la)
-    for (int lb = 0; lb <= LMAX; ++lb) {
-      const int c = la * (LMAX + 1) + lb;
-      const long np = pl.start[c + 1] - pl.start[c];
-      if (np == 0) continue;
-      for (int lc = 0; lc <= LMAX; ++lc) {
-        const long nk = kl.start[lc + 1] - kl.start[lc];
-        if (nk == 0) continue;
-        EriLaunch P = base;
-        P.la = la;
-        P.lb = lb;
-        P.lc = lc;
-        P.G = group_lanes(la, lb, lc);
-        P.gsize = group_doubles(la, lb, lc);
-        P.pairs = pairs_dev + pl.start[c];
-        P.npair = np;
-        P.kets = kets_dev + kl.start[lc];
-        P.nket = nk;
-        const size_t per_warp = static_cast<size_t>(32 / P.G) * P.gsize * sizeof(double);
-        int warps = static_cast<int>(std::min<size_t>(ERI_THREADS / 32, static_cast<size_t>(maxsm) / per_warp));
-        if (warps < 1) return set_err(ctx, RIJK_ERR_ARG, "integral class (%d %d|%d) needs too much shared memory", la, lb, lc);
-        const size_t smem = per_warp * warps;
-        if (smem > 48 * 1024) {
-          cudaError_t e = cudaFuncSetAttribute(k_eri, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-          if (e != cudaSuccess) return cuda_check(ctx, e, "integral kernel shared memory");
-        }
-        const long gpb = static_cast<long>(warps) * 32 / P.G;
-        const long ntask = np * nk;
-        long blocks = (ntask + gpb - 1) / gpb;
-        blocks = std::min<long>(blocks, 148L * 32);
-        k_eri<<<static_cast<unsigned>(blocks), warps * 32, smem, s>>>(P);
+  for (int lab = 0; lab <= 2 * LMAX; ++lab) {
+    const long np = pl.lab_start[lab + 1] - pl.lab_start[lab];
+    if (np == 0) continue;
+    for (int g = 0; g < 2 * (LMAX + 1); ++g) {
+      const int lc = g / 2;
+      EriLaunch P = base;
+      P.kets = kets_dev + kl.start[g];
+      P.nket = kl.start[g + 1] - kl.start[g];
+      if (P.nket == 0) continue;
+      P.pairs = pairs_dev + pl.lab_start[lab];
+      P.npair = np;
+      // the thread-per-aux-shell kernel: its expansions, and the accumulators of contracted pairs, must fit
+      const int side = lab / 2 + 1;  // (la + 1)(lb + 1) is at most side * (lab + 2 - side)
+      P.e1size = (3 * side * (lab + 2 - side) * (lab + 1) + 1) & ~1;
+      P.esize = pl.wide[lab] * ((tet(lab) + 1) & ~1);
+      const int contracted = kl.nprim[g] > 1 ? pl.wide[lab] : pl.wide_contracted[lab];
+      const size_t smem = (static_cast<size_t>(P.e1size) + P.esize + static_cast<size_t>(contracted) * NT * (2 * lc + 1)) *
+                          sizeof(double);
+      if (g % 2 == 0 && lab <= LAB_MAX && smem <= static_cast<size_t>(maxsm)) {
+        const cudaError_t e = kLaunchThread[lc](lab, P, smem, ctx->stream);
+        if (e != cudaSuccess) return cuda_check(ctx, e, "integral kernel launch");
+        ++*launches;
+        continue;
+      }
+      for (int la = std::max(0, lab - LMAX); la <= std::min(lab, LMAX); ++la) {
+        if (pl.count[la * (LMAX + 1) + lab - la] == 0) continue;
+        if (const int rc = launch_group(ctx, P, pl, pairs_dev, la, lab - la, lc, maxsm)) return rc;
         ++*launches;
       }
     }
+  }
   return cuda_check(ctx, cudaGetLastError(), "integral kernel launch");
 }
 
@@ -610,6 +628,8 @@ EriLaunch base_launch(const DevTables& t) {
   P.term_off = t.term_off;
   P.tuv = t.tuv;
   P.cart = t.cart;
+  P.sph_rows = t.rows;
+  P.harm_norm = t.norm;
   return P;
 }
 
@@ -672,7 +692,8 @@ int eri2c_device(rijk_ctx* ctx, EriPlan& p, double* dV, long ld, int* launches) 
   for (int a = 0; a < na; ++a) cand[a] = make_int2(a, na);  // (P, unit)
   PairLists pl;
   std::vector<EriShell> bra = p.aux.sh;
-  EriShell u{};
+  EriShell u{};  // the unit s function of dauxu
+  u.nprim = u.nfunc = u.pure = 1;
   bra.push_back(u);
   pair_lists(bra, cand, [](const int2&) { return true; }, pl);
   DeviceBuf dp;
