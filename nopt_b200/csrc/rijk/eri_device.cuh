@@ -63,6 +63,7 @@ struct EriLaunch {
   const SphRow* sph_rows;   // [spherical, Cartesian][SPH_ROWS]
   const double* harm_norm;  // [l][9]: norms of the integer harmonics (harm in eri_thread.cuh)
   int e1size, esize;        // k_eri_thread: doubles of its 1-D and pair expansions in shared memory
+  int tile;                 // k_eri_thread: aux shells of a CTA, a power of two up to its 64 threads
 };
 
 __host__ __device__ inline int tet(int L) { return (L + 1) * (L + 2) * (L + 3) / 6; }

@@ -7,8 +7,10 @@
 // with q_mc the integer coefficients of the polynomial, s_m its norm and E^ab the bra's spherical (or
 // Cartesian) functions in Hermite Gaussians.
 //
-// One CTA takes a bra shell pair and 64 aux shells of one l.  Its threads form E for each bra primitive
-// pair in shared memory once, for all those aux shells; each thread then runs its own aux shell: the Boys
+// One CTA of 64 threads takes a bra shell pair and a tile of 8 to 64 aux shells of one l (eri_tile); with fewer
+// than 64, several threads share an aux shell and divide the bra functions between them (each forms R and W
+// again, which costs no time on lanes that would idle).  The threads form E for each bra primitive
+// pair in shared memory once, for all those aux shells; each thread then runs its aux shell: the Boys
 // values, the R recursion in place in registers (entries in falling order: a layer's entry of order k reads
 // only entries of order k - 1 and k - 2, not yet overwritten; local memory from total order 7 on), W, and
 // the product with E, whose entries all threads read as 16-byte broadcasts.  la + lb and lc are template
@@ -17,8 +19,8 @@
 // What bounds it: the FP64 pipe and its latency at 8 to 16 warps per SM.  Measured against a group of lanes per
 // shell triple with everything in shared memory (k_eri, kept for Cartesian aux shells and la + lb > 6), whose
 // Boys values one lane formed while the others waited and whose E was formed again for every aux shell: at
-// (H2O)8 cc-pVTZ/cc-pVTZ-JKFIT all of (P|Q) and (mu nu|P) 31.8 -> 9.4 ms, (H2O)16
-// cc-pVDZ/cc-pVDZ-JKFIT 32.7 -> 5.4 ms, (H2O)32 cc-pVTZ 1.02 -> 0.225 s.
+// (H2O)8 cc-pVTZ/cc-pVTZ-JKFIT all of (P|Q) and (mu nu|P) 31.8 -> 4.0 ms, (H2O)16
+// cc-pVDZ/cc-pVDZ-JKFIT 32.7 -> 3.1 ms, (H2O)32 cc-pVTZ 1.02 -> 0.130 s.
 #pragma once
 #include <utility>
 
@@ -27,7 +29,7 @@
 namespace rijk {
 namespace eri {
 
-constexpr int NT = 64;        // threads, and aux shells, of a CTA
+constexpr int NT = 64;        // threads of a CTA
 constexpr int LAB_MAX = 6;    // la + lb handled here (f f)
 
 // Hermite index -> (t, u, v), the order of tet_index
@@ -183,16 +185,23 @@ __device__ __forceinline__ double dot_row(const double* __restrict__ E, const do
   return a + b;
 }
 
-// The aux functions ROW .. 2 LC of one thread: out(ab, m, value) for every bra function pair
+// The aux functions ROW .. 2 LC of one thread: out(ab, m, value) for its bra function pairs ab0, ab0 + dab, ..
 template <int LAB, int LC, int ROW, typename Out>
 __device__ __forceinline__ void rows(const double* R, double f, const double* __restrict__ norm,
-                                     const double* __restrict__ E, int nab, Out out) {
+                                     const double* __restrict__ E, int ab0, int dab, int nab, Out out) {
   constexpr int NH = tetc(LAB), NHP = (NH + 1) & ~1;
   double W[NH];
   w_all<LC, ROW>(R, f * __ldg(norm + ROW), W, std::make_integer_sequence<int, NH>());
 #pragma unroll 1
-  for (int ab = 0; ab < nab; ++ab) out(ab, ROW, dot_row<NH>(E + ab * NHP, W));
-  if constexpr (ROW < 2 * LC) rows<LAB, LC, ROW + 1>(R, f, norm, E, nab, out);
+  for (int ab = ab0; ab < nab; ab += dab) out(ab, ROW, dot_row<NH>(E + ab * NHP, W));
+  if constexpr (ROW < 2 * LC) rows<LAB, LC, ROW + 1>(R, f, norm, E, ab0, dab, nab, out);
+}
+
+// s s: every aux function of the thread, added to acc
+template <int LC, int ROW>
+__device__ __forceinline__ void sums(const double* R, double f, const double* __restrict__ norm, double* acc) {
+  acc[ROW] = fma(f * __ldg(norm + ROW), w_entry<0, LC, ROW>(R), acc[ROW]);
+  if constexpr (ROW < 2 * LC) sums<LC, ROW + 1>(R, f, norm, acc);
 }
 
 template <int LAB, int LC>
@@ -201,19 +210,21 @@ __global__ void __launch_bounds__(NT) k_eri_thread(const EriLaunch P) {
   extern __shared__ __align__(16) double sm[];
   double* E1 = sm;                      // 3 x (la+1)(lb+1)(LAB+1)
   double* E = sm + P.e1size;            // nab x NHP
-  double* acc = E + P.esize;            // nab x NT NF, contracted pairs only
   const int tid = threadIdx.x;
-  const long ntile = (P.nket + NT - 1) / NT;
+  const int tile = P.tile, kt = tid & (tile - 1), part = tid / tile, parts = NT / tile;
+  double* acc = E + P.esize;            // nab x tile NF, contracted pairs only
+  const int arow = tile * NF;
+  const long ntile = (P.nket + tile - 1) / tile;
   const long ip = blockIdx.x / ntile;
-  const long k0 = (blockIdx.x - ip * ntile) * NT;
+  const long k0 = (blockIdx.x - ip * ntile) * tile;
   const int2 pair = P.pairs[ip];
   const EriShell A = P.bra[pair.x];
   const EriShell B = P.bra[pair.y];
-  const bool live = k0 + tid < P.nket;
-  const EriShell C = P.ket[P.kets[live ? k0 + tid : P.nket - 1]];
+  const bool live = k0 + kt < P.nket;
+  const EriShell C = P.ket[P.kets[live ? k0 + kt : P.nket - 1]];
   const int la = A.l, lb = B.l, nfb = B.nfunc, nab = A.nfunc * nfb;
   // the tile's largest primitive count: the aux shells are sorted by it
-  const int nprim_k = P.ket[P.kets[min(k0 + NT, P.nket) - 1]].nprim;
+  const int nprim_k = P.ket[P.kets[min(k0 + tile, P.nket) - 1]].nprim;
   const bool direct = A.nprim * B.nprim * nprim_k == 1;
   const double* norm = P.harm_norm + LC * 9;
   const double two_pi_25 = 2.0 * 17.493418327624862;  // 2 pi^(5/2)
@@ -237,8 +248,11 @@ __global__ void __launch_bounds__(NT) k_eri_thread(const EriLaunch P) {
     }
   };
 
-  if (!direct)
-    for (int o = tid; o < nab * NT * NF; o += NT) acc[o] = 0.0;
+  double racc[NF] = {};  // LAB = 0: the sums stay in registers, E is one number
+  if (LAB > 0 && !direct) {
+    for (int o = tid; o < nab * arow; o += NT) acc[o] = 0.0;
+    __syncthreads();
+  }
   const double ABx = A.x - B.x, ABy = A.y - B.y, ABz = A.z - B.z;
   const double r2 = ABx * ABx + ABy * ABy + ABz * ABz;
   bool any = false;
@@ -251,55 +265,57 @@ __global__ void __launch_bounds__(NT) k_eri_thread(const EriLaunch P) {
     if (fabs(cc * K) < 1e-22) continue;  // contributes below double precision (host rule); the same for all threads
     any = true;
     const double Px = (a * A.x + b * B.x) * ip1, Py = (a * A.y + b * B.y) * ip1, Pz = (a * A.z + b * B.z) * ip1;
-    // E1[d][i][j][t]: 1-D Hermite expansion of the primitive product
-    const int ts = LAB + 1, n1 = (la + 1) * (lb + 1) * ts;
-    __syncthreads();  // the previous primitive pair's readers of E are done
-    if (tid < 3) {
-      const double pd = tid == 0 ? Px : (tid == 1 ? Py : Pz);
-      const double ad = tid == 0 ? A.x : (tid == 1 ? A.y : A.z);
-      const double bd = tid == 0 ? B.x : (tid == 1 ? B.y : B.z);
-      const double xpa = pd - ad, xpb = pd - bd, o2p = 0.5 * ip1;
-      double* e1 = E1 + tid * n1;
-      e1[0] = tid == 0 ? K * cc : 1.0;
-      for (int q = 0; q <= la; ++q)
-        for (int r = 0; r <= lb; ++r) {
-          if (q + r == 0) continue;
-          const double* src = e1 + (r > 0 ? (q * (lb + 1) + r - 1) : ((q - 1) * (lb + 1))) * ts;
-          double* dst = e1 + (q * (lb + 1) + r) * ts;
-          const double x = r > 0 ? xpb : xpa;
-          const int o = q + r;  // the source has entries t <= o - 1
-          for (int t = 0; t <= o; ++t) {
-            double v = t < o ? x * src[t] : 0.0;
-            if (t + 1 < o) v += (t + 1) * src[t + 1];
-            if (t > 0) v += o2p * src[t - 1];
-            dst[t] = v;
+    if constexpr (LAB > 0) {
+      // E1[d][i][j][t]: 1-D Hermite expansion of the primitive product
+      const int ts = LAB + 1, n1 = (la + 1) * (lb + 1) * ts;
+      __syncthreads();  // the previous primitive pair's readers of E are done
+      if (tid < 3) {
+        const double pd = tid == 0 ? Px : (tid == 1 ? Py : Pz);
+        const double ad = tid == 0 ? A.x : (tid == 1 ? A.y : A.z);
+        const double bd = tid == 0 ? B.x : (tid == 1 ? B.y : B.z);
+        const double xpa = pd - ad, xpb = pd - bd, o2p = 0.5 * ip1;
+        double* e1 = E1 + tid * n1;
+        e1[0] = tid == 0 ? K * cc : 1.0;
+        for (int q = 0; q <= la; ++q)
+          for (int r = 0; r <= lb; ++r) {
+            if (q + r == 0) continue;
+            const double* src = e1 + (r > 0 ? (q * (lb + 1) + r - 1) : ((q - 1) * (lb + 1))) * ts;
+            double* dst = e1 + (q * (lb + 1) + r) * ts;
+            const double x = r > 0 ? xpb : xpa;
+            const int o = q + r;  // the source has entries t <= o - 1
+            for (int t = 0; t <= o; ++t) {
+              double v = t < o ? x * src[t] : 0.0;
+              if (t + 1 < o) v += (t + 1) * src[t + 1];
+              if (t > 0) v += o2p * src[t - 1];
+              dst[t] = v;
+            }
+          }
+      }
+      __syncthreads();
+      // E[ab][tuv] over the spherical (or Cartesian) functions of the pair
+      for (int o = tid; o < nab * NH; o += NT) {
+        const int ab = o / NH, h = o - ab * NH;
+        const int c = __ldg(P.tuv + h);
+        const int t = c & 0xff, u = (c >> 8) & 0xff, v = c >> 16;
+        const int fa = ab / nfb, fb = ab - fa * nfb;
+        const SphRow& ra = P.sph_rows[(A.pure ? 0 : 1) * SPH_ROWS + la * 15 + fa];
+        const SphRow& rb = P.sph_rows[(B.pure ? 0 : 1) * SPH_ROWS + lb * 15 + fb];
+        double s = 0.0;
+        for (int x = 0; x < ra.n; ++x) {
+          const int ka = ra.cart[x];
+          const int ax = ka & 15, ay = (ka >> 4) & 15, az = ka >> 8;
+          for (int y = 0; y < rb.n; ++y) {
+            const int kb = rb.cart[y];
+            const int bx = kb & 15, by = (kb >> 4) & 15, bz = kb >> 8;
+            if (t > ax + bx || u > ay + by || v > az + bz) continue;
+            s += ra.c[x] * rb.c[y] * E1[(ax * (lb + 1) + bx) * ts + t] * E1[n1 + (ay * (lb + 1) + by) * ts + u] *
+                 E1[2 * n1 + (az * (lb + 1) + bz) * ts + v];
           }
         }
-    }
-    __syncthreads();
-    // E[ab][tuv] over the spherical (or Cartesian) functions of the pair
-    for (int o = tid; o < nab * NH; o += NT) {
-      const int ab = o / NH, h = o - ab * NH;
-      const int c = __ldg(P.tuv + h);
-      const int t = c & 0xff, u = (c >> 8) & 0xff, v = c >> 16;
-      const int fa = ab / nfb, fb = ab - fa * nfb;
-      const SphRow& ra = P.sph_rows[(A.pure ? 0 : 1) * SPH_ROWS + la * 15 + fa];
-      const SphRow& rb = P.sph_rows[(B.pure ? 0 : 1) * SPH_ROWS + lb * 15 + fb];
-      double s = 0.0;
-      for (int x = 0; x < ra.n; ++x) {
-        const int ka = ra.cart[x];
-        const int ax = ka & 15, ay = (ka >> 4) & 15, az = ka >> 8;
-        for (int y = 0; y < rb.n; ++y) {
-          const int kb = rb.cart[y];
-          const int bx = kb & 15, by = (kb >> 4) & 15, bz = kb >> 8;
-          if (t > ax + bx || u > ay + by || v > az + bz) continue;
-          s += ra.c[x] * rb.c[y] * E1[(ax * (lb + 1) + bx) * ts + t] * E1[n1 + (ay * (lb + 1) + by) * ts + u] *
-               E1[2 * n1 + (az * (lb + 1) + bz) * ts + v];
-        }
+        E[ab * NHP + h] = s;
       }
-      E[ab * NHP + h] = s;
+      __syncthreads();
     }
-    __syncthreads();
     const double X = Px - C.x, Y = Py - C.y, Z = Pz - C.z;
     const double d2 = X * X + Y * Y + Z * Z;
 #pragma unroll 1
@@ -308,6 +324,7 @@ __global__ void __launch_bounds__(NT) k_eri_thread(const EriLaunch P) {
       const double gam = has ? P.kexp[C.prim0 + k] : 1.0, ck = has ? P.kcoef[C.prim0 + k] : 0.0;
       const double rs = rsqrt(p + gam), al = p * gam * rs * rs, ig = 1.0 / gam;
       double f = two_pi_25 * ip1 * ig * rs * ck;
+      if (LAB == 0) f *= K * cc;
       const double o2g = -0.5 * ig;
 #pragma unroll
       for (int q = 0; q < LC; ++q) f *= o2g;
@@ -322,23 +339,29 @@ __global__ void __launch_bounds__(NT) k_eri_thread(const EriLaunch P) {
       }
       double R[NR];
       r_layers<L>(R, G, X, Y, Z);
-      if (direct) {
-        rows<LAB, LC, 0>(R, f, norm, E, nab, [&](int ab, int m, double v) {
+      if constexpr (LAB == 0) {
+        sums<LC, 0>(R, f, norm, racc);
+      } else if (direct) {
+        rows<LAB, LC, 0>(R, f, norm, E, part, parts, nab, [&](int ab, int m, double v) {
           if (live) store(ab, C.off + m, v);
         });
       } else {
-        double* mine = acc + tid * NF;
-        rows<LAB, LC, 0>(R, f, norm, E, nab, [&](int ab, int m, double v) { mine[ab * (NT * NF) + m] += v; });
+        double* mine = acc + kt * NF;
+        rows<LAB, LC, 0>(R, f, norm, E, part, parts, nab, [&](int ab, int m, double v) { mine[ab * arow + m] += v; });
       }
     }
   }
   if (!live) return;
-  if (!direct) {
-    for (int ab = 0; ab < nab; ++ab)
+  if constexpr (LAB == 0) {
+    if (part == 0)
 #pragma unroll
-      for (int m = 0; m < NF; ++m) store(ab, C.off + m, acc[ab * (NT * NF) + tid * NF + m]);
+      for (int m = 0; m < NF; ++m) store(0, C.off + m, racc[m]);
+  } else if (!direct) {
+    for (int ab = part; ab < nab; ab += parts)
+#pragma unroll
+      for (int m = 0; m < NF; ++m) store(ab, C.off + m, acc[ab * arow + kt * NF + m]);
   } else if (!any) {  // every primitive pair is below double precision
-    for (int ab = 0; ab < nab; ++ab)
+    for (int ab = part; ab < nab; ab += parts)
 #pragma unroll
       for (int m = 0; m < NF; ++m) store(ab, C.off + m, 0.0);
   }
@@ -357,7 +380,7 @@ cudaError_t launch(const EriLaunch& P, size_t smem, cudaStream_t s) {
   const cudaError_t e = ensure_smem_limit(fn, smem);
   if (e != cudaSuccess) return e;
   // P.npair * tiles is far below 2^31: a call's row block holds at most 2 GiB of integrals
-  const long blocks = P.npair * ((P.nket + NT - 1) / NT);
+  const long blocks = P.npair * ((P.nket + P.tile - 1) / P.tile);
   k_eri_thread<LAB, LC><<<static_cast<unsigned>(blocks), NT, smem, s>>>(P);
   return cudaGetLastError();
 }

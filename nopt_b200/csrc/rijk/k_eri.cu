@@ -530,12 +530,13 @@ struct PairLists {
 
 template <typename Keep>
 void pair_lists(const std::vector<EriShell>& bra, const std::vector<int2>& cand, Keep keep, PairLists& out) {
-  std::vector<int2> by[NCLASS];
+  // pairs of many primitives first: a launch's longest CTAs then start with it
+  std::vector<int2> by[NCLASS], heavy[NCLASS];
   out = PairLists();
   for (const int2& pr : cand) {
     if (!keep(pr)) continue;
     const EriShell &A = bra[pr.x], &B = bra[pr.y];
-    by[A.l * (LMAX + 1) + B.l].push_back(pr);
+    (A.nprim * B.nprim >= 8 ? heavy : by)[A.l * (LMAX + 1) + B.l].push_back(pr);
     const int lab = A.l + B.l, nab = A.nfunc * B.nfunc;
     out.wide[lab] = std::max(out.wide[lab], nab);
     if (A.nprim * B.nprim > 1) out.wide_contracted[lab] = std::max(out.wide_contracted[lab], nab);
@@ -545,7 +546,8 @@ void pair_lists(const std::vector<EriShell>& bra, const std::vector<int2>& cand,
     for (int la = std::max(0, lab - LMAX); la <= std::min(lab, LMAX); ++la) {
       const int c = la * (LMAX + 1) + lab - la;
       out.start[c] = static_cast<long>(out.pairs.size());
-      out.count[c] = static_cast<long>(by[c].size());
+      out.count[c] = static_cast<long>(by[c].size() + heavy[c].size());
+      out.pairs.insert(out.pairs.end(), heavy[c].begin(), heavy[c].end());
       out.pairs.insert(out.pairs.end(), by[c].begin(), by[c].end());
     }
   }
@@ -557,7 +559,7 @@ const LaunchThread kLaunchThread[LMAX + 1] = {launch_lc<0>, launch_lc<1>, launch
 
 // The class (la, lb | group g of the kets) on k_eri.
 int launch_group(rijk_ctx* ctx, EriLaunch P, const PairLists& pl, const int2* pairs_dev, int la, int lb, int lc,
-                 int maxsm) {
+                 int maxsm, cudaStream_t s) {
   const int c = la * (LMAX + 1) + lb;
   if (pl.count[c] == 0) return RIJK_OK;
   P.la = la;
@@ -577,20 +579,45 @@ int launch_group(rijk_ctx* ctx, EriLaunch P, const PairLists& pl, const int2* pa
   }
   const long gpb = static_cast<long>(warps) * 32 / P.G;
   const long blocks = std::min<long>((P.npair * P.nket + gpb - 1) / gpb, 148L * 32);
-  k_eri<<<static_cast<unsigned>(blocks), warps * 32, smem, ctx->stream>>>(P);
+  k_eri<<<static_cast<unsigned>(blocks), warps * 32, smem, s>>>(P);
   return RIJK_OK;
 }
 
-// Launches every class of one output block.  pairs_dev holds PairLists::pairs on the device.
+// Aux shells of a k_eri_thread CTA.  64, one a thread, while that gives the GPU four CTAs an SM; fewer where the
+// class has fewer, or where the launch would leave SMs idle and the bra functions can be shared out instead
+// (each thread keeps at least three of them).
+int eri_tile(long npair, long nket, int wide) {
+  int tile = NT;
+  while (tile > 8 && (tile / 2 >= nket || (npair * ((nket + tile - 1) / tile) < 4 * 148 && wide * tile >= 6 * NT)))
+    tile /= 2;
+  return tile;
+}
+
+// Launches every class of one output block.  pairs_dev holds PairLists::pairs on the device.  The classes are
+// independent, and many are too small or end too raggedly to fill the GPU alone: they run on three streams.
+// With the shared tiles, s s sums in registers, long pairs first and the streams, all of (P|Q) and (mu nu|P) took
+// 4.0 instead of 9.4 ms at (H2O)8 cc-pVTZ/cc-pVTZ-JKFIT and 0.13 instead of 0.225 s at (H2O)32.
 int launch_classes(rijk_ctx* ctx, const EriLaunch& base, const PairLists& pl, const int2* pairs_dev,
                    const KetLists& kl, const int* kets_dev, int* launches) {
   int maxsm = 0;
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-  for (int lab = 0; lab <= 2 * LMAX; ++lab) {
+  const cudaStream_t streams[3] = {ctx->stream, ctx->j_stream, ctx->copy_stream};
+  cudaEventRecord(ctx->ev_pk, ctx->stream);
+  cudaStreamWaitEvent(ctx->j_stream, ctx->ev_pk, 0);
+  cudaStreamWaitEvent(ctx->copy_stream, ctx->ev_pk, 0);
+  auto join = [&]() {
+    cudaEventRecord(ctx->ev_jside, ctx->j_stream);
+    cudaEventRecord(ctx->ev_j, ctx->copy_stream);
+    cudaStreamWaitEvent(ctx->stream, ctx->ev_jside, 0);
+    cudaStreamWaitEvent(ctx->stream, ctx->ev_j, 0);
+  };
+  int turn = 0;
+  for (int lab = 2 * LMAX; lab >= 0; --lab) {
     const long np = pl.lab_start[lab + 1] - pl.lab_start[lab];
     if (np == 0) continue;
-    for (int g = 0; g < 2 * (LMAX + 1); ++g) {
+    for (int g = 2 * (LMAX + 1) - 1; g >= 0; --g) {
       const int lc = g / 2;
+      const cudaStream_t s = streams[turn++ % 3];
       EriLaunch P = base;
       P.kets = kets_dev + kl.start[g];
       P.nket = kl.start[g + 1] - kl.start[g];
@@ -602,21 +629,29 @@ int launch_classes(rijk_ctx* ctx, const EriLaunch& base, const PairLists& pl, co
       P.e1size = (3 * side * (lab + 2 - side) * (lab + 1) + 1) & ~1;
       P.esize = pl.wide[lab] * ((tet(lab) + 1) & ~1);
       const int contracted = kl.nprim[g] > 1 ? pl.wide[lab] : pl.wide_contracted[lab];
-      const size_t smem = (static_cast<size_t>(P.e1size) + P.esize + static_cast<size_t>(contracted) * NT * (2 * lc + 1)) *
-                          sizeof(double);
+      P.tile = eri_tile(np, P.nket, pl.wide[lab]);
+      const size_t smem = (static_cast<size_t>(P.e1size) + P.esize +
+                           static_cast<size_t>(contracted) * P.tile * (2 * lc + 1)) * sizeof(double);
       if (g % 2 == 0 && lab <= LAB_MAX && smem <= static_cast<size_t>(maxsm)) {
-        const cudaError_t e = kLaunchThread[lc](lab, P, smem, ctx->stream);
-        if (e != cudaSuccess) return cuda_check(ctx, e, "integral kernel launch");
+        const cudaError_t e = kLaunchThread[lc](lab, P, smem, s);
+        if (e != cudaSuccess) {
+          join();
+          return cuda_check(ctx, e, "integral kernel launch");
+        }
         ++*launches;
         continue;
       }
       for (int la = std::max(0, lab - LMAX); la <= std::min(lab, LMAX); ++la) {
         if (pl.count[la * (LMAX + 1) + lab - la] == 0) continue;
-        if (const int rc = launch_group(ctx, P, pl, pairs_dev, la, lab - la, lc, maxsm)) return rc;
+        if (const int rc = launch_group(ctx, P, pl, pairs_dev, la, lab - la, lc, maxsm, s)) {
+          join();
+          return rc;
+        }
         ++*launches;
       }
     }
   }
+  join();
   return cuda_check(ctx, cudaGetLastError(), "integral kernel launch");
 }
 
