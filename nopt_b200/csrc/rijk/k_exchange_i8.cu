@@ -2,29 +2,28 @@
 // with FP64 accuracy from exact int8 products (the Ozaki splitting scheme).
 //
 // tcgen05 has no FP64 kind.  Each row nu of X^T (the half-transformed tensor, k = Q n_c + i
-// contiguous) is written, over the k range of one split-K part r, as
-//     X[nu][k] = 2^e(r,nu) * sum_{s=0}^{7} d_s[nu][k] 2^{-7(s+1)},   d_s integer in [-64, 64],
-// with e chosen so that max_k |X[nu][k]| / 2^e < 1/2 (k_slice_x).  The digits are exact: each
-// step scales by 2^7, rounds to the nearest integer and keeps the exact remainder, so the value
-// left after 8 digits is at most 2^-57 of 2^e, which is below 2^-55 of the row maximum.  Then
-//     K_mu,nu = 2^(e_mu + e_nu) sum_g 2^{-7(g+2)} sum_{s+t=g} (d_s[mu] . d_t[nu]),
-// where every (d_s . d_t) is an exact s32 tensor-core sum (|d_s d_t| <= 4096; a part spans at
-// most 65504 k, and a group sums at most 8 pairs: 8 * 4096 * 65504 < 2^31 - 1).  The groups g < 8
-// (36 digit pairs) are kept; the dropped ones are below 9 * 2^-58 of 2^(e_mu + e_nu) per k,
-// the level of FP64 rounding in a sum of products.
+// contiguous) is written, over the k range of one split-K part r, as the 56-bit integers
+//     v = rint(X[nu][k] 2^-x(r,nu)),  |v| <= 127.49 2^48,   v = sum_{s=0}^{6} d_s 256^(6-s),
+// with balanced byte digits d_s in [-128, 127] (k_slice_x: one conversion, one 64-bit add that propagates
+// the carries, one exclusive or).  The rounding is at most 2^-55 of the row's maximum.  Then
+//     K_mu,nu = 2^(x_mu + x_nu) sum_g 256^(12-g) sum_{s+t=g} (d_s[mu] . d_t[nu]),
+// where every (d_s . d_t) is an exact s32 tensor-core sum (|d_s d_t| <= 2^14, a group sums at most 7
+// pairs, and a part spans at most 18720 k: 7 2^14 18720 < 2^31 - 1).  The groups g < 8 (34 digit pairs) are
+// kept.  The digits of a small value are as large as any other's, so a dropped group's products do not
+// shrink with the values: those of g = 8, 5 pairs of about 74^2, come to 2^-66 of the scales' product per k and
+// to 2^-57 over 7e5 k.  (Dropping g = 7 too would leave 2^-49, above the rounding of an FP64 sum.)
 //
-// Digit layout: row nu of the planes is kdim/32 blocks of 256 bytes, block c holding the 8 digits
-// of k in [32c, 32c + 32) as 8 runs of 32 bytes (digit-major).  A stage then moves two 128-byte
-// halves per row (digits 0-3, 4-7) with 128-byte-swizzled TMA boxes, and the K-major descriptor
-// of digit d points 32 (d mod 4) bytes into its half, as a 16-bit operand steps through K.
+// Digit layout: for 128 rows and 32 k, one block of 28 KB holding the 7 digits' 128 x 32 matrices as the
+// 8-row x 16-byte core matrices that an unswizzled K-major descriptor steps through.  A stage is then a
+// bulk copy of the A panel's block and 7 of the B panel's 64 rows, with no tensor map.
 //
-// k_syrk_i8: one CTA per (128 x 128 block (a, b), b <= a, split part r), in two passes over the
-// part: groups 0-3 (10 products, digits 0-3 only) and groups 4-7 (26 products), each into 4 TMEM
-// accumulators of 128 columns.  Every MMA is M 128, N 128, K 32: it reads 128 bytes of shared
-// memory operands per tensor clock, which the SM sustains (N 64 would need 192).  The epilogue of
-// pass 0 stores the scaled FP64 partial of its tiles, that of pass 1 adds to it (the same thread
-// and elements); the partials have the layout of k_syrk_f64, summed and unpacked by
-// launch_unpack_sym.
+// k_syrk_i8: one CTA per (128 x 64 tile (a, b), b <= 2 a + 1, split part).  TMEM holds the 8 groups'
+// 64 columns side by side, and B's digits lie side by side in shared memory, so one MMA multiplies a digit s
+// of A by several digits t of B, each result landing in the columns of its group s + t: 11 MMAs of up to
+// 256 columns a chunk instead of 34, which read 103 bytes of shared memory a tensor clock (one digit pair per
+// 128 x 128 MMA read 128, all that an SM delivers, before the copies into it).  One pass over the part fills
+// every group.  The epilogue joins the groups in two 64-bit integers, scales, and stores the FP64 partials
+// in the layout of k_syrk_f64, summed and unpacked by launch_unpack_sym.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -44,82 +43,20 @@ int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);
 
 namespace {
 
-constexpr int kDigits = 8;                     // digit planes per value
-constexpr int kChunk = 32;                     // k per stage and per MMA (one 32-byte swizzle atom row)
-constexpr int kI8Threads = 192;                // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
-constexpr int kBlock = kDigits * kChunk;       // bytes per row and 32 k: 8 digits x 32 B
-constexpr uint32_t kHalf = 128 * 128;          // 4 digits of a 128-row panel: 128 rows x 128 B
-constexpr uint32_t kI8Stage = 4 * kHalf;       // A digits 0-3, A 4-7, B 0-3, B 4-7: 64 KB
-constexpr long kMaxPart = 65504;               // k per split part: 8 * 4096 * 65504 < 2^31 - 1, every s32 sum exact
-constexpr int kI8SmemBudget = 225 * 1024;
+constexpr int kDigits = 7;                     // byte digits of a value
+constexpr int kGroups = 8;                     // groups s + t kept
+constexpr int kChunk = 32;                     // k per stage and per MMA
+constexpr int kI8Threads = 192;                // warp 0 copies, warp 1 MMA, warps 2-5 epilogue
+constexpr uint32_t kDigitA = 128 * kChunk;     // one digit of a 128-row panel: 4 KB
+constexpr uint32_t kDigitB = 64 * kChunk;      // one digit of a 64-row panel: 2 KB
+constexpr uint32_t kBlockBytes = kDigits * kDigitA;             // 28 KB
+constexpr uint32_t kI8Stage = kDigits * (kDigitA + kDigitB);    // 42 KB
+constexpr int kI8Stages = 5;
+constexpr long kMaxPart = 18720;               // k per split part: 7 2^14 18720 < 2^31 - 1, every s32 sum exact
+constexpr int kNonFinite = 1 << 20;            // row exponent of a row with an infinity or NaN
 
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
-}
-
-// ------------------------------------------------------------------ digit planes ----
-// One CTA per (row nu, part r), part length up to kMaxPart: a first sweep takes the row's maximum
-// over the part (from HBM), a second one re-reads the part (now in L2) and writes each thread's
-// 8 digits of 4 consecutive k as packed 4-byte words into the k's block.  Rows at or past npad
-// (the padding of the 128-row blocks), and k from kdim to the end of the last block, get zero
-// digits.
-constexpr int kSliceThreads = 256;
-
-__global__ void __launch_bounds__(kSliceThreads) k_slice_x(const double* __restrict__ XT, long npad, long npad2,
-                                                           long kdim, long kper, int8_t* __restrict__ Xs,
-                                                           int* __restrict__ E) {
-  __shared__ double wmax[kSliceThreads / 32];
-  const long row = blockIdx.x, part = blockIdx.y;
-  const long k0 = part * kper, k1 = std::min(k0 + kper, kdim);
-  const long kend = k1 == kdim ? (kdim + kChunk - 1) / kChunk * kChunk : k1;  // zero digits fill the last block
-  const long nblk = (kdim + kChunk - 1) / kChunk;
-  int8_t* out = Xs + static_cast<size_t>(row) * nblk * kBlock;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const bool live = row < npad;
-  const double* x = XT + static_cast<size_t>(live ? row : 0) * kdim;
-  double m = 0.0;
-  if (live)
-    for (long k = k0 + 4L * t; k < k1; k += 4L * kSliceThreads) {  // k1 and k are multiples of 4
-      const double2 a = *reinterpret_cast<const double2*>(x + k);
-      const double2 b = *reinterpret_cast<const double2*>(x + k + 2);
-      m = fmax(m, fmax(fmax(fabs(a.x), fabs(a.y)), fmax(fabs(b.x), fabs(b.y))));
-    }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) wmax[warp] = m;
-  __syncthreads();
-  m = wmax[0];
-#pragma unroll
-  for (int w = 1; w < kSliceThreads / 32; ++w) m = fmax(m, wmax[w]);
-  // m = f 2^(b+1) with f in [1/2, 1) (b = ilogb(m)); dividing by 2^(b+2) leaves |x| < 1/2
-  const int e = m > 0.0 ? ilogb(m) + 2 : 0;
-  if (t == 0) E[part * npad2 + row] = e;
-  for (long k = k0 + 4L * t; k < kend; k += 4L * kSliceThreads) {
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
-    if (live && k < k1) {
-      const double2 a = *reinterpret_cast<const double2*>(x + k);
-      const double2 b = *reinterpret_cast<const double2*>(x + k + 2);
-      v[0] = a.x;
-      v[1] = a.y;
-      v[2] = b.x;
-      v[3] = b.y;
-    }
-    uint32_t packed[kDigits] = {};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      double r = ldexp(v[q], -e);
-#pragma unroll
-      for (int d = 0; d < kDigits; ++d) {
-        const double tt = r * 128.0;
-        const double dg = rint(tt);
-        r = tt - dg;
-        packed[d] |= (static_cast<uint32_t>(static_cast<int>(dg)) & 0xFFu) << (8 * q);
-      }
-    }
-    int8_t* blk = out + (k / kChunk) * kBlock + (k % kChunk);
-#pragma unroll
-    for (int d = 0; d < kDigits; ++d) *reinterpret_cast<uint32_t*>(blk + d * kChunk) = packed[d];
-  }
 }
 
 // 2^e exactly for |e| <= 1000 (the exponent bits), else through ldexp.
@@ -127,64 +64,198 @@ __device__ __forceinline__ double pow2i(int e) {
   return (e >= -1000 && e <= 1000) ? __longlong_as_double(static_cast<long long>(e + 1023) << 52) : ldexp(1.0, e);
 }
 
+// ------------------------------------------------------------------ digits ----
+// The exponent x of a row whose largest magnitude has the bits `top`: max / 2^x <= 127.49 2^48.
+__device__ __forceinline__ int row_exponent(unsigned long long top) {
+  if (top >= 0x7ff0000000000000ull) return kNonFinite;
+  if (top == 0) return 0;
+  const double m = __longlong_as_double(static_cast<long long>(top));
+  const int e = ilogb(m) + 1;  // m < 2^e
+  return (ldexp(m, -e) <= 0.995 ? e : e + 1) - 55;
+}
+
+// 16 values of one row as 16 bytes of each digit, digit 0 the leading one.
+__device__ __forceinline__ void digits16(const double (&x)[16], int ex, uint4 (&d)[kDigits]) {
+  uint32_t* out = reinterpret_cast<uint32_t*>(d);
+  const bool plain = ex > -1000 && ex < 1000;
+  const double f = plain ? pow2i(-ex) : 0.0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const double y = plain ? x[4 * q + j] * f : ldexp(x[4 * q + j], -ex);
+      const unsigned long long u =
+          (static_cast<unsigned long long>(__double2ll_rn(y)) + 0x0080808080808080ull) ^ 0x0080808080808080ull;
+      lo[j] = static_cast<uint32_t>(u);
+      hi[j] = static_cast<uint32_t>(u >> 32);
+    }
+    // byte b of the four words, b = 0 .. 3 (of lo: digits 6 .. 3; of hi: digits 2 .. 0)
+    const uint32_t l01 = __byte_perm(lo[0], lo[1], 0x5140), l23 = __byte_perm(lo[2], lo[3], 0x5140);
+    const uint32_t m01 = __byte_perm(lo[0], lo[1], 0x7362), m23 = __byte_perm(lo[2], lo[3], 0x7362);
+    const uint32_t h01 = __byte_perm(hi[0], hi[1], 0x5140), h23 = __byte_perm(hi[2], hi[3], 0x5140);
+    const uint32_t n01 = __byte_perm(hi[0], hi[1], 0x7362), n23 = __byte_perm(hi[2], hi[3], 0x7362);
+    out[6 * 4 + q] = __byte_perm(l01, l23, 0x5410);
+    out[5 * 4 + q] = __byte_perm(l01, l23, 0x7632);
+    out[4 * 4 + q] = __byte_perm(m01, m23, 0x5410);
+    out[3 * 4 + q] = __byte_perm(m01, m23, 0x7632);
+    out[2 * 4 + q] = __byte_perm(h01, h23, 0x5410);
+    out[1 * 4 + q] = __byte_perm(h01, h23, 0x7632);
+    out[0 * 4 + q] = __byte_perm(n01, n23, 0x5410);
+  }
+}
+
+// Digits of X^T.  One CTA per (8 rows, part): a first sweep takes the rows' maxima over the part (from
+// HBM), a second one re-reads it (now in L2) and writes the digits, a lane per row and 16 k, so that 8
+// lanes fill a 128-byte core matrix.  Rows at or past npad (the padding of the 128-row blocks), and k from
+// kdim to the end of the last block, get zero digits.  HBM bounds it: 8 bytes read and 7 written per value.
+constexpr int kSliceThreads = 256;
+
+__global__ void __launch_bounds__(kSliceThreads) k_slice_x(const double* __restrict__ XT, long npad, long npad2,
+                                                           long kdim, long kper, uint8_t* __restrict__ Xs,
+                                                           int* __restrict__ E) {
+  __shared__ unsigned long long top[8][kSliceThreads / 32];
+  __shared__ int ex[8];
+  const long r0 = static_cast<long>(blockIdx.x) * 8, part = blockIdx.y;
+  const long k0 = part * kper, k1 = std::min(k0 + kper, kdim);
+  const long kend = k1 == kdim ? (kdim + kChunk - 1) / kChunk * kChunk : k1;  // zero digits fill the last block
+  const long nblk = (kdim + kChunk - 1) / kChunk;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const bool live = r0 < npad;  // npad is a multiple of 8
+#pragma unroll 1
+  for (int r = 0; r < 8; ++r) {
+    unsigned long long m = 0;  // magnitudes order as their bit patterns, infinities and NaN above all
+    if (live) {
+      const double* x = XT + (r0 + r) * kdim;
+      for (long k = k0 + 2L * t; k < k1; k += 2L * kSliceThreads) {  // kdim and kper are even
+        const double2 a = *reinterpret_cast<const double2*>(x + k);
+        const unsigned long long u = __double_as_longlong(a.x) & 0x7fffffffffffffffull;
+        const unsigned long long v = __double_as_longlong(a.y) & 0x7fffffffffffffffull;
+        m = max(m, max(u, v));
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) top[r][warp] = m;
+  }
+  __syncthreads();
+  if (t < 8) {
+    unsigned long long m = 0;
+    for (int w = 0; w < kSliceThreads / 32; ++w) m = max(m, top[t][w]);
+    ex[t] = row_exponent(m);
+    E[part * npad2 + r0 + t] = ex[t];
+  }
+  __syncthreads();
+  // lane: row lane % 8, 16-k group warp * 4 + lane / 8 of each 512 k
+  const int r = lane & 7;
+  const int x = ex[r] == kNonFinite ? 0 : ex[r];
+  const double* src = XT + (live ? r0 + r : 0) * kdim;
+  uint8_t* base = Xs + (r0 / 128) * nblk * kBlockBytes + ((r0 % 128) / 8) * 256 + r * 16;
+  for (long k = k0 + 16L * (warp * 4 + (lane >> 3)); k < kend; k += 16L * kSliceThreads / 8) {
+    double v[16];
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      double2 a = make_double2(0.0, 0.0);
+      if (live && k + j < k1) a = *reinterpret_cast<const double2*>(src + k + j);
+      v[j] = a.x;
+      v[j + 1] = a.y;
+    }
+    uint4 d[kDigits];
+    digits16(v, x, d);
+    uint8_t* out = base + (k / kChunk) * kBlockBytes + ((k / 16) & 1) * 128;
+#pragma unroll
+    for (int s = 0; s < kDigits; ++s) *reinterpret_cast<uint4*>(out + s * kDigitA) = d[s];
+  }
+}
+
 // ------------------------------------------------------------------ int8 SYRK ----
+// The 8 groups of 16 columns (group g 64 columns after group g - 1) of this thread's TMEM lane, joined:
+// sum_g v_g 256^(3-g), groups 0 - 3 and 4 - 7 each in one 64-bit integer (|v_g| < 2^31, so below 2^56).
+__device__ __forceinline__ void join_groups16(uint32_t taddr, double (&w)[16]) {
+  long long hi[16], lo[16];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t v[4][16];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) tmem_ld16_nowait(taddr + (4 * h + g) * 64, v[g]);
+    tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      long long x = static_cast<int32_t>(v[0][j]);
+#pragma unroll
+      for (int g = 1; g < 4; ++g) x = x * 256 + static_cast<int32_t>(v[g][j]);
+      (h == 0 ? hi[j] : lo[j]) = x;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) w[j] = fma(static_cast<double>(lo[j]), 1.0 / 4294967296.0, static_cast<double>(hi[j]));
+}
+
+// x 2^e
+__device__ __forceinline__ double scale2(double x, int e) { return (e > -1000 && e < 1000) ? x * pow2i(e) : ldexp(x, e); }
+
 struct I8Params {
+  const uint8_t* Xs;
   long kdim, kper;
-  int npad2, nt, stages;
+  int npad2, nt;
   double* Kpart;  // FP64 partials [part][ntile][64][64]
   long ntile;
   const int* E;   // row exponents [part][npad2]
   int* err;
 };
 
-// One stage's MMAs of pass `pass` (groups 4 pass .. 4 pass + 3).  Digit d of a panel sits in half
-// d / 4, 32 (d mod 4) bytes into each 128-byte swizzled row.  The first product of a group in a
-// pass (digits (0, g), first chunk) starts its accumulator.
-__device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t sa, uint32_t sb, int pass, bool later) {
-  constexpr uint64_t kDesc = sw128_desc_bits(16, 1024);
-  constexpr uint32_t id = idesc_s8_s32(128, 128);
+// One chunk's MMAs: digit s of A against digits 0 .. min(6, 7 - s) of B, group s + t in the columns 64 (s + t).
+// The chunk that starts the sums (first) overwrites each group on its first product: digit s = 0 starts
+// groups 0 - 6, and (1, 6) starts group 7.
+__device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t sa, uint32_t sb, bool first) {
+  constexpr uint64_t kDesc = plain_desc_bits(128, 256);  // core matrices 128 B apart along k, 256 B along rows
 #pragma unroll
   for (int s = 0; s < kDigits; ++s) {
-    const uint64_t da = sw128_desc(sa + (s / 4) * kHalf + (s % 4) * 32, kDesc);
+    const uint64_t da = sw128_desc(sa + s * kDigitA, kDesc);
+    const int n = kGroups - s < kDigits ? kGroups - s : kDigits;  // digits of B
 #pragma unroll
-    for (int t = 0; t < kDigits - s; ++t) {
-      if ((s + t) / 4 != pass) continue;
-      const uint64_t db = sw128_desc(sb + (t / 4) * kHalf + (t % 4) * 32, kDesc);
-      umma_s8(tmem + ((s + t) % 4) * 128, da, db, id, (later || s != 0) ? 1u : 0u);
+    for (int t = 0; t < n; t += 4) {
+      const int m = n - t < 4 ? n - t : 4;  // up to 256 columns
+      const uint64_t db = sw128_desc(sb + t * kDigitB, kDesc);
+      const uint32_t d = tmem + (s + t) * 64;
+      if (s == 1 && t + m == kDigits) {  // its last digit is group 7's first product
+        if (m > 1) umma_s8(d, da, db, idesc_s8_s32(128, 64 * (m - 1)), 1u);
+        umma_s8(d + 64 * (m - 1), da, sw128_desc(sb + (t + m - 1) * kDigitB, kDesc), idesc_s8_s32(128, 64), first ? 0u : 1u);
+      } else {
+        umma_s8(d, da, db, idesc_s8_s32(128, 64 * m), (first && s == 0) ? 0u : 1u);
+      }
     }
   }
 }
 
-__global__ void __launch_bounds__(kI8Threads, 1)
-    k_syrk_i8(const __grid_constant__ CUtensorMap mapX, I8Params p) {
+__global__ void __launch_bounds__(kI8Threads, 1) k_syrk_i8(I8Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  const int S = p.stages;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * kI8Stage);
-  uint64_t* empty = full + S;
-  uint64_t* tfull = empty + S;   // a pass's accumulators are final (phase = pass)
-  uint64_t* tempty = tfull + 1;  // pass 0's accumulators have been read
-  uint64_t* drain = tempty + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kI8Stages * kI8Stage);
+  uint64_t* empty = full + kI8Stages;
+  uint64_t* tfull = empty + kI8Stages;  // the accumulators are final
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  long a, b;
-  tri_decode(blockIdx.x, a, b);  // 128-row blocks, b <= a
-  const bool diag = a == b;
+  // tile (a, b): 128-row block a, 64-row block b <= 2 a + 1; blocks a' < a hold a (a + 1) tiles
+  const int tile = blockIdx.x;
+  int a = static_cast<int>((sqrtf(4.0f * tile + 1.0f) - 1.0f) * 0.5f);
+  while (a * (a + 1) > tile) --a;
+  while ((a + 1) * (a + 2) <= tile) ++a;
+  const int b = tile - a * (a + 1);
   const long part = blockIdx.y;
   const long k0 = part * p.kper;
   const long k1 = std::min(k0 + p.kper, p.kdim);
   const int nch = static_cast<int>((k1 - k0 + kChunk - 1) / kChunk);
+  const long nblk = (p.kdim + kChunk - 1) / kChunk;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < S; ++i) {
+    for (int i = 0; i < kI8Stages; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
     mbar_init(tfull, 1);
-    mbar_init(tempty, 4);
-    mbar_init(drain, 1);
     *abort = 0;
     fence_barrier_init();
   }
@@ -199,38 +270,35 @@ __global__ void __launch_bounds__(kI8Threads, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      tma_prefetch_desc(&mapX);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int pass = 0; pass < 2 && ok; ++pass) {
-        const int halves = pass + 1;  // pass 0 needs digits 0-3 only
-        const uint32_t bytes = (diag ? 1u : 2u) * halves * kHalf;
-        for (int c = 0; c < nch; ++c) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort)) {
-            ok = false;
-            break;
-          }
-          uint8_t* st = smem + stage * kI8Stage;
-          const int x = static_cast<int>((k0 / kChunk + c) * kBlock);  // byte column of chunk c
-          mbar_expect_tx(&full[stage], bytes);
-          for (int h = 0; h < halves; ++h) {
-            tma_load_2d(st + h * kHalf, &mapX, &full[stage], x + 128 * h, static_cast<int>(a * 128));
-            if (!diag)
-              tma_load_2d(st + (2 + h) * kHalf, &mapX, &full[stage], x + 128 * h, static_cast<int>(b * 128));
-          }
-          if (++stage == S) {
-            stage = 0;
-            phase ^= 1;
-          }
+      const uint8_t* pa = p.Xs + (a * nblk + k0 / kChunk) * kBlockBytes;
+      const uint8_t* pb = p.Xs + ((b / 2) * nblk + k0 / kChunk) * kBlockBytes + (b & 1) * kDigitB;
+      for (int c = 0; c < nch; ++c) {
+        if (!mbar_wait(&empty[stage], phase ^ 1, abort)) {
+          ok = false;
+          break;
+        }
+        uint8_t* st = smem + stage * kI8Stage;
+        mbar_expect_tx(&full[stage], kI8Stage);
+        bulk_load(st, pa, kBlockBytes, &full[stage]);
+#pragma unroll
+        for (int d = 0; d < kDigits; ++d)
+          bulk_load(st + kBlockBytes + d * kDigitB, pb + d * kDigitA, kDigitB, &full[stage]);
+        pa += kBlockBytes;
+        pb += kBlockBytes;
+        if (++stage == kI8Stages) {
+          stage = 0;
+          phase ^= 1;
         }
       }
       if (!ok) {
         *abort = 1;
         atomicOr(p.err, DEVERR_TIMEOUT);
       }
-      volatile int never = 0;
-      for (int i = 0; i < S; ++i) {
+      volatile int never = 0;  // every issued copy has landed before the CTA exits
+      for (int i = 0; i < kI8Stages; ++i) {
         uint32_t par = (i < stage) ? phase : (phase ^ 1);
         mbar_wait(&full[i], par, &never);
       }
@@ -240,89 +308,57 @@ __global__ void __launch_bounds__(kI8Threads, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int pass = 0; pass < 2 && ok; ++pass) {
-        if (pass == 1) {  // the epilogue has read pass 0's accumulators
-          if (!mbar_wait(tempty, 0, abort)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
+      for (int c = 0; c < nch; ++c) {
+        if (!mbar_wait(&full[stage], phase, abort)) {
+          ok = false;
+          break;
         }
-        for (int c = 0; c < nch; ++c) {
-          if (!mbar_wait(&full[stage], phase, abort)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * kI8Stage);
-          issue_chunk(tmem, sa, diag ? sa : sa + 2 * kHalf, pass, c != 0);
-          umma_commit(&empty[stage]);
-          if (++stage == S) {
-            stage = 0;
-            phase ^= 1;
-          }
+        tc_fence_after();
+        const uint32_t sa = smem_u32(smem + stage * kI8Stage);
+        issue_chunk(tmem, sa, sa + kBlockBytes, c == 0);
+        umma_commit(&empty[stage]);
+        if (++stage == kI8Stages) {
+          stage = 0;
+          phase ^= 1;
         }
-        if (ok) umma_commit(tfull);
       }
       if (!ok) {
         *abort = 1;
         atomicOr(p.err, DEVERR_TIMEOUT);
       }
-      umma_commit(drain);
+      umma_commit(tfull);  // also after a give-up: every MMA issued ends before TMEM is freed
       volatile int never = 0;
-      if (!mbar_wait(drain, 0, &never)) atomicOr(p.err, DEVERR_TIMEOUT);
+      if (!mbar_wait(tfull, 0, &never)) atomicOr(p.err, DEVERR_TIMEOUT);
     }
   } else {
     const int q = warp & 3;
     const int row = q * 32 + lane;     // row of the 128-row block
     const long ra = 2 * a + row / 64;  // 64-row tile, the same for the warp's 32 lanes
     const int r = row % 64;
-    const int* Ep = p.E + part * p.npad2;
-    const double rs = pow2i(Ep[a * 128 + row]);  // row scale 2^e
-    const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16);
-    bool ok = true;
-    for (int pass = 0; pass < 2; ++pass) {
-      if (!__all_sync(0xffffffffu, mbar_wait(tfull, pass, abort)) || __any_sync(0xffffffffu, *abort)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
-      double gf[4];  // 2^-7(4 pass + g + 2)
-#pragma unroll
-      for (int g = 0; g < 4; ++g) gf[g] = pow2i(-7 * (4 * pass + g + 2));
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(tfull, 0, abort)) && !__any_sync(0xffffffffu, *abort);
+    tc_fence_after();
+    // tiles above the diagonal (their mirror is stored) and rows past npad are left out
+    if (ok && b <= ra && ra < p.nt) {
+      const int* Ep = p.E + part * p.npad2;
+      const int ea = Ep[a * 128 + row];
+      const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16);
+      double* out = p.Kpart + (part * p.ntile + tri_index(ra, b)) * TILE2 + static_cast<long>(r) * TILE;
 #pragma unroll 1
-      for (int c0 = 0; c0 < 128; c0 += 16) {
-        const long cb = 2 * b + c0 / 64;
-        // upper-right sub-tile of a diagonal block (its mirror is stored), or rows past npad
-        if ((diag && ra < cb) || ra >= p.nt) continue;
-        uint32_t v[4][16];
-#pragma unroll
-        for (int g = 0; g < 4; ++g) tmem_ld16_nowait(lane_base + g * 128 + c0, v[g]);
-        tmem_wait_ld();
-        double* out = p.Kpart + (part * p.ntile + tri_index(ra, cb)) * TILE2 + static_cast<long>(r) * TILE + (c0 % 64);
+      for (int c0 = 0; c0 < 64; c0 += 16) {
+        double v[16];
+        join_groups16(lane_base + c0, v);
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
           double w[2];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            double acc = 0.0;
-#pragma unroll
-            for (int g = 3; g >= 0; --g)  // smallest first; the group factors are exact powers of two
-              acc = fma(static_cast<double>(static_cast<int32_t>(v[g][j + h])), gf[g], acc);
-            w[h] = acc * (rs * pow2i(__ldg(Ep + b * 128 + c0 + j + h)));
+            const int eb = __ldg(Ep + b * 64 + c0 + j + h);
+            w[h] = (ea == kNonFinite || eb == kNonFinite) ? __longlong_as_double(0x7ff8000000000000ll)
+                                                          : scale2(v[j + h], 72 + ea + eb);
           }
-          double2* o = reinterpret_cast<double2*>(out + j);
-          if (pass == 1) {
-            const double2 prev = *o;
-            w[0] += prev.x;
-            w[1] += prev.y;
-          }
-          *o = make_double2(w[0], w[1]);
+          *reinterpret_cast<double2*>(out + c0 + j) = make_double2(w[0], w[1]);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (pass == 0 && lane == 0) mbar_arrive(tempty);
     }
     if (!ok && lane == 0) {
       *abort = 1;
@@ -335,38 +371,6 @@ __global__ void __launch_bounds__(kI8Threads, 1)
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
-}
-
-// ------------------------------------------------------------------ tensor maps ----
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn_i8() {
-  // looked up once (thread-safe static initialisation: contexts may live on several host threads)
-  static const EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      return reinterpret_cast<EncodeTiledFn>(p);
-    return static_cast<EncodeTiledFn>(nullptr);
-  }();
-  return fn;
-}
-
-// 2-D map of the digit rows [rows][cols bytes], box {128 bytes, box_rows}, 128-byte swizzle.
-bool make_map_i8(CUtensorMap* m, const void* base, uint64_t cols, uint64_t rows, uint32_t box_rows) {
-  EncodeTiledFn fn = encode_fn_i8();
-  if (!fn) return false;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols};
-  cuuint32_t box[2] = {128, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
 }
 
 int sm_count(int device) {
@@ -382,14 +386,14 @@ int sm_count(int device) {
 
 }  // namespace
 
-// Split-K parts of the int8 SYRK: chunk-aligned, at most kMaxPart k each, and enough CTAs for
-// about two waves (one CTA per SM), chosen among [want, 4 want] so that the last wave is fullest.
+// Split-K parts of the int8 SYRK: chunk-aligned, at most kMaxPart k each; among up to four times the fewest
+// parts (or parts for one wave), the count whose last wave of CTAs, one an SM, is fullest.
 int syrk_i8_parts(long nt, long kdim, int device, long* kper_out) {
-  const long nb = (nt + 1) / 2, ctas_per_part = nb * (nb + 1) / 2;
+  const long nb = (nt + 1) / 2, ctas_per_part = nb * (nb + 1);
   const long sms = sm_count(device);
   const long nchunks = (kdim + kChunk - 1) / kChunk;
   const long min_parts = (kdim + kMaxPart - 1) / kMaxPart;
-  const long want = std::max(min_parts, (2 * sms + ctas_per_part - 1) / ctas_per_part);
+  const long want = std::max(min_parts, sms / ctas_per_part);
   long best = want;
   double best_eff = 0.0;
   for (long sp = want; sp <= 4 * want && sp <= std::max<long>(1, nchunks); ++sp) {
@@ -406,26 +410,22 @@ int syrk_i8_parts(long nt, long kdim, int device, long* kper_out) {
   return static_cast<int>((kdim + kper - 1) / kper);
 }
 
-// K partials of the FP64 form from X^T (npad x kdim doubles) through the int8 digit planes.
+// K partials of the FP64 form from X^T (npad x kdim doubles) through its digits.
 int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int nparts, long kper, double* Kpart,
             cudaStream_t s) {
   const long npad2 = round_up(npad, 128);
   const long nblk = (kdim + kChunk - 1) / kChunk;
-  const size_t planes = static_cast<size_t>(npad2) * nblk * kBlock;
   int rc;
-  if ((rc = ensure(ctx, ctx->Xs, planes, "int8 digit planes")) ||
+  if ((rc = ensure(ctx, ctx->Xs, static_cast<size_t>(npad2 / 128) * nblk * kBlockBytes, "int8 digits of X")) ||
       (rc = ensure(ctx, ctx->Xe, static_cast<size_t>(nparts) * npad2 * sizeof(int), "digit exponents")))
     return rc;
-  int8_t* Xs = static_cast<int8_t*>(ctx->Xs.p);
+  uint8_t* Xs = static_cast<uint8_t*>(ctx->Xs.p);
   int* E = static_cast<int*>(ctx->Xe.p);
-  k_slice_x<<<dim3(static_cast<unsigned>(npad2), static_cast<unsigned>(nparts)), kSliceThreads, 0, s>>>(
+  k_slice_x<<<dim3(static_cast<unsigned>(npad2 / 8), static_cast<unsigned>(nparts)), kSliceThreads, 0, s>>>(
       XT, npad, npad2, kdim, kper, Xs, E);
   prof_mark(ctx, "slice_x");
-  CUtensorMap mA;
-  const uint64_t cols = static_cast<uint64_t>(nblk) * kBlock;
-  if (!make_map_i8(&mA, Xs, cols, static_cast<uint64_t>(npad2), 128))
-    return set_err(ctx, RIJK_ERR_CUDA, "tensor map encoding failed (int8 digits)");
   I8Params ip{};
+  ip.Xs = Xs;
   ip.kdim = kdim;
   ip.kper = kper;
   ip.npad2 = static_cast<int>(npad2);
@@ -434,12 +434,11 @@ int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int 
   ip.ntile = nt * (nt + 1) / 2;
   ip.E = E;
   ip.err = static_cast<int*>(ctx->err.p);
-  ip.stages = std::min(4, static_cast<int>((kI8SmemBudget - 2048) / kI8Stage));
-  const size_t smem = static_cast<size_t>(ip.stages) * kI8Stage + 1024 + 256;
+  const size_t smem = static_cast<size_t>(kI8Stages) * kI8Stage + 1024 + 256;
   ensure_smem_limit(reinterpret_cast<const void*>(k_syrk_i8), smem);
   const long nb = npad2 / 128;
-  dim3 grid(static_cast<unsigned>(nb * (nb + 1) / 2), static_cast<unsigned>(nparts));
-  k_syrk_i8<<<grid, kI8Threads, smem, s>>>(mA, ip);
+  dim3 grid(static_cast<unsigned>(nb * (nb + 1)), static_cast<unsigned>(nparts));
+  k_syrk_i8<<<grid, kI8Threads, smem, s>>>(ip);
   return cuda_check(ctx, cudaGetLastError(), "int8 SYRK launch");
 }
 

@@ -72,6 +72,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
+// Contiguous global -> shared copy of `bytes` (a multiple of 16; both addresses 16-byte aligned).
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar))
+      : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];\n" ::"l"(map) : "memory");
 }
@@ -161,11 +168,12 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr, uint64_t bits) {
   return bits | static_cast<uint64_t>((saddr >> 4) & 0x3FFF);
 }
 
-// Descriptor bits of a K-major operand with 32-byte swizzle (layout code 6): 8-row x 32-byte
-// atoms, SBO = 256 B between atoms.  One atom row holds the 32 int8 K-elements of one kind::i8 MMA.
-__host__ __device__ constexpr uint64_t sw32_desc_bits(uint32_t sbo_bytes) {
-  return (static_cast<uint64_t>(1) << 16) | (static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32) | (1ULL << 46) |
-         (6ULL << 61);
+// Descriptor bits of an unswizzled operand of 8-row x 16-byte core matrices (layout code 0).  K-major: LBO between
+// the core matrices along k, SBO between 8-row groups.  MN-major (a core matrix is 8 k x 16 bytes of M or N): SBO
+// between the core matrices along M or N, LBO between groups of 8 k.
+__host__ __device__ constexpr uint64_t plain_desc_bits(uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return (static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16) |
+         (static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32) | (1ULL << 46);
 }
 
 // Instruction descriptor of kind::i8: D s32 (bits 4-5 = 2), A and B signed 8-bit (bits 7-9 and
