@@ -61,13 +61,15 @@ extern "C" {
 #define RIJK_LAYOUT_PACKED 1    /* I3[(mu*(mu+1)/2 + nu)*naux + P], mu >= nu                    */
 
 /* Arithmetic of one Fock build. */
-#define RIJK_PREC_FP64 0  /* FP64 throughout: the drop-in form                                   */
+#define RIJK_PREC_FP64 0  /* FP64 throughout: the drop-in form.  Large exchanges (from about 1e10 FLOPs
+                             on) run on tcgen05 tensor cores: operands as seven int8 digits with
+                             power-of-two scales, 34 exact s32 digit products, FP64 scaling and sums
+                             (the Ozaki splitting scheme), with smaller errors than FP64 FMAs; the
+                             half-transform so only while the digits of B (0.9 to 1.1 times its
+                             bytes) find room in device memory                                  */
 #define RIJK_PREC_MIXED 1 /* exchange half-transform and K on tcgen05 tensor cores with split-BF16
                              (3-term) operands and FP32 accumulation; Coulomb in FP64          */
-#define RIJK_PREC_FP64_TC 2 /* FP64 results, with K = X^T X on tcgen05 tensor cores: X^T split
-                             into 8 int8 digit planes per row and split-K part (a power-of-two
-                             exponent each), 36 exact s32 digit products, FP64 scaling and sums
-                             (the Ozaki splitting scheme); J and the half-transform as FP64   */
+#define RIJK_PREC_FP64_TC 2 /* RIJK_PREC_FP64 with K = X^T X from int8 digits at every size       */
 
 typedef struct rijk_ctx rijk_ctx;
 
@@ -77,7 +79,7 @@ typedef struct {
   double ms_last_fock;    /* last Fock build, device time                                   */
   double ms_coulomb;      /* from its start until J is complete (the w and J passes)        */
   double ms_exchange;     /* from then until its end.  FP64 and FP64_TC builds run the
-                             Coulomb pair beside the half-transform, so there the exchange
+                             Coulomb pair beside the exchange, so there the exchange
                              starts before J is complete; mixed builds run them in turn    */
   double flops_last_fock; /* algorithmic FLOPs of the last build                            */
   double bytes_last_fock; /* algorithmic HBM bytes of the last build                        */
@@ -103,7 +105,7 @@ int rijk_create(rijk_ctx** ctx, int device);
 int rijk_destroy(rijk_ctx* ctx);
 /* Run on the caller's CUDA stream (a cudaStream_t) instead of the context's own.  An FP64 or FP64_TC
  * build also runs its Coulomb passes on a second stream the context owns: that stream waits on the
- * caller's stream at the start of the build, and the caller's stream waits on it before the build's
+ * caller's stream in the build, and the caller's stream waits on it before the build's
  * end, so work queued after the build on the caller's stream sees J and K. */
 int rijk_set_stream(rijk_ctx* ctx, void* stream);
 int rijk_last_error(const rijk_ctx* ctx, char* buf, int len);

@@ -32,8 +32,8 @@
 #include <cmath>
 #include <cstdint>
 
+#include "i8_digits.cuh"
 #include "rijk_internal.h"
-#include "tc_util.cuh"
 
 namespace rijk {
 
@@ -43,78 +43,23 @@ int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);
 
 namespace {
 
-constexpr int kDigits = 7;                     // byte digits of a value
-constexpr int kGroups = 8;                     // groups s + t kept
-constexpr int kChunk = 32;                     // k per stage and per MMA
 constexpr int kI8Threads = 192;                // warp 0 copies, warp 1 MMA, warps 2-5 epilogue
-constexpr uint32_t kDigitA = 128 * kChunk;     // one digit of a 128-row panel: 4 KB
 constexpr uint32_t kDigitB = 64 * kChunk;      // one digit of a 64-row panel: 2 KB
-constexpr uint32_t kBlockBytes = kDigits * kDigitA;             // 28 KB
 constexpr uint32_t kI8Stage = kDigits * (kDigitA + kDigitB);    // 42 KB
 constexpr int kI8Stages = 5;
 constexpr long kMaxPart = 18720;               // k per split part: 7 2^14 18720 < 2^31 - 1, every s32 sum exact
-constexpr int kNonFinite = 1 << 20;            // row exponent of a row with an infinity or NaN
 
-__device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
-  return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
-}
-
-// 2^e exactly for |e| <= 1000 (the exponent bits), else through ldexp.
-__device__ __forceinline__ double pow2i(int e) {
-  return (e >= -1000 && e <= 1000) ? __longlong_as_double(static_cast<long long>(e + 1023) << 52) : ldexp(1.0, e);
-}
-
-// ------------------------------------------------------------------ digits ----
-// The exponent x of a row whose largest magnitude has the bits `top`: max / 2^x <= 127.49 2^48.
-__device__ __forceinline__ int row_exponent(unsigned long long top) {
-  if (top >= 0x7ff0000000000000ull) return kNonFinite;
-  if (top == 0) return 0;
-  const double m = __longlong_as_double(static_cast<long long>(top));
-  const int e = ilogb(m) + 1;  // m < 2^e
-  return (ldexp(m, -e) <= 0.995 ? e : e + 1) - 55;
-}
-
-// 16 values of one row as 16 bytes of each digit, digit 0 the leading one.
-__device__ __forceinline__ void digits16(const double (&x)[16], int ex, uint4 (&d)[kDigits]) {
-  uint32_t* out = reinterpret_cast<uint32_t*>(d);
-  const bool plain = ex > -1000 && ex < 1000;
-  const double f = plain ? pow2i(-ex) : 0.0;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    uint32_t lo[4], hi[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const double y = plain ? x[4 * q + j] * f : ldexp(x[4 * q + j], -ex);
-      const unsigned long long u =
-          (static_cast<unsigned long long>(__double2ll_rn(y)) + 0x0080808080808080ull) ^ 0x0080808080808080ull;
-      lo[j] = static_cast<uint32_t>(u);
-      hi[j] = static_cast<uint32_t>(u >> 32);
-    }
-    // byte b of the four words, b = 0 .. 3 (of lo: digits 6 .. 3; of hi: digits 2 .. 0)
-    const uint32_t l01 = __byte_perm(lo[0], lo[1], 0x5140), l23 = __byte_perm(lo[2], lo[3], 0x5140);
-    const uint32_t m01 = __byte_perm(lo[0], lo[1], 0x7362), m23 = __byte_perm(lo[2], lo[3], 0x7362);
-    const uint32_t h01 = __byte_perm(hi[0], hi[1], 0x5140), h23 = __byte_perm(hi[2], hi[3], 0x5140);
-    const uint32_t n01 = __byte_perm(hi[0], hi[1], 0x7362), n23 = __byte_perm(hi[2], hi[3], 0x7362);
-    out[6 * 4 + q] = __byte_perm(l01, l23, 0x5410);
-    out[5 * 4 + q] = __byte_perm(l01, l23, 0x7632);
-    out[4 * 4 + q] = __byte_perm(m01, m23, 0x5410);
-    out[3 * 4 + q] = __byte_perm(m01, m23, 0x7632);
-    out[2 * 4 + q] = __byte_perm(h01, h23, 0x5410);
-    out[1 * 4 + q] = __byte_perm(h01, h23, 0x7632);
-    out[0 * 4 + q] = __byte_perm(n01, n23, 0x5410);
-  }
-}
-
-// Digits of X^T.  One CTA per (8 rows, part): a first sweep takes the rows' maxima over the part (from
-// HBM), a second one re-reads it (now in L2) and writes the digits, a lane per row and 16 k, so that 8
+// Digits of X^T.  One CTA per (8 rows, part).  The rows' maxima over the part come with X (known: k_xform_i8
+// leaves them in `tops`), or from a first sweep over it; then the digits are written, a lane per row and 16 k, so that 8
 // lanes fill a 128-byte core matrix.  Rows at or past npad (the padding of the 128-row blocks), and k from
 // kdim to the end of the last block, get zero digits.  HBM bounds it: 8 bytes read and 7 written per value.
 constexpr int kSliceThreads = 256;
 
+template <bool KNOWN>
 __global__ void __launch_bounds__(kSliceThreads) k_slice_x(const double* __restrict__ XT, long npad, long npad2,
-                                                           long kdim, long kper, uint8_t* __restrict__ Xs,
-                                                           int* __restrict__ E) {
-  __shared__ unsigned long long top[8][kSliceThreads / 32];
+                                                           long kdim, long kper, const uint32_t* tops,
+                                                           uint8_t* __restrict__ Xs, int* __restrict__ E) {
+  __shared__ uint32_t top[8][kSliceThreads / 32];
   __shared__ int ex[8];
   const long r0 = static_cast<long>(blockIdx.x) * 8, part = blockIdx.y;
   const long k0 = part * kper, k1 = std::min(k0 + kper, kdim);
@@ -123,15 +68,13 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_x(const double* __restr
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const bool live = r0 < npad;  // npad is a multiple of 8
 #pragma unroll 1
-  for (int r = 0; r < 8; ++r) {
-    unsigned long long m = 0;  // magnitudes order as their bit patterns, infinities and NaN above all
+  for (int r = 0; r < 8 && !KNOWN; ++r) {
+    uint32_t m = 0;
     if (live) {
       const double* x = XT + (r0 + r) * kdim;
       for (long k = k0 + 2L * t; k < k1; k += 2L * kSliceThreads) {  // kdim and kper are even
         const double2 a = *reinterpret_cast<const double2*>(x + k);
-        const unsigned long long u = __double_as_longlong(a.x) & 0x7fffffffffffffffull;
-        const unsigned long long v = __double_as_longlong(a.y) & 0x7fffffffffffffffull;
-        m = max(m, max(u, v));
+        m = max(m, max(magnitude(a.x), magnitude(a.y)));
       }
     }
 #pragma unroll
@@ -140,9 +83,12 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_x(const double* __restr
   }
   __syncthreads();
   if (t < 8) {
-    unsigned long long m = 0;
-    for (int w = 0; w < kSliceThreads / 32; ++w) m = max(m, top[t][w]);
-    ex[t] = row_exponent(m);
+    uint32_t m = 0;
+    if (KNOWN)
+      m = live ? tops[part * npad2 + r0 + t] : 0;
+    else
+      for (int w = 0; w < kSliceThreads / 32; ++w) m = max(m, top[t][w]);
+    ex[t] = value_exponent(m);
     E[part * npad2 + r0 + t] = ex[t];
   }
   __syncthreads();
@@ -169,31 +115,6 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_x(const double* __restr
 }
 
 // ------------------------------------------------------------------ int8 SYRK ----
-// The 8 groups of 16 columns (group g 64 columns after group g - 1) of this thread's TMEM lane, joined:
-// sum_g v_g 256^(3-g), groups 0 - 3 and 4 - 7 each in one 64-bit integer (|v_g| < 2^31, so below 2^56).
-__device__ __forceinline__ void join_groups16(uint32_t taddr, double (&w)[16]) {
-  long long hi[16], lo[16];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint32_t v[4][16];
-#pragma unroll
-    for (int g = 0; g < 4; ++g) tmem_ld16_nowait(taddr + (4 * h + g) * 64, v[g]);
-    tmem_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      long long x = static_cast<int32_t>(v[0][j]);
-#pragma unroll
-      for (int g = 1; g < 4; ++g) x = x * 256 + static_cast<int32_t>(v[g][j]);
-      (h == 0 ? hi[j] : lo[j]) = x;
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 16; ++j) w[j] = fma(static_cast<double>(lo[j]), 1.0 / 4294967296.0, static_cast<double>(hi[j]));
-}
-
-// x 2^e
-__device__ __forceinline__ double scale2(double x, int e) { return (e > -1000 && e < 1000) ? x * pow2i(e) : ldexp(x, e); }
-
 struct I8Params {
   const uint8_t* Xs;
   long kdim, kper;
@@ -203,30 +124,6 @@ struct I8Params {
   const int* E;   // row exponents [part][npad2]
   int* err;
 };
-
-// One chunk's MMAs: digit s of A against digits 0 .. min(6, 7 - s) of B, group s + t in the columns 64 (s + t).
-// The chunk that starts the sums (first) overwrites each group on its first product: digit s = 0 starts
-// groups 0 - 6, and (1, 6) starts group 7.
-__device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t sa, uint32_t sb, bool first) {
-  constexpr uint64_t kDesc = plain_desc_bits(128, 256);  // core matrices 128 B apart along k, 256 B along rows
-#pragma unroll
-  for (int s = 0; s < kDigits; ++s) {
-    const uint64_t da = sw128_desc(sa + s * kDigitA, kDesc);
-    const int n = kGroups - s < kDigits ? kGroups - s : kDigits;  // digits of B
-#pragma unroll
-    for (int t = 0; t < n; t += 4) {
-      const int m = n - t < 4 ? n - t : 4;  // up to 256 columns
-      const uint64_t db = sw128_desc(sb + t * kDigitB, kDesc);
-      const uint32_t d = tmem + (s + t) * 64;
-      if (s == 1 && t + m == kDigits) {  // its last digit is group 7's first product
-        if (m > 1) umma_s8(d, da, db, idesc_s8_s32(128, 64 * (m - 1)), 1u);
-        umma_s8(d + 64 * (m - 1), da, sw128_desc(sb + (t + m - 1) * kDigitB, kDesc), idesc_s8_s32(128, 64), first ? 0u : 1u);
-      } else {
-        umma_s8(d, da, db, idesc_s8_s32(128, 64 * m), (first && s == 0) ? 0u : 1u);
-      }
-    }
-  }
-}
 
 __global__ void __launch_bounds__(kI8Threads, 1) k_syrk_i8(I8Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -315,7 +212,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_syrk_i8(I8Params p) {
         }
         tc_fence_after();
         const uint32_t sa = smem_u32(smem + stage * kI8Stage);
-        issue_chunk(tmem, sa, sa + kBlockBytes, c == 0);
+        issue_digit_products<64, plain_desc_bits(128, 256), false>(tmem, sa, sa + kBlockBytes, c == 0);
         umma_commit(&empty[stage]);
         if (++stage == kI8Stages) {
           stage = 0;
@@ -340,22 +237,27 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_syrk_i8(I8Params p) {
     // tiles above the diagonal (their mirror is stored) and rows past npad are left out
     if (ok && b <= ra && ra < p.nt) {
       const int* Ep = p.E + part * p.npad2;
-      const int ea = Ep[a * 128 + row];
+      const double sa = value_scale(Ep[a * 128 + row]) * kJoined;
       const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16);
       double* out = p.Kpart + (part * p.ntile + tri_index(ra, b)) * TILE2 + static_cast<long>(r) * TILE;
 #pragma unroll 1
       for (int c0 = 0; c0 < 64; c0 += 16) {
-        double v[16];
-        join_groups16(lane_base + c0, v);
+        long long hi[16], lo[16];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t v[4][16];
+#pragma unroll
+          for (int g = 0; g < 4; ++g) tmem_ld16_nowait(lane_base + (4 * h + g) * 64 + c0, v[g]);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) (h == 0 ? hi[j] : lo[j]) = join4(v[0][j], v[1][j], v[2][j], v[3][j]);
+        }
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
           double w[2];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int eb = __ldg(Ep + b * 64 + c0 + j + h);
-            w[h] = (ea == kNonFinite || eb == kNonFinite) ? __longlong_as_double(0x7ff8000000000000ll)
-                                                          : scale2(v[j + h], 72 + ea + eb);
-          }
+          for (int h = 0; h < 2; ++h)
+            w[h] = join8(hi[j + h], lo[j + h]) * sa * value_scale(__ldg(Ep + b * 64 + c0 + j + h));
           *reinterpret_cast<double2*>(out + c0 + j) = make_double2(w[0], w[1]);
         }
       }
@@ -388,15 +290,20 @@ int sm_count(int device) {
 
 // Split-K parts of the int8 SYRK: chunk-aligned, at most kMaxPart k each; among up to four times the fewest
 // parts (or parts for one wave), the count whose last wave of CTAs, one an SM, is fullest.
-int syrk_i8_parts(long nt, long kdim, int device, long* kper_out) {
+// Parts are whole aux functions (noccp k each) where a part can hold an even number of them, so that
+// k_xform_i8 can keep each part's row maxima.
+int syrk_i8_parts(long nt, long naux, long noccp, int device, long* kper_out) {
+  const long kdim = naux * noccp;
   const long nb = (nt + 1) / 2, ctas_per_part = nb * (nb + 1);
   const long sms = sm_count(device);
-  const long nchunks = (kdim + kChunk - 1) / kChunk;
-  const long min_parts = (kdim + kMaxPart - 1) / kMaxPart;
+  const long unit = noccp % kChunk == 0 ? noccp : 2 * noccp;  // aligned to chunks and aux functions
+  const long grain = unit <= kMaxPart ? unit : kChunk;
+  const long max_part = kMaxPart / grain * grain;
+  const long min_parts = (kdim + max_part - 1) / max_part;
   const long want = std::max(min_parts, sms / ctas_per_part);
   long best = want;
   double best_eff = 0.0;
-  for (long sp = want; sp <= 4 * want && sp <= std::max<long>(1, nchunks); ++sp) {
+  for (long sp = want; sp <= 4 * want && sp <= std::max<long>(1, kdim / grain); ++sp) {
     const long ctas = ctas_per_part * sp, waves = (ctas + sms - 1) / sms;
     const double eff = static_cast<double>(ctas) / static_cast<double>(waves * sms);
     if (eff > best_eff + 0.02) {
@@ -404,15 +311,15 @@ int syrk_i8_parts(long nt, long kdim, int device, long* kper_out) {
       best = sp;
     }
   }
-  long kper = round_up((kdim + best - 1) / best, kChunk);
-  kper = std::min(kper, kMaxPart);
+  const long kper = std::min(round_up((kdim + best - 1) / best, grain), max_part);
   *kper_out = kper;
   return static_cast<int>((kdim + kper - 1) / kper);
 }
 
 // K partials of the FP64 form from X^T (npad x kdim doubles) through its digits.
-int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int nparts, long kper, double* Kpart,
-            cudaStream_t s) {
+// tops: the rows' largest magnitudes in every part (k_xform_i8), or null.
+int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int nparts, long kper,
+            const uint32_t* tops, double* Kpart, cudaStream_t s) {
   const long npad2 = round_up(npad, 128);
   const long nblk = (kdim + kChunk - 1) / kChunk;
   int rc;
@@ -421,8 +328,11 @@ int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int 
     return rc;
   uint8_t* Xs = static_cast<uint8_t*>(ctx->Xs.p);
   int* E = static_cast<int*>(ctx->Xe.p);
-  k_slice_x<<<dim3(static_cast<unsigned>(npad2 / 8), static_cast<unsigned>(nparts)), kSliceThreads, 0, s>>>(
-      XT, npad, npad2, kdim, kper, Xs, E);
+  const dim3 sgrid(static_cast<unsigned>(npad2 / 8), static_cast<unsigned>(nparts));
+  if (tops)
+    k_slice_x<true><<<sgrid, kSliceThreads, 0, s>>>(XT, npad, npad2, kdim, kper, tops, Xs, E);
+  else
+    k_slice_x<false><<<sgrid, kSliceThreads, 0, s>>>(XT, npad, npad2, kdim, kper, tops, Xs, E);
   prof_mark(ctx, "slice_x");
   I8Params ip{};
   ip.Xs = Xs;

@@ -12,6 +12,7 @@
 #include <algorithm>
 
 #include "gemm_f64.cuh"
+#include "i8_digits.cuh"
 #include "rijk_internal.h"
 
 namespace rijk {
@@ -21,7 +22,7 @@ constexpr int K1_THREADS = 128;
 __global__ void __launch_bounds__(K1_THREADS)
     k_metric_contract(const double* __restrict__ M, long nauxp, long mrows, const double* __restrict__ I3, int layout,
                       long n, long naux, long I0, long t0, long rows_in_chunk_base, double* __restrict__ B,
-                      long tile_elems, long tri) {
+                      long tile_elems, long tri, uint32_t* __restrict__ top) {
   extern __shared__ __align__(16) double smem_k1[];
   double* sA[2] = {smem_k1, smem_k1 + 64 * LDK};
   double* sB[2] = {smem_k1 + 2 * 64 * LDK, smem_k1 + 3 * 64 * LDK};
@@ -92,19 +93,24 @@ __global__ void __launch_bounds__(K1_THREADS)
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     long q = q0 + wm * 32 + i * 8 + g;
-    if (q >= naux) continue;
+    uint32_t m = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       int c = wn * 32 + j * 8 + 2 * tq;
-      *reinterpret_cast<double2*>(Bt + q * tile_elems + c) = make_double2(acc[i][j][0], acc[i][j][1]);
+      if (q < naux) *reinterpret_cast<double2*>(Bt + q * tile_elems + c) = make_double2(acc[i][j][0], acc[i][j][1]);
+      m = max(m, max(magnitude(acc[i][j][0]), magnitude(acc[i][j][1])));
     }
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    if (tq == 0 && q < naux) atomicMax(top + q, m);
   }
 }
 
 // I3 holds the tile rows I in [I0, I1): full layout rows (mu - I0*64)*n + nu, packed layout
 // pair rows starting at pair_base = (I0*64)(I0*64+1)/2.
 void launch_metric_contract_chunk(const double* M, long nauxp, long mrows, const double* I3, int layout, long n,
-                                  long naux, long nt, long I0, long I1, double* B, cudaStream_t s, long tri) {
+                                  long naux, long nt, long I0, long I1, double* B, uint32_t* top, cudaStream_t s,
+                                  long tri) {
   long t0 = tri_index(I0, 0);
   long t1 = tri_index(I1, 0);
   long ntile = nt * (nt + 1) / 2;
@@ -114,7 +120,7 @@ void launch_metric_contract_chunk(const double* M, long nauxp, long mrows, const
   const size_t smem = 4 * 64 * LDK * sizeof(double);
   ensure_smem_limit(reinterpret_cast<const void*>(k_metric_contract), smem);
   k_metric_contract<<<grid, K1_THREADS, smem, s>>>(M, nauxp, mrows, I3, layout, n, naux, I0, t0, pair_base, B,
-                                                   ntile * TILE2, tri);
+                                                   ntile * TILE2, tri, top);
 }
 
 }  // namespace rijk

@@ -65,6 +65,11 @@ int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
     cudaMemPoolTrimTo(ctx->pool, 0);
     e = cudaMalloc(&b.p, bytes);
   }
+  if (e == cudaErrorMemoryAllocation && ctx->Bdig.p && &b != &ctx->Bdig) {  // ... and without the digits of B
+    cudaGetLastError();
+    drop_bdig(ctx);
+    e = cudaMalloc(&b.p, bytes);
+  }
   if (e != cudaSuccess) {
     b.p = nullptr;
     return cuda_check(ctx, e, what);
@@ -260,18 +265,32 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   const bool tc = precision == RIJK_PREC_FP64_TC;
   long kper_tc = 0;
   int nsK = 1;
+  bool i8x = false, i8k = tc;
   if (nocc > 0 && precision != RIJK_PREC_MIXED) {
-    nsK = tc ? syrk_i8_parts(nt, kdim, ctx->device, &kper_tc) : syrk_nsplit(nt, kdim);
+    // The int8 tensor cores from about 1e10 FLOPs of exchange and more than 192 functions on (128-row blocks).
+    // Whole FP64 builds, DMMA against int8: 278 against 294 us at n = 192, n_c = 40; 233 against 246 at 232, 20; 580
+    // against 564 at 348, 30; 534 against 449 at 250, 41; 628 against 457 at 240, 50; 2.30 against 1.56 ms at 384, 80;
+    // 80.3 against 33.6 ms at 970, 161.  Without room for the digits of B the half-transform stays on DMMA.
+    const bool large = npad > 192 && 3.0 * npad * npad * kdim >= 1e10;
+    i8k = tc || large;
+    nsK = i8k ? syrk_i8_parts(nt, naux, noccp, ctx->device, &kper_tc) : syrk_nsplit(nt, kdim);
+    i8x = large && kper_tc % noccp == 0 && bdig_prepare(ctx);
+    if (i8x && (rc = xform_i8_buffers(ctx, noccp, nsK))) return rc;
     if ((rc = ensure(ctx, ctx->MOp, noccp * npad * sizeof(double), "MOp")) ||
         (rc = ensure(ctx, ctx->XT, static_cast<size_t>(npad) * kdim * sizeof(double), "XT")) ||
         (rc = ensure(ctx, ctx->Kpart, static_cast<size_t>(nsK) * tile_elems * sizeof(double), "Kpart")))
       return rc;
+    i8x = i8x && ctx->have_bdig;  // a buffer above may have needed their memory
   }
-  // FP64 and FP64_TC: the Coulomb pair runs on the high-priority stream beside the half-transform, one
-  // 256-thread CTA per SM, in the registers and warps the half-transform's two CTAs per SM leave free;
+  // FP64 and FP64_TC: the Coulomb pair runs on the high-priority stream beside the DMMA half-transform, one
+  // or two 256-thread CTAs per SM, in the registers and warps the half-transform's CTAs leave free;
   // the pair is bound by HBM, the half-transform by the FP64 tensor pipe.  With per-kernel timing on,
   // the kernels run one after another instead.
   const bool side_j = precision != RIJK_PREC_MIXED && nocc > 0 && !ctx->profiling;
+  // The int8 half-transform's registers leave no room for the pair's CTAs, and it reads L2 at its limit: there the
+  // pair starts behind it, beside the digits of X and K, three CTAs an SM (C40H82 33.6 ms, the pair first and
+  // alone 33.7, one CTA an SM 38; (H2O)16 1.56, 1.59 ms; C25H52 6.5, 7.0 ms).
+  const bool late_j = side_j && i8x;
   cudaEventRecord(ctx->ev0, s);
   prof_begin(ctx);
   launch_pack_density(dD, n, npad, nt, static_cast<double*>(ctx->Dt.p), s);
@@ -279,7 +298,7 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   // The pair's CTAs (one or two an SM): the half-transform's time per byte of B grows with the orbitals,
   // so fewer orbitals leave a shorter window for the same bytes
   const int side_ctas = noccp <= 96 ? 2 * ctx->sms : ctx->sms;
-  if (side_j) {
+  auto run_side_j = [&](int side_ctas) {
     cudaStream_t js = ctx->j_stream;
     cudaEventRecord(ctx->ev_pk, s);
     cudaStreamWaitEvent(js, ctx->ev_pk, 0);
@@ -293,6 +312,9 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
     cudaEventRecord(ctx->ev1, js);
     if (j_done) cudaEventRecord(j_done, js);
     cudaEventRecord(ctx->ev_jside, js);
+  };
+  if (side_j) {
+    if (!late_j) run_side_j(side_ctas);
   } else if (precision == RIJK_PREC_MIXED) {
     // mixed form: both passes over the split-BF16 copy (half the bytes of the FP64 passes)
     const long ntile2 = round_up(nt, 2) * (round_up(nt, 2) + 1) / 2;
@@ -330,17 +352,30 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
     // About 20 us, so that the Coulomb CTAs, whose stream waits on an event, are resident before the
     // half-transform's thousands of CTAs queue (builds queued back to back: 240.5 -> 235.2 ms at
     // n_ao = 1856, where the pair alone takes 17.7 ms)
-    if (side_j) {
+    if (side_j && !late_j) {
       launch_delay(40000, s);
       ++launches;
     }
     launch_pack_mo(dMO, nocc, n, noccp, npad, static_cast<double*>(ctx->MOp.p), s);
     prof_mark(ctx, "pack_mo");
-    launches += launch_xform_f64(static_cast<const double*>(ctx->B.p), static_cast<const double*>(ctx->MOp.p), naux,
-                                 nt, noccp, static_cast<double*>(ctx->XT.p), s);
-    prof_mark(ctx, "xform_f64");
-    if (tc) {  // int8 digit planes of X^T, then K on tcgen05 (exact s32 products)
+    if (i8x) {
+      rc = xform_i8(ctx, static_cast<const double*>(ctx->MOp.p), noccp, static_cast<double*>(ctx->XT.p), kper_tc / noccp,
+                    nsK, s);
+      if (rc) {
+        if (side_j) cudaStreamWaitEvent(s, ctx->ev_jside, 0);  // nothing of the side stream outlives the call
+        return rc;
+      }
+      launches += 2;
+      if (late_j) run_side_j(3 * ctx->sms);
+      prof_mark(ctx, "xform_i8");
+    } else {
+      launches += launch_xform_f64(static_cast<const double*>(ctx->B.p), static_cast<const double*>(ctx->MOp.p), naux,
+                                   nt, noccp, static_cast<double*>(ctx->XT.p), s);
+      prof_mark(ctx, "xform_f64");
+    }
+    if (i8k) {  // int8 digits of X^T, then K on tcgen05 (exact s32 products)
       rc = syrk_i8(ctx, static_cast<const double*>(ctx->XT.p), npad, nt, kdim, nsK, kper_tc,
+                   i8x ? static_cast<const uint32_t*>(ctx->Xtop.p) : nullptr,
                    static_cast<double*>(ctx->Kpart.p), s);
       if (rc) {
         if (side_j) cudaStreamWaitEvent(s, ctx->ev_jside, 0);  // nothing of the side stream outlives the call
@@ -458,6 +493,7 @@ RIJK_API int rijk_destroy(rijk_ctx* ctx) {
   DeviceBuf* bufs[] = {&ctx->M,  &ctx->B,     &ctx->Bmix,  &ctx->stageD, &ctx->stageMO, &ctx->stageJ,
                        &ctx->stageK, &ctx->Dt, &ctx->w,     &ctx->Jpart, &ctx->MOp,    &ctx->XT,
                        &ctx->Kpart, &ctx->err, &ctx->scratch, &ctx->eri_tab, &ctx->Xs, &ctx->Xe,
+                       &ctx->Bdig, &ctx->Btop, &ctx->Bexp, &ctx->Cdig, &ctx->Xtop,
                        &ctx->s3.raw};
   for (DeviceBuf* b : bufs) release(*b);
   for (DeviceBuf& b : ctx->scf) release(b);
@@ -526,7 +562,7 @@ RIJK_API int rijk_set_aux_range(rijk_ctx* ctx, long q0, long q1) {
   ctx->q0 = q0;
   ctx->nq = q1 - q0;
   ctx->have_b = false;
-  ctx->have_bmix = false;
+  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = false;
   return RIJK_OK;
 }
 
@@ -639,7 +675,7 @@ int set_metric_impl(rijk_ctx* ctx, const double* PQ, cudaMemcpyKind kind, long n
   ctx->metric_form = form;
   ctx->have_metric = true;
   ctx->have_b = false;
-  ctx->have_bmix = false;
+  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = false;
   ctx->stats.naux = naux;
   if (hinfo[1] > 0) ctx->last_error = "warning: metric eigenvalues <= 0 dropped";
   return RIJK_OK;
@@ -695,10 +731,12 @@ int set_3c_impl(rijk_ctx* ctx, long n, long naux, int layout, const ChunkFill& f
   const long nq = ctx->nq, q0 = ctx->q0;
   int rc;
   ctx->have_b = false;
-  ctx->have_bmix = false;
+  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = false;
   release(ctx->Bmix);
-  if ((rc = ensure(ctx, ctx->B, static_cast<size_t>(nq) * ntile * TILE2 * sizeof(double), "fitted tensor B")))
+  if ((rc = ensure(ctx, ctx->B, static_cast<size_t>(nq) * ntile * TILE2 * sizeof(double), "fitted tensor B")) ||
+      (rc = ensure(ctx, ctx->Btop, nq * sizeof(uint32_t), "magnitudes of B")))
     return rc;
+  cudaMemsetAsync(ctx->Btop.p, 0, nq * sizeof(uint32_t), s);
   // Raw integrals come in blocks of whole tile rows, at most ~2 GiB each.
   const long rows_per = rows_per_chunk(n, nauxp, layout);
   auto pairs_of = [&](long I0, long I1, long& first, long& count) {
@@ -725,7 +763,7 @@ int set_3c_impl(rijk_ctx* ctx, long n, long naux, int layout, const ChunkFill& f
     cudaEventRecord(ctx->ev0, s);
     launch_metric_contract_chunk(static_cast<const double*>(ctx->M.p) + q0 * nauxp, nauxp, nauxp - q0,
                                  static_cast<const double*>(raw.p), layout, n, nq, nt, I0, I1,
-                                 static_cast<double*>(ctx->B.p), s,
+                                 static_cast<double*>(ctx->B.p), static_cast<uint32_t*>(ctx->Btop.p), s,
                                  ctx->metric_form == RIJK_METRIC_CHOLESKY ? q0 : -1);
     cudaEventRecord(ctx->ev1, s);
     rc = cuda_check(ctx, cudaStreamSynchronize(s), "metric contraction");
@@ -737,7 +775,7 @@ int set_3c_impl(rijk_ctx* ctx, long n, long naux, int layout, const ChunkFill& f
   ctx->npad = npad;
   ctx->nt = nt;
   ctx->ntile = ntile;
-  ctx->have_b = true;
+  ctx->have_b = ctx->have_btop = true;
   ctx->stats.ms_setup_3c = ms;
   ctx->stats.n = n;
   ctx->stats.npad = npad;

@@ -99,8 +99,15 @@ struct rijk_ctx {
   rijk::DeviceBuf err;    // int device error word
   rijk::DeviceBuf scratch;  // misc small
   rijk::DeviceBuf eri_tab;  // integral tables (Boys grid, harmonics, aux term lists)
-  rijk::DeviceBuf Xs;       // int8 digits of X^T for the tensor-core FP64 exchange: npad2 rows of kdim/32
-                            // blocks of 8 digits x 32 bytes
+  rijk::DeviceBuf Bdig;     // int8 digits of B for the FP64 half-transform on tcgen05 (k_xform_i8.cu), when there is room
+  rijk::DeviceBuf Bexp;     // the scales and the exponents of every B^Q's digits
+  rijk::DeviceBuf Btop;     // leading words of the largest magnitude of every B^Q, kept by the metric contraction
+  bool have_btop = false;
+  bool have_bdig = false;   // Bdig holds the digits of the present B
+  bool no_bdig = false;     // there was no room for them with the present B
+  rijk::DeviceBuf Cdig;     // exponents and int8 digits of the orbitals
+  rijk::DeviceBuf Xtop;     // largest magnitudes of X^T's rows in each split part
+  rijk::DeviceBuf Xs;       // int8 digits of X^T: blocks of 128 rows x 32 k, 7 digits each
   rijk::DeviceBuf Xe;       // their row exponents, parts x npad2
   rijk::DeviceBuf scf[32];  // rijk_scf's work buffers, kept between calls
   double* noalloc_scratch = nullptr;  // device address of rijk_coulomb_noalloc's fixed scratch on `device`
@@ -225,11 +232,13 @@ void launch_scan_nonfinite(const double* x, long count, int* err, cudaStream_t s
 
 // ---- k_metric.cu
 // B[Q][tile-packed e] = sum_P M[Q][P] * I3(pair(e), P) for the raw rows of tile rows [I0, I1).
+// top[Q] is raised to the leading word of the largest |B[Q]| written (see magnitude in i8_digits.cuh).
 // M may start at a row offset q0 (mrows = rows left after it); B receives naux rows.  tri >= 0 declares
 // M lower triangular with its first row at global row tri (the Cholesky form): the contraction then
 // stops at each row block's last nonzero column, half the products, the same result.
 void launch_metric_contract_chunk(const double* M, long nauxp, long mrows, const double* I3, int layout, long n,
-                                  long naux, long nt, long I0, long I1, double* B, cudaStream_t s, long tri = -1);
+                                  long naux, long nt, long I0, long I1, double* B, uint32_t* top, cudaStream_t s,
+                                  long tri = -1);
 
 // ---- k_coulomb.cu
 // Loads the FP64 Coulomb kernels' module on the current device (see preload_density_kernels).
@@ -256,9 +265,19 @@ int launch_xform_f64(const double* B, const double* MOp, long naux, long nt, lon
 int syrk_nsplit(long nt, long kdim);
 void launch_syrk_f64(const double* XT, long npad, long nt, long kdim, int nsplit, double* Kpart, cudaStream_t s);
 
-// ---- k_exchange_i8.cu (RIJK_PREC_FP64_TC): K partials from int8 digit planes on tcgen05
-int syrk_i8_parts(long nt, long kdim, int device, long* kper);
-int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int nparts, long kper, double* Kpart,
-            cudaStream_t s);
+// ---- k_exchange_i8.cu: K partials of the FP64 form from int8 digits on tcgen05
+int syrk_i8_parts(long nt, long naux, long noccp, int device, long* kper);
+int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int nparts, long kper,
+            const uint32_t* tops, double* Kpart, cudaStream_t s);
+
+// ---- k_xform_i8.cu: the FP64 half-transform from int8 digits on tcgen05
+// The digits of the present B, made on the first call; false when there is no room for them (the caller
+// then takes the DMMA kernel).  drop_bdig gives their memory back, until B changes.
+bool bdig_prepare(rijk_ctx* ctx);
+void drop_bdig(rijk_ctx* ctx);
+// Buffers of a build, before anything is queued, and the build's half-transform: XT as launch_xform_f64 writes it,
+// and in ctx->Xtop the largest magnitude of each row over every qper aux functions.
+int xform_i8_buffers(rijk_ctx* ctx, long noccp, long parts);
+int xform_i8(rijk_ctx* ctx, const double* MOp, long noccp, double* XT, long qper, long parts, cudaStream_t s);
 
 }  // namespace rijk

@@ -54,11 +54,13 @@ RIJK_API int rijk_begin_3c(rijk_ctx* ctx, long n, long naux, int layout) {
   const long nauxp = round_up(naux, KC);
   const long nq = ctx->nq;
   ctx->have_b = false;
-  ctx->have_bmix = false;
+  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = false;
   release(ctx->Bmix);
   int rc;
-  if ((rc = ensure(ctx, ctx->B, static_cast<size_t>(nq) * ntile * TILE2 * sizeof(double), "fitted tensor B")))
+  if ((rc = ensure(ctx, ctx->B, static_cast<size_t>(nq) * ntile * TILE2 * sizeof(double), "fitted tensor B")) ||
+      (rc = ensure(ctx, ctx->Btop, nq * sizeof(uint32_t), "magnitudes of B")))
     return fail(ctx, rc);
+  cudaMemsetAsync(ctx->Btop.p, 0, nq * sizeof(uint32_t), s);
   const long rows_per = rows_per_chunk(n, nauxp, layout);
   long maxcount = 0;
   for (long I0 = 0; I0 < nt; I0 += rows_per) {
@@ -119,8 +121,8 @@ RIJK_API int rijk_add_3c_block(rijk_ctx* ctx, long mu0, long mu1, const double* 
       cudaEventRecord(ctx->ev0, s);
       launch_metric_contract_chunk(static_cast<const double*>(ctx->M.p) + q0 * nauxp, nauxp, nauxp - q0,
                                    static_cast<const double*>(ctx->s3.raw.p), layout, n, nq, nt, I0, I1,
-                                   static_cast<double*>(ctx->B.p), s,
-                                 ctx->metric_form == RIJK_METRIC_CHOLESKY ? q0 : -1);
+                                   static_cast<double*>(ctx->B.p), static_cast<uint32_t*>(ctx->Btop.p), s,
+                                   ctx->metric_form == RIJK_METRIC_CHOLESKY ? q0 : -1);
       cudaEventRecord(ctx->ev1, s);
       rc = cuda_check(ctx, cudaStreamSynchronize(s), "metric contraction");
       if (rc) return fail(ctx, rc);
@@ -141,7 +143,7 @@ RIJK_API int rijk_add_3c_block(rijk_ctx* ctx, long mu0, long mu1, const double* 
   ctx->npad = npad;
   ctx->nt = nt;
   ctx->ntile = ntile;
-  ctx->have_b = true;
+  ctx->have_b = ctx->have_btop = true;
   ctx->stats.ms_setup_3c = ctx->s3.ms;
   ctx->stats.n = n;
   ctx->stats.npad = npad;
