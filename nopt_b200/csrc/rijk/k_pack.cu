@@ -11,21 +11,28 @@
 
 namespace rijk {
 
-__global__ void k_pack_density(const double* __restrict__ D, long n, long npad, double* __restrict__ Dt) {
-  long t = blockIdx.x;
+// Four CTAs a tile, each a 32 x 32 block of it: the transposed elements are read row-wise into shared memory.
+// (One CTA a tile, its transposed reads strided by n, took 5.7 us at n = 48 and 12 us at n = 384; now 3 and 4.)
+__global__ void __launch_bounds__(256) k_pack_density(const double* __restrict__ D, long n, long npad,
+                                                      double* __restrict__ Dt) {
+  __shared__ double tr[32][33];
   long I, J;
-  tri_decode(t, I, J);
-  double* out = Dt + t * TILE2;
-  for (int e = threadIdx.x; e < TILE2; e += blockDim.x) {
-    int r = e / TILE, c = e % TILE;
-    long mu = I * TILE + r, nu = J * TILE + c;
-    double v = 0.0;
-    if (mu < n && nu < n) {
-      v = D[mu * n + nu];
-      if (I != J) v += D[nu * n + mu];
-    }
-    out[e] = v;
+  tri_decode(blockIdx.x >> 2, I, J);
+  const int r0 = (blockIdx.x & 2) * 16, c0 = (blockIdx.x & 1) * 32;  // the block inside the tile
+  const long mu0 = I * TILE + r0, nu0 = J * TILE + c0;
+  double* out = Dt + (blockIdx.x >> 2) * TILE2 + r0 * TILE + c0;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  double v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const long mu = mu0 + y + 8 * k, nu = nu0 + x;
+    v[k] = mu < n && nu < n ? D[mu * n + nu] : 0.0;
+    const long nt = nu0 + y + 8 * k, mt = mu0 + x;  // row nt of the transposed block
+    if (I != J) tr[y + 8 * k][x] = mt < n && nt < n ? D[nt * n + mt] : 0.0;
   }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 4; ++k) out[(y + 8 * k) * TILE + x] = I != J ? v[k] + tr[x][y + 8 * k] : v[k];
 }
 
 __global__ void k_pack_mo(const double* __restrict__ MO, long nocc, long n, long noccp, long npad,
@@ -83,8 +90,9 @@ __global__ void __launch_bounds__(256) k_sum_splits(const T* partial, int nsplit
   }
 }
 
-__global__ void __launch_bounds__(256) k_unpack_blocks(const double* __restrict__ packed, long n, long nb,
-                                                      double* __restrict__ out) {
+// nsplit > 1: the split partials, `total` elements apart, are summed here, in order.
+__global__ void __launch_bounds__(256) k_unpack_blocks(const double* __restrict__ packed, int nsplit, long total, long n,
+                                                      long nb, double* __restrict__ out) {
   __shared__ double blk[32][33];
   const long bi = blockIdx.x / nb, bj = blockIdx.x % nb;  // 32-blocks of the output
   const long I = bi / 2, J = bj / 2;                       // 64-tiles
@@ -94,10 +102,20 @@ __global__ void __launch_bounds__(256) k_unpack_blocks(const double* __restrict_
   const long rs = lower ? (bi & 1) * 32 : (bj & 1) * 32;  // row offset inside the stored tile
   const long cs = lower ? (bj & 1) * 32 : (bi & 1) * 32;
   const double* src = packed + tri_index(a, b) * TILE2;
-  for (int e = threadIdx.x; e < 1024; e += 256) {
-    const int r = e / 32, c = e % 32;
-    blk[r][c] = src[(rs + r) * TILE + cs + c];
+  double v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int e = threadIdx.x + 256 * k;
+    v[k] = src[(rs + e / 32) * TILE + cs + e % 32];
   }
+  for (int sp = 1; sp < nsplit; ++sp)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int e = threadIdx.x + 256 * k;
+      v[k] += src[sp * total + (rs + e / 32) * TILE + cs + e % 32];
+    }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) blk[(threadIdx.x + 256 * k) / 32][threadIdx.x % 32] = v[k];
   __syncthreads();
   for (int e = threadIdx.x; e < 1024; e += 256) {
     const int r = e / 32, c = e % 32;
@@ -122,7 +140,7 @@ static int grid_for(long total, int threads) {
 
 void launch_pack_density(const double* D, long n, long npad, long nt, double* Dt, cudaStream_t s) {
   long ntile = nt * (nt + 1) / 2;
-  k_pack_density<<<static_cast<unsigned>(ntile), 256, 0, s>>>(D, n, npad, Dt);
+  k_pack_density<<<static_cast<unsigned>(4 * ntile), 256, 0, s>>>(D, n, npad, Dt);
 }
 
 cudaError_t preload_density_kernels() {
@@ -145,13 +163,18 @@ void launch_pack_mo(const double* MO, long nocc, long n, long noccp, long npad, 
   k_pack_mo<<<grid_for(noccp * npad, 256), 256, 0, s>>>(MO, nocc, n, noccp, npad, MOp);
 }
 
-// Sums the split partials in place (into split 0) and writes the full symmetric n x n matrix.
+// A launch of its own for the sum costs 4 to 5 us; up to 16 splits the unpacking adds them as it reads (every
+// partial twice, for both triangles: still L2 traffic of microseconds).
+bool sum_apart(int nsplit) { return nsplit > 16; }
+
+// Sums the split partials (in place, into split 0, where there are many) and writes the full symmetric n x n matrix.
 void launch_unpack_sym(double* partial, int nsplit, long ntile, long n, double* out, cudaStream_t s) {
   double* p = partial;
   const long total = ntile * TILE2;
-  if (nsplit > 1) k_sum_splits<double><<<static_cast<unsigned>((total + 127) / 128), 256, 0, s>>>(p, nsplit, total, p);
+  const bool apart = sum_apart(nsplit);
+  if (apart) k_sum_splits<double><<<static_cast<unsigned>((total + 127) / 128), 256, 0, s>>>(p, nsplit, total, p);
   const long nb = (n + 31) / 32;
-  k_unpack_blocks<<<static_cast<unsigned>(nb * nb), 256, 0, s>>>(p, n, nb, out);
+  k_unpack_blocks<<<static_cast<unsigned>(nb * nb), 256, 0, s>>>(p, apart ? 1 : nsplit, total, n, nb, out);
 }
 
 // fp32 split partials -> their fp64 sum (into `sum`, ntile tiles) -> the full symmetric n x n matrix.
@@ -160,7 +183,7 @@ void launch_unpack_sym_f32(const float* partial, int nsplit, long ntile, long n,
   const long total = ntile * TILE2;
   k_sum_splits<float><<<static_cast<unsigned>((total + 127) / 128), 256, 0, s>>>(partial, nsplit, total, sum);
   const long nb = (n + 31) / 32;
-  k_unpack_blocks<<<static_cast<unsigned>(nb * nb), 256, 0, s>>>(sum, n, nb, out);
+  k_unpack_blocks<<<static_cast<unsigned>(nb * nb), 256, 0, s>>>(sum, 1, total, n, nb, out);
 }
 
 void launch_scan_nonfinite(const double* x, long count, int* err, cudaStream_t s) {

@@ -185,20 +185,26 @@ FILE* g_log = nullptr;
 bool g_log_checked = false;
 }  // namespace
 
-void log_line(const std::string& json) {
+static bool log_on() {
   std::lock_guard<std::mutex> lock(g_log_mu);
   if (!g_log_checked) {
     g_log_checked = true;
     const char* path = std::getenv("RIJK_LOG");
     if (path && *path) g_log = std::fopen(path, "a");
   }
-  if (!g_log) return;
+  return g_log != nullptr;
+}
+
+void log_line(const std::string& json) {
+  if (!log_on()) return;
+  std::lock_guard<std::mutex> lock(g_log_mu);
   std::fputs(json.c_str(), g_log);
   std::fputc('\n', g_log);
   std::fflush(g_log);
 }
 
 void log_build(rijk_ctx* ctx, const char* call, long nocc, int precision) {
+  if (!log_on()) return;
   const rijk_stats_t& st = ctx->stats;
   const char* prec = precision == RIJK_PREC_MIXED ? "mixed" : precision == RIJK_PREC_FP64_TC ? "fp64_tc" : "fp64";
   const double ms = st.ms_last_fock;
@@ -308,7 +314,7 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
     launch_coulomb_j(static_cast<const double*>(ctx->B.p), static_cast<const double*>(ctx->w.p), naux, tile_elems, nsJ,
                      static_cast<double*>(ctx->Jpart.p), js, side_ctas);
     launch_unpack_sym(static_cast<double*>(ctx->Jpart.p), nsJ, ntile, n, dJ, js);
-    launches += 4 + (nsJ > 1 ? 1 : 0);  // pack, w, j, unpack (+ split sum)
+    launches += 4 + (sum_apart(nsJ) ? 1 : 0);  // pack, w, j, unpack (+ split sum)
     cudaEventRecord(ctx->ev1, js);
     if (j_done) cudaEventRecord(j_done, js);
     cudaEventRecord(ctx->ev_jside, js);
@@ -336,7 +342,7 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   if (!side_j) {
     launch_unpack_sym(static_cast<double*>(ctx->Jpart.p), nsJ, ntile, n, dJ, s);
     prof_mark(ctx, "unpack_j");
-    launches += (precision == RIJK_PREC_MIXED ? 5 : 4) + (nsJ > 1 ? 1 : 0);  // pack, w (+ chunk sum), j, unpack (+ split sum)
+    launches += (precision == RIJK_PREC_MIXED ? 5 : 4) + (sum_apart(nsJ) ? 1 : 0);  // pack, w (+ chunk sum), j, unpack (+ split sum)
     cudaEventRecord(ctx->ev1, s);
     if (j_done) cudaEventRecord(j_done, s);
   }
@@ -351,8 +357,11 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   } else {
     // About 20 us, so that the Coulomb CTAs, whose stream waits on an event, are resident before the
     // half-transform's thousands of CTAs queue (builds queued back to back: 240.5 -> 235.2 ms at
-    // n_ao = 1856, where the pair alone takes 17.7 ms)
-    if (side_j && !late_j) {
+    // n_ao = 1856, where the pair alone takes 17.7 ms).  Below some ten waves of those CTAs the pair gets its
+    // slots soon enough without, and the wait is lost time (81 -> 61 us a build at n_ao = 72, 191 -> 174 at 144,
+    // 278 -> 270 at 192).
+    const long xform_ctas = nt * ((noccp + 95) / 96) * naux;
+    if (side_j && !late_j && xform_ctas > 30L * ctx->sms) {
       launch_delay(40000, s);
       ++launches;
     }
@@ -390,7 +399,7 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
     }
     launch_unpack_sym(static_cast<double*>(ctx->Kpart.p), nsK, ntile, n, dK, s);
     prof_mark(ctx, "unpack_k");
-    launches += 3 + (nsK > 1 ? 1 : 0);  // pack_mo, syrk, unpack (+ split sum); the half-transform counted above
+    launches += 3 + (sum_apart(nsK) ? 1 : 0);  // pack_mo, syrk, unpack (+ split sum); the half-transform counted above
   }
   if (side_j) cudaStreamWaitEvent(s, ctx->ev_jside, 0);  // J joins the build's stream
   cudaEventRecord(ctx->ev2, s);
@@ -478,6 +487,11 @@ RIJK_API int rijk_create(rijk_ctx** out, int device) {
     rijk_destroy(ctx);
     return RIJK_ERR_ALLOC;
   }
+  if (cudaHostAlloc(&ctx->host_err, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+    rijk_destroy(ctx);
+    return RIJK_ERR_ALLOC;
+  }
+  *ctx->host_err = 0;
   cudaMemsetAsync(ctx->err.p, 0, sizeof(int), ctx->stream);
   cudaStreamSynchronize(ctx->stream);
   *out = ctx;
@@ -510,6 +524,7 @@ RIJK_API int rijk_destroy(rijk_ctx* ctx) {
     if (ev) cudaEventDestroy(ev);
   for (cudaEvent_t ev : ctx->pev)
     if (ev) cudaEventDestroy(ev);
+  if (ctx->host_err) cudaFreeHost(ctx->host_err);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -878,12 +893,14 @@ RIJK_API int rijk_fock(rijk_ctx* ctx, const double* D, const double* MO, long no
     return rc;
   }
   cudaStreamWaitEvent(c, ctx->ev_j, 0);
+  // the error word comes with K: a copy of its own after the build would wait for the device once more
+  cudaMemcpyAsync(ctx->host_err, ctx->err.p, sizeof(int), cudaMemcpyDeviceToHost, s);
   rc = cuda_check(ctx, cudaMemcpyAsync(J, ctx->stageJ.p, nn, cudaMemcpyDeviceToHost, c), "D2H J");
   if (!rc) rc = cuda_check(ctx, cudaMemcpyAsync(K, ctx->stageK.p, nn, cudaMemcpyDeviceToHost, s), "D2H K");
   const int rc_c = cuda_check(ctx, cudaStreamSynchronize(c), "rijk_fock copies");
   if (!rc) rc = cuda_check(ctx, cudaStreamSynchronize(s), "rijk_fock");
   if (!rc) rc = rc_c;
-  if (!rc) rc = check_device_error(ctx);
+  if (!rc && *ctx->host_err) rc = check_device_error(ctx);
   if (rc) return rc;
   ctx->stats.ms_coulomb = elapsed(ctx->ev0, ctx->ev1);
   ctx->stats.ms_exchange = elapsed(ctx->ev1, ctx->ev2);

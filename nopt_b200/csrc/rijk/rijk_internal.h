@@ -111,6 +111,7 @@ struct rijk_ctx {
   rijk::DeviceBuf Xe;       // their row exponents, parts x npad2
   rijk::DeviceBuf scf[32];  // rijk_scf's work buffers, kept between calls
   double* noalloc_scratch = nullptr;  // device address of rijk_coulomb_noalloc's fixed scratch on `device`
+  int* host_err = nullptr;     // pinned copy of the device error word
   long fail_alloc_after = -1;  // rijk_selftest_alloc_failure: allocations left before one is refused (-1: off)
   // a device build queued by rijk_fock_device, written to the metrics log by the next rijk_sync
   bool log_pending = false;
@@ -225,6 +226,7 @@ void launch_pack_density(const double* D, long n, long npad, long nt, double* Dt
 void launch_pack_mo(const double* MO, long nocc, long n, long noccp, long npad, double* MOp, cudaStream_t s);
 // One warp that sleeps for `cycles` SM clock cycles and exits (a fixed delay on a stream).
 void launch_delay(long long cycles, cudaStream_t s);
+bool sum_apart(int nsplit);  // whether launch_unpack_sym sums the splits in a launch of its own
 void launch_unpack_sym(double* partial, int nsplit, long ntile, long n, double* out, cudaStream_t s);
 void launch_unpack_sym_f32(const float* partial, int nsplit, long ntile, long n, double* sum, double* out,
                            cudaStream_t s);
