@@ -17,7 +17,7 @@
 // parameters, so the recursion and the harmonic sums are straight-line code without index tables.
 //
 // What bounds it: the FP64 pipe and its latency at 8 to 16 warps per SM.  Measured against a group of lanes per
-// shell triple with everything in shared memory (k_eri, kept for Cartesian aux shells and la + lb > 6), whose
+// shell triple with everything in shared memory (k_eri, kept for (P|Q), Cartesian aux shells and la + lb > 6), whose
 // Boys values one lane formed while the others waited and whose E was formed again for every aux shell: at
 // (H2O)8 cc-pVTZ/cc-pVTZ-JKFIT all of (P|Q) and (mu nu|P) 31.8 -> 4.0 ms, (H2O)16
 // cc-pVDZ/cc-pVDZ-JKFIT 32.7 -> 3.1 ms, (H2O)32 cc-pVTZ 1.02 -> 0.130 s.
@@ -232,10 +232,6 @@ __global__ void __launch_bounds__(NT) k_eri_thread(const EriLaunch P) {
   // one value of the thread's aux function m and the bra functions ab to its place
   auto store = [&](int ab, long col, double v) {
     const int fa = ab / nfb, fb = ab - fa * nfb;
-    if (P.mode == 2) {
-      P.out[(static_cast<long>(A.off + fa) - P.rowbase) * P.ld + col] = v;
-      return;
-    }
     const long mu = A.off + fa, nu = B.off + fb;
     if (P.mode == 0) {
       if (pair.x == pair.y && nu > mu) return;

@@ -7,7 +7,7 @@
 // (gto_ints.cpp): bra primitive pairs expanded in Hermite Gaussians (E coefficients), Hermite
 // Coulomb integrals R_tuv from the Boys function, aux functions as one-centre Hermite sums.
 //
-// Spherical aux shells with la + lb <= 6, all of the usual bases, take k_eri_thread (eri_thread.cuh), one launch
+// (mu nu|P) over spherical aux shells with la + lb <= 6, all of the usual bases, takes k_eri_thread (eri_thread.cuh), one launch
 // per (la + lb, lc).  The rest of this comment is about k_eri here, which takes the others.
 //
 // Work decomposition.  One launch per angular class (l_A, l_B, l_C); a task is one shell triple
@@ -624,7 +624,9 @@ int launch_classes(rijk_ctx* ctx, const EriLaunch& base, const PairLists& pl, co
       if (P.nket == 0) continue;
       P.pairs = pairs_dev + pl.lab_start[lab];
       P.npair = np;
-      // the thread-per-aux-shell kernel: its expansions, and the accumulators of contracted pairs, must fit
+      // The thread-per-aux-shell kernel: its expansions, and the accumulators of contracted pairs, must fit.  (P|Q) stays
+      // on k_eri: it is 1 % of the integrals (its 25 launches 0.4 of 4.1 ms at (H2O)8 cc-pVTZ, 0.3 with this kernel), and
+      // through the metric's condition another rounding of it moves the derivatives by 1e-9.
       const int side = lab / 2 + 1;  // (la + 1)(lb + 1) is at most side * (lab + 2 - side)
       P.e1size = (3 * side * (lab + 2 - side) * (lab + 1) + 1) & ~1;
       P.esize = pl.wide[lab] * ((tet(lab) + 1) & ~1);
@@ -632,7 +634,8 @@ int launch_classes(rijk_ctx* ctx, const EriLaunch& base, const PairLists& pl, co
       P.tile = eri_tile(np, P.nket, pl.wide[lab]);
       const size_t smem = (static_cast<size_t>(P.e1size) + P.esize +
                            static_cast<size_t>(contracted) * P.tile * (2 * lc + 1)) * sizeof(double);
-      if (g % 2 == 0 && lab <= LAB_MAX && smem <= static_cast<size_t>(maxsm)) {
+      if (base.mode != 2 && g % 2 == 0 && lab <= LAB_MAX &&
+          smem <= static_cast<size_t>(maxsm)) {
         const cudaError_t e = kLaunchThread[lc](lab, P, smem, s);
         if (e != cudaSuccess) {
           join();
@@ -727,8 +730,7 @@ int eri2c_device(rijk_ctx* ctx, EriPlan& p, double* dV, long ld, int* launches) 
   for (int a = 0; a < na; ++a) cand[a] = make_int2(a, na);  // (P, unit)
   PairLists pl;
   std::vector<EriShell> bra = p.aux.sh;
-  EriShell u{};  // the unit s function of dauxu
-  u.nprim = u.nfunc = u.pure = 1;
+  EriShell u{};
   bra.push_back(u);
   pair_lists(bra, cand, [](const int2&) { return true; }, pl);
   DeviceBuf dp;
