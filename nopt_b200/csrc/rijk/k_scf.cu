@@ -358,17 +358,24 @@ __global__ void __launch_bounds__(256) k_tc2_update_sym(double* __restrict__ P, 
 
 // ---- one TC2 step in one kernel, for n' <= 512.  At n' = 384 a step of the form above (the library
 // product, then the trace and update kernels) took about 23 us, most of it launch latency.  Here a CTA of
-// 4 warps forms a 32 x 32 tile of P^2 on DMMA (warps 2 x 2, 16 x 16 each) over 32-wide chunks of k
-// staged [k][row] (stride T2_LD, conflict-free as in dmma.cuh) through a three-stage cp.async pipeline.
+// 8 warps forms a 32 x 32 tile of P^2 on DMMA over 64-wide chunks of k staged [k][row] (stride T2_LD,
+// conflict-free as in dmma.cuh) through a three-stage cp.async pipeline.  What bounds it is the chain of
+// chunks, so the two groups of four warps (2 x 2, 16 x 16 each) take half of every chunk's k and add their
+// tiles at the end (10.9 instead of 12.0 us a step at n' = 384; what is left is mostly the 28 MB that the tiles'
+// panels move from L2).  Queueing the steps of a density without a host wait every four took the density
+// phase of a (H2O)16 SCF from 16.0 to 14.2 ms with that.
 // P is symmetric, so P(k, j) = P(j, k):
 // both operands are columns of P, with the rows contiguous.  The choice between P^2 and 2P - P^2 needs
 // tr P and tr P^2 = ||P||_F^2 of the input, which the previous step (or k_tc2_norms) left as partial sums,
 // one pair per tile: lane 0 of warp 0 of every CTA adds them in the same fixed order, so every CTA, and
 // every rank of a sharded SCF, takes the same branch.  The epilogue writes Pn and its tile's own partial
-// sums; CTA (0, 0) also writes tr P and tr P^2 to sc[1], sc[2] for the host's convergence test.
+// sums; CTA (0, 0) also writes tr P and tr P^2 to sc[1], sc[2].
+// Steps are queued without waiting for the host: sc[8 + step parity] counts the steps still to take (-1: the
+// idempotency error is not small yet), and once it is 0 a step only passes P on.
 constexpr int T2 = 32;
 constexpr int T2_LD = 36;
-constexpr int T2_THREADS = 128;
+constexpr int T2_THREADS = 256;
+constexpr int T2_K = 64;  // k of one stage
 
 __device__ __forceinline__ void t2_cp8(double* smem, const double* gmem, bool valid) {
   const uint32_t d = smem_u32(smem);
@@ -401,9 +408,10 @@ __device__ __forceinline__ void t2_tile_sums(double sdg, double ssq, double* __r
   }
 }
 
-// The partial sums of P0 (column-major n x n), one pair per 32 x 32 tile of the step's grid.
+// The partial sums of P0 (column-major n x n), one pair per 32 x 32 tile of the step's grid; no step taken yet.
 __global__ void __launch_bounds__(T2_THREADS) k_tc2_norms(const double* __restrict__ P, long n,
-                                                          double* __restrict__ part_out) {
+                                                          double* __restrict__ part_out, double* __restrict__ sc) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) sc[8 + threadIdx.x] = -1.0;
   const long r0 = static_cast<long>(blockIdx.y) * T2, c0 = static_cast<long>(blockIdx.x) * T2;
   double sdg = 0.0, ssq = 0.0;
   for (int e = threadIdx.x; e < T2 * T2; e += T2_THREADS) {
@@ -418,7 +426,7 @@ __global__ void __launch_bounds__(T2_THREADS) k_tc2_norms(const double* __restri
 }
 
 constexpr int T2_STAGES = 3;
-constexpr size_t T2_SMEM = static_cast<size_t>(T2_STAGES) * 2 * T2 * T2_LD * sizeof(double);
+constexpr size_t T2_SMEM = static_cast<size_t>(T2_STAGES) * 2 * T2_K * T2_LD * sizeof(double);
 
 // 16-byte copy of which the first `bytes` (0, 8 or 16) come from global memory, the rest zero
 __device__ __forceinline__ void t2_cp16(double* smem, const double* gmem, int bytes) {
@@ -430,13 +438,47 @@ __device__ __forceinline__ void t2_cp16(double* smem, const double* gmem, int by
 template <bool PAIRS>
 __global__ void __launch_bounds__(T2_THREADS) k_tc2_step(const double* __restrict__ P, double* __restrict__ Pn, long n,
                                                          const double* __restrict__ part_in,
-                                                         double* __restrict__ part_out, double nocc,
+                                                         double* __restrict__ part_out, double nocc, int step,
                                                          double* __restrict__ sc) {
   extern __shared__ __align__(16) double t2s[];  // T2_STAGES x {A, B} chunks of [k][row]
   __shared__ double tr[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long r0 = static_cast<long>(blockIdx.y) * T2, c0 = static_cast<long>(blockIdx.x) * T2;
   const int nblk = gridDim.x * gridDim.y;
+  const double left = sc[8 + (step & 1)];
+  auto stage_a = [&](int st) { return t2s + static_cast<size_t>(st) * 2 * T2_K * T2_LD; };
+  auto load = [&](int st, long k0) {  // element (row, k) of a column block: P[row + k n]
+    double* sA = stage_a(st);
+    double* sB = sA + T2_K * T2_LD;
+    if (PAIRS) {
+      for (int e = tid; e < T2 * T2_K / 2; e += T2_THREADS) {
+        const int kk = e >> 4, rr = (e & 15) * 2;
+        const long k = k0 + kk, ra = r0 + rr, rb = c0 + rr;
+        const int ba = k < n ? static_cast<int>(8 * std::max<long>(0, std::min<long>(2, n - ra))) : 0;
+        const int bb = k < n ? static_cast<int>(8 * std::max<long>(0, std::min<long>(2, n - rb))) : 0;
+        t2_cp16(&sA[kk * T2_LD + rr], ba ? P + ra + k * n : P, ba);
+        t2_cp16(&sB[kk * T2_LD + rr], bb ? P + rb + k * n : P, bb);
+      }
+    } else {
+      for (int e = tid; e < T2 * T2_K; e += T2_THREADS) {
+        const int kk = e >> 5, rr = e & 31;
+        const long k = k0 + kk, ra = r0 + rr, rb = c0 + rr;
+        const bool va = k < n && ra < n, vb = k < n && rb < n;
+        t2_cp8(&sA[kk * T2_LD + rr], va ? P + ra + k * n : P, va);
+        t2_cp8(&sB[kk * T2_LD + rr], vb ? P + rb + k * n : P, vb);
+      }
+    }
+  };
+  const bool go = left != 0.0;
+  const long nk = go ? (n + T2_K - 1) / T2_K : 0;
+  if (go) {
+    load(0, 0);
+    cp_async_commit();
+    if (nk > 1) {
+      load(1, T2_K);
+      cp_async_commit();
+    }
+  }
   if (warp == 0) {  // tr P and ||P||_F^2 from the input's partial sums, in a fixed order
     double a = 0.0, b = 0.0;
     for (int i = lane; i < nblk; i += 32) {
@@ -454,44 +496,26 @@ __global__ void __launch_bounds__(T2_THREADS) k_tc2_step(const double* __restric
       if (blockIdx.x == 0 && blockIdx.y == 0) {
         sc[1] = a;
         sc[2] = b;
+        // quadratic once the idempotency error is small: this step and two more reach rounding
+        sc[8 + ((step + 1) & 1)] = left < 0.0 ? (fabs(a - b) < 1e-8 ? 2.0 : -1.0) : fmax(left - 1.0, 0.0);
+        if (go) sc[10] = step;
       }
     }
   }
-  auto stage_a = [&](int st) { return t2s + static_cast<size_t>(st) * 2 * T2 * T2_LD; };
-  auto load = [&](int st, long k0) {  // element (row, k) of a column block: P[row + k n]
-    double* sA = stage_a(st);
-    double* sB = sA + T2 * T2_LD;
-    if (PAIRS) {
-      for (int e = tid; e < T2 * T2 / 2; e += T2_THREADS) {
-        const int kk = e >> 4, rr = (e & 15) * 2;
-        const long k = k0 + kk, ra = r0 + rr, rb = c0 + rr;
-        const int ba = k < n ? static_cast<int>(8 * std::max<long>(0, std::min<long>(2, n - ra))) : 0;
-        const int bb = k < n ? static_cast<int>(8 * std::max<long>(0, std::min<long>(2, n - rb))) : 0;
-        t2_cp16(&sA[kk * T2_LD + rr], ba ? P + ra + k * n : P, ba);
-        t2_cp16(&sB[kk * T2_LD + rr], bb ? P + rb + k * n : P, bb);
-      }
-    } else {
-      for (int e = tid; e < T2 * T2; e += T2_THREADS) {
-        const int kk = e >> 5, rr = e & 31;
-        const long k = k0 + kk, ra = r0 + rr, rb = c0 + rr;
-        const bool va = k < n && ra < n, vb = k < n && rb < n;
-        t2_cp8(&sA[kk * T2_LD + rr], va ? P + ra + k * n : P, va);
-        t2_cp8(&sB[kk * T2_LD + rr], vb ? P + rb + k * n : P, vb);
-      }
+  if (!go) {  // done: hand the tile and its sums on
+    for (int e = tid; e < T2 * T2; e += T2_THREADS) {
+      const long r = r0 + (e & 31), c = c0 + (e >> 5);
+      if (r < n && c < n) Pn[r + c * n] = P[r + c * n];
     }
-  };
-  const int wm = warp >> 1, wn = warp & 1, g = lane >> 2, t = lane & 3;
+    const long blk = static_cast<long>(blockIdx.y) * gridDim.x + blockIdx.x;
+    if (tid < 2) part_out[2 * blk + tid] = part_in[2 * blk + tid];
+    return;
+  }
+  const int grp = warp >> 2, wm = (warp >> 1) & 1, wn = warp & 1, g = lane >> 2, t = lane & 3;
   double acc[2][2][2] = {};
-  const long nk = (n + T2 - 1) / T2;
-  load(0, 0);
-  cp_async_commit();
-  if (nk > 1) {
-    load(1, T2);
-    cp_async_commit();
-  }
   for (long kc = 0; kc < nk; ++kc) {
     if (kc + 2 < nk) {
-      load(static_cast<int>((kc + 2) % T2_STAGES), (kc + 2) * T2);
+      load(static_cast<int>((kc + 2) % T2_STAGES), (kc + 2) * T2_K);
       cp_async_commit();
       cp_async_wait<2>();
     } else if (kc + 1 < nk) {
@@ -500,10 +524,10 @@ __global__ void __launch_bounds__(T2_THREADS) k_tc2_step(const double* __restric
       cp_async_wait<0>();
     }
     __syncthreads();
-    const double* a_ = stage_a(static_cast<int>(kc % T2_STAGES));
-    const double* b_ = a_ + T2 * T2_LD;
+    const double* a_ = stage_a(static_cast<int>(kc % T2_STAGES)) + grp * (T2_K / 2) * T2_LD;
+    const double* b_ = a_ + T2_K * T2_LD;
 #pragma unroll
-    for (int k = 0; k < T2; k += 4) {
+    for (int k = 0; k < T2_K / 2; k += 4) {
       double a[2], b[2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) a[i] = a_[(k + t) * T2_LD + wm * 16 + i * 8 + g];
@@ -516,37 +540,46 @@ __global__ void __launch_bounds__(T2_THREADS) k_tc2_step(const double* __restric
     }
     __syncthreads();
   }
-  const double t1 = tr[0], t2 = tr[1];
-  const bool square = fabs(t2 - nocc) < fabs(2.0 * t1 - t2 - nocc);
+  // the second group's half of the sums, through the first stage's memory
+  double* half = t2s + (warp & 3) * 32 * 8 + lane;
+  if (grp == 1) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) half[e * 32] = acc[e >> 2][(e >> 1) & 1][e & 1];
+  }
+  __syncthreads();
   double sdg = 0.0, ssq = 0.0;
+  if (grp == 0) {
+    const double t1 = tr[0], t2 = tr[1];
+    const bool square = fabs(t2 - nocc) < fabs(2.0 * t1 - t2 - nocc);
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const long r = r0 + wm * 16 + i * 8 + g, c = c0 + wn * 16 + j * 8 + 2 * t + h;
-        if (r < n && c < n) {
-          const double s2 = acc[i][j][h];
-          const double v = square ? s2 : 2.0 * P[r + c * n] - s2;
-          Pn[r + c * n] = v;
-          ssq += v * v;
-          if (r == c) sdg += v;
+        for (int h = 0; h < 2; ++h) {
+          const long r = r0 + wm * 16 + i * 8 + g, c = c0 + wn * 16 + j * 8 + 2 * t + h;
+          const double s2 = acc[i][j][h] + half[(i * 4 + j * 2 + h) * 32];
+          if (r < n && c < n) {
+            const double v = square ? s2 : 2.0 * P[r + c * n] - s2;
+            Pn[r + c * n] = v;
+            ssq += v * v;
+            if (r == c) sdg += v;
+          }
         }
-      }
+  }
   t2_tile_sums(sdg, ssq, part_out);
 }
 
 // One fused step; the launch configuration for n' (even n': 16-byte copies).
 void launch_tc2_step(const double* P, double* Pn, long n, const double* part_in, double* part_out, double nocc,
-                     double* sc, cudaStream_t s) {
+                     int step, double* sc, cudaStream_t s) {
   const unsigned nb = static_cast<unsigned>((n + T2 - 1) / T2);
   if (n % 2 == 0) {
     ensure_smem_limit(reinterpret_cast<const void*>(k_tc2_step<true>), T2_SMEM);
-    k_tc2_step<true><<<dim3(nb, nb), T2_THREADS, T2_SMEM, s>>>(P, Pn, n, part_in, part_out, nocc, sc);
+    k_tc2_step<true><<<dim3(nb, nb), T2_THREADS, T2_SMEM, s>>>(P, Pn, n, part_in, part_out, nocc, step, sc);
   } else {
     ensure_smem_limit(reinterpret_cast<const void*>(k_tc2_step<false>), T2_SMEM);
-    k_tc2_step<false><<<dim3(nb, nb), T2_THREADS, T2_SMEM, s>>>(P, Pn, n, part_in, part_out, nocc, sc);
+    k_tc2_step<false><<<dim3(nb, nb), T2_THREADS, T2_SMEM, s>>>(P, Pn, n, part_in, part_out, nocc, step, sc);
   }
 }
 
@@ -842,6 +875,7 @@ RIJK_API int rijk_scf(rijk_ctx* ctx, const double* H, const double* S, long nocc
   // Returns 0, 1 when the caller should use the eigensolver (no convergence, a subspace too far
   // from the previous one), or a (negative) error code.
   int purified = 0;
+  int tc2_steps = 40;  // fused steps the last density took
   auto purify_occ = [&](const double* Fm) -> int {
     constexpr int kMaxSteps = 100;
     if (o.density_by_eigenvectors || nocc <= 0 || nocc >= nm) return 1;
@@ -866,22 +900,33 @@ RIJK_API int rijk_scf(rijk_ctx* ctx, const double* H, const double* S, long nocc
     const long pstride = 2L * nb2 * nb2;
     double* Pa = P;   // the current iterate of the fused steps
     double* Pb = P2;
-    if (fused) k_tc2_norms<<<dim3(nb2, nb2), T2_THREADS, 0, s>>>(P, nm, part);
-    for (int step = 1; step <= kMaxSteps && !done; ++step) {
-      if (fused) {
-        launch_tc2_step(Pa, Pb, nm, part + ((step - 1) & 1) * pstride, part + (step & 1) * pstride,
-                        static_cast<double>(nocc), pPur, s);
-        std::swap(Pa, Pb);
-      } else {
-        // P^2: its upper triangle is read.  DSYRK forms half the products; below n' = 1024 cuBLAS's DGEMM
-        // was the faster of the two (21 against 25 ms of steps per SCF at n' = 384)
-        if (nm >= 1024)
-          cublasDsyrk(cb, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, nmi, nmi, &one, P, nmi, &zero, P2, nmi);
-        else
-          cublasDgemm(cb, CUBLAS_OP_N, CUBLAS_OP_N, nmi, nmi, nmi, &one, P, nmi, P, nmi, &zero, P2, nmi);
-        k_tc2_traces<<<1, 256, 0, s>>>(P, P2, nm, pPur);
-        k_tc2_update_sym<<<static_cast<unsigned>(ntiles32), 256, 0, s>>>(P, P2, nm, pPur, static_cast<double>(nocc));
+    if (fused) {
+      // as many steps as the last density took and one more, then eight at a time, without waiting in between
+      k_tc2_norms<<<dim3(nb2, nb2), T2_THREADS, 0, s>>>(P, nm, part, pPur);
+      for (int step = 1; step <= kMaxSteps && !done;) {
+        const int until = std::min(kMaxSteps, step == 1 ? tc2_steps + 1 : step + 7);
+        for (; step <= until; ++step) {
+          launch_tc2_step(Pa, Pb, nm, part + ((step - 1) & 1) * pstride, part + (step & 1) * pstride,
+                          static_cast<double>(nocc), step, pPur, s);
+          std::swap(Pa, Pb);
+        }
+        double st[11];
+        cudaMemcpyAsync(st, pPur, sizeof(st), cudaMemcpyDeviceToHost, s);
+        if (const cudaError_t e = cudaStreamSynchronize(s); e != cudaSuccess)
+          return cuda_check(ctx, e, "rijk_scf purification");
+        done = st[8 + (step & 1)] == 0.0;
+        if (done) tc2_steps = static_cast<int>(st[10]);
       }
+    }
+    for (int step = 1; step <= kMaxSteps && !done && !fused; ++step) {
+      // P^2: its upper triangle is read.  DSYRK forms half the products; below n' = 1024 cuBLAS's DGEMM
+      // was the faster of the two (21 against 25 ms of steps per SCF at n' = 384)
+      if (nm >= 1024)
+        cublasDsyrk(cb, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, nmi, nmi, &one, P, nmi, &zero, P2, nmi);
+      else
+        cublasDgemm(cb, CUBLAS_OP_N, CUBLAS_OP_N, nmi, nmi, nmi, &one, P, nmi, P, nmi, &zero, P2, nmi);
+      k_tc2_traces<<<1, 256, 0, s>>>(P, P2, nm, pPur);
+      k_tc2_update_sym<<<static_cast<unsigned>(ntiles32), 256, 0, s>>>(P, P2, nm, pPur, static_cast<double>(nocc));
       if (left > 0) {
         done = --left == 0;
       } else if (step >= 16 && step % 4 == 0) {
