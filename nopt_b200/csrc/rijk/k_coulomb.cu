@@ -103,13 +103,25 @@ __global__ void __launch_bounds__(J_THREADS) k_coulomb_j(const double* __restric
   }
 }
 
+// The fewest aux ranges (at most 32) that fill whole waves of the pass's resident CTAs (eight an SM, four of the mixed
+// pass) to 93 %, else those that fill them best.  About 8 CTAs an SM whatever the waves ran the mixed pass at (H2O)16
+// in 2.06 waves (124 us, now 103; C31H64 900, 726 us; the FP64 pass at (H2O)16 215, 180 us).
 int coulomb_nsplit(long tile_elems, long naux, int elems_per_thread) {
-  long blocks = (tile_elems / elems_per_thread + J_THREADS - 1) / J_THREADS;
-  long want = (148L * 8 + blocks - 1) / blocks;  // about 8 CTAs per SM in flight
-  if (want < 1) want = 1;
-  if (want > 32) want = 32;
-  if (want > naux) want = naux;
-  return static_cast<int>(want);
+  const long blocks = (tile_elems / elems_per_thread + J_THREADS - 1) / J_THREADS;
+  const long slots = 148L * (elems_per_thread == 2 ? 8 : 4);
+  const long most = std::min<long>(32, naux);
+  long best = 1;
+  double best_eff = 0.0;
+  for (long ns = 1; ns <= most; ++ns) {
+    const long ctas = blocks * ns, waves = (ctas + slots - 1) / slots;
+    const double eff = static_cast<double>(ctas) / static_cast<double>(waves * slots);
+    if (eff > best_eff + 1e-9) {
+      best_eff = eff;
+      best = ns;
+    }
+    if (best_eff >= 0.93) break;
+  }
+  return static_cast<int>(best);
 }
 
 // The capped forms ask for the largest shared-memory carveout, the one the half-transform runs with, so that
@@ -183,17 +195,17 @@ __device__ __forceinline__ long mix_off(long e) { return (e >> 12) * 8192 + (e &
 
 constexpr int WM_THREADS = 256;  // 8 warps; each warp reduces one aux function over the chunk at a time
 constexpr int WM_OCT = 1024;     // octets (8 elements) per chunk: two tiles, 32 KB of fp32 Dt in shared memory
-constexpr int WM_QR = 32;        // aux functions per CTA
+constexpr int WM_QR = 32;        // aux functions per CTA, fewer where that leaves SMs idle (launch_coulomb_w_mixed)
 
 int coulomb_w_mixed_chunks(long ntile) { return static_cast<int>((ntile * TILE2 / 8 + WM_OCT - 1) / WM_OCT); }
 
-// wpart[c][q] = sum over octet chunk c (blockIdx.x) of Bmix[q][e] Dt[e], q in the WM_QR aux functions
+// wpart[c][q] = sum over octet chunk c (blockIdx.x) of Bmix[q][e] Dt[e], q in the qr aux functions
 // of blockIdx.y.  The chunk's Dt is staged once as fp32 in two planes (elements 0-3 and 4-7 of each
 // octet), so a warp's 16-byte reads of it are conflict-free; each warp then streams one aux
 // function's hi/lo planes over the chunk with four octets per lane in flight and reduces by shuffle.
 __global__ void __launch_bounds__(WM_THREADS) k_coulomb_w_mixed(const __nv_bfloat16* __restrict__ Bmix,
                                                                  const double* __restrict__ Dt, long naux, long ntile,
-                                                                 long ntile2, double* __restrict__ wpart) {
+                                                                 long ntile2, int qr, double* __restrict__ wpart) {
   __shared__ __align__(16) float sd[2][WM_OCT * 4];
   const long n8 = ntile * TILE2 / 8;
   const long c0 = static_cast<long>(blockIdx.x) * WM_OCT;
@@ -207,10 +219,10 @@ __global__ void __launch_bounds__(WM_THREADS) k_coulomb_w_mixed(const __nv_bfloa
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long qstride = ntile2 * 2 * TILE2;
-  const long qa = static_cast<long>(blockIdx.y) * WM_QR;
+  const long qa = static_cast<long>(blockIdx.y) * qr;
   const float4* s0 = reinterpret_cast<const float4*>(sd[0]);
   const float4* s1 = reinterpret_cast<const float4*>(sd[1]);
-  for (int j = warp; j < WM_QR; j += WM_THREADS / 32) {
+  for (int j = warp; j < qr; j += WM_THREADS / 32) {
     const long q = qa + j;
     if (q >= naux) break;
     const __nv_bfloat16* qb = Bmix + q * qstride;
@@ -309,8 +321,11 @@ __global__ void __launch_bounds__(J_THREADS) k_coulomb_j_mixed(const __nv_bfloat
 void launch_coulomb_w_mixed(const __nv_bfloat16* Bmix, const double* Dt, long naux, long ntile, long ntile2, double* w,
                             cudaStream_t s) {
   const int chunks = coulomb_w_mixed_chunks(ntile);
-  dim3 grid(static_cast<unsigned>(chunks), static_cast<unsigned>((naux + WM_QR - 1) / WM_QR));
-  k_coulomb_w_mixed<<<grid, WM_THREADS, 0, s>>>(Bmix, Dt, naux, ntile, ntile2, w + naux);
+  // a warp's aux functions run one after another: one each below four CTAs an SM (40 -> 14 us at n_ao = 72, 54 -> 25 at 144)
+  int qr = WM_QR;
+  while (qr > WM_THREADS / 32 && chunks * ((naux + qr - 1) / qr) < 4 * 148) qr /= 2;
+  dim3 grid(static_cast<unsigned>(chunks), static_cast<unsigned>((naux + qr - 1) / qr));
+  k_coulomb_w_mixed<<<grid, WM_THREADS, 0, s>>>(Bmix, Dt, naux, ntile, ntile2, qr, w + naux);
   k_sum_chunks<<<static_cast<unsigned>((naux + 255) / 256), 256, 0, s>>>(w + naux, chunks, naux, w);
 }
 

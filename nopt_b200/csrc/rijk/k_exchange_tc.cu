@@ -881,7 +881,9 @@ static SyrkPlan syrk_plan_waves(long kdim, long tiles, long slots) {
   const long nchunks = (kdim + 63) / 64;
   const long smin = std::max<long>(1, (nchunks + kMaxChunks - 1) / kMaxChunks);
   const long smax = std::max<long>(smin, nchunks / 2);
-  long sp = smin;
+  // too few chunks for one full wave: as many ranges as there are (at n_ao = 72 one tile's 43 instead of a single
+  // CTA, 66 -> 9 us)
+  long sp = std::min(smax, std::max(smin, slots / tiles));
   for (long w = 1; w <= 64; ++w) {
     const long cand = std::min(smax, (w * slots) / tiles);
     if (cand < smin) continue;
@@ -894,10 +896,16 @@ static SyrkPlan syrk_plan_waves(long kdim, long tiles, long slots) {
   return {kper, static_cast<int>((kdim + kper - 1) / kper)};
 }
 
+// Whether K's kernel leaves registers on every SM for a J pass beside it: k_syrk_tc does (192 threads), the pair
+// kernel's 320 threads hold all but 12K of them.
+bool mixed_k_leaves_room(long nt) { return round_up(nt, 2) * TILE < 1024; }
+
 // K = sum over orbital batches of X_b^T X_b.  The half-transform holds all orbitals of one batch in
 // the MMA's N dimension (at most 192), so n_c beyond that runs as several batches of equal size; each
 // batch's split-K partials go to their own slots and one reduction sums them all.
-int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK) {
+// beside_k is called once, in the build's order right before the (first batch's) K kernel: what it queues on other
+// streams after an event recorded then runs beside K.
+int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK, const std::function<void()>& beside_k) {
   int rc = mixed_prepare(ctx);
   if (rc) return rc;
   const long n = ctx->n, naux = ctx->nq;
@@ -959,6 +967,7 @@ int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK) {
     kXformTable[noccp / 16](mB, mC, xp, ctx->device, s);
     ++launches;
     prof_mark(ctx, "xform_tc");
+    if (b0 == 0) beside_k();
     float* part = Kpart32 + static_cast<size_t>(slot) * ntile2 * TILE2;
     if (pair_syrk) {
       const SyrkPlan pl = syrk_plan(kdim, tiles256, sms / 2);

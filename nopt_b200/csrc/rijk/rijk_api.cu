@@ -20,7 +20,8 @@
 namespace rijk {
 
 int mixed_prepare(rijk_ctx* ctx);
-int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK);
+int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK, const std::function<void()>& beside_k);
+bool mixed_k_leaves_room(long nt);
 
 int set_err(rijk_ctx* ctx, int code, const char* fmt, ...) {
   if (ctx) {
@@ -297,6 +298,9 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   // pair starts behind it, beside the digits of X and K, three CTAs an SM (C40H82 33.6 ms, the pair first and
   // alone 33.7, one CTA an SM 38; (H2O)16 1.56, 1.59 ms; C25H52 6.5, 7.0 ms).
   const bool late_j = side_j && i8x;
+  // Mixed: the J pass (HBM) beside K (tensor pipe and shared memory) where K's kernel leaves registers for it.
+  // Mixed builds, in turn against beside: 0.53 against 0.49 ms at (H2O)16, 4.26 against 3.94 at C31H64.
+  const bool mixed_side_j = precision == RIJK_PREC_MIXED && nocc > 0 && !ctx->profiling && mixed_k_leaves_room(nt);
   cudaEventRecord(ctx->ev0, s);
   prof_begin(ctx);
   launch_pack_density(dD, n, npad, nt, static_cast<double*>(ctx->Dt.p), s);
@@ -328,9 +332,11 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
     launch_coulomb_w_mixed(Bm, static_cast<const double*>(ctx->Dt.p), naux, ntile, ntile2,
                            static_cast<double*>(ctx->w.p), s);
     prof_mark(ctx, "coulomb_w_mixed");
-    launch_coulomb_j_mixed(Bm, static_cast<const double*>(ctx->w.p), naux, ntile, ntile2, nsJ,
-                           static_cast<double*>(ctx->Jpart.p), s);
-    prof_mark(ctx, "coulomb_j_mixed");
+    if (!mixed_side_j) {
+      launch_coulomb_j_mixed(Bm, static_cast<const double*>(ctx->w.p), naux, ntile, ntile2, nsJ,
+                             static_cast<double*>(ctx->Jpart.p), s);
+      prof_mark(ctx, "coulomb_j_mixed");
+    }
   } else {
     launch_coulomb_w(static_cast<const double*>(ctx->B.p), static_cast<const double*>(ctx->Dt.p), naux, tile_elems,
                      static_cast<double*>(ctx->w.p), s);
@@ -339,7 +345,9 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
                      nsJ, static_cast<double*>(ctx->Jpart.p), s);
     prof_mark(ctx, "coulomb_j");
   }
-  if (!side_j) {
+  if (mixed_side_j) {
+    launches += 5 + (sum_apart(nsJ) ? 1 : 0);  // pack, w (+ chunk sum), j, unpack (+ split sum)
+  } else if (!side_j) {
     launch_unpack_sym(static_cast<double*>(ctx->Jpart.p), nsJ, ntile, n, dJ, s);
     prof_mark(ctx, "unpack_j");
     launches += (precision == RIJK_PREC_MIXED ? 5 : 4) + (sum_apart(nsJ) ? 1 : 0);  // pack, w (+ chunk sum), j, unpack (+ split sum)
@@ -351,7 +359,20 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   if (nocc == 0) {
     cudaMemsetAsync(dK, 0, n * n * sizeof(double), s);
   } else if (precision == RIJK_PREC_MIXED) {
-    rc = mixed_exchange(ctx, dMO, nocc, dK);
+    auto j_beside_k = [&]() {
+      if (!mixed_side_j) return;
+      cudaStream_t js = ctx->j_stream;
+      cudaEventRecord(ctx->ev_pk, s);
+      cudaStreamWaitEvent(js, ctx->ev_pk, 0);
+      launch_coulomb_j_mixed(static_cast<const __nv_bfloat16*>(ctx->Bmix.p), static_cast<const double*>(ctx->w.p), naux, ntile,
+                             round_up(nt, 2) * (round_up(nt, 2) + 1) / 2, nsJ, static_cast<double*>(ctx->Jpart.p), js);
+      launch_unpack_sym(static_cast<double*>(ctx->Jpart.p), nsJ, ntile, n, dJ, js);
+      cudaEventRecord(ctx->ev1, js);
+      if (j_done) cudaEventRecord(j_done, js);
+      cudaEventRecord(ctx->ev_jside, js);
+    };
+    rc = mixed_exchange(ctx, dMO, nocc, dK, j_beside_k);
+    if (mixed_side_j) cudaStreamWaitEvent(s, ctx->ev_jside, 0);  // J joins the build's stream
     if (rc) return rc;
     launches += ctx->stats.kernels_last_fock;
   } else {
