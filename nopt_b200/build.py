@@ -21,7 +21,6 @@ CUDA_SOURCES = [
     "rijk/rijk_api.cu",
     "rijk/k_pack.cu",
     "rijk/k_metric.cu",
-    "rijk/k_metric_i8.cu",
     "rijk/k_coulomb.cu",
     "rijk/k_exchange_f64.cu",
     "rijk/k_exchange_tc.cu",

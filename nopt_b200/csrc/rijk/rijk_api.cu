@@ -528,8 +528,8 @@ RIJK_API int rijk_destroy(rijk_ctx* ctx) {
   DeviceBuf* bufs[] = {&ctx->M,  &ctx->B,     &ctx->Bmix,  &ctx->stageD, &ctx->stageMO, &ctx->stageJ,
                        &ctx->stageK, &ctx->Dt, &ctx->w,     &ctx->Jpart, &ctx->MOp,    &ctx->XT,
                        &ctx->Kpart, &ctx->err, &ctx->scratch, &ctx->eri_tab, &ctx->Xs, &ctx->Xe,
-                       &ctx->Bdig, &ctx->Btop, &ctx->Bexp, &ctx->Mdig, &ctx->Cdig, &ctx->Xtop,
-                       &ctx->s3.raw, &ctx->s3.digits};
+                       &ctx->Bdig, &ctx->Btop, &ctx->Bexp, &ctx->Cdig, &ctx->Xtop,
+                       &ctx->s3.raw};
   for (DeviceBuf* b : bufs) release(*b);
   for (DeviceBuf& b : ctx->scf) release(b);
   if (ctx->cublas) cublasDestroy(ctx->cublas);
@@ -635,7 +635,6 @@ int set_metric_impl(rijk_ctx* ctx, const double* PQ, cudaMemcpyKind kind, long n
     cleanup();
     return rc;
   }
-  ctx->have_mdig = false;
   cudaEventRecord(ctx->ev0, s);
   rc = cuda_check(ctx, cudaMemcpyAsync(V.p, PQ, naux * naux * sizeof(double), kind, s), "copy (P|Q)");
   if (rc) { cleanup(); return rc; }
@@ -765,7 +764,7 @@ int set_3c_impl(rijk_ctx* ctx, long n, long naux, int layout, const ChunkFill& f
   cudaStream_t s = ctx->stream;
   const long npad = round_up(n, TILE), nt = npad / TILE, ntile = nt * (nt + 1) / 2;
   const long nauxp = round_up(naux, KC);
-  const long nq = ctx->nq;
+  const long nq = ctx->nq, q0 = ctx->q0;
   int rc;
   ctx->have_b = false;
   ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = false;
@@ -785,7 +784,7 @@ int set_3c_impl(rijk_ctx* ctx, long n, long naux, int layout, const ChunkFill& f
     pairs_of(I0, std::min(nt, I0 + rows_per), f, c);
     maxcount = std::max(maxcount, c);
   }
-  DeviceBuf raw, digits;
+  DeviceBuf raw;
   if ((rc = ensure_tmp(ctx, raw, static_cast<size_t>(std::max<long>(maxcount, 1)) * nauxp * sizeof(double), "raw 3c block")))
     return rc;
   cudaMemsetAsync(raw.p, 0, raw.bytes, s);
@@ -796,17 +795,18 @@ int set_3c_impl(rijk_ctx* ctx, long n, long naux, int layout, const ChunkFill& f
     long first, count;
     pairs_of(I0, I1, first, count);
     rc = fill(I0 * TILE, std::min(I1 * TILE, n), first, count, static_cast<double*>(raw.p), nauxp);
-    if (rc) { release(raw); release(digits); return rc; }
+    if (rc) { release(raw); return rc; }
     cudaEventRecord(ctx->ev0, s);
-    metric_contract(ctx, static_cast<const double*>(raw.p), layout, n, I0, I1, digits);
+    launch_metric_contract_chunk(static_cast<const double*>(ctx->M.p) + q0 * nauxp, nauxp, nauxp - q0,
+                                 static_cast<const double*>(raw.p), layout, n, nq, nt, I0, I1,
+                                 static_cast<double*>(ctx->B.p), static_cast<uint32_t*>(ctx->Btop.p), s,
+                                 ctx->metric_form == RIJK_METRIC_CHOLESKY ? q0 : -1);
     cudaEventRecord(ctx->ev1, s);
     rc = cuda_check(ctx, cudaStreamSynchronize(s), "metric contraction");
-    if (rc) { release(raw); release(digits); return rc; }
+    if (rc) { release(raw); return rc; }
     ms += elapsed(ctx->ev0, ctx->ev1);
   }
   release(raw);
-  release(digits);
-  if ((rc = check_device_error(ctx))) return rc;
   ctx->n = n;
   ctx->npad = npad;
   ctx->nt = nt;

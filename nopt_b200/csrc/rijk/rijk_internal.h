@@ -101,8 +101,6 @@ struct rijk_ctx {
   rijk::DeviceBuf eri_tab;  // integral tables (Boys grid, harmonics, aux term lists)
   rijk::DeviceBuf Bdig;     // int8 digits of B for the FP64 half-transform on tcgen05 (k_xform_i8.cu), when there is room
   rijk::DeviceBuf Bexp;     // the scales and the exponents of every B^Q's digits
-  rijk::DeviceBuf Mdig;     // scales and int8 digits of the metric factor's rows (k_metric_i8.cu)
-  bool have_mdig = false;   // they are the present factor's
   rijk::DeviceBuf Btop;     // leading words of the largest magnitude of every B^Q, kept by the metric contraction
   bool have_btop = false;
   bool have_bdig = false;   // Bdig holds the digits of the present B
@@ -128,7 +126,7 @@ struct rijk_ctx {
     long next_mu = 0;   // first orbital row the next block must start at
     long chunk_I0 = 0;  // tile rows [chunk_I0, chunk_I0 + rows_per) fill the staging buffer
     double ms = 0.0;
-    rijk::DeviceBuf raw, digits;
+    rijk::DeviceBuf raw;
   } s3;
 
   rijk_stats_t stats{};
@@ -243,12 +241,6 @@ void launch_scan_nonfinite(const double* x, long count, int* err, cudaStream_t s
 void launch_metric_contract_chunk(const double* M, long nauxp, long mrows, const double* I3, int layout, long n,
                                   long naux, long nt, long I0, long I1, double* B, uint32_t* top, cudaStream_t s,
                                   long tri = -1);
-
-// ---- k_metric_i8.cu
-// B's tile rows [I0, I1) from their raw integrals in ctx's present metric and aux range, on ctx->stream: on the int8
-// tensor cores where the contraction is large, else (or without room for the digits) launch_metric_contract_chunk.
-// digits: scratch of the caller's, kept between the blocks of one tensor.
-void metric_contract(rijk_ctx* ctx, const double* raw, int layout, long n, long I0, long I1, DeviceBuf& digits);
 
 // ---- k_coulomb.cu
 // Loads the FP64 Coulomb kernels' module on the current device (see preload_density_kernels).

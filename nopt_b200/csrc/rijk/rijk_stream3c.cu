@@ -23,7 +23,6 @@ void stream3c_cancel(rijk_ctx* ctx) {
   if (!ctx->s3.active && !ctx->s3.raw.p) return;
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   release(ctx->s3.raw);
-  release(ctx->s3.digits);
   ctx->s3.active = false;
 }
 
@@ -99,7 +98,7 @@ RIJK_API int rijk_add_3c_block(rijk_ctx* ctx, long mu0, long mu1, const double* 
   cudaStream_t s = ctx->stream;
   const long npad = round_up(n, TILE), nt = npad / TILE, ntile = nt * (nt + 1) / 2;
   const long nauxp = round_up(naux, KC);
-  const long nq = ctx->nq;
+  const long nq = ctx->nq, q0 = ctx->q0;
   long blk_first, blk_count;
   pair_rows(layout, n, mu0, mu1, &blk_first, &blk_count);
   int rc;
@@ -120,7 +119,10 @@ RIJK_API int rijk_add_3c_block(rijk_ctx* ctx, long mu0, long mu1, const double* 
     if (rc) return fail(ctx, rc);
     if (r1 == cmu1) {  // the chunk is complete: contract it with the metric factor
       cudaEventRecord(ctx->ev0, s);
-      metric_contract(ctx, static_cast<const double*>(ctx->s3.raw.p), layout, n, I0, I1, ctx->s3.digits);
+      launch_metric_contract_chunk(static_cast<const double*>(ctx->M.p) + q0 * nauxp, nauxp, nauxp - q0,
+                                   static_cast<const double*>(ctx->s3.raw.p), layout, n, nq, nt, I0, I1,
+                                   static_cast<double*>(ctx->B.p), static_cast<uint32_t*>(ctx->Btop.p), s,
+                                   ctx->metric_form == RIJK_METRIC_CHOLESKY ? q0 : -1);
       cudaEventRecord(ctx->ev1, s);
       rc = cuda_check(ctx, cudaStreamSynchronize(s), "metric contraction");
       if (rc) return fail(ctx, rc);
@@ -136,9 +138,7 @@ RIJK_API int rijk_add_3c_block(rijk_ctx* ctx, long mu0, long mu1, const double* 
   if (mu1 < n) return RIJK_OK;
   // the last row: the fitted tensor is complete
   release(ctx->s3.raw);
-  release(ctx->s3.digits);
   ctx->s3.active = false;
-  if ((rc = check_device_error(ctx))) return rc;
   ctx->n = n;
   ctx->npad = npad;
   ctx->nt = nt;
