@@ -881,9 +881,7 @@ static SyrkPlan syrk_plan_waves(long kdim, long tiles, long slots) {
   const long nchunks = (kdim + 63) / 64;
   const long smin = std::max<long>(1, (nchunks + kMaxChunks - 1) / kMaxChunks);
   const long smax = std::max<long>(smin, nchunks / 2);
-  // too few chunks for one full wave: as many ranges as there are (at n_ao = 72 one tile's 43 instead of a single
-  // CTA, 66 -> 9 us)
-  long sp = std::min(smax, std::max(smin, slots / tiles));
+  long sp = smin;
   for (long w = 1; w <= 64; ++w) {
     const long cand = std::min(smax, (w * slots) / tiles);
     if (cand < smin) continue;
