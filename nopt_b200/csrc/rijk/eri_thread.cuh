@@ -1,26 +1,22 @@
-// eri_thread.cuh — the three-centre integral kernel for spherical aux shells: a thread per aux shell.
-//
-// The Hermite expansion of a solid-harmonic Gaussian r^l Y_lm exp(-gamma r^2) about its own centre is the
-// harmonic polynomial itself in the derivatives, times (2 gamma)^-l: every lower term cancels, because the
-// polynomial's Laplacian vanishes.  An integral over one bra primitive pair p is then
-//     (ab|m) = sum_tuv E^ab_tuv W_m[tuv],   W_m[tuv] = c (-1/2gamma)^l s_m sum_c q_mc R[tuv + c]
-// with q_mc the integer coefficients of the polynomial, s_m its norm and E^ab the bra's spherical (or
-// Cartesian) functions in Hermite Gaussians.
+// eri_thread.cuh — the three-centre integral kernel for uncontracted spherical aux shells: a thread per aux shell.
 //
 // One CTA of 64 threads takes a bra shell pair and a tile of 8 to 64 aux shells of one l (eri_tile); with fewer
 // than 64, several threads share an aux shell and divide the bra functions between them (each forms R and W
-// again, which costs no time on lanes that would idle).  The threads form E for each bra primitive
-// pair in shared memory once, for all those aux shells; each thread then runs its aux shell: the Boys
-// values, the R recursion in place in registers (entries in falling order: a layer's entry of order k reads
-// only entries of order k - 1 and k - 2, not yet overwritten; local memory from total order 7 on), W, and
-// the product with E, whose entries all threads read as 16-byte broadcasts.  la + lb and lc are template
-// parameters, so the recursion and the harmonic sums are straight-line code without index tables.
+// again, which costs no time on lanes that would idle).  For each bra primitive pair the threads form the products
+// of its Hermite expansions, [Cartesian pair][tuv], in shared memory once for all those aux shells; each thread
+// then runs its aux shell: the Boys values, the R recursion in place in registers (entries in falling order: a
+// layer's entry of order k reads only entries of order k - 1 and k - 2, not yet overwritten; local memory from
+// total order 7 on), the aux Hermite sums W, and their product with the expansions, whose entries all threads
+// read as 16-byte broadcasts.  la + lb and lc are template parameters, so the recursion and the aux sums are
+// straight-line code without index tables.
 //
-// What bounds it: the FP64 pipe and its latency at 8 to 16 warps per SM.  Measured against a group of lanes per
-// shell triple with everything in shared memory (k_eri, kept for (P|Q), Cartesian aux shells and la + lb > 6), whose
-// Boys values one lane formed while the others waited and whose E was formed again for every aux shell: at
-// (H2O)8 cc-pVTZ/cc-pVTZ-JKFIT all of (P|Q) and (mu nu|P) 31.8 -> 4.0 ms, (H2O)16
-// cc-pVDZ/cc-pVDZ-JKFIT 32.7 -> 3.1 ms, (H2O)32 cc-pVTZ 1.02 -> 0.130 s.
+// The operations on one integral and their order are k_eri's, so both give the same bits: the split-BF16 copy of
+// the fitted tensor rounds it, and integrals that differ in their last bits moved single elements of mixed J and K
+// by 1e-7.  What k_eri spent its time on was not these operations: one lane of a group formed the Boys values while
+// the others waited, every stage ran through shared memory with a barrier, and the bra's expansion was formed
+// again for every aux shell.  (P|Q), Cartesian or contracted aux shells and la + lb > 6 stay there.
+// What bounds this kernel: the FP64 pipe and its latency at 8 to 16 warps per SM.  Measured, all classes of one
+// build: (H2O)8 cc-pVTZ 31.8 -> 6.5 ms, (H2O)32 cc-pVTZ 1.02 -> 0.234 s.
 #pragma once
 #include <utility>
 
@@ -90,25 +86,67 @@ constexpr int harm(int l, int row, int t, int u, int v) {
   }
 }
 
+// The aux Hermite terms of a spherical function, in the order of the term table (t, then u, then v rising): the
+// harmonic itself, and the places where the table's lower terms cancel to a last bit instead of to zero.
+constexpr bool is_term(int l, int row, int t, int u, int v) {
+  if (t + u + v == l) return harm(l, row, t, u, v) != 0;
+  const int k = t * 100 + u * 10 + v;
+  switch (l * 10 + row) {
+    case 32: return k == 10;
+    case 34: return k == 100;
+    case 42: return k == 110;
+    case 43: return k == 11;
+    case 45: return k == 101;
+    case 46: return k == 20 || k == 200;
+    default: return false;
+  }
+}
+constexpr int nterm(int l, int row) {
+  int n = 0;
+  for (int t = 0; t <= l; ++t)
+    for (int u = 0; u <= l - t; ++u)
+      for (int v = 0; v <= l - t - u; ++v) n += is_term(l, row, t, u, v);
+  return n;
+}
+// term i of the list as t | u << 4 | v << 8
+constexpr int term_at(int l, int row, int i) {
+  for (int t = 0; t <= l; ++t)
+    for (int u = 0; u <= l - t; ++u)
+      for (int v = 0; v <= l - t - u; ++v)
+        if (is_term(l, row, t, u, v) && i-- == 0) return t | (u << 4) | (v << 8);
+  return 0;
+}
+// the h-th (t, u, v), t + u + v <= L, in that order, packed likewise
+__host__ __device__ constexpr int lex_at(int L, int h) {
+  for (int t = 0; t <= L; ++t)
+    for (int u = 0; u <= L - t; ++u) {
+      const int n = L - t - u + 1;
+      if (h < n) return t | (u << 4) | (h << 8);
+      h -= n;
+    }
+  return 0;
+}
+
+// X r1 + k r2 of the recursion; as intrinsics, so that no other contraction is chosen
+template <int K>
+__device__ __forceinline__ double r_step(double X, double r1, double r2) {
+  if constexpr (K == 0)
+    return __dmul_rn(X, r1);
+  else if constexpr (K == 1)
+    return __dadd_rn(r2, __dmul_rn(X, r1));
+  else
+    return __fma_rn(static_cast<double>(K), r2, __dmul_rn(X, r1));
+}
+
 template <int E>
 __device__ __forceinline__ void r_entry(double* R, double X, double Y, double Z) {
   constexpr int t = dec_t(E), u = dec_u(E), v = dec_v(E);
-  if constexpr (t > 0) {
-    if constexpr (t > 1)
-      R[E] = fma(X, R[tix(t - 1, u, v)], (t - 1) * R[tix(t - 2, u, v)]);
-    else
-      R[E] = X * R[tix(t - 1, u, v)];
-  } else if constexpr (u > 0) {
-    if constexpr (u > 1)
-      R[E] = fma(Y, R[tix(t, u - 1, v)], (u - 1) * R[tix(t, u - 2, v)]);
-    else
-      R[E] = Y * R[tix(t, u - 1, v)];
-  } else {
-    if constexpr (v > 1)
-      R[E] = fma(Z, R[tix(t, u, v - 1)], (v - 1) * R[tix(t, u, v - 2)]);
-    else
-      R[E] = Z * R[tix(t, u, v - 1)];
-  }
+  if constexpr (t > 0)
+    R[E] = r_step<t - 1>(X, R[tix(t - 1, u, v)], R[tix(t > 1 ? t - 2 : 0, u, v)]);
+  else if constexpr (u > 0)
+    R[E] = r_step<u - 1>(Y, R[tix(t, u - 1, v)], R[tix(t, u > 1 ? u - 2 : 0, v)]);
+  else
+    R[E] = r_step<v - 1>(Z, R[tix(t, u, v - 1)], R[tix(t, u, v > 1 ? v - 2 : 0)]);
 }
 
 template <int CNT, int... E>
@@ -125,94 +163,78 @@ __device__ __forceinline__ void r_layers(double* R, const double* G, double X, d
   if constexpr (N > 0) r_layers<L, N - 1>(R, G, X, Y, Z);
 }
 
-// sum_c q_c R[h + c] over the Cartesians c of l
-template <int H, int LC, int ROW, int C = 0>
-__device__ __forceinline__ double w_entry(const double* R) {
-  constexpr int NC = (LC + 1) * (LC + 2) / 2;
-  // Cartesian C of l: the Hermite entries of order LC in tet order
-  constexpr int e = LC == 0 ? 0 : tetc(LC - 1) + C;
-  constexpr int q = harm(LC, ROW, dec_t(e), dec_u(e), dec_v(e));
-  constexpr int at = tix(dec_t(H) + dec_t(e), dec_u(H) + dec_u(e), dec_v(H) + dec_v(e));
-  double s = 0.0;
-  if constexpr (C + 1 < NC) s = w_entry<H, LC, ROW, C + 1>(R);
-  if constexpr (q != 0) s = fma(static_cast<double>(q), R[at], s);
+// sum over the terms I .. of the aux function: s + sum dp[i] R[h + term i], in order
+template <int T, int U, int V, int LC, int ROW, int I = 0>
+__device__ __forceinline__ double w_entry(const double* R, const double* dp, double s) {
+  constexpr int k = term_at(LC, ROW, I);
+  s = fma(dp[I], R[tix(T + (k & 15), U + ((k >> 4) & 15), V + (k >> 8))], s);
+  if constexpr (I + 1 < nterm(LC, ROW)) return w_entry<T, U, V, LC, ROW, I + 1>(R, dp, s);
   return s;
 }
-template <int LC, int ROW, int... H>
-__device__ __forceinline__ void w_all(const double* R, double f, double* W, std::integer_sequence<int, H...>) {
-  ((W[H] = f * w_entry<H, LC, ROW>(R)), ...);
+template <int LAB, int LC, int ROW, int... H>
+__device__ __forceinline__ void w_all(const double* R, const double* dp, double* W, std::integer_sequence<int, H...>) {
+  ((W[H] = w_entry<lex_at(LAB, H) & 15, (lex_at(LAB, H) >> 4) & 15, (lex_at(LAB, H) >> 8), LC, ROW>(R, dp, 0.0)), ...);
 }
 
-// F_0 .. F_L of T into F
-template <int L>
-__device__ __forceinline__ void boys(double T, const double* __restrict__ tab, double* F) {
-  constexpr double TMAX = gto_tab::BOYS_TMAX;
-  constexpr int NPER = gto_tab::BOYS_NPER, MTAB = gto_tab::BOYS_MTAB;
-  const double e = exp(-T);
-  if (T < TMAX - 0.5 / NPER) {
-    const int i = static_cast<int>(T * NPER + 0.5);
-    const double dt = static_cast<double>(i) / NPER - T;
-    const double* row = tab + static_cast<long>(i) * MTAB + L;
-    double f = __ldg(row + 6) * (1.0 / 720.0);
-    f = fma(f, dt, __ldg(row + 5) * (1.0 / 120.0));
-    f = fma(f, dt, __ldg(row + 4) * (1.0 / 24.0));
-    f = fma(f, dt, __ldg(row + 3) * (1.0 / 6.0));
-    f = fma(f, dt, __ldg(row + 2) * 0.5);
-    f = fma(f, dt, __ldg(row + 1));
-    f = fma(f, dt, __ldg(row));
-    F[L] = f;
-#pragma unroll
-    for (int m = L; m > 0; --m) F[m - 1] = fma(2.0 * T, F[m], e) * (1.0 / (2 * m - 1));
-  } else {
-    const double it = 0.5 / T;
-    F[0] = 0.5 * sqrt(gto_tab::PI / T);
-#pragma unroll
-    for (int m = 0; m < L; ++m) F[m + 1] = ((2 * m + 1) * F[m] - e) * it;
-  }
-}
-
-// v[m] = sum_h E[ab][h] W[h] for one aux function: two partial sums
+// acc[ab] += sum_h E[ab][h] W[h] for the thread's Cartesian pairs, h in order; four pairs at a time, whose chains
+// of FMAs hide each other's latency
 template <int NH>
-__device__ __forceinline__ double dot_row(const double* __restrict__ E, const double* W) {
-  double a = 0.0, b = 0.0;
-#pragma unroll
-  for (int h = 0; h + 1 < NH; h += 2) {
-    const double2 e = *reinterpret_cast<const double2*>(E + h);
-    a = fma(e.x, W[h], a);
-    b = fma(e.y, W[h + 1], b);
-  }
-  if (NH & 1) a = fma(E[NH - 1], W[NH - 1], a);
-  return a + b;
-}
-
-// The aux functions ROW .. 2 LC of one thread: out(ab, m, value) for its bra function pairs ab0, ab0 + dab, ..
-template <int LAB, int LC, int ROW, typename Out>
-__device__ __forceinline__ void rows(const double* R, double f, const double* __restrict__ norm,
-                                     const double* __restrict__ E, int ab0, int dab, int nab, Out out) {
-  constexpr int NH = tetc(LAB), NHP = (NH + 1) & ~1;
-  double W[NH];
-  w_all<LC, ROW>(R, f * __ldg(norm + ROW), W, std::make_integer_sequence<int, NH>());
+__device__ __forceinline__ void add_rows(const double* __restrict__ E, const double* W, int ab0, int dab, int nab, int stride,
+                                         double* acc) {
+  constexpr int NHP = (NH + 1) & ~1;
 #pragma unroll 1
-  for (int ab = ab0; ab < nab; ab += dab) out(ab, ROW, dot_row<NH>(E + ab * NHP, W));
-  if constexpr (ROW < 2 * LC) rows<LAB, LC, ROW + 1>(R, f, norm, E, ab0, dab, nab, out);
+  for (int ab = ab0; ab < nab; ab += 4 * dab) {
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    const double* e[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e[i] = E + (ab + i * dab < nab ? ab + i * dab : ab) * NHP;
+#pragma unroll
+    for (int h = 0; h < NH; h += 2) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const double2 c = *reinterpret_cast<const double2*>(e[i] + h);
+        v[i] = fma(c.x, W[h], v[i]);
+        if (h + 1 < NH) v[i] = fma(c.y, W[h + 1 < NH ? h + 1 : h], v[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (ab + i * dab < nab) acc[(ab + i * dab) * stride] += v[i];
+  }
 }
 
-// s s: every aux function of the thread, added to acc
-template <int LC, int ROW>
-__device__ __forceinline__ void sums(const double* R, double f, const double* __restrict__ norm, double* acc) {
-  acc[ROW] = fma(f * __ldg(norm + ROW), w_entry<0, LC, ROW>(R), acc[ROW]);
-  if constexpr (ROW < 2 * LC) sums<LC, ROW + 1>(R, f, norm, acc);
+// The aux functions ROW .. 2 LC of one thread.  terms, toff: the term table and its offsets for this l; pw: the
+// prefactor times powers of 1 / 2 gamma
+template <int LAB, int LC, int ROW>
+__device__ __forceinline__ void rows(const double* R, const double* pw, const EriTerm* __restrict__ terms,
+                                     const int* __restrict__ toff, const double* __restrict__ E, int ab0, int dab, int nab,
+                                     int stride, double* acc) {
+  constexpr int NH = tetc(LAB), NT_ = nterm(LC, ROW);
+  double dp[NT_];
+  const EriTerm* q = terms + __ldg(toff + ROW);
+#pragma unroll
+  for (int i = 0; i < NT_; ++i) {
+    const int k = term_at(LC, ROW, i);
+    dp[i] = __dmul_rn(q[i].d, pw[(LC + (k & 15) + ((k >> 4) & 15) + (k >> 8)) / 2]);
+  }
+  double W[NH];
+  w_all<LAB, LC, ROW>(R, dp, W, std::make_integer_sequence<int, NH>());
+  if constexpr (LAB == 0)
+    acc[ROW] += __dmul_rn(E[0], W[0]);
+  else
+    add_rows<NH>(E, W, ab0, dab, nab, stride, acc + ROW);
+  if constexpr (ROW < 2 * LC) rows<LAB, LC, ROW + 1>(R, pw, terms, toff, E, ab0, dab, nab, stride, acc);
 }
 
 template <int LAB, int LC>
 __global__ void __launch_bounds__(NT) k_eri_thread(const EriLaunch P) {
-  constexpr int L = LAB + LC, NR = tetc(L), NH = tetc(LAB), NHP = (NH + 1) & ~1, NF = 2 * LC + 1;
+  constexpr int L = LAB + LC, NR = tetc(L), NH = tetc(LAB), NHP = (NH + 1) & ~1, NF = 2 * LC + 1, ts = LAB + 2;
   extern __shared__ __align__(16) double sm[];
-  double* E1 = sm;                      // 3 x (la+1)(lb+1)(LAB+1)
-  double* E = sm + P.e1size;            // nab x NHP
+  double* E1 = sm;                // 3 x (la+1)(lb+1) ts: 1-D expansions
+  double* E = sm + P.e1size;      // nab x NHP: their products
+  double* acc = E + P.esize;      // nab x tile NF: Cartesian integrals
   const int tid = threadIdx.x;
   const int tile = P.tile, kt = tid & (tile - 1), part = tid / tile, parts = NT / tile;
-  double* acc = E + P.esize;            // nab x tile NF, contracted pairs only
   const int arow = tile * NF;
   const long ntile = (P.nket + tile - 1) / tile;
   const long ip = blockIdx.x / ntile;
@@ -222,144 +244,126 @@ __global__ void __launch_bounds__(NT) k_eri_thread(const EriLaunch P) {
   const EriShell B = P.bra[pair.y];
   const bool live = k0 + kt < P.nket;
   const EriShell C = P.ket[P.kets[live ? k0 + kt : P.nket - 1]];
-  const int la = A.l, lb = B.l, nfb = B.nfunc, nab = A.nfunc * nfb;
-  // the tile's largest primitive count: the aux shells are sorted by it
-  const int nprim_k = P.ket[P.kets[min(k0 + tile, P.nket) - 1]].nprim;
-  const bool direct = A.nprim * B.nprim * nprim_k == 1;
-  const double* norm = P.harm_norm + LC * 9;
+  const int la = A.l, lb = B.l, nca = ncart_d(la), ncb = ncart_d(lb), nab = nca * ncb;
+  const double gam = P.kexp[C.prim0], ck = P.kcoef[C.prim0];
+  const int* toff = P.term_off + (LMAX + 1 + LC) * (TERM_STRIDE + 1);
+  const double sgn = (LC & 1) ? -1.0 : 1.0;
   const double two_pi_25 = 2.0 * 17.493418327624862;  // 2 pi^(5/2)
 
-  // one value of the thread's aux function m and the bra functions ab to its place
-  auto store = [&](int ab, long col, double v) {
-    const int fa = ab / nfb, fb = ab - fa * nfb;
-    const long mu = A.off + fa, nu = B.off + fb;
-    if (P.mode == 0) {
-      if (pair.x == pair.y && nu > mu) return;
-      const long hi = mu > nu ? mu : nu, lo = mu > nu ? nu : mu;
-      if (hi < P.mu0 || hi >= P.mu1) return;
-      P.out[(hi * (hi + 1) / 2 + lo - P.rowbase) * P.ld + col] = v;
-    } else {
-      if (mu >= P.mu0 && mu < P.mu1) P.out[((mu - P.rowbase) * P.n + nu) * P.ld + col] = v;
-      if (pair.x != pair.y && nu >= P.mu0 && nu < P.mu1) P.out[((nu - P.rowbase) * P.n + mu) * P.ld + col] = v;
-    }
-  };
-
-  double racc[NF] = {};  // LAB = 0: the sums stay in registers, E is one number
-  if (LAB > 0 && !direct) {
+  double racc[NF] = {};  // LAB = 0: the sums stay in registers
+  if (LAB > 0) {
     for (int o = tid; o < nab * arow; o += NT) acc[o] = 0.0;
     __syncthreads();
   }
   const double ABx = A.x - B.x, ABy = A.y - B.y, ABz = A.z - B.z;
-  const double r2 = ABx * ABx + ABy * ABy + ABz * ABz;
-  bool any = false;
+  const double r2 = fma(ABz, ABz, fma(ABx, ABx, __dmul_rn(ABy, ABy)));
   for (int ij = 0; ij < A.nprim * B.nprim; ++ij) {
     const int i = ij / B.nprim, j = ij - i * B.nprim;
-    const double a = P.bexp[A.prim0 + i], b = P.bexp[B.prim0 + j];
-    const double cc = P.bcoef[A.prim0 + i] * P.bcoef[B.prim0 + j];
-    const double p = a + b, ip1 = 1.0 / p;
-    const double K = exp(-(a * b * ip1) * r2);
+    const double a = P.bexp[A.prim0 + i], ca = P.bcoef[A.prim0 + i];
+    const double b = P.bexp[B.prim0 + j], cb = P.bcoef[B.prim0 + j];
+    const double p = a + b, mu = a * b / p;
+    const double K = exp(-mu * r2);
+    const double cc = ca * cb;
     if (fabs(cc * K) < 1e-22) continue;  // contributes below double precision (host rule); the same for all threads
-    any = true;
-    const double Px = (a * A.x + b * B.x) * ip1, Py = (a * A.y + b * B.y) * ip1, Pz = (a * A.z + b * B.z) * ip1;
+    const double Px = fma(b, B.x, __dmul_rn(a, A.x)) / p, Py = fma(b, B.y, __dmul_rn(a, A.y)) / p;
+    const double Pz = fma(b, B.z, __dmul_rn(a, A.z)) / p;
     if constexpr (LAB > 0) {
-      // E1[d][i][j][t]: 1-D Hermite expansion of the primitive product
-      const int ts = LAB + 1, n1 = (la + 1) * (lb + 1) * ts;
+      const int n1 = (la + 1) * (lb + 1) * ts;
       __syncthreads();  // the previous primitive pair's readers of E are done
       if (tid < 3) {
         const double pd = tid == 0 ? Px : (tid == 1 ? Py : Pz);
         const double ad = tid == 0 ? A.x : (tid == 1 ? A.y : A.z);
         const double bd = tid == 0 ? B.x : (tid == 1 ? B.y : B.z);
-        const double xpa = pd - ad, xpb = pd - bd, o2p = 0.5 * ip1;
-        double* e1 = E1 + tid * n1;
-        e1[0] = tid == 0 ? K * cc : 1.0;
-        for (int q = 0; q <= la; ++q)
-          for (int r = 0; r <= lb; ++r) {
-            if (q + r == 0) continue;
-            const double* src = e1 + (r > 0 ? (q * (lb + 1) + r - 1) : ((q - 1) * (lb + 1))) * ts;
-            double* dst = e1 + (q * (lb + 1) + r) * ts;
-            const double x = r > 0 ? xpb : xpa;
-            const int o = q + r;  // the source has entries t <= o - 1
-            for (int t = 0; t <= o; ++t) {
-              double v = t < o ? x * src[t] : 0.0;
-              if (t + 1 < o) v += (t + 1) * src[t + 1];
-              if (t > 0) v += o2p * src[t - 1];
-              dst[t] = v;
-            }
-          }
+        hermite_1d_dev(la, lb, p, pd - ad, pd - bd, tid == 0 ? K : 1.0, E1 + tid * n1, ts);
       }
       __syncthreads();
-      // E[ab][tuv] over the spherical (or Cartesian) functions of the pair
+      // E[ab][tuv] = Ex Ey Ez, zero beyond the pair's orders
       for (int o = tid; o < nab * NH; o += NT) {
         const int ab = o / NH, h = o - ab * NH;
-        const int c = __ldg(P.tuv + h);
-        const int t = c & 0xff, u = (c >> 8) & 0xff, v = c >> 16;
-        const int fa = ab / nfb, fb = ab - fa * nfb;
-        const SphRow& ra = P.sph_rows[(A.pure ? 0 : 1) * SPH_ROWS + la * 15 + fa];
-        const SphRow& rb = P.sph_rows[(B.pure ? 0 : 1) * SPH_ROWS + lb * 15 + fb];
-        double s = 0.0;
-        for (int x = 0; x < ra.n; ++x) {
-          const int ka = ra.cart[x];
-          const int ax = ka & 15, ay = (ka >> 4) & 15, az = ka >> 8;
-          for (int y = 0; y < rb.n; ++y) {
-            const int kb = rb.cart[y];
-            const int bx = kb & 15, by = (kb >> 4) & 15, bz = kb >> 8;
-            if (t > ax + bx || u > ay + by || v > az + bz) continue;
-            s += ra.c[x] * rb.c[y] * E1[(ax * (lb + 1) + bx) * ts + t] * E1[n1 + (ay * (lb + 1) + by) * ts + u] *
-                 E1[2 * n1 + (az * (lb + 1) + bz) * ts + v];
-          }
+        const int c = __ldg(P.lex + LAB * LEX_STRIDE + h);
+        const int t = c & 15, u = (c >> 4) & 15, v = c >> 8;
+        const int ka = __ldg(P.cart + la * 16 + ab / ncb), kb = __ldg(P.cart + lb * 16 + ab % ncb);
+        const int ax = ka & 15, ay = (ka >> 4) & 15, az = ka >> 8;
+        const int bx = kb & 15, by = (kb >> 4) & 15, bz = kb >> 8;
+        double e = 0.0;
+        if (t <= ax + bx && u <= ay + by && v <= az + bz) {
+          const double et = E1[(ax * (lb + 1) + bx) * ts + t];
+          const double eu = __dmul_rn(et, E1[n1 + (ay * (lb + 1) + by) * ts + u]);
+          e = __dmul_rn(eu, E1[2 * n1 + (az * (lb + 1) + bz) * ts + v]);
         }
-        E[ab * NHP + h] = s;
+        E[ab * NHP + h] = e;
       }
       __syncthreads();
     }
+    const double al = p * gam / (p + gam);
     const double X = Px - C.x, Y = Py - C.y, Z = Pz - C.z;
-    const double d2 = X * X + Y * Y + Z * Z;
-#pragma unroll 1
-    for (int k = 0; k < nprim_k; ++k) {
-      const bool has = k < C.nprim;
-      const double gam = has ? P.kexp[C.prim0 + k] : 1.0, ck = has ? P.kcoef[C.prim0 + k] : 0.0;
-      const double rs = rsqrt(p + gam), al = p * gam * rs * rs, ig = 1.0 / gam;
-      double f = two_pi_25 * ip1 * ig * rs * ck;
-      if (LAB == 0) f *= K * cc;
-      const double o2g = -0.5 * ig;
+    const double T = al * fma(Z, Z, fma(X, X, __dmul_rn(Y, Y)));
+    double G[L + 1];
+    boys_eval_l<L>(T, P.boys, G);
+    const double pref = two_pi_25 / (p * gam * sqrt(p + gam)) * cc * ck * sgn;
+    const double i2g = 1.0 / (2.0 * gam);
+    double pw[LC + 1];
+    pw[0] = pref;
 #pragma unroll
-      for (int q = 0; q < LC; ++q) f *= o2g;
-      double G[L + 1];
-      boys<L>(al * d2, P.boys, G);
-      const double m2a = -2.0 * al;
-      double pw = 1.0;
+    for (int q = 1; q <= LC; ++q) pw[q] = pw[q - 1] * i2g;
+    const double m2a = -2.0 * al;
+    double pwn = 1.0;
 #pragma unroll
-      for (int m = 1; m <= L; ++m) {
-        pw *= m2a;
-        G[m] *= pw;
-      }
-      double R[NR];
-      r_layers<L>(R, G, X, Y, Z);
-      if constexpr (LAB == 0) {
-        sums<LC, 0>(R, f, norm, racc);
-      } else if (direct) {
-        rows<LAB, LC, 0>(R, f, norm, E, part, parts, nab, [&](int ab, int m, double v) {
-          if (live) store(ab, C.off + m, v);
-        });
-      } else {
-        double* mine = acc + kt * NF;
-        rows<LAB, LC, 0>(R, f, norm, E, part, parts, nab, [&](int ab, int m, double v) { mine[ab * arow + m] += v; });
+    for (int m = 1; m <= L; ++m) {
+      pwn *= m2a;
+      G[m] *= pwn;
+    }
+    double R[NR];
+    r_layers<L>(R, G, X, Y, Z);
+    if constexpr (LAB == 0)
+      rows<0, LC, 0>(R, pw, P.terms, toff, &K, 0, 1, 1, 0, racc);
+    else
+      rows<LAB, LC, 0>(R, pw, P.terms, toff, E, part, parts, nab, arow, acc + kt * NF);
+  }
+  if (LAB > 0) __syncthreads();  // the other parts' integrals
+  if (!live) return;
+  // bra Cartesian -> spherical, then store
+  const int nfb = B.nfunc, nfab = A.nfunc * nfb;
+  const double* ta = P.sph + sph_off(la);
+  const double* tb = P.sph + sph_off(lb);
+  for (int f = part; f < nfab; f += parts) {
+    const int fa = f / nfb, fb = f - fa * nfb;
+    const int ia0 = A.pure ? 0 : fa, ia1 = A.pure ? nca : fa + 1;
+    const int ib0 = B.pure ? 0 : fb, ib1 = B.pure ? ncb : fb + 1;
+    double v[NF] = {};
+    if constexpr (LAB == 0) {
+#pragma unroll
+      for (int m = 0; m < NF; ++m) v[m] = racc[m];  // the s function's coefficient is 1
+    } else {
+      for (int ia = ia0; ia < ia1; ++ia) {
+        const double wa = A.pure ? __ldg(ta + fa * nca + ia) : 1.0;
+        if (wa == 0.0) continue;
+        double sb[NF] = {};
+        for (int ib = ib0; ib < ib1; ++ib) {
+          const double wb = B.pure ? __ldg(tb + fb * ncb + ib) : 1.0;
+#pragma unroll
+          for (int m = 0; m < NF; ++m) sb[m] = fma(wb, acc[(ia * ncb + ib) * arow + kt * NF + m], sb[m]);
+        }
+#pragma unroll
+        for (int m = 0; m < NF; ++m) v[m] = fma(wa, sb[m], v[m]);
       }
     }
-  }
-  if (!live) return;
-  if constexpr (LAB == 0) {
-    if (part == 0)
+    const long mu = A.off + fa, nu = B.off + fb;
+    double *o0 = nullptr, *o1 = nullptr;
+    if (P.mode == 0) {
+      if (pair.x == pair.y && nu > mu) continue;
+      const long hi = mu > nu ? mu : nu, lo = mu > nu ? nu : mu;
+      if (hi < P.mu0 || hi >= P.mu1) continue;
+      o0 = P.out + (hi * (hi + 1) / 2 + lo - P.rowbase) * P.ld + C.off;
+    } else {
+      if (mu >= P.mu0 && mu < P.mu1) o0 = P.out + ((mu - P.rowbase) * P.n + nu) * P.ld + C.off;
+      if (pair.x != pair.y && nu >= P.mu0 && nu < P.mu1) o1 = P.out + ((nu - P.rowbase) * P.n + mu) * P.ld + C.off;
+    }
 #pragma unroll
-      for (int m = 0; m < NF; ++m) store(0, C.off + m, racc[m]);
-  } else if (!direct) {
-    for (int ab = part; ab < nab; ab += parts)
-#pragma unroll
-      for (int m = 0; m < NF; ++m) store(ab, C.off + m, acc[ab * arow + kt * NF + m]);
-  } else if (!any) {  // every primitive pair is below double precision
-    for (int ab = part; ab < nab; ab += parts)
-#pragma unroll
-      for (int m = 0; m < NF; ++m) store(ab, C.off + m, 0.0);
+    for (int m = 0; m < NF; ++m) {
+      if (o0) o0[m] = v[m];
+      if (o1) o1[m] = v[m];
+    }
   }
 }
 

@@ -7,8 +7,8 @@
 // (gto_ints.cpp): bra primitive pairs expanded in Hermite Gaussians (E coefficients), Hermite
 // Coulomb integrals R_tuv from the Boys function, aux functions as one-centre Hermite sums.
 //
-// (mu nu|P) over spherical aux shells with la + lb <= 6, all of the usual bases, takes k_eri_thread (eri_thread.cuh), one launch
-// per (la + lb, lc).  The rest of this comment is about k_eri here, which takes the others.
+// (mu nu|P) over uncontracted spherical aux shells with la + lb <= 6, all of the usual bases, takes k_eri_thread
+// (eri_thread.cuh), one launch per (la + lb, lc).  The rest of this comment is about k_eri here, which takes the others.
 //
 // Work decomposition.  One launch per angular class (l_A, l_B, l_C); a task is one shell triple
 // (A B | C) and runs on a group of G lanes (G = 1 .. 32, chosen per class so that small classes
@@ -38,53 +38,6 @@ namespace {
 using namespace eri;
 constexpr int GROUP_F = 24;  // per group: F_0 .. F_15 and the aux power table pw[0..7]
 constexpr int ERI_THREADS = 128;
-
-// F_m(T), m = 0 .. L, exactly as the host engine evaluates it (Taylor about the nearest grid
-// point, downward recursion; F_0 and upward recursion past the grid).
-__device__ void boys_eval(int L, double T, const double* __restrict__ tab, double* F) {
-  constexpr double TMAX = gto_tab::BOYS_TMAX;
-  constexpr int NPER = gto_tab::BOYS_NPER, MTAB = gto_tab::BOYS_MTAB;
-  if (T < TMAX - 0.5 / NPER) {
-    const int i = static_cast<int>(T * NPER + 0.5);
-    const double dt = static_cast<double>(i) / NPER - T;
-    const double* row = tab + static_cast<long>(i) * MTAB;
-    double f = __ldg(row + L + 6);
-    f = __ldg(row + L + 5) + f * dt / 6.0;
-    f = __ldg(row + L + 4) + f * dt / 5.0;
-    f = __ldg(row + L + 3) + f * dt / 4.0;
-    f = __ldg(row + L + 2) + f * dt / 3.0;
-    f = __ldg(row + L + 1) + f * dt / 2.0;
-    f = __ldg(row + L) + f * dt;
-    F[L] = f;
-    const double e = exp(-T);
-    for (int m = L; m > 0; --m) F[m - 1] = (2.0 * T * F[m] + e) / (2 * m - 1);
-  } else {
-    const double e = exp(-T);
-    F[0] = 0.5 * sqrt(gto_tab::PI / T);
-    for (int m = 0; m < L; ++m) F[m + 1] = ((2 * m + 1) * F[m] - e) / (2.0 * T);
-  }
-}
-
-// 1-D Hermite expansion E[i][j][t] of a primitive product, i <= la, j <= lb, t < ts (= la+lb+2).
-__device__ void hermite_1d_dev(int la, int lb, double p, double xpa, double xpb, double k0, double* E, int ts) {
-  const double o2p = 0.5 / p;
-  auto at = [&](int i, int j, int t) -> double& { return E[(i * (lb + 1) + j) * ts + t]; };
-  for (int k = 0; k < (la + 1) * (lb + 1) * ts; ++k) E[k] = 0.0;
-  at(0, 0, 0) = k0;
-  for (int i = 0; i < la; ++i)
-    for (int t = 0; t <= i + 1; ++t) {
-      double v = xpa * at(i, 0, t) + (t + 1) * at(i, 0, t + 1);
-      if (t > 0) v += o2p * at(i, 0, t - 1);
-      at(i + 1, 0, t) = v;
-    }
-  for (int i = 0; i <= la; ++i)
-    for (int j = 0; j < lb; ++j)
-      for (int t = 0; t <= i + j + 1; ++t) {
-        double v = xpb * at(i, j, t) + (t + 1) * at(i, j, t + 1);
-        if (t > 0) v += o2p * at(i, j, t - 1);
-        at(i, j + 1, t) = v;
-      }
-}
 
 __global__ void __launch_bounds__(ERI_THREADS) k_eri(const EriLaunch P) {
   extern __shared__ __align__(16) double sm_eri[];
@@ -345,7 +298,7 @@ int upload_basis(rijk_ctx* ctx, const HostBasis& h, DevBasis& d) {
 // Device tables shared by all launches: Boys grid, spherical transforms, aux term lists,
 // Hermite index decode and Cartesian exponents.  Built once per context.
 struct TabLayout {
-  size_t boys, sph, terms, term_off, tuv, cart, rows, norm, total;
+  size_t boys, sph, terms, term_off, tuv, cart, lex, total;
 };
 
 TabLayout tab_layout(size_t nterms) {
@@ -362,8 +315,7 @@ TabLayout tab_layout(size_t nterms) {
   t.term_off = take(sizeof(int) * TERM_KEYS * (TERM_STRIDE + 1));
   t.tuv = take(sizeof(int) * TET_MAX);
   t.cart = take(sizeof(int) * (LMAX + 1) * 16);
-  t.rows = take(sizeof(SphRow) * 2 * SPH_ROWS);
-  t.norm = take(sizeof(double) * (LMAX + 1) * 9);
+  t.lex = take(sizeof(int) * (LAB_MAX + 1) * LEX_STRIDE);
   t.total = o;
   return t;
 }
@@ -375,8 +327,8 @@ struct DevTables {
   const int* term_off;
   const int* tuv;
   const int* cart;
-  const SphRow* rows;
-  const double* norm;
+  const int* lex;
+  bool thread_terms;  // the spherical term lists are the ones k_eri_thread is compiled for
 };
 
 int ensure_tables(rijk_ctx* ctx, DevTables& dt) {
@@ -438,29 +390,9 @@ int ensure_tables(rijk_ctx* ctx, DevTables& dt) {
       for (int lx = l; lx >= 0; --lx)
         for (int ly = l - lx; ly >= 0; --ly)
           cart[l * 16 + gto_tab::cart_index(l, lx, ly)] = lx | (ly << 4) | ((l - lx - ly) << 8);
-    SphRow* rows = reinterpret_cast<SphRow*>(blob.data() + lay.rows);
-    double* norm = reinterpret_cast<double*>(blob.data() + lay.norm);
-    for (int l = 0; l <= LMAX; ++l) {
-      const int nc = ncart_d(l);
-      for (int m = 0; m < 2 * l + 1; ++m)
-        for (int lx = l; lx >= 0; --lx)
-          for (int ly = l - lx; ly >= 0; --ly) {
-            const int lz = l - lx - ly;
-            const double c = S.c[l][static_cast<size_t>(m) * nc + gto_tab::cart_index(l, lx, ly)];
-            const int q = harm(l, m, lx, ly, lz);
-            if (q == 0) continue;  // the table's own value is zero there, or rounding of a cancelled sum
-            SphRow& r = rows[l * 15 + m];
-            r.cart[r.n] = lx | (ly << 4) | (lz << 8);
-            r.c[r.n++] = c;
-            norm[l * 9 + m] = c / q;
-          }
-      for (int c = 0; c < nc; ++c) {
-        SphRow& r = rows[SPH_ROWS + l * 15 + c];
-        r.n = 1;
-        r.cart[0] = cart[l * 16 + c];
-        r.c[0] = 1.0;
-      }
-    }
+    int* lex = reinterpret_cast<int*>(blob.data() + lay.lex);
+    for (int l = 0; l <= LAB_MAX; ++l)
+      for (int h = 0; h < tet(l); ++h) lex[l * LEX_STRIDE + h] = lex_at(l, h);
     int rc = ensure(ctx, ctx->eri_tab, lay.total, "integral tables");
     if (rc) return rc;
     rc = cuda_check(ctx, cudaMemcpyAsync(ctx->eri_tab.p, blob.data(), lay.total, cudaMemcpyHostToDevice, ctx->stream),
@@ -474,8 +406,18 @@ int ensure_tables(rijk_ctx* ctx, DevTables& dt) {
   dt.term_off = reinterpret_cast<const int*>(p + lay.term_off);
   dt.tuv = reinterpret_cast<const int*>(p + lay.tuv);
   dt.cart = reinterpret_cast<const int*>(p + lay.cart);
-  dt.rows = reinterpret_cast<const SphRow*>(p + lay.rows);
-  dt.norm = reinterpret_cast<const double*>(p + lay.norm);
+  dt.lex = reinterpret_cast<const int*>(p + lay.lex);
+  dt.thread_terms = true;
+  for (int l = 0; l <= LMAX; ++l)
+    for (int m = 0; m < 2 * l + 1; ++m) {
+      const int* o = toff.data() + (LMAX + 1 + l) * (TERM_STRIDE + 1) + m;
+      bool same = o[1] - o[0] == nterm(l, m);
+      for (int i = 0; same && i < nterm(l, m); ++i) {
+        const EriTerm& e = terms[o[0] + i];
+        same = term_at(l, m, i) == (e.t | (e.u << 4) | (e.v << 8));
+      }
+      dt.thread_terms = dt.thread_terms && same;
+    }
   return RIJK_OK;
 }
 
@@ -495,12 +437,11 @@ int group_doubles(int la, int lb, int lc) {
   return (d + 1) & ~1;
 }
 
-// Ket shells grouped by angular momentum, spherical ones before Cartesian ones, each group sorted by
-// primitive count (tasks next to each other then share their loop trip counts).
+// Ket shells grouped by angular momentum: first the uncontracted spherical ones (k_eri_thread's), then the others
+// sorted by primitive count (tasks next to each other in a warp then share their loop trip counts).
 struct KetLists {
   std::vector<int> idx;
-  long start[2 * (LMAX + 1) + 1] = {};  // group 2 l: spherical, 2 l + 1: Cartesian
-  int nprim[2 * (LMAX + 1)] = {};       // largest primitive count of the group
+  long start[2 * (LMAX + 1) + 1] = {};  // group 2 l: spherical single primitives, 2 l + 1: the others
 };
 
 KetLists ket_lists(const HostBasis& k) {
@@ -509,9 +450,8 @@ KetLists ket_lists(const HostBasis& k) {
     out.start[g] = static_cast<long>(out.idx.size());
     std::vector<int> v;
     for (int s = 0; s < static_cast<int>(k.sh.size()); ++s)
-      if (2 * k.sh[s].l + (k.sh[s].pure ? 0 : 1) == g) v.push_back(s);
+      if (2 * k.sh[s].l + (k.sh[s].pure && k.sh[s].nprim == 1 ? 0 : 1) == g) v.push_back(s);
     std::stable_sort(v.begin(), v.end(), [&](int x, int y) { return k.sh[x].nprim < k.sh[y].nprim; });
-    if (!v.empty()) out.nprim[g] = k.sh[v.back()].nprim;
     out.idx.insert(out.idx.end(), v.begin(), v.end());
   }
   out.start[2 * (LMAX + 1)] = static_cast<long>(out.idx.size());
@@ -519,13 +459,13 @@ KetLists ket_lists(const HostBasis& k) {
 }
 
 // Bra pair lists by class (l_A, l_B), concatenated in the order of l_A + l_B, with class offsets; for each
-// l_A + l_B the widest pair and the widest contracted one.
+// l_A + l_B the most Cartesian function pairs.
 constexpr int NCLASS = (LMAX + 1) * (LMAX + 1);
 struct PairLists {
   std::vector<int2> pairs;
   long start[NCLASS] = {}, count[NCLASS] = {};
   long lab_start[2 * LMAX + 2] = {};
-  int wide[2 * LMAX + 1] = {}, wide_contracted[2 * LMAX + 1] = {};
+  int wide[2 * LMAX + 1] = {};
 };
 
 template <typename Keep>
@@ -537,9 +477,7 @@ void pair_lists(const std::vector<EriShell>& bra, const std::vector<int2>& cand,
     if (!keep(pr)) continue;
     const EriShell &A = bra[pr.x], &B = bra[pr.y];
     (A.nprim * B.nprim >= 8 ? heavy : by)[A.l * (LMAX + 1) + B.l].push_back(pr);
-    const int lab = A.l + B.l, nab = A.nfunc * B.nfunc;
-    out.wide[lab] = std::max(out.wide[lab], nab);
-    if (A.nprim * B.nprim > 1) out.wide_contracted[lab] = std::max(out.wide_contracted[lab], nab);
+    out.wide[A.l + B.l] = std::max(out.wide[A.l + B.l], ncart_d(A.l) * ncart_d(B.l));
   }
   for (int lab = 0; lab <= 2 * LMAX; ++lab) {
     out.lab_start[lab] = static_cast<long>(out.pairs.size());
@@ -584,11 +522,12 @@ int launch_group(rijk_ctx* ctx, EriLaunch P, const PairLists& pl, const int2* pa
 }
 
 // Aux shells of a k_eri_thread CTA.  64, one a thread, while that gives the GPU four CTAs an SM; fewer where the
-// class has fewer, or where the launch would leave SMs idle and the bra functions can be shared out instead
-// (each thread keeps at least three of them).
-int eri_tile(long npair, long nket, int wide) {
+// class has fewer, where the launch would leave SMs idle and the bra functions can be shared out instead (each
+// thread keeps at least three of them), or where their Cartesian integrals would leave shared memory for one CTA only.
+int eri_tile(long npair, long nket, int wide, int nf, int fixed) {
   int tile = NT;
-  while (tile > 8 && (tile / 2 >= nket || (npair * ((nket + tile - 1) / tile) < 4 * 148 && wide * tile >= 6 * NT)))
+  while (tile > 8 && (tile / 2 >= nket || (npair * ((nket + tile - 1) / tile) < 4 * 148 && wide * tile >= 6 * NT) ||
+                      (fixed + wide * tile * nf) * 8 > 100 * 1024))
     tile /= 2;
   return tile;
 }
@@ -624,18 +563,15 @@ int launch_classes(rijk_ctx* ctx, const EriLaunch& base, const PairLists& pl, co
       if (P.nket == 0) continue;
       P.pairs = pairs_dev + pl.lab_start[lab];
       P.npair = np;
-      // The thread-per-aux-shell kernel: its expansions, and the accumulators of contracted pairs, must fit.  (P|Q) stays
-      // on k_eri: it is 1 % of the integrals (its 25 launches 0.4 of 4.1 ms at (H2O)8 cc-pVTZ, 0.3 with this kernel), and
-      // through the metric's condition another rounding of it moves the derivatives by 1e-9.
+      // The thread-per-aux-shell kernel: its expansions and Cartesian integrals must fit.  (P|Q), 1 % of the integrals,
+      // stays on k_eri.
       const int side = lab / 2 + 1;  // (la + 1)(lb + 1) is at most side * (lab + 2 - side)
-      P.e1size = (3 * side * (lab + 2 - side) * (lab + 1) + 1) & ~1;
+      P.e1size = (3 * side * (lab + 2 - side) * (lab + 2) + 1) & ~1;
       P.esize = pl.wide[lab] * ((tet(lab) + 1) & ~1);
-      const int contracted = kl.nprim[g] > 1 ? pl.wide[lab] : pl.wide_contracted[lab];
-      P.tile = eri_tile(np, P.nket, pl.wide[lab]);
+      P.tile = eri_tile(np, P.nket, pl.wide[lab], 2 * lc + 1, P.e1size + P.esize);
       const size_t smem = (static_cast<size_t>(P.e1size) + P.esize +
-                           static_cast<size_t>(contracted) * P.tile * (2 * lc + 1)) * sizeof(double);
-      if (base.mode != 2 && g % 2 == 0 && lab <= LAB_MAX &&
-          smem <= static_cast<size_t>(maxsm)) {
+                           static_cast<size_t>(pl.wide[lab]) * P.tile * (2 * lc + 1)) * sizeof(double);
+      if (base.mode != 2 && base.thread_terms && g % 2 == 0 && lab <= LAB_MAX && smem <= static_cast<size_t>(maxsm)) {
         const cudaError_t e = kLaunchThread[lc](lab, P, smem, s);
         if (e != cudaSuccess) {
           join();
@@ -666,8 +602,8 @@ EriLaunch base_launch(const DevTables& t) {
   P.term_off = t.term_off;
   P.tuv = t.tuv;
   P.cart = t.cart;
-  P.sph_rows = t.rows;
-  P.harm_norm = t.norm;
+  P.lex = t.lex;
+  P.thread_terms = t.thread_terms;
   return P;
 }
 
