@@ -356,9 +356,12 @@ def grad_report(fb, si, MOc, nocc, fp64_peak, reps=3):
     n, naux = si.n, si.naux
     npad = st["npad"]
     noccp = (nocc + 15) // 16 * 16
+    te = st["ntile"] * 4096
     pairs = nocc * (nocc + 1) // 2 + 1  # packed (i, j), and the row of w
     flops = {"y_t": 2.0 * noccp * nocc * npad * naux, "gamma": 2.0 * pairs * naux * naux + 2.0 * n * nocc * nocc * naux,
-             "d3c_M_gamma": 1.0 * n * (n + 1) * nocc * naux, "dV_MtGM": 2.0 * pairs * naux * naux}
+             "d3c_M_gamma": 1.0 * n * (n + 1) * nocc * naux,
+             "g_gamma_B": 2.0 * noccp * nocc * npad * naux + 2.0 * te * noccp * naux + 2.0 * te * naux * naux,
+             "dV_MtGM": 4.0 * naux ** 3}
     stages = {}
     for k, ms in st["grad_stages"].items():
         e = {"ms": ms}

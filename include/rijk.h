@@ -96,7 +96,7 @@ typedef struct {
   long grad_qchunk;       /* aux functions per chunk of the last rijk_grad (naux: one chunk)    */
   /* Device time of the stages of the last rijk_grad (with profiling on): [0] the FP64 Fock build,
    * energy and dE/dC, [1] 0, [2] Y^Q = X^Q C^T, [3] Z^P = sum_Q M_QP Y^Q and C^T Z^P,
-   * [4] dE/d(P|mu nu) with its copies to the host, [5] 0, [6] dE/d(P|Q) from Z.                     */
+   * [4] dE/d(P|mu nu) with its copies to the host, [5] T^Q, Gamma and G = Gamma B, [6] -M^T G M.    */
   double ms_grad_stage[7];
   double ms_grad_total;   /* device time of rijk_grad before its host copies (profiling on)     */
 } rijk_stats_t;

@@ -253,7 +253,7 @@ static void prof_collect(rijk_ctx* ctx) {
 }
 
 int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long nocc, double* dJ, double* dK,
-                     int precision, cudaEvent_t mo_ready, cudaEvent_t j_done) {
+                     int precision, cudaEvent_t mo_ready, cudaEvent_t j_done, bool dmma_x) {
   // naux here is the number of aux functions this context holds (a slice under rijk_set_aux_range)
   const long n = ctx->n, naux = ctx->nq, nt = ctx->nt, npad = ctx->npad, ntile = ctx->ntile;
   const long tile_elems = ntile * TILE2;
@@ -281,7 +281,7 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
     const bool large = npad > 192 && 3.0 * npad * npad * kdim >= 1e10;
     i8k = tc || large;
     nsK = i8k ? syrk_i8_parts(nt, naux, noccp, ctx->device, &kper_tc) : syrk_nsplit(nt, kdim);
-    i8x = large && kper_tc % noccp == 0 && bdig_prepare(ctx);
+    i8x = large && !dmma_x && kper_tc % noccp == 0 && bdig_prepare(ctx);
     if (i8x && (rc = xform_i8_buffers(ctx, noccp, nsK))) return rc;
     if ((rc = ensure(ctx, ctx->MOp, noccp * npad * sizeof(double), "MOp")) ||
         (rc = ensure(ctx, ctx->XT, static_cast<size_t>(npad) * kdim * sizeof(double), "XT")) ||

@@ -169,9 +169,10 @@ void log_build(rijk_ctx* ctx, const char* call, long nocc, int precision);
 void log_line(const std::string& json);
 // One Fock build on device pointers (J into dJ, K into dK), asynchronous on ctx->stream.  With
 // mo_ready the exchange waits for that event (dMO is written on another stream); with j_done the
-// event is recorded once J is complete, before the exchange kernels.
+// event is recorded once J is complete, before the exchange kernels.  dmma_x keeps an FP64 build's half-transform on
+// DMMA (its XT is then the same for every size; the int8 form's differs in last bits).
 int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long nocc, double* dJ, double* dK,
-                     int precision, cudaEvent_t mo_ready = nullptr, cudaEvent_t j_done = nullptr);
+                     int precision, cudaEvent_t mo_ready = nullptr, cudaEvent_t j_done = nullptr, bool dmma_x = false);
 // Metric factor from (P|Q) held in host memory (cudaMemcpyHostToDevice) or device memory.
 int set_metric_impl(rijk_ctx* ctx, const double* PQ, cudaMemcpyKind kind, long naux, int form);
 // Fitted tensor from three-centre integrals that `fill` writes, one block of tile rows at a time:
