@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "dmma.cuh"
 #include "rijk_internal.h"
 
 #define RIJK_API extern "C" __attribute__((visibility("default")))
@@ -46,18 +47,51 @@ __global__ void k_gather_pa(const double* __restrict__ R, long nb, long n2, long
   }
 }
 
-// out[r][Q] = sum_nu XT[nu][Q p2 + r] C[r][nu] for r < nr: the diagonal (rr|Q) of a batch of rows.
-__global__ void k_diag_pair(const double* __restrict__ XT, const double* __restrict__ C, long nr, long p2, long naux,
-                            long npad, double* __restrict__ out) {
-  const long kdim = naux * p2, total = naux * p2;
+// out[r][Q] = sum_nu XT[nu][Q p2 + r] C[r][nu] for r < nr: the diagonal (rr|Q) of a batch of rows.  A CTA takes 32
+// neighbouring (Q, r) and shares the sum over nu between its 8 warps: with a thread to each sum the few thousand
+// threads waited for one load after another (131 us for 96 rows at C10H22 cc-pVDZ).
+__global__ void __launch_bounds__(256) k_diag_pair(const double* __restrict__ XT, const double* __restrict__ C, long nr,
+                                                   long p2, long naux, long npad, double* __restrict__ out) {
+  __shared__ double part[8][32];
+  const long kdim = naux * p2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (long i0 = static_cast<long>(blockIdx.x) * 32; i0 < kdim; i0 += static_cast<long>(gridDim.x) * 32) {
+    const long idx = i0 + lane, Q = idx / p2, r = idx % p2;
+    const bool live = idx < kdim && r < nr;
+    double s = 0.0;
+    if (live) {
+      const double* c = C + r * npad;
+#pragma unroll 4
+      for (long nu = warp; nu < npad; nu += 8) s += XT[nu * kdim + idx] * c[nu];
+    }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && live) {
+      for (int w = 1; w < 8; ++w) s += part[w][lane];
+      out[r * naux + Q] = s;
+    }
+    __syncthreads();
+  }
+}
+
+// Yp[(t (t + 1) / 2 + u)][Q] = Yt[(t n_a + u)][Q], u <= t
+__global__ void k_pack_tu(const double* __restrict__ Yt, long na, long naux, double* __restrict__ Yp) {
+  const long total = na * (na + 1) / 2 * naux;
   for (long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
        idx += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long Q = idx / p2, r = idx % p2;
-    if (r >= nr) continue;
-    const double* c = C + r * npad;
-    double s = 0.0;
-    for (long nu = 0; nu < npad; ++nu) s += XT[nu * kdim + Q * p2 + r] * c[nu];
-    out[r * naux + Q] = s;
+    long t, u;
+    tri_decode(idx / naux, t, u);
+    Yp[idx] = Yt[(t * na + u) * naux + idx % naux];
+  }
+}
+
+// out[p][(t u)] = Jp[p][tu], tu the packed pair of t and u
+__global__ void k_expand_tu(const double* __restrict__ Jp, long nmo, long na, double* __restrict__ out) {
+  const long T = na * (na + 1) / 2, total = nmo * na * na;
+  for (long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
+       idx += static_cast<long>(gridDim.x) * blockDim.x) {
+    const long p = idx / (na * na), t = idx / na % na, u = idx % na;
+    out[idx] = Jp[p * T + (t > u ? t * (t + 1) / 2 + u : u * (u + 1) / 2 + t)];
   }
 }
 
@@ -296,27 +330,51 @@ RIJK_API int rijk_soscf_hess_ints(rijk_ctx* ctx, double* aa_J, double* aa_K, con
     g.C = dK, g.ldc = n_a, g.sC = n_a * n_a;
     gemm_f64(g, n_mo, ctx->stream);
   }
-  // (pp|Q) for every orbital, by half-transforms of batches of rows
-  double* Rpp = sc.get(ctx, static_cast<size_t>(n_mo) * naux, "(pp|Q)", &rc);
+  double* dJ = sc.get(ctx, static_cast<size_t>(n_mo) * n_a * n_a, "aa_J", &rc);
   if (rc) return rc;
-  const long batch = 96;
+  // aa_J[p][(t u)] = sum_Q (pp|Q)(t u|Q), by the cheaper of two orders.  J^{tu}_{mu nu} = sum_Q (t u|Q) B^Q_{mu nu} for
+  // the T = n_a (n_a + 1) / 2 pairs first costs n^2 n_aux T and their diagonals (pp| 2 n^2 n_mo T FLOPs; the diagonals
+  // (pp|Q) of every B^Q first, 2 n^2 n_mo n_aux.  The pairs also must not take more scratch than the other's batch
+  // of 96 rows.  Whole calls at C10H22 cc-pVDZ (n = 250, n_aux = 1206), pairs against diagonals: 0.74 against 2.18 ms at
+  // n_a = 6, 0.80, 2.21 at 10, 1.59, 2.44 at 18, 1.95, 2.49 at 22, and even at the line, 2.50, 2.52 at 26.
+  const long te = ctx->ntile * TILE2, T = n_a * (n_a + 1) / 2;
+  const bool pairs_first = T * (naux + 2 * n_mo) < 2 * n_mo * naux && T * te <= 96 * npad * naux;
+  const long nd = pairs_first ? T : naux;  // tensors whose diagonals are formed, by half-transforms of batches of rows
+  const double* tens = static_cast<const double*>(ctx->B.p);
+  if (pairs_first) {
+    double* Yp = sc.get(ctx, static_cast<size_t>(T) * naux, "packed (t u|Q)", &rc);
+    if (rc) return rc;
+    double* Jtu = sc.get(ctx, static_cast<size_t>(T) * te, "J^{tu}", &rc);
+    if (rc) return rc;
+    k_pack_tu<<<grid_of(T * naux), 256, 0, ctx->stream>>>(ap.Yt, n_a, naux, Yp);
+    GemmF64Args g;
+    g.M = T, g.N = te, g.K = naux;
+    g.A = Yp, g.lda = naux, g.a_kmajor = true;
+    g.B = tens, g.ldb = te, g.b_kmajor = false;
+    g.C = Jtu, g.ldc = te;
+    gemm_f64(g, 1, ctx->stream);
+    tens = Jtu;
+  }
+  double* Rpp = sc.get(ctx, static_cast<size_t>(n_mo) * nd, "(pp| diagonals", &rc);
+  if (rc) return rc;
+  // 96 rows a batch, or all of them while their half-transform is no larger than 256 MB
+  const long all = round_up(n_mo, 16);
+  const long batch = npad * nd * all <= (32L << 20) ? all : 96;
   {
     Scratch sb;
-    double* XT = sb.get(ctx, static_cast<size_t>(npad) * naux * batch, "batch half-transform", &rc);
+    double* XT = sb.get(ctx, static_cast<size_t>(npad) * nd * std::min(batch, all), "batch half-transform", &rc);
     if (rc) return rc;
     for (long p0 = 0; p0 < n_mo; p0 += batch) {
       const long nr = std::min(batch, n_mo - p0), pb = round_up(nr, 16);
       const double* rows = ap.rows_all + p0 * npad;
-      launch_xform_f64(static_cast<const double*>(ctx->B.p), rows, naux, ctx->nt, pb, XT, ctx->stream);
-      k_diag_pair<<<grid_of(naux * pb), 256, 0, ctx->stream>>>(XT, rows, nr, pb, naux, npad, Rpp + p0 * naux);
+      launch_xform_f64(tens, rows, nd, ctx->nt, pb, XT, ctx->stream);
+      k_diag_pair<<<grid_of(nd * pb * 8), 256, 0, ctx->stream>>>(XT, rows, nr, pb, nd, npad, Rpp + p0 * nd);
     }
     // p0 + pb <= round_up(n_mo, 16): the last batch's padding rows are the zero rows of rows_all
-    if ((rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "(pp|Q)"))) return rc;
   }
-  // aa_J[p][(t u)] = sum_Q (pp|Q)(t u|Q)
-  double* dJ = sc.get(ctx, static_cast<size_t>(n_mo) * n_a * n_a, "aa_J", &rc);
-  if (rc) return rc;
-  {
+  if (pairs_first) {
+    k_expand_tu<<<grid_of(n_mo * n_a * n_a), 256, 0, ctx->stream>>>(Rpp, n_mo, n_a, dJ);
+  } else {
     GemmF64Args g;
     g.M = n_mo, g.N = n_a * n_a, g.K = naux;
     g.A = Rpp, g.lda = naux, g.a_kmajor = true;

@@ -6,9 +6,8 @@
 // takes MO_INTS = RI_aa RI_aa^T over the aux index.  With B already fitted:
 //     Y^Q = C1 B^Q C2^T  (n_a x n_a),   MO_INTS[(b n_a + a) n_a^2 + d n_a + c] = sum_Q Y^Q_ab Y^Q_cd
 // (a, c from MO_VEC1; b, d from MO_VEC2, as the reference's RI_aa index order (b, a)).
-// Device work: the FP64 half-transform kernel (C1 as the orbital block), a batched DMMA GEMM
-// (k_gemm.cu) with one product per aux function for Y^Q, one GEMM Z Z^T over Q, and a gather into
-// the reference's order.
+// Device work: the FP64 half-transform kernel (C1 as the orbital block), one DMMA GEMM over the AO index for Y of
+// all aux functions (k_gemm.cu), a gather, and one GEMM Y Y^T over Q, which is the reference's order already.
 // The core J and K come from the ordinary FP64 Fock build with D_core and the first n_c rows of
 // MO_VEC, exactly the reference's tail (src/RI.cpp:235-287).
 #include <vector>
@@ -34,14 +33,13 @@ __global__ void k_rows_from(const double* __restrict__ C, int t, long na, long n
   }
 }
 
-// out[(b na + a) na^2 + d na + c] = G[(a + b p) + (c + d p) * p^2], p = noccp (column-major G)
-__global__ void k_gather_moints(const double* __restrict__ G, long na, long p, double* __restrict__ out) {
-  const long na2 = na * na, p2 = p * p;
-  long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  for (; idx < na2 * na2; idx += static_cast<long>(gridDim.x) * blockDim.x) {
-    long r = idx / na2, c2 = idx % na2;
-    long b = r / na, a = r % na, d = c2 / na, c = c2 % na;
-    out[idx] = G[(a + b * p) + (c + d * p) * p2];
+// Yt[(b na + a)][Q] = R[b][Q p + a]
+__global__ void k_gather_ba(const double* __restrict__ R, long na, long p, long naux, double* __restrict__ Yt) {
+  const long total = na * na * naux;
+  for (long idx = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
+       idx += static_cast<long>(gridDim.x) * blockDim.x) {
+    const long Q = idx % naux, b = idx / naux / na, a = idx / naux % na;
+    Yt[idx] = R[b * naux * p + Q * p + a];
   }
 }
 
@@ -72,12 +70,12 @@ RIJK_API int rijk_mo_ints(rijk_ctx* ctx, const double* DM_D, double* J, double* 
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
   const long n = ctx->n, naux = ctx->nq, npad = ctx->npad, nt = ctx->nt;
-  const long p = round_up(n_a, 16), kdim = naux * p, p2 = p * p;
+  const long p = round_up(n_a, 16), kdim = naux * p, na2 = n_a * n_a;
   const size_t cbytes = static_cast<size_t>(n_a) * n * sizeof(double);
   int rc;
-  DeviceBuf dC1, dC2, R1, R2, XTa, Y, G, out;
+  DeviceBuf dC1, dC2, R1, R2, XTa, Y, Yt, out;
   auto cleanup = [&]() {
-    DeviceBuf* all[] = {&dC1, &dC2, &R1, &R2, &XTa, &Y, &G, &out};
+    DeviceBuf* all[] = {&dC1, &dC2, &R1, &R2, &XTa, &Y, &Yt, &out};
     for (DeviceBuf* b : all) release(*b);
   };
   auto chk = [&](int r) {
@@ -88,8 +86,8 @@ RIJK_API int rijk_mo_ints(rijk_ctx* ctx, const double* DM_D, double* J, double* 
       (rc = chk(ensure_tmp(ctx, R1, p * npad * sizeof(double), "mo_ints rows1"))) ||
       (rc = chk(ensure_tmp(ctx, R2, p * npad * sizeof(double), "mo_ints rows2"))) ||
       (rc = chk(ensure_tmp(ctx, XTa, static_cast<size_t>(npad) * kdim * sizeof(double), "mo_ints XT"))) ||
-      (rc = chk(ensure_tmp(ctx, Y, static_cast<size_t>(naux) * p2 * sizeof(double), "mo_ints Y"))) ||
-      (rc = chk(ensure_tmp(ctx, G, static_cast<size_t>(p2) * p2 * sizeof(double), "mo_ints G"))) ||
+      (rc = chk(ensure_tmp(ctx, Y, static_cast<size_t>(n_a) * kdim * sizeof(double), "mo_ints Y"))) ||
+      (rc = chk(ensure_tmp(ctx, Yt, static_cast<size_t>(na2) * naux * sizeof(double), "mo_ints Y^T"))) ||
       (rc = chk(ensure_tmp(ctx, out, static_cast<size_t>(n_a * n_a) * n_a * n_a * sizeof(double), "mo_ints out"))))
     return rc;
   cudaMemcpyAsync(dC1.p, MO_VEC1, cbytes, cudaMemcpyHostToDevice, s);
@@ -101,24 +99,25 @@ RIJK_API int rijk_mo_ints(rijk_ctx* ctx, const double* DM_D, double* J, double* 
   // X1^Q: XT[nu][Q p + a] = sum_mu B^Q_{nu mu} C1_{a mu}
   launch_xform_f64(static_cast<const double*>(ctx->B.p), static_cast<const double*>(R1.p), naux, nt, p,
                    static_cast<double*>(XTa.p), s);
-  {  // Y^Q[b][a] = sum_nu C2_{b nu} X1^Q_{a nu}  (p x p per aux function)
+  {  // Y[b][Q p + a] = sum_nu C2_{b nu} X1^Q_{a nu}, every Q in one product: a 64 x 64 tile of it holds 64 / p aux
+     // functions, where a product per aux function filled n_a x n_a of a tile
     GemmF64Args g;
-    g.M = p, g.N = p, g.K = npad;
-    g.A = static_cast<const double*>(R2.p), g.lda = npad, g.sA = 0, g.a_kmajor = true;
-    g.B = static_cast<const double*>(XTa.p), g.ldb = kdim, g.sB = p, g.b_kmajor = false;
-    g.C = static_cast<double*>(Y.p), g.ldc = p, g.sC = p2;
-    gemm_f64(g, naux, s);
-  }
-  {  // G[x][y] = sum_Q Y^Q[x] Y^Q[y] over the flattened p^2 entries
-    GemmF64Args g;
-    g.M = p2, g.N = p2, g.K = naux;
-    g.A = static_cast<const double*>(Y.p), g.lda = p2, g.a_kmajor = false;
-    g.B = static_cast<const double*>(Y.p), g.ldb = p2, g.b_kmajor = false;
-    g.C = static_cast<double*>(G.p), g.ldc = p2;
+    g.M = n_a, g.N = kdim, g.K = npad;
+    g.A = static_cast<const double*>(R2.p), g.lda = npad, g.a_kmajor = true;
+    g.B = static_cast<const double*>(XTa.p), g.ldb = kdim, g.b_kmajor = false;
+    g.C = static_cast<double*>(Y.p), g.ldc = kdim;
     gemm_f64(g, 1, s);
   }
-  k_gather_moints<<<grid_of(n_a * n_a * n_a * n_a), 256, 0, s>>>(static_cast<const double*>(G.p), n_a, p,
-                                                                   static_cast<double*>(out.p));
+  k_gather_ba<<<grid_of(na2 * naux), 256, 0, s>>>(static_cast<const double*>(Y.p), n_a, p, naux,
+                                                  static_cast<double*>(Yt.p));
+  {  // out[(b a)][(d c)] = sum_Q Y^Q[b][a] Y^Q[d][c]
+    GemmF64Args g;
+    g.M = na2, g.N = na2, g.K = naux;
+    g.A = static_cast<const double*>(Yt.p), g.lda = naux, g.a_kmajor = true;
+    g.B = static_cast<const double*>(Yt.p), g.ldb = naux, g.b_kmajor = true;
+    g.C = static_cast<double*>(out.p), g.ldc = na2;
+    gemm_f64(g, 1, s);
+  }
   cudaMemcpyAsync(MO_INTS, out.p, static_cast<size_t>(n_a * n_a) * n_a * n_a * sizeof(double), cudaMemcpyDeviceToHost,
                   s);
   if ((rc = chk(cuda_check(ctx, cudaStreamSynchronize(s), "rijk_mo_ints")))) return rc;
