@@ -264,7 +264,11 @@ int syrk_ctas_per_sm() {
 int syrk_nsplit(long nt, long kdim) {
   const long ntile = nt * (nt + 1) / 2;
   const long slots = syrk_ctas_per_sm();
-  const long maxs = std::max<long>(1, kdim / (KC * 8));
+  // at least 8 chunks of k a CTA, but as few as 2 where that leaves SMs idle: the chunks of a CTA are a serial chain
+  // of 1.7 us each (14 CTAs 20 us, 58 CTAs 11 us at n = 48, n_aux = 232)
+  const long chunks = kdim / KC;
+  long maxs = std::max<long>(1, chunks / 8);
+  if (ntile * maxs < 148) maxs = std::max(maxs, std::min(chunks / 2, 148 / ntile));
   const long need = slots * 19 / 10;
   const long smin = std::min(maxs, std::max<long>(1, (need + ntile - 1) / ntile));
   long best = smin;
