@@ -193,44 +193,46 @@ __device__ __forceinline__ uint4 ldg_stream_u4(const void* p) {
 // Element offset of packed element e (tile t = e / 4096) inside one aux function's Bmix block.
 __device__ __forceinline__ long mix_off(long e) { return (e >> 12) * 8192 + (e & 4095); }
 
-constexpr int WM_THREADS = 256;  // 8 warps; each warp reduces one aux function over the chunk at a time
-constexpr int WM_OCT = 1024;     // octets (8 elements) per chunk: two tiles, 32 KB of fp32 Dt in shared memory
-constexpr int WM_QR = 32;        // aux functions per CTA, fewer where that leaves SMs idle (launch_coulomb_w_mixed)
+constexpr int WM_THREADS = 256;  // 8 warps; each warp reduces NQ aux functions over the chunk at a time
+constexpr int WM_OCT = 1024;     // octets (8 elements) per chunk: two tiles, 32 KB of the fp32 density
 
 int coulomb_w_mixed_chunks(long ntile) { return static_cast<int>((ntile * TILE2 / 8 + WM_OCT - 1) / WM_OCT); }
 
-// wpart[c][q] = sum over octet chunk c (blockIdx.x) of Bmix[q][e] Dt[e], q in the qr aux functions
-// of blockIdx.y.  The chunk's Dt is staged once as fp32 in two planes (elements 0-3 and 4-7 of each
-// octet), so a warp's 16-byte reads of it are conflict-free; each warp then streams one aux
-// function's hi/lo planes over the chunk with four octets per lane in flight and reduces by shuffle.
+// wpart[c][q] = sum over octet chunk c (blockIdx.x) of Bmix[q][e] D[e], for the 8 NQ aux functions of blockIdx.y.
+// The density comes as fp32 in two planes (elements 0-3 and 4-7 of each octet) through L1, each octet for NQ aux
+// functions whose hi/lo planes a warp streams beside each other; reduced by shuffle.  No shared memory, so the CTAs
+// find room beside the half-transform, which takes all of it and 12K of the registers.
+template <int NQ>
 __global__ void __launch_bounds__(WM_THREADS) k_coulomb_w_mixed(const __nv_bfloat16* __restrict__ Bmix,
-                                                                 const double* __restrict__ Dt, long naux, long ntile,
-                                                                 long ntile2, int qr, double* __restrict__ wpart) {
-  __shared__ __align__(16) float sd[2][WM_OCT * 4];
+                                                                 const float* __restrict__ Df, long naux, long ntile,
+                                                                 long ntile2, double* __restrict__ wpart) {
   const long n8 = ntile * TILE2 / 8;
   const long c0 = static_cast<long>(blockIdx.x) * WM_OCT;
   const int cnt = static_cast<int>(n8 - c0 < WM_OCT ? n8 - c0 : WM_OCT);
-  const double4* D4 = reinterpret_cast<const double4*>(Dt + c0 * 8);
-  for (int i = threadIdx.x; i < 2 * cnt; i += WM_THREADS) {  // i = 2 * octet + half
-    const double4 d = D4[i];
-    reinterpret_cast<float4*>(sd[i & 1])[i >> 1] =
-        make_float4(static_cast<float>(d.x), static_cast<float>(d.y), static_cast<float>(d.z), static_cast<float>(d.w));
-  }
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long qstride = ntile2 * 2 * TILE2;
-  const long qa = static_cast<long>(blockIdx.y) * qr;
-  const float4* s0 = reinterpret_cast<const float4*>(sd[0]);
-  const float4* s1 = reinterpret_cast<const float4*>(sd[1]);
-  for (int j = warp; j < qr; j += WM_THREADS / 32) {
-    const long q = qa + j;
-    if (q >= naux) break;
-    const __nv_bfloat16* qb = Bmix + q * qstride;
-    double acc = 0.0;  // each octet's 8 products are summed in fp32, the octets in fp64
-    auto dot = [&](const uint4 h, const uint4 l, int o) {
+  const long q0 = (static_cast<long>(blockIdx.y) * (WM_THREADS / 32) + warp) * NQ;
+  if (q0 >= naux) return;
+  const float4* s0 = reinterpret_cast<const float4*>(Df) + c0;
+  const float4* s1 = s0 + n8;
+  const __nv_bfloat16* qb[NQ];
+#pragma unroll
+  for (int u = 0; u < NQ; ++u) qb[u] = Bmix + (q0 + u < naux ? q0 + u : q0) * qstride;
+  double acc[NQ] = {};  // each octet's 8 products are summed in fp32, the octets in fp64
+#pragma unroll 4
+  for (int o = lane; o < cnt; o += 32) {
+    const long off = mix_off((c0 + o) * 8);
+    uint4 h[NQ], l[NQ];
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+      h[u] = ldg_stream_u4(qb[u] + off);
+      l[u] = ldg_stream_u4(qb[u] + off + TILE2);
+    }
+    const float4 d0 = __ldg(s0 + o), d1 = __ldg(s1 + o);
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
       float b[8];
-      bf16x8_sum(h, l, b);
-      const float4 d0 = s0[o], d1 = s1[o];
+      bf16x8_sum(h[u], l[u], b);
       float t = b[0] * d0.x;
       t = fmaf(b[1], d0.y, t);
       t = fmaf(b[2], d0.z, t);
@@ -239,26 +241,13 @@ __global__ void __launch_bounds__(WM_THREADS) k_coulomb_w_mixed(const __nv_bfloa
       t = fmaf(b[5], d1.y, t);
       t = fmaf(b[6], d1.z, t);
       t = fmaf(b[7], d1.w, t);
-      acc += static_cast<double>(t);
-    };
-    int o = lane;
-    for (; o + 96 < cnt; o += 128) {
-      uint4 h[4], l[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const long off = mix_off((c0 + o + 32 * u) * 8);
-        h[u] = ldg_stream_u4(qb + off);
-        l[u] = ldg_stream_u4(qb + off + TILE2);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) dot(h[u], l[u], o + 32 * u);
+      acc[u] += static_cast<double>(t);
     }
-    for (; o < cnt; o += 32) {
-      const long off = mix_off((c0 + o) * 8);
-      dot(ldg_stream_u4(qb + off), ldg_stream_u4(qb + off + TILE2), o);
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) wpart[blockIdx.x * naux + q] = acc;
+  }
+#pragma unroll
+  for (int u = 0; u < NQ; ++u) {
+    const double v = warp_sum(acc[u]);
+    if (lane == 0 && q0 + u < naux) wpart[blockIdx.x * naux + q0 + u] = v;
   }
 }
 
@@ -318,14 +307,16 @@ __global__ void __launch_bounds__(J_THREADS) k_coulomb_j_mixed(const __nv_bfloat
 }
 
 // w needs room for (1 + coulomb_w_mixed_chunks(ntile)) * naux doubles: w, then the chunk partials.
-void launch_coulomb_w_mixed(const __nv_bfloat16* Bmix, const double* Dt, long naux, long ntile, long ntile2, double* w,
+void launch_coulomb_w_mixed(const __nv_bfloat16* Bmix, const float* Df, long naux, long ntile, long ntile2, double* w,
                             cudaStream_t s) {
   const int chunks = coulomb_w_mixed_chunks(ntile);
-  // a warp's aux functions run one after another: one each below four CTAs an SM (40 -> 14 us at n_ao = 72, 54 -> 25 at 144)
-  int qr = WM_QR;
-  while (qr > WM_THREADS / 32 && chunks * ((naux + qr - 1) / qr) < 4 * 148) qr /= 2;
-  dim3 grid(static_cast<unsigned>(chunks), static_cast<unsigned>((naux + qr - 1) / qr));
-  k_coulomb_w_mixed<<<grid, WM_THREADS, 0, s>>>(Bmix, Dt, naux, ntile, ntile2, qr, w + naux);
+  // two aux functions a warp (alone, (H2O)16: 121 us, four of them 145), one below four CTAs an SM (40 -> 14 us at
+  // n_ao = 72, 54 -> 25 at 144)
+  const int per_cta = WM_THREADS / 32;
+  const bool wide = chunks * ((naux + 2 * per_cta - 1) / (2 * per_cta)) >= 4 * 148;
+  const long rows = wide ? 2 * per_cta : per_cta;
+  dim3 grid(static_cast<unsigned>(chunks), static_cast<unsigned>((naux + rows - 1) / rows));
+  (wide ? k_coulomb_w_mixed<2> : k_coulomb_w_mixed<1>)<<<grid, WM_THREADS, 0, s>>>(Bmix, Df, naux, ntile, ntile2, w + naux);
   k_sum_chunks<<<static_cast<unsigned>((naux + 255) / 256), 256, 0, s>>>(w + naux, chunks, naux, w);
 }
 

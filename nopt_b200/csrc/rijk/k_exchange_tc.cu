@@ -894,16 +894,12 @@ static SyrkPlan syrk_plan_waves(long kdim, long tiles, long slots) {
   return {kper, static_cast<int>((kdim + kper - 1) / kper)};
 }
 
-// Whether K's kernel leaves registers on every SM for a J pass beside it: k_syrk_tc does (192 threads), the pair
-// kernel's 320 threads hold all but 12K of them.
-bool mixed_k_leaves_room(long nt) { return round_up(nt, 2) * TILE < 1024; }
-
 // K = sum over orbital batches of X_b^T X_b.  The half-transform holds all orbitals of one batch in
 // the MMA's N dimension (at most 192), so n_c beyond that runs as several batches of equal size; each
 // batch's split-K partials go to their own slots and one reduction sums them all.
-// beside_k is called once, in the build's order right before the (first batch's) K kernel: what it queues on other
-// streams after an event recorded then runs beside K.
-int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK, const std::function<void()>& beside_k) {
+// `beside` is called once, when the (first batch's) half-transform is queued: what it queues on other streams runs beside
+// that kernel, whose CTAs are one an SM and there first, and beside K.
+int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK, const std::function<void()>& beside) {
   int rc = mixed_prepare(ctx);
   if (rc) return rc;
   const long n = ctx->n, naux = ctx->nq;
@@ -962,10 +958,11 @@ int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK, cons
     xp.XTh = XT;
     xp.XTl = XT + npad2 * kdim;
     xp.err = static_cast<int*>(ctx->err.p);
+    if (b0 == 0) cudaEventRecord(ctx->ev_pk, s);
     kXformTable[noccp / 16](mB, mC, xp, ctx->device, s);
     ++launches;
     prof_mark(ctx, "xform_tc");
-    if (b0 == 0) beside_k();
+    if (b0 == 0) beside();
     float* part = Kpart32 + static_cast<size_t>(slot) * ntile2 * TILE2;
     if (pair_syrk) {
       const SyrkPlan pl = syrk_plan(kdim, tiles256, sms / 2);

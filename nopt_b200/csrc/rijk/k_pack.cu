@@ -14,7 +14,7 @@ namespace rijk {
 // Four CTAs a tile, each a 32 x 32 block of it: the transposed elements are read row-wise into shared memory.
 // (One CTA a tile, its transposed reads strided by n, took 5.7 us at n = 48 and 12 us at n = 384; now 3 and 4.)
 __global__ void __launch_bounds__(256) k_pack_density(const double* __restrict__ D, long n, long npad,
-                                                      double* __restrict__ Dt) {
+                                                      double* __restrict__ Dt, float* __restrict__ Df) {
   __shared__ double tr[32][33];
   long I, J;
   tri_decode(blockIdx.x >> 2, I, J);
@@ -32,7 +32,14 @@ __global__ void __launch_bounds__(256) k_pack_density(const double* __restrict__
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < 4; ++k) out[(y + 8 * k) * TILE + x] = I != J ? v[k] + tr[x][y + 8 * k] : v[k];
+  for (int k = 0; k < 4; ++k) {
+    const double d = I != J ? v[k] + tr[x][y + 8 * k] : v[k];
+    out[(y + 8 * k) * TILE + x] = d;
+    if (Df) {  // elements 0-3 and 4-7 of every eight in a plane each
+      const long e = out - Dt + (y + 8 * k) * TILE + x;
+      Df[((e >> 2) & 1) * (gridDim.x / 4 * (TILE2 / 2)) + (e >> 3) * 4 + (e & 3)] = static_cast<float>(d);
+    }
+  }
 }
 
 __global__ void k_pack_mo(const double* __restrict__ MO, long nocc, long n, long noccp, long npad,
@@ -138,9 +145,9 @@ static int grid_for(long total, int threads) {
   return static_cast<int>(b);
 }
 
-void launch_pack_density(const double* D, long n, long npad, long nt, double* Dt, cudaStream_t s) {
+void launch_pack_density(const double* D, long n, long npad, long nt, double* Dt, cudaStream_t s, float* Df) {
   long ntile = nt * (nt + 1) / 2;
-  k_pack_density<<<static_cast<unsigned>(4 * ntile), 256, 0, s>>>(D, n, npad, Dt);
+  k_pack_density<<<static_cast<unsigned>(4 * ntile), 256, 0, s>>>(D, n, npad, Dt, Df);
 }
 
 cudaError_t preload_density_kernels() {

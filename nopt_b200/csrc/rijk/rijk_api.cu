@@ -20,8 +20,7 @@
 namespace rijk {
 
 int mixed_prepare(rijk_ctx* ctx);
-int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK, const std::function<void()>& beside_k);
-bool mixed_k_leaves_room(long nt);
+int mixed_exchange(rijk_ctx* ctx, const double* dMO, long nocc, double* dK, const std::function<void()>& beside);
 
 int set_err(rijk_ctx* ctx, int code, const char* fmt, ...) {
   if (ctx) {
@@ -261,7 +260,7 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   int rc;
   int launches = 0;
   const int nsJ = coulomb_nsplit(tile_elems, naux, precision == RIJK_PREC_MIXED ? 8 : 2);
-  if ((rc = ensure(ctx, ctx->Dt, tile_elems * sizeof(double), "Dt")) ||
+  if ((rc = ensure(ctx, ctx->Dt, tile_elems * (sizeof(double) + sizeof(float)), "Dt")) ||
       (rc = ensure(ctx, ctx->w, (1 + coulomb_w_mixed_chunks(ntile)) * naux * sizeof(double), "w")) ||  // w, partials
       (rc = ensure(ctx, ctx->Jpart, static_cast<size_t>(nsJ) * tile_elems * sizeof(double), "Jpart")))
     return rc;
@@ -298,12 +297,15 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   // pair starts behind it, beside the digits of X and K, three CTAs an SM (C40H82 33.6 ms, the pair first and
   // alone 33.7, one CTA an SM 38; (H2O)16 1.56, 1.59 ms; C25H52 6.5, 7.0 ms).
   const bool late_j = side_j && i8x;
-  // Mixed: the J pass (HBM) beside K (tensor pipe and shared memory) where K's kernel leaves registers for it.
-  // Mixed builds, in turn against beside: 0.53 against 0.49 ms at (H2O)16, 4.26 against 3.94 at C31H64.
-  const bool mixed_side_j = precision == RIJK_PREC_MIXED && nocc > 0 && !ctx->profiling && mixed_k_leaves_room(nt);
+  // Mixed: the Coulomb pair on the high-priority stream beside the exchange, whose kernels leave registers for it
+  // (not the CTA pairs of K from n = 1024 on, but the half-transform before them).
+  // In turn, J beside K only, and the pair beside both: 113, 113 and 100 us at (H2O)3, 530, 490 and 442 at (H2O)16, 4.26,
+  // 4.09 and 3.99 ms at C31H64.
+  const bool mixed_side_j = precision == RIJK_PREC_MIXED && nocc > 0 && !ctx->profiling;
   cudaEventRecord(ctx->ev0, s);
   prof_begin(ctx);
-  launch_pack_density(dD, n, npad, nt, static_cast<double*>(ctx->Dt.p), s);
+  float* Df = reinterpret_cast<float*>(static_cast<double*>(ctx->Dt.p) + tile_elems);
+  launch_pack_density(dD, n, npad, nt, static_cast<double*>(ctx->Dt.p), s, precision == RIJK_PREC_MIXED ? Df : nullptr);
   prof_mark(ctx, "pack_density");
   // The pair's CTAs (one or two an SM): the half-transform's time per byte of B grows with the orbitals,
   // so fewer orbitals leave a shorter window for the same bytes
@@ -323,20 +325,20 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
     if (j_done) cudaEventRecord(j_done, js);
     cudaEventRecord(ctx->ev_jside, js);
   };
+  auto mixed_pair = [&](cudaStream_t js) {
+    const long ntile2 = round_up(nt, 2) * (round_up(nt, 2) + 1) / 2;
+    const __nv_bfloat16* Bm = static_cast<const __nv_bfloat16*>(ctx->Bmix.p);
+    launch_coulomb_w_mixed(Bm, Df, naux, ntile, ntile2, static_cast<double*>(ctx->w.p), js);
+    prof_mark(ctx, "coulomb_w_mixed");
+    launch_coulomb_j_mixed(Bm, static_cast<const double*>(ctx->w.p), naux, ntile, ntile2, nsJ,
+                           static_cast<double*>(ctx->Jpart.p), js);
+    prof_mark(ctx, "coulomb_j_mixed");
+  };
   if (side_j) {
     if (!late_j) run_side_j(side_ctas);
   } else if (precision == RIJK_PREC_MIXED) {
     // mixed form: both passes over the split-BF16 copy (half the bytes of the FP64 passes)
-    const long ntile2 = round_up(nt, 2) * (round_up(nt, 2) + 1) / 2;
-    const __nv_bfloat16* Bm = static_cast<const __nv_bfloat16*>(ctx->Bmix.p);
-    launch_coulomb_w_mixed(Bm, static_cast<const double*>(ctx->Dt.p), naux, ntile, ntile2,
-                           static_cast<double*>(ctx->w.p), s);
-    prof_mark(ctx, "coulomb_w_mixed");
-    if (!mixed_side_j) {
-      launch_coulomb_j_mixed(Bm, static_cast<const double*>(ctx->w.p), naux, ntile, ntile2, nsJ,
-                             static_cast<double*>(ctx->Jpart.p), s);
-      prof_mark(ctx, "coulomb_j_mixed");
-    }
+    if (!mixed_side_j) mixed_pair(s);
   } else {
     launch_coulomb_w(static_cast<const double*>(ctx->B.p), static_cast<const double*>(ctx->Dt.p), naux, tile_elems,
                      static_cast<double*>(ctx->w.p), s);
@@ -359,19 +361,17 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   if (nocc == 0) {
     cudaMemsetAsync(dK, 0, n * n * sizeof(double), s);
   } else if (precision == RIJK_PREC_MIXED) {
-    auto j_beside_k = [&]() {
+    auto beside = [&]() {
       if (!mixed_side_j) return;
       cudaStream_t js = ctx->j_stream;
-      cudaEventRecord(ctx->ev_pk, s);
       cudaStreamWaitEvent(js, ctx->ev_pk, 0);
-      launch_coulomb_j_mixed(static_cast<const __nv_bfloat16*>(ctx->Bmix.p), static_cast<const double*>(ctx->w.p), naux, ntile,
-                             round_up(nt, 2) * (round_up(nt, 2) + 1) / 2, nsJ, static_cast<double*>(ctx->Jpart.p), js);
+      mixed_pair(js);
       launch_unpack_sym(static_cast<double*>(ctx->Jpart.p), nsJ, ntile, n, dJ, js);
       cudaEventRecord(ctx->ev1, js);
       if (j_done) cudaEventRecord(j_done, js);
       cudaEventRecord(ctx->ev_jside, js);
     };
-    rc = mixed_exchange(ctx, dMO, nocc, dK, j_beside_k);
+    rc = mixed_exchange(ctx, dMO, nocc, dK, beside);
     if (mixed_side_j) cudaStreamWaitEvent(s, ctx->ev_jside, 0);  // J joins the build's stream
     if (rc) return rc;
     launches += ctx->stats.kernels_last_fock;

@@ -223,7 +223,8 @@ void gemm_f64(const GemmF64Args& p, long batch, cudaStream_t s);
 // Loads (CUDA loads modules lazily, on a kernel's first use) the density packing and symmetric unpacking
 // kernels on the current device.
 cudaError_t preload_density_kernels();
-void launch_pack_density(const double* D, long n, long npad, long nt, double* Dt, cudaStream_t s);
+// Df: the same in fp32, in two planes of half the elements (mixed builds), or null
+void launch_pack_density(const double* D, long n, long npad, long nt, double* Dt, cudaStream_t s, float* Df = nullptr);
 void launch_pack_mo(const double* MO, long nocc, long n, long noccp, long npad, double* MOp, cudaStream_t s);
 // One warp that sleeps for `cycles` SM clock cycles and exits (a fixed delay on a stream).
 void launch_delay(long long cycles, cudaStream_t s);
@@ -257,7 +258,7 @@ void launch_coulomb_j(const double* B, const double* w, long naux, long tile_ele
                       cudaStream_t s, int max_ctas = 0);
 
 // Mixed form: the same passes over the split-BF16 copy (Bmix[Q][t][hl][64][64], ntile2 tiles per Q).
-void launch_coulomb_w_mixed(const __nv_bfloat16* Bmix, const double* Dt, long naux, long ntile, long ntile2, double* w,
+void launch_coulomb_w_mixed(const __nv_bfloat16* Bmix, const float* Df, long naux, long ntile, long ntile2, double* w,
                             cudaStream_t s);
 void launch_coulomb_j_mixed(const __nv_bfloat16* Bmix, const double* w, long naux, long ntile, long ntile2,
                             int nsplit, double* Jpart, cudaStream_t s);
