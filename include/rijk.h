@@ -204,6 +204,12 @@ int rijk_selftest_wait_timeout(rijk_ctx* ctx, long long cycles);
  * failed call leaves the context usable once allocations succeed again. */
 int rijk_selftest_alloc_failure(rijk_ctx* ctx, long after);
 
+/* The same one step further down: after `after` more requests of this context to the driver for device
+ * memory, the next `times` requests are answered with "out of memory" (times = 0: off).  The library
+ * then does what it does on an exhausted device: it asks again without the memory it can spare, and a
+ * build takes the form that needs less. */
+int rijk_selftest_alloc_refuse(rijk_ctx* ctx, long after, long times);
+
 /* Size of the fixed device scratch used by rijk_coulomb_noalloc (per GPU, held until exit). */
 #define RIJK_NOALLOC_SCRATCH_BYTES (32L * 1024 * 1024)
 

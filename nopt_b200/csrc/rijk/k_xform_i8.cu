@@ -424,23 +424,23 @@ bool bdig_prepare(rijk_ctx* ctx) {
   if (ctx->no_bdig || !encode_tiled()) return false;
   const long nb = (ctx->nt + 1) / 2, nsb = nb * (nb + 1) / 2;
   const size_t bytes = static_cast<size_t>(ctx->nq) * nsb * kSuper;
-  if (ctx->Bdig.bytes < bytes) {
-    size_t free_b = 0, total_b = 0;
-    cudaMemGetInfo(&free_b, &total_b);
-    if (free_b + ctx->Bdig.bytes < bytes + total_b / 24) {
-      ctx->no_bdig = true;
-      return false;
-    }
-  }
   const std::string keep = ctx->last_error;  // running out of room here is no error
-  if (ensure(ctx, ctx->Bdig, bytes, "int8 digits of B") ||
-      ensure(ctx, ctx->Bexp, static_cast<size_t>(ctx->nq) * (sizeof(double) + sizeof(int)), "digit exponents of B") ||
-      ensure(ctx, ctx->Btop, ctx->nq * sizeof(uint32_t), "magnitudes of B")) {
+  auto no_room = [&]() {
     ctx->last_error = keep;
     drop_bdig(ctx);
     ctx->no_bdig = true;
     return false;
+  };
+  // The small buffers first: short of memory, `ensure` gives Bdig's back (drop_bdig) and still succeeds.
+  if (ensure(ctx, ctx->Bexp, static_cast<size_t>(ctx->nq) * (sizeof(double) + sizeof(int)), "digit exponents of B") ||
+      ensure(ctx, ctx->Btop, ctx->nq * sizeof(uint32_t), "magnitudes of B"))
+    return no_room();
+  if (ctx->Bdig.bytes < bytes) {
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    if (free_b + ctx->Bdig.bytes < bytes + total_b / 24) return no_room();
   }
+  if (ensure(ctx, ctx->Bdig, bytes, "int8 digits of B")) return no_room();
   cudaStream_t s = ctx->stream;
   double* scale = static_cast<double*>(ctx->Bexp.p);
   int* ex = reinterpret_cast<int*>(scale + ctx->nq);

@@ -43,6 +43,15 @@ int cuda_check(rijk_ctx* ctx, cudaError_t e, const char* what) {
   return set_err(ctx, RIJK_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+// One request to the driver (rijk_selftest_alloc_refuse answers some of them with "out of memory").
+static cudaError_t device_malloc(rijk_ctx* ctx, void** p, size_t bytes) {
+  if (ctx->refuse_times > 0 && ctx->refuse_after-- <= 0) {
+    --ctx->refuse_times;
+    return cudaErrorMemoryAllocation;
+  }
+  return cudaMalloc(p, bytes);
+}
+
 int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
   if (b.bytes >= bytes && b.p) return RIJK_OK;
   if (bytes > 0 && ctx->fail_alloc_after >= 0) {  // rijk_selftest_alloc_failure
@@ -58,17 +67,17 @@ int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
   b.p = nullptr;
   b.bytes = 0;
   if (bytes == 0) return RIJK_OK;
-  cudaError_t e = cudaMalloc(&b.p, bytes);
+  cudaError_t e = device_malloc(ctx, &b.p, bytes);
   if (e == cudaErrorMemoryAllocation && ctx->pool) {  // once more without what the scratch pool keeps
     cudaGetLastError();
     cudaStreamSynchronize(ctx->stream);
     cudaMemPoolTrimTo(ctx->pool, 0);
-    e = cudaMalloc(&b.p, bytes);
+    e = device_malloc(ctx, &b.p, bytes);
   }
   if (e == cudaErrorMemoryAllocation && ctx->Bdig.p && &b != &ctx->Bdig) {  // ... and without the digits of B
     cudaGetLastError();
     drop_bdig(ctx);
-    e = cudaMalloc(&b.p, bytes);
+    e = device_malloc(ctx, &b.p, bytes);
   }
   if (e != cudaSuccess) {
     b.p = nullptr;

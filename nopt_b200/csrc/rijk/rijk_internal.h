@@ -113,6 +113,7 @@ struct rijk_ctx {
   double* noalloc_scratch = nullptr;  // device address of rijk_coulomb_noalloc's fixed scratch on `device`
   int* host_err = nullptr;     // pinned copy of the device error word
   long fail_alloc_after = -1;  // rijk_selftest_alloc_failure: allocations left before one is refused (-1: off)
+  long refuse_after = 0, refuse_times = 0;  // rijk_selftest_alloc_refuse: requests left before, and to be refused
   // a device build queued by rijk_fock_device, written to the metrics log by the next rijk_sync
   bool log_pending = false;
   long log_nocc = 0;

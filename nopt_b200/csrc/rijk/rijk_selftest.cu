@@ -70,3 +70,11 @@ RIJK_API int rijk_selftest_alloc_failure(rijk_ctx* ctx, long after) {
   ctx->fail_alloc_after = after < 0 ? -1 : after;
   return RIJK_OK;
 }
+
+RIJK_API int rijk_selftest_alloc_refuse(rijk_ctx* ctx, long after, long times) {
+  if (!ctx) return RIJK_ERR_ARG;
+  if (after < 0 || times < 0) return rijk::set_err(ctx, RIJK_ERR_ARG, "rijk_selftest_alloc_refuse: negative count");
+  ctx->refuse_after = after;
+  ctx->refuse_times = times;
+  return RIJK_OK;
+}
