@@ -419,15 +419,20 @@ bool map_digits(CUtensorMap* m, const void* base, uint64_t blocks, uint32_t x, u
 
 }  // namespace
 
+static size_t bdig_bytes(long nq, long nt) {
+  const long nb = (nt + 1) / 2;
+  return static_cast<size_t>(nq) * (nb * (nb + 1) / 2) * kSuper;
+}
+
 bool bdig_prepare(rijk_ctx* ctx) {
   if (ctx->have_bdig) return true;
   if (ctx->no_bdig || !encode_tiled()) return false;
   const long nb = (ctx->nt + 1) / 2, nsb = nb * (nb + 1) / 2;
-  const size_t bytes = static_cast<size_t>(ctx->nq) * nsb * kSuper;
+  const size_t bytes = bdig_bytes(ctx->nq, ctx->nt);
   const std::string keep = ctx->last_error;  // running out of room here is no error
   auto no_room = [&]() {
     ctx->last_error = keep;
-    drop_bdig(ctx);
+    drop_bdig(ctx, true);
     ctx->no_bdig = true;
     return false;
   };
@@ -459,11 +464,16 @@ bool bdig_prepare(rijk_ctx* ctx) {
   return true;
 }
 
-void drop_bdig(rijk_ctx* ctx) {
-  ctx->no_bdig = ctx->no_bdig || ctx->have_bdig;  // (without them it is memory of an earlier tensor)
+void drop_bdig(rijk_ctx* ctx, bool for_good) {
+  ctx->no_bdig = ctx->no_bdig || (for_good && ctx->have_bdig);  // (without them it is memory of an earlier tensor)
   ctx->have_bdig = false;
   cudaStreamSynchronize(ctx->stream);
   release(ctx->Bdig);
+}
+
+void forget_bdig(rijk_ctx* ctx, long nq, long nt) {
+  ctx->have_bdig = ctx->no_bdig = false;
+  if (ctx->Bdig.p && ctx->Bdig.bytes != bdig_bytes(nq, nt)) drop_bdig(ctx, false);
 }
 
 int xform_i8_buffers(rijk_ctx* ctx, long noccp, long parts) {

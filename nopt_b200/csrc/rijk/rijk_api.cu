@@ -43,13 +43,37 @@ int cuda_check(rijk_ctx* ctx, cudaError_t e, const char* what) {
   return set_err(ctx, RIJK_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
-// One request to the driver (rijk_selftest_alloc_refuse answers some of them with "out of memory").
-static cudaError_t device_malloc(rijk_ctx* ctx, void** p, size_t bytes) {
+// One request for device memory (rijk_selftest_alloc_refuse answers some of them with "out of memory").
+static cudaError_t device_malloc(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, bool pooled) {
   if (ctx->refuse_times > 0 && ctx->refuse_after-- <= 0) {
     --ctx->refuse_times;
     return cudaErrorMemoryAllocation;
   }
-  return cudaMalloc(p, bytes);
+  return pooled ? cudaMallocFromPoolAsync(&b.p, bytes, ctx->pool, ctx->stream) : cudaMalloc(&b.p, bytes);
+}
+
+// Memory for the empty buffer b, if need be what the context can spare: the blocks its scratch pool keeps, then the
+// digits of B.  A scratch buffer is free again after its call, so the digits may come back with the next build.
+static int acquire(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what, bool pooled) {
+  cudaError_t e = device_malloc(ctx, b, bytes, pooled);
+  if (e == cudaErrorMemoryAllocation && ctx->pool) {
+    cudaGetLastError();
+    cudaStreamSynchronize(ctx->stream);
+    cudaMemPoolTrimTo(ctx->pool, 0);
+    e = device_malloc(ctx, b, bytes, pooled);
+  }
+  if (e == cudaErrorMemoryAllocation && ctx->Bdig.p && &b != &ctx->Bdig) {
+    cudaGetLastError();
+    drop_bdig(ctx, !pooled);
+    e = device_malloc(ctx, b, bytes, pooled);
+  }
+  if (e != cudaSuccess) {
+    b.p = nullptr;
+    return cuda_check(ctx, e, what);
+  }
+  b.bytes = bytes;
+  b.pool = pooled ? ctx : nullptr;
+  return RIJK_OK;
 }
 
 int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
@@ -67,24 +91,7 @@ int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
   b.p = nullptr;
   b.bytes = 0;
   if (bytes == 0) return RIJK_OK;
-  cudaError_t e = device_malloc(ctx, &b.p, bytes);
-  if (e == cudaErrorMemoryAllocation && ctx->pool) {  // once more without what the scratch pool keeps
-    cudaGetLastError();
-    cudaStreamSynchronize(ctx->stream);
-    cudaMemPoolTrimTo(ctx->pool, 0);
-    e = device_malloc(ctx, &b.p, bytes);
-  }
-  if (e == cudaErrorMemoryAllocation && ctx->Bdig.p && &b != &ctx->Bdig) {  // ... and without the digits of B
-    cudaGetLastError();
-    drop_bdig(ctx);
-    e = device_malloc(ctx, &b.p, bytes);
-  }
-  if (e != cudaSuccess) {
-    b.p = nullptr;
-    return cuda_check(ctx, e, what);
-  }
-  b.bytes = bytes;
-  return RIJK_OK;
+  return acquire(ctx, b, bytes, what, false);
 }
 
 // The largest single scratch buffer is a 2 GiB block of raw integrals (rows_per_chunk), beside a few
@@ -102,14 +109,7 @@ int ensure_tmp(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
   }
   release(b);
   if (bytes == 0) return RIJK_OK;
-  const cudaError_t e = cudaMallocFromPoolAsync(&b.p, bytes, ctx->pool, ctx->stream);
-  if (e != cudaSuccess) {
-    b.p = nullptr;
-    return cuda_check(ctx, e, what);
-  }
-  b.bytes = bytes;
-  b.pool = ctx;
-  return RIJK_OK;
+  return acquire(ctx, b, bytes, what, true);
 }
 
 cudaError_t ensure_smem_limit(const void* fn, size_t bytes) {
@@ -776,8 +776,9 @@ int set_3c_impl(rijk_ctx* ctx, long n, long naux, int layout, const ChunkFill& f
   const long nq = ctx->nq, q0 = ctx->q0;
   int rc;
   ctx->have_b = false;
-  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = false;
+  ctx->have_bmix = false;
   release(ctx->Bmix);
+  forget_bdig(ctx, nq, nt);
   if ((rc = ensure(ctx, ctx->B, static_cast<size_t>(nq) * ntile * TILE2 * sizeof(double), "fitted tensor B")) ||
       (rc = ensure(ctx, ctx->Btop, nq * sizeof(uint32_t), "magnitudes of B")))
     return rc;

@@ -188,8 +188,9 @@ RIJK_API int rijk_load(rijk_ctx* ctx, const char* path) {
   if ((rc = stream_in(ctx, nullptr, bM + bB, static_cast<char*>(st.p), f.f, h))) return rc;
   if (h != hd.checksum) return set_err(ctx, RIJK_ERR_ARG, "rijk_load: checksum mismatch in %s", path);
   if (fseek(f.f, sizeof hd, SEEK_SET) != 0) return set_err(ctx, RIJK_ERR_ARG, "rijk_load: seek failed");
-  ctx->have_metric = ctx->have_b = ctx->have_bmix = ctx->have_btop = ctx->have_bdig = ctx->no_bdig = false;
+  ctx->have_metric = ctx->have_b = ctx->have_bmix = ctx->have_btop = false;
   release(ctx->Bmix);
+  forget_bdig(ctx, hd.nq, hd.nt);
   if ((rc = ensure(ctx, ctx->M, bM, "metric M")) || (rc = ensure(ctx, ctx->B, bB, "fitted tensor B"))) return rc;
   h = 1469598103934665603ull;
   if ((rc = stream_in(ctx, static_cast<char*>(ctx->M.p), bM, static_cast<char*>(st.p), f.f, h))) return rc;

@@ -277,9 +277,12 @@ int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int 
 
 // ---- k_xform_i8.cu: the FP64 half-transform from int8 digits on tcgen05
 // The digits of the present B, made on the first call; false when there is no room for them (the caller
-// then takes the DMMA kernel).  drop_bdig gives their memory back, until B changes.
+// then takes the DMMA kernel).  drop_bdig gives their memory back, for_good: until B changes.  forget_bdig: a new B of nq
+// aux functions and nt tile rows is to come; the memory stays only where the new digits fit it exactly (the next
+// geometry of a molecule).
 bool bdig_prepare(rijk_ctx* ctx);
-void drop_bdig(rijk_ctx* ctx);
+void drop_bdig(rijk_ctx* ctx, bool for_good);
+void forget_bdig(rijk_ctx* ctx, long nq, long nt);
 // Buffers of a build, before anything is queued, and the build's half-transform: XT as launch_xform_f64 writes it,
 // and in ctx->Xtop the largest magnitude of each row over every qper aux functions.
 int xform_i8_buffers(rijk_ctx* ctx, long noccp, long parts);

@@ -54,8 +54,9 @@ RIJK_API int rijk_begin_3c(rijk_ctx* ctx, long n, long naux, int layout) {
   const long nauxp = round_up(naux, KC);
   const long nq = ctx->nq;
   ctx->have_b = false;
-  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = false;
+  ctx->have_bmix = false;
   release(ctx->Bmix);
+  forget_bdig(ctx, nq, nt);
   int rc;
   if ((rc = ensure(ctx, ctx->B, static_cast<size_t>(nq) * ntile * TILE2 * sizeof(double), "fitted tensor B")) ||
       (rc = ensure(ctx, ctx->Btop, nq * sizeof(uint32_t), "magnitudes of B")))

@@ -40,9 +40,9 @@ def _build(fb, system, nocc, precision=rijk.PREC_FP64):
 
 
 def test_more_aux_functions_in_the_memory_of_earlier_digits():
-    """The second tensor's digits fit the memory of the first's, its exponents do not: the request for these is
+    """The second tensor's digits fit the memory of the first's exactly, its exponents do not: the request for these is
     refused until the digits' memory has been given back."""
-    first, second = _system(450, 700, 20), _system(300, 1100, 32)
+    first, second = _system(450, 660, 20), _system(300, 1100, 32)  # 660 x 10 and 1100 x 6 blocks
     with rijk.FockBuilder(0) as fb:
         _set(fb, first, 450)
         assert "xform_i8" in _build(fb, first, 20)
@@ -81,3 +81,54 @@ def test_digits_make_room_for_a_larger_build():
         if k > 0 and "xform_i8" in stages:  # no such request any more
             break
     assert k < 19 and {"xform_i8", "xform_f64"} <= seen
+
+
+CALLS = {
+    "mo_tensor": lambda fb, s: fb.mo_tensor(s[3][:5], s[3][:3]),
+    "mo_calc": lambda fb, s: tuple(fb.mo_calc(s[3][:60], 3, 4, 53).values()),
+    "mo_ints": lambda fb, s: fb.calc_2el_mo_ints_ri(None, s[3], s[3][:4], s[3][:4], 3, 4, want_jk=False)[0],
+    "hess_ints": lambda fb, s: fb.soscf_hess_ints(s[3][:40], 3, 4),
+    "grad": lambda fb, s: fb.grad(s[3], 4, np.eye(300), 0.0, want_3c=True, want_metric=True),
+    "metric": lambda fb, s: fb.set_metric(s[0]),
+    "three_centre": lambda fb, s: fb.set_3c(s[1], 300),
+}
+
+
+@pytest.mark.parametrize("name", list(CALLS))
+def test_scratch_takes_the_memory_of_the_digits(name):
+    """Scratch that is refused twice, the second time with the pool's spare blocks gone, has the digits' memory; refused
+    once, the pool's alone.  The results are those of a call that met no shortage, and the next build forms the
+    digits again."""
+    n, nocc = 300, 32
+    system = _system(n, 1100, nocc)
+    call = CALLS[name]
+    with rijk.FockBuilder(0) as fb:
+        _set(fb, system, n)
+        want = call(fb, system)
+        for times in (1, 2):
+            for after in (0, 3):
+                if name == "metric":
+                    _set(fb, system, n)
+                assert "xform_i8" in _build(fb, system, nocc)
+                fb.selftest_alloc_refuse(after, times)
+                got = call(fb, system)
+                fb.selftest_alloc_refuse(0, 0)
+                if want is not None:
+                    for a, b in zip(np.atleast_1d(want) if not isinstance(want, tuple) else want,
+                                    np.atleast_1d(got) if not isinstance(got, tuple) else got):
+                        assert np.array_equal(a, b)
+        if name == "metric":
+            _set(fb, system, n)
+        assert "xform_i8" in _build(fb, system, nocc)
+
+
+def test_digits_of_an_old_tensor_are_released():
+    import torch
+    system, small = _system(450, 700, 20), _system(70, 60, 5)
+    with rijk.FockBuilder(0) as fb:
+        _set(fb, system, 450)
+        assert "xform_i8" in _build(fb, system, 20)
+        before = torch.cuda.mem_get_info()[0]
+        _set(fb, small, 70)
+        # 700 aux functions x 10 blocks of 128 x 128 elements in 7 bytes each: 0.8 GB
+        assert torch.cuda.mem_get_info()[0] - before > 700 * 10 * 128 * 128 * 7 // 2
