@@ -33,6 +33,7 @@
 #include <cstdint>
 
 #include "i8_digits.cuh"
+#include "i8_rule.h"
 #include "rijk_internal.h"
 
 namespace rijk {
@@ -47,7 +48,6 @@ constexpr int kI8Threads = 192;                // warp 0 copies, warp 1 MMA, war
 constexpr uint32_t kDigitB = 64 * kChunk;      // one digit of a 64-row panel: 2 KB
 constexpr uint32_t kI8Stage = kDigits * (kDigitA + kDigitB);    // 42 KB
 constexpr int kI8Stages = 5;
-constexpr long kMaxPart = 18720;               // k per split part: 7 2^14 18720 < 2^31 - 1, every s32 sum exact
 
 // Digits of X^T.  One CTA per (8 rows, part).  The rows' maxima over the part come with X (known: k_xform_i8
 // leaves them in `tops`), or from a first sweep over it; then the digits are written, a lane per row and 16 k, so that 8
@@ -288,7 +288,7 @@ int sm_count(int device) {
 
 }  // namespace
 
-// Split-K parts of the int8 SYRK: chunk-aligned, at most kMaxPart k each; among up to four times the fewest
+// Split-K parts of the int8 SYRK: chunk-aligned, at most kMaxDigitSum k each; among up to four times the fewest
 // parts (or parts for one wave), the count whose last wave of CTAs, one an SM, is fullest.
 // Parts are whole aux functions (noccp k each) where a part can hold an even number of them, so that
 // k_xform_i8 can keep each part's row maxima.
@@ -297,8 +297,8 @@ int syrk_i8_parts(long nt, long naux, long noccp, int device, long* kper_out) {
   const long nb = (nt + 1) / 2, ctas_per_part = nb * (nb + 1);
   const long sms = sm_count(device);
   const long unit = noccp % kChunk == 0 ? noccp : 2 * noccp;  // aligned to chunks and aux functions
-  const long grain = unit <= kMaxPart ? unit : kChunk;
-  const long max_part = kMaxPart / grain * grain;
+  const long grain = unit <= kMaxDigitSum ? unit : kChunk;
+  const long max_part = kMaxDigitSum / grain * grain;
   const long min_parts = (kdim + max_part - 1) / max_part;
   const long want = std::max(min_parts, sms / ctas_per_part);
   long best = want;

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "gemm_f64.cuh"
+#include "i8_rule.h"
 #include "rijk_internal.h"
 
 #define RIJK_API extern "C" __attribute__((visibility("default")))
@@ -282,14 +283,10 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   int nsK = 1;
   bool i8x = false, i8k = tc;
   if (nocc > 0 && precision != RIJK_PREC_MIXED) {
-    // The int8 tensor cores from about 1e10 FLOPs of exchange and more than 192 functions on (128-row blocks).
-    // Whole FP64 builds, DMMA against int8: 278 against 294 us at n = 192, n_c = 40; 233 against 246 at 232, 20; 580
-    // against 564 at 348, 30; 534 against 449 at 250, 41; 628 against 457 at 240, 50; 2.30 against 1.56 ms at 384, 80;
-    // 80.3 against 33.6 ms at 970, 161.  Without room for the digits of B the half-transform stays on DMMA.
-    const bool large = npad > 192 && 3.0 * npad * npad * kdim >= 1e10;
-    i8k = tc || large;
+    // The int8 tensor cores for large exchanges; without room for the digits of B the half-transform stays on DMMA.
+    i8k = tc || int8_exchange(npad, kdim);
     nsK = i8k ? syrk_i8_parts(nt, naux, noccp, ctx->device, &kper_tc) : syrk_nsplit(nt, kdim);
-    i8x = large && !dmma_x && kper_tc % noccp == 0 && bdig_prepare(ctx);
+    i8x = int8_half_transform(n, npad, kdim, noccp, kper_tc) && !dmma_x && bdig_prepare(ctx);
     if (i8x && (rc = xform_i8_buffers(ctx, noccp, nsK))) return rc;
     if ((rc = ensure(ctx, ctx->MOp, noccp * npad * sizeof(double), "MOp")) ||
         (rc = ensure(ctx, ctx->XT, static_cast<size_t>(npad) * kdim * sizeof(double), "XT")) ||
