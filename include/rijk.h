@@ -64,9 +64,14 @@ extern "C" {
 #define RIJK_PREC_FP64 0  /* FP64 throughout: the drop-in form.  Large exchanges (from about 1e10 FLOPs
                              on) run on tcgen05 tensor cores: operands as seven int8 digits with
                              power-of-two scales, 34 exact s32 digit products, FP64 scaling and sums
-                             (the Ozaki splitting scheme), with smaller errors than FP64 FMAs; the
-                             half-transform so only while the digits of B (0.9 to 1.1 times its
-                             bytes) find room in device memory                                  */
+                             (the Ozaki splitting scheme); the half-transform so only while the
+                             digits of B (0.9 to 1.1 times its bytes) find room in device memory.
+                             The digits are fixed-point numbers, scaled so that multiplying a basis
+                             function by a power of two does not matter: the error of K_mn is below
+                             that of FP64 FMAs against sqrt(K_mm K_nn) (4e-16 and 1.4e-15 at the
+                             most for C12H26 cc-pVDZ), but not against each K_mn of its own.  Elements
+                             far below that size, of functions far apart, keep fewer digits of their
+                             own than FMAs leave them: 1.2e-13 in the median there, against 1.5e-15 */
 #define RIJK_PREC_MIXED 1 /* exchange half-transform and K on tcgen05 tensor cores with split-BF16
                              (3-term) operands and FP32 accumulation; Coulomb in FP64          */
 #define RIJK_PREC_FP64_TC 2 /* RIJK_PREC_FP64 with K = X^T X from int8 digits at every size       */

@@ -111,10 +111,11 @@ __global__ void __launch_bounds__(K1_THREADS)
   }
 
   const int g = lane >> 2, tq = lane & 3;
+  uint32_t m[4][2] = {};  // of this thread's 8 columns
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     long q = q0 + wm * 32 + i * 8 + g;
-    uint32_t m = 0;
+    uint32_t mq = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
 #pragma unroll
@@ -124,14 +125,24 @@ __global__ void __launch_bounds__(K1_THREADS)
         if (q < naux && dst[c] >= 0) {
           B[q * tile_elems + dst[c]] = x;
           if (mirror[c] >= 0) B[q * tile_elems + mirror[c]] = x;
+          m[j][e] = max(m[j][e], magnitude(x));
+          mq = max(mq, magnitude(x));
         }
-        m = max(m, magnitude(x));
       }
     }
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
-    if (tq == 0 && q < naux) atomicMax(top + q, m);
+    mq = max(mq, __shfl_xor_sync(0xffffffffu, mq, 1));
+    mq = max(mq, __shfl_xor_sync(0xffffffffu, mq, 2));
+    if (tq == 0 && q < naux) atomicMax(top + tile_elems + q, mq);
   }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) m[j][e] = max(m[j][e], __shfl_xor_sync(0xffffffffu, m[j][e], o));
+      const long d = dst[wn * 32 + j * 8 + 2 * tq + e];
+      if (g == 0 && d >= 0) atomicMax(top + d, m[j][e]);
+    }
 }
 
 // I3 holds the tile rows I in [I0, I1): full layout rows (mu - I0*64)*n + nu, packed layout

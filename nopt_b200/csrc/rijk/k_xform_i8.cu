@@ -7,9 +7,18 @@
 // one rectangular copy of 28 KB into the unswizzled canonical layouts:
 //   rows as M   32 columns = 2 column groups of 2 KB             K-major:  SBO 128 (rows), LBO 2048 (columns)
 //   columns as M  32 rows = 4 row groups of each column group     MN-major: SBO 512 (columns), LBO 128 (rows)
-// so the stored lower triangle serves the full symmetric matrix, as in the other half-transforms.  One exponent
-// per Q (a block is read both ways) leaves every element an absolute rounding of 2^-55 of the largest of
-// B^Q; in K these add at random over Q and i.
+// so the stored lower triangle serves the full symmetric matrix, as in the other half-transforms.
+//
+// Row scales.  One exponent per Q (a block is read both ways) leaves every element an absolute rounding of 2^-55 of the
+// largest of B^Q.  So that this means as much to every function, whatever the sizes of the functions, the digits are
+// those of 2^-(e_mu + e_nu) B^Q_{mu nu}, with e_mu such that every row's largest element over all Q is about 1
+// (k_balance, from the magnitudes the metric contraction keeps).  The factors are exact: those of the summed index go into
+// the digits of C, those of the row nu into X.  The rounding of K_{mu nu} against sqrt(K_mu,mu K_nu,nu) is then the same for
+// any scaling of the functions (C12H26, emulated: 3.8e-16 at the most, 1.4e-15 with FP64 FMAs; without the scales
+// 3.7e-10 when the functions' sizes spread over 2^12).  An element far below that, of functions far apart, keeps fewer
+// digits of its own than FP64 FMAs would leave it (1.2e-13 in the median there, against 1.5e-15).
+// Where the rows' largest elements lie within a factor of 16, e = 0 serves as well (6.4e-16 at that factor; of
+// normalised functions in double- and triple-zeta bases they lie within 4 to 10) and saves a pass over B.
 //
 // k_xform_i8: persistent, one CTA per SM, over items (Q, 128 rows nu, batch of at most 64 orbitals), the batches of
 // one (Q, rows) next to each other so that the later ones find B's digits in L2.  Warp 0 copies stages of
@@ -46,13 +55,105 @@ constexpr int kOutLd = 18;  // doubles a row of the epilogue's transposing buffe
 constexpr size_t kXSmem = static_cast<size_t>(kXStages) * kXStage + 8 * 32 * kOutLd * sizeof(double) + 1024 + 256;
 
 // ------------------------------------------------------------------ digits of B ----
-// top[Q] = the largest magnitude of B^Q
-__global__ void __launch_bounds__(256) k_bmax(const double* __restrict__ B, long tile_elems, uint32_t* top) {
-  const double2* b = reinterpret_cast<const double2*>(B + blockIdx.y * tile_elems);
+// top[e] = the largest magnitude over Q of element e, for a tensor that no metric contraction has left it for.
+__global__ void __launch_bounds__(256) k_element_max(const double* __restrict__ B, long nq, long tile_elems, uint32_t* top) {
+  const long e = static_cast<long>(blockIdx.x) * 256 + threadIdx.x;  // a double2; tile_elems / 2 is a multiple of 256
+  const double2* b = reinterpret_cast<const double2*>(B) + e;
+  uint32_t mx = 0, my = 0;
+#pragma unroll 4
+  for (long q = blockIdx.y; q < nq; q += gridDim.y) {
+    const double2 v = ldg_stream(b + q * (tile_elems / 2));
+    mx = max(mx, magnitude(v.x));
+    my = max(my, magnitude(v.y));
+  }
+  atomicMax(top + 2 * e, mx);
+  atomicMax(top + 2 * e + 1, my);
+}
+
+// log2 of a magnitude; nothing to balance where it is zero or not finite
+__device__ __forceinline__ float log2_magnitude(uint32_t top) {
+  if (top == 0 || top >= 0x7ff00000u) return -INFINITY;
+  return static_cast<float>(static_cast<int>(top >> 20) - 1023) + __log2f(__uint_as_float(0x3f800000u | ((top & 0xfffffu) << 3)));
+}
+
+// Whether e = 0 will do (kPlain), from the first step's logarithms: half those of the rows' largest elements.  The
+// aux functions' own maxima are then those of the metric contraction, if it has left any.
+enum { kPlain = 0, kScaled = 1, kPlainNoTops = 2 };
+__global__ void __launch_bounds__(256) k_spread(const float* __restrict__ e, long n, int have_tops, int* __restrict__ how) {
+  __shared__ float lo[8], hi[8];
+  float a = INFINITY, b = -INFINITY;
+  for (long i = threadIdx.x; i < n; i += 256) {
+    a = fminf(a, e[i]);
+    b = fmaxf(b, e[i]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
+    b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    lo[threadIdx.x >> 5] = a;
+    hi[threadIdx.x >> 5] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      a = fminf(a, lo[w]);
+      b = fmaxf(b, hi[w]);
+    }
+    *how = b - a > 2.0f ? kScaled : have_tops ? kPlain : kPlainNoTops;
+  }
+}
+
+// One step towards row scales: e_mu grows by half the logarithm of its row's largest scaled element, so that a pair
+// of rows meets in the middle (Ruiz's scaling; it converges by halving, in one step where diagonals lead).  A warp a row.
+__global__ void __launch_bounds__(256) k_balance(const uint32_t* __restrict__ top, long n, const int* how,
+                                                 const float* __restrict__ e0, float* __restrict__ e1) {
+  if (how && *how != kScaled) return;
+  const long mu = static_cast<long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (mu >= n) return;
+  const long I = mu / TILE, r = mu % TILE;
+  float m = -INFINITY;
+  for (long nu = threadIdx.x & 31; nu < n; nu += 32) {
+    const long J = nu / TILE, c = nu % TILE;
+    uint32_t t = top[I >= J ? tri_index(I, J) * TILE2 + r * TILE + c : tri_index(J, I) * TILE2 + c * TILE + r];
+    if (I == J) t = max(t, top[tri_index(I, I) * TILE2 + c * TILE + r]);
+    m = fmaxf(m, log2_magnitude(t) - e0[nu]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) e1[mu] = m == -INFINITY ? e0[mu] : 0.5f * (e0[mu] + m);
+}
+constexpr int kBalanceSteps = 8;  // even: the result is where the first step read
+
+// The scales as powers of two, down = 2^-e for B and up = 2^e for C and X.
+__global__ void k_balance_scales(const float* __restrict__ e, long n, long npad2, const int* how,
+                                 double* __restrict__ down, double* __restrict__ up) {
+  const long mu = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (mu >= npad2) return;
+  const int x = mu < n && *how == kScaled ? static_cast<int>(rintf(fminf(fmaxf(e[mu], -600.f), 600.f))) : 0;
+  down[mu] = pow2i(-x);
+  up[mu] = pow2i(x);
+}
+
+// top[Q] = the largest magnitude of the scaled B^Q
+__global__ void __launch_bounds__(256) k_bmax(const double* __restrict__ B, long ntile, const int* how,
+                                              const double* __restrict__ down, uint32_t* top) {
+  if (*how == kPlain) return;
   uint32_t m = 0;
-  for (long e = static_cast<long>(blockIdx.x) * 256 + threadIdx.x; e < tile_elems / 2; e += static_cast<long>(gridDim.x) * 256) {
-    const double2 v = ldg_stream(b + e);
-    m = max(m, max(magnitude(v.x), magnitude(v.y)));
+  for (long t = blockIdx.x; t < ntile; t += gridDim.x) {
+    long I, J;
+    tri_decode(t, I, J);
+    const double2* b = reinterpret_cast<const double2*>(B + (blockIdx.y * ntile + t) * TILE2);
+    const int c = 2 * (threadIdx.x & 31);
+    const double2 dc = __ldg(reinterpret_cast<const double2*>(down + J * TILE + c));
+#pragma unroll
+    for (int k = 0; k < TILE / 8; ++k) {
+      const int r = (threadIdx.x >> 5) + 8 * k;
+      const double dr = __ldg(down + I * TILE + r);
+      const double2 v = ldg_stream(b + (r * TILE + c) / 2);
+      m = max(m, max(magnitude(v.x * dr * dc.x), magnitude(v.y * dr * dc.y)));
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -60,7 +161,9 @@ __global__ void __launch_bounds__(256) k_bmax(const double* __restrict__ B, long
 }
 
 // Their exponents, and the scales that go with the digits.
-__global__ void k_exponents(const uint32_t* __restrict__ top, long count, int* __restrict__ ex, double* __restrict__ scale) {
+__global__ void k_exponents(const uint32_t* __restrict__ plain, const uint32_t* __restrict__ scaled, const int* how,
+                            long count, int* __restrict__ ex, double* __restrict__ scale) {
+  const uint32_t* top = *how == kPlain ? plain : scaled;
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
     ex[i] = value_exponent(top[i]);
@@ -71,7 +174,8 @@ __global__ void k_exponents(const uint32_t* __restrict__ top, long count, int* _
 // One CTA per (128 x 128 block, Q): a lane per row and 16 columns, consecutive lanes on consecutive rows, so a
 // warp writes 512 contiguous bytes of each digit.
 __global__ void __launch_bounds__(256) k_slice_b(const double* __restrict__ B, long nt, long tile_elems, long nsb,
-                                                 const int* __restrict__ ex, uint8_t* __restrict__ out) {
+                                                 const int* __restrict__ ex, const double* __restrict__ down,
+                                                 uint8_t* __restrict__ out) {
   long a, b;
   tri_decode(blockIdx.x, a, b);
   const long Q = blockIdx.y;
@@ -79,6 +183,7 @@ __global__ void __launch_bounds__(256) k_slice_b(const double* __restrict__ B, l
   const double* BQ = B + Q * tile_elems;
   uint8_t* img = out + (Q * nsb + blockIdx.x) * kSuper;
   const int r = threadIdx.x & 127;
+  const double dr = down[a * 128 + r];
   for (int cg = threadIdx.x >> 7; cg < 8; cg += 2) {
     const long I = 2 * a + (r >> 6), J = 2 * b + (cg >> 2);
     double v[16];
@@ -98,6 +203,13 @@ __global__ void __launch_bounds__(256) k_slice_b(const double* __restrict__ B, l
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = src[j * TILE];
     }
+    const double2* dc = reinterpret_cast<const double2*>(down + b * 128 + cg * 16);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double2 f = __ldg(dc + j);
+      v[2 * j] = v[2 * j] * dr * f.x;
+      v[2 * j + 1] = v[2 * j + 1] * dr * f.y;
+    }
     uint4 d[kDigits];
     digits16(v, e, d);
     uint8_t* p = img + cg * 2048 + r * 16;  // 8-row groups of 128 B
@@ -114,14 +226,15 @@ struct Batches {
   __host__ __device__ int rows(int b) const { return 16 * (base + (b < extra ? 1 : 0)); }
 };
 
-// One CTA per 16 orbital rows: their maxima over the n columns, then digits, [chunk][digit][8-row group][2][8][16].
+// One CTA per 16 orbital rows: their maxima over the n scaled columns, then digits, [chunk][digit][8-row group][2][8][16].
 __global__ void __launch_bounds__(128) k_slice_c(const double* __restrict__ MOp, long n, long npad, long nk, Batches bt,
-                                                 double* __restrict__ scale, uint8_t* __restrict__ out) {
+                                                 const double* __restrict__ up, double* __restrict__ scale,
+                                                 uint8_t* __restrict__ out) {
   __shared__ uint32_t top[16];
   const int i0 = blockIdx.x * 16, t = threadIdx.x, lane = t & 31, warp = t >> 5;
   for (int r = warp; r < 16; r += 4) {
     uint32_t m = 0;
-    for (long k = lane; k < n; k += 32) m = max(m, magnitude(MOp[(i0 + r) * npad + k]));
+    for (long k = lane; k < n; k += 32) m = max(m, magnitude(MOp[(i0 + r) * npad + k] * up[k]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (lane == 0) top[r] = m;
@@ -138,7 +251,7 @@ __global__ void __launch_bounds__(128) k_slice_c(const double* __restrict__ MOp,
   for (long g = t >> 4; g < 2 * nk; g += 8) {  // 16 columns; the rows are zero from n to npad
     double v[16];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = MOp[(i0 + r) * npad + g * 16 + j];
+    for (int j = 0; j < 16; ++j) v[j] = MOp[(i0 + r) * npad + g * 16 + j] * up[g * 16 + j];
     uint4 d[kDigits];
     digits16(v, e, d);
     const long row = row0 + r;
@@ -153,6 +266,7 @@ struct XformI8Params {
   const uint8_t* C;
   const double* scaleB;
   const double* scaleC;
+  const double* up;          // row scales of B's digits
   double* XT;
   uint32_t* tops;            // [part][npad2]
   long qper;                 // aux functions of a part
@@ -346,7 +460,7 @@ __global__ void __launch_bounds__(kXThreads, 1)
       const long nu0 = static_cast<long>(M) * 128 + q * 32;
       const int i0 = p.bt.first(b) + half * units * 8;
       if (nu0 >= p.npad) continue;  // npad is a multiple of 64: the whole warp
-      const double sb = p.scaleB[Q] * kJoined;
+      const double sb = p.scaleB[Q] * kJoined * p.up[nu0 + lane];
       double* out = p.XT + (nu0 + (lane >> 3)) * p.kdim + static_cast<long>(Q) * p.noccp + i0 + 2 * (lane & 7);
       const long step = 4 * p.kdim;
       const double2* sc = reinterpret_cast<const double2*>(p.scaleC + i0);
@@ -419,6 +533,30 @@ bool map_digits(CUtensorMap* m, const void* base, uint64_t blocks, uint32_t x, u
 
 }  // namespace
 
+// What Bexp holds.
+struct BScales {
+  double *scale, *down, *up;  // of the aux functions (value_scale), of the orbital functions
+  int* ex;                    // exponents of the aux functions
+  uint32_t* top;
+  int* how;                   // kPlain, kScaled, kPlainNoTops
+  float *e0, *e1;             // the balancing's logarithms
+};
+static size_t scales_bytes(long nq, long npad2) {
+  return (round_up(nq, 2) + 2 * npad2) * sizeof(double) + (2 * nq + 1 + 2 * npad2) * sizeof(int);
+}
+static BScales scales_of(void* p, long nq, long npad2) {
+  BScales s{};
+  s.scale = static_cast<double*>(p);
+  s.down = s.scale + round_up(nq, 2);  // read 16 bytes at a time
+  s.up = s.down + npad2;
+  s.ex = reinterpret_cast<int*>(s.up + npad2);
+  s.top = reinterpret_cast<uint32_t*>(s.ex + nq);
+  s.how = reinterpret_cast<int*>(s.top + nq);
+  s.e0 = reinterpret_cast<float*>(s.how + 1);
+  s.e1 = s.e0 + npad2;
+  return s;
+}
+
 static size_t bdig_bytes(long nq, long nt) {
   const long nb = (nt + 1) / 2;
   return static_cast<size_t>(nq) * (nb * (nb + 1) / 2) * kSuper;
@@ -436,9 +574,10 @@ bool bdig_prepare(rijk_ctx* ctx) {
     ctx->no_bdig = true;
     return false;
   };
+  const long te = ctx->ntile * TILE2, npad2 = nb * 128;
   // The small buffers first: short of memory, `ensure` gives Bdig's back (drop_bdig) and still succeeds.
-  if (ensure(ctx, ctx->Bexp, static_cast<size_t>(ctx->nq) * (sizeof(double) + sizeof(int)), "digit exponents of B") ||
-      ensure(ctx, ctx->Btop, ctx->nq * sizeof(uint32_t), "magnitudes of B"))
+  if (ensure(ctx, ctx->Bexp, scales_bytes(ctx->nq, npad2), "digit scales of B") ||
+      ensure(ctx, ctx->Btop, (te + ctx->nq) * sizeof(uint32_t), "magnitudes of B"))
     return no_room();
   if (ctx->Bdig.bytes < bytes) {
     size_t free_b = 0, total_b = 0;
@@ -447,19 +586,27 @@ bool bdig_prepare(rijk_ctx* ctx) {
   }
   if (ensure(ctx, ctx->Bdig, bytes, "int8 digits of B")) return no_room();
   cudaStream_t s = ctx->stream;
-  double* scale = static_cast<double*>(ctx->Bexp.p);
-  int* ex = reinterpret_cast<int*>(scale + ctx->nq);
+  const BScales sc = scales_of(ctx->Bexp.p, ctx->nq, npad2);
   uint32_t* top = static_cast<uint32_t*>(ctx->Btop.p);
-  const long te = ctx->ntile * TILE2;
   const double* B = static_cast<const double*>(ctx->B.p);
   const unsigned q = static_cast<unsigned>(ctx->nq);
   if (!ctx->have_btop) {  // a tensor read from a file
-    cudaMemsetAsync(top, 0, ctx->nq * sizeof(uint32_t), s);
-    k_bmax<<<dim3(static_cast<unsigned>(std::min<long>((te / 2 + 1023) / 1024, 64)), q), 256, 0, s>>>(B, te, top);
-    ctx->have_btop = true;
+    cudaMemsetAsync(top, 0, te * sizeof(uint32_t), s);
+    k_element_max<<<dim3(static_cast<unsigned>(te / 512), static_cast<unsigned>(std::min<long>(ctx->nq, 16))), 256, 0, s>>>(
+        B, ctx->nq, te, top);
   }
-  k_exponents<<<static_cast<unsigned>((ctx->nq + 255) / 256), 256, 0, s>>>(top, ctx->nq, ex, scale);
-  k_slice_b<<<dim3(static_cast<unsigned>(nsb), q), 256, 0, s>>>(B, ctx->nt, te, nsb, ex, static_cast<uint8_t*>(ctx->Bdig.p));
+  const unsigned rows = static_cast<unsigned>((ctx->n + 7) / 8);
+  cudaMemsetAsync(sc.e0, 0, ctx->n * sizeof(float), s);
+  k_balance<<<rows, 256, 0, s>>>(top, ctx->n, nullptr, sc.e0, sc.e1);
+  k_spread<<<1, 256, 0, s>>>(sc.e1, ctx->n, ctx->have_btop, sc.how);
+  for (int i = 1; i < kBalanceSteps; ++i)
+    k_balance<<<rows, 256, 0, s>>>(top, ctx->n, sc.how, i & 1 ? sc.e1 : sc.e0, i & 1 ? sc.e0 : sc.e1);
+  k_balance_scales<<<static_cast<unsigned>(nb), 128, 0, s>>>(sc.e0, ctx->n, npad2, sc.how, sc.down, sc.up);
+  cudaMemsetAsync(sc.top, 0, ctx->nq * sizeof(uint32_t), s);
+  k_bmax<<<dim3(static_cast<unsigned>(std::min<long>(ctx->ntile, 8)), q), 256, 0, s>>>(B, ctx->ntile, sc.how, sc.down, sc.top);
+  k_exponents<<<static_cast<unsigned>((ctx->nq + 255) / 256), 256, 0, s>>>(top + te, sc.top, sc.how, ctx->nq, sc.ex, sc.scale);
+  k_slice_b<<<dim3(static_cast<unsigned>(nsb), q), 256, 0, s>>>(B, ctx->nt, te, nsb, sc.ex, sc.down,
+                                                                 static_cast<uint8_t*>(ctx->Bdig.p));
   ctx->have_bdig = true;
   return true;
 }
@@ -494,15 +641,17 @@ int xform_i8(rijk_ctx* ctx, const double* MOp, long noccp, double* XT, long qper
   uint8_t* C = reinterpret_cast<uint8_t*>(scaleC + noccp);
   uint32_t* tops = static_cast<uint32_t*>(ctx->Xtop.p);
   cudaMemsetAsync(tops, 0, static_cast<size_t>(parts) * nb * 128 * sizeof(uint32_t), s);
-  k_slice_c<<<static_cast<unsigned>(units), 128, 0, s>>>(MOp, ctx->n, ctx->npad, nk, bt, scaleC, C);
+  const BScales sc = scales_of(ctx->Bexp.p, ctx->nq, nb * 128);
+  k_slice_c<<<static_cast<unsigned>(units), 128, 0, s>>>(MOp, ctx->n, ctx->npad, nk, bt, sc.up, scaleC, C);
   CUtensorMap rows, cols;
   const uint64_t blocks = static_cast<uint64_t>(ctx->nq) * nsb;
   if (!map_digits(&rows, ctx->Bdig.p, blocks, 256, 2) || !map_digits(&cols, ctx->Bdig.p, blocks, 64, 8))
     return set_err(ctx, RIJK_ERR_CUDA, "tensor map encoding failed (digits of B)");
   XformI8Params p{};
   p.C = C;
-  p.scaleB = static_cast<const double*>(ctx->Bexp.p);
+  p.scaleB = sc.scale;
   p.scaleC = scaleC;
+  p.up = sc.up;
   p.XT = XT;
   p.tops = tops;
   p.qper = qper;

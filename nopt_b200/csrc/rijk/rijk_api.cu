@@ -777,9 +777,9 @@ int set_3c_impl(rijk_ctx* ctx, long n, long naux, int layout, const ChunkFill& f
   release(ctx->Bmix);
   forget_bdig(ctx, nq, nt);
   if ((rc = ensure(ctx, ctx->B, static_cast<size_t>(nq) * ntile * TILE2 * sizeof(double), "fitted tensor B")) ||
-      (rc = ensure(ctx, ctx->Btop, nq * sizeof(uint32_t), "magnitudes of B")))
+      (rc = ensure(ctx, ctx->Btop, (ntile * TILE2 + nq) * sizeof(uint32_t), "magnitudes of B")))
     return rc;
-  cudaMemsetAsync(ctx->Btop.p, 0, nq * sizeof(uint32_t), s);
+  cudaMemsetAsync(ctx->Btop.p, 0, (ntile * TILE2 + nq) * sizeof(uint32_t), s);
   // Raw integrals come in blocks of whole tile rows, at most ~2 GiB each.
   const long rows_per = rows_per_chunk(n, nauxp, layout);
   auto pairs_of = [&](long I0, long I1, long& first, long& count) {

@@ -100,8 +100,8 @@ struct rijk_ctx {
   rijk::DeviceBuf scratch;  // misc small
   rijk::DeviceBuf eri_tab;  // integral tables (Boys grid, harmonics, aux term lists)
   rijk::DeviceBuf Bdig;     // int8 digits of B for the FP64 half-transform on tcgen05 (k_xform_i8.cu), when there is room
-  rijk::DeviceBuf Bexp;     // the scales and the exponents of every B^Q's digits
-  rijk::DeviceBuf Btop;     // leading words of the largest magnitude of every B^Q, kept by the metric contraction
+  rijk::DeviceBuf Bexp;     // the scales of its digits: of every B^Q, and of the orbital functions
+  rijk::DeviceBuf Btop;     // leading words of the largest magnitudes of B's elements over Q, and of every B^Q (the metric contraction's)
   bool have_btop = false;
   bool have_bdig = false;   // Bdig holds the digits of the present B
   bool no_bdig = false;     // there was no room for them with the present B
@@ -237,7 +237,9 @@ void launch_scan_nonfinite(const double* x, long count, int* err, cudaStream_t s
 
 // ---- k_metric.cu
 // B[Q][tile-packed e] = sum_P M[Q][P] * I3(pair(e), P) for the raw rows of tile rows [I0, I1).
-// top[Q] is raised to the leading word of the largest |B[Q]| written (see magnitude in i8_digits.cuh).
+// top[e] is raised to the leading word of the largest magnitude over Q of the tile set's element e (see magnitude in
+// i8_digits.cuh; where a column is written twice, in a diagonal tile, only at (mu, nu), mu >= nu), and
+// top[tile elements + Q] to that of the largest of B[Q].
 // M may start at a row offset q0 (mrows = rows left after it); B receives naux rows.  tri >= 0 declares
 // M lower triangular with its first row at global row tri (the Cholesky form): the contraction then
 // stops at each row block's last nonzero column, half the products, the same result.

@@ -59,9 +59,9 @@ RIJK_API int rijk_begin_3c(rijk_ctx* ctx, long n, long naux, int layout) {
   forget_bdig(ctx, nq, nt);
   int rc;
   if ((rc = ensure(ctx, ctx->B, static_cast<size_t>(nq) * ntile * TILE2 * sizeof(double), "fitted tensor B")) ||
-      (rc = ensure(ctx, ctx->Btop, nq * sizeof(uint32_t), "magnitudes of B")))
+      (rc = ensure(ctx, ctx->Btop, (ntile * TILE2 + nq) * sizeof(uint32_t), "magnitudes of B")))
     return fail(ctx, rc);
-  cudaMemsetAsync(ctx->Btop.p, 0, nq * sizeof(uint32_t), s);
+  cudaMemsetAsync(ctx->Btop.p, 0, (ntile * TILE2 + nq) * sizeof(uint32_t), s);
   const long rows_per = rows_per_chunk(n, nauxp, layout);
   long maxcount = 0;
   for (long I0 = 0; I0 < nt; I0 += rows_per) {
