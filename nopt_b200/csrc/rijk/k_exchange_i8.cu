@@ -316,16 +316,17 @@ int syrk_i8_parts(long nt, long naux, long noccp, int device, long* kper_out) {
   return static_cast<int>((kdim + kper - 1) / kper);
 }
 
+int syrk_i8_buffers(rijk_ctx* ctx, long npad, long kdim, int nparts) {
+  const long npad2 = round_up(npad, 128), nblk = (kdim + kChunk - 1) / kChunk;
+  const int rc = ensure(ctx, ctx->Xs, static_cast<size_t>(npad2 / 128) * nblk * kBlockBytes, "int8 digits of X");
+  return rc ? rc : ensure(ctx, ctx->Xe, static_cast<size_t>(nparts) * npad2 * sizeof(int), "digit exponents");
+}
+
 // K partials of the FP64 form from X^T (npad x kdim doubles) through its digits.
 // tops: the rows' largest magnitudes in every part (k_xform_i8), or null.
 int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int nparts, long kper,
             const uint32_t* tops, double* Kpart, cudaStream_t s) {
   const long npad2 = round_up(npad, 128);
-  const long nblk = (kdim + kChunk - 1) / kChunk;
-  int rc;
-  if ((rc = ensure(ctx, ctx->Xs, static_cast<size_t>(npad2 / 128) * nblk * kBlockBytes, "int8 digits of X")) ||
-      (rc = ensure(ctx, ctx->Xe, static_cast<size_t>(nparts) * npad2 * sizeof(int), "digit exponents")))
-    return rc;
   uint8_t* Xs = static_cast<uint8_t*>(ctx->Xs.p);
   int* E = static_cast<int*>(ctx->Xe.p);
   const dim3 sgrid(static_cast<unsigned>(npad2 / 8), static_cast<unsigned>(nparts));

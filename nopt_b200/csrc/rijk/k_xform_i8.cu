@@ -619,7 +619,7 @@ void drop_bdig(rijk_ctx* ctx, bool for_good) {
 }
 
 void forget_bdig(rijk_ctx* ctx, long nq, long nt) {
-  ctx->have_bdig = ctx->no_bdig = false;
+  ctx->have_bdig = ctx->no_bdig = ctx->no_i8k = false;
   if (ctx->Bdig.p && ctx->Bdig.bytes != bdig_bytes(nq, nt)) drop_bdig(ctx, false);
 }
 

@@ -283,16 +283,41 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   int nsK = 1;
   bool i8x = false, i8k = tc;
   if (nocc > 0 && precision != RIJK_PREC_MIXED) {
-    // The int8 tensor cores for large exchanges; without room for the digits of B the half-transform stays on DMMA.
-    i8k = tc || int8_exchange(npad, kdim);
-    nsK = i8k ? syrk_i8_parts(nt, naux, noccp, ctx->device, &kper_tc) : syrk_nsplit(nt, kdim);
-    i8x = int8_half_transform(n, npad, kdim, noccp, kper_tc) && !dmma_x && bdig_prepare(ctx);
-    if (i8x && (rc = xform_i8_buffers(ctx, noccp, nsK))) return rc;
-    if ((rc = ensure(ctx, ctx->MOp, noccp * npad * sizeof(double), "MOp")) ||
-        (rc = ensure(ctx, ctx->XT, static_cast<size_t>(npad) * kdim * sizeof(double), "XT")) ||
-        (rc = ensure(ctx, ctx->Kpart, static_cast<size_t>(nsK) * tile_elems * sizeof(double), "Kpart")))
-      return rc;
-    i8x = i8x && ctx->have_bdig;  // a buffer above may have needed their memory
+    auto buffers = [&]() {
+      int r = ensure(ctx, ctx->MOp, noccp * npad * sizeof(double), "MOp");
+      if (!r) r = ensure(ctx, ctx->XT, static_cast<size_t>(npad) * kdim * sizeof(double), "XT");
+      return r ? r : ensure(ctx, ctx->Kpart, static_cast<size_t>(nsK) * tile_elems * sizeof(double), "Kpart");
+    };
+    // The int8 tensor cores for large exchanges.  Without room for the digits of B the half-transform stays on DMMA,
+    // without room for those of X, about 0.9 times its bytes, all of the exchange.
+    const std::string keep = ctx->last_error;
+    i8k = tc || (int8_exchange(npad, kdim) && !ctx->no_i8k);
+    if (i8k) {
+      nsK = syrk_i8_parts(nt, naux, noccp, ctx->device, &kper_tc);
+      i8x = int8_half_transform(n, npad, kdim, noccp, kper_tc) && !ctx->no_i8k && !dmma_x && bdig_prepare(ctx);
+      if (!(rc = buffers())) rc = syrk_i8_buffers(ctx, npad, kdim, nsK);
+      if (rc && (tc || rc != RIJK_ERR_ALLOC)) return rc;
+      i8k = !rc;
+      if (i8k && i8x && xform_i8_buffers(ctx, noccp, nsK)) {
+        i8x = false;
+        ctx->last_error = keep;
+      }
+      i8x = i8x && ctx->have_bdig;  // a buffer above may have needed their memory
+    }
+    if (!i8k) {
+      const bool refused = rc != RIJK_OK;
+      if (refused) {
+        i8x = false;
+        cudaStreamSynchronize(s);  // an earlier build may still read them
+        for (DeviceBuf* b : {&ctx->Xs, &ctx->Xe, &ctx->Cdig, &ctx->Xtop}) release(*b);
+      }
+      nsK = syrk_nsplit(nt, kdim);
+      if ((rc = buffers())) return rc;
+      if (refused) {
+        ctx->last_error = keep;
+        ctx->no_i8k = true;
+      }
+    }
   }
   // FP64 and FP64_TC: the Coulomb pair runs on the high-priority stream beside the DMMA half-transform, one
   // or two 256-thread CTAs per SM, in the registers and warps the half-transform's CTAs leave free;
@@ -604,7 +629,7 @@ RIJK_API int rijk_set_aux_range(rijk_ctx* ctx, long q0, long q1) {
   ctx->q0 = q0;
   ctx->nq = q1 - q0;
   ctx->have_b = false;
-  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = false;
+  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = ctx->no_i8k = false;
   return RIJK_OK;
 }
 
@@ -717,7 +742,7 @@ int set_metric_impl(rijk_ctx* ctx, const double* PQ, cudaMemcpyKind kind, long n
   ctx->metric_form = form;
   ctx->have_metric = true;
   ctx->have_b = false;
-  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = false;
+  ctx->have_bmix = ctx->have_bdig = ctx->no_bdig = ctx->no_i8k = false;
   ctx->stats.naux = naux;
   if (hinfo[1] > 0) ctx->last_error = "warning: metric eigenvalues <= 0 dropped";
   return RIJK_OK;

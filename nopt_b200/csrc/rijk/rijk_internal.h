@@ -105,6 +105,7 @@ struct rijk_ctx {
   bool have_btop = false;
   bool have_bdig = false;   // Bdig holds the digits of the present B
   bool no_bdig = false;     // there was no room for them with the present B
+  bool no_i8k = false;      // ... nor for the digits of X
   rijk::DeviceBuf Cdig;     // exponents and int8 digits of the orbitals
   rijk::DeviceBuf Xtop;     // largest magnitudes of X^T's rows in each split part
   rijk::DeviceBuf Xs;       // int8 digits of X^T: blocks of 128 rows x 32 k, 7 digits each
@@ -274,6 +275,7 @@ void launch_syrk_f64(const double* XT, long npad, long nt, long kdim, int nsplit
 
 // ---- k_exchange_i8.cu: K partials of the FP64 form from int8 digits on tcgen05
 int syrk_i8_parts(long nt, long naux, long noccp, int device, long* kper);
+int syrk_i8_buffers(rijk_ctx* ctx, long npad, long kdim, int nparts);  // before anything is queued
 int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int nparts, long kper,
             const uint32_t* tops, double* Kpart, cudaStream_t s);
 

@@ -132,3 +132,27 @@ def test_digits_of_an_old_tensor_are_released():
         _set(fb, small, 70)
         # 700 aux functions x 10 blocks of 128 x 128 elements in 7 bytes each: 0.8 GB
         assert torch.cuda.mem_get_info()[0] - before > 700 * 10 * 128 * 128 * 7 // 2
+
+
+def test_no_room_for_the_int8_exchange():
+    """Each request of a first large build is refused three times: neither the pool's blocks nor the digits of B then
+    make room, and the exchange runs on the FP64 units, which need less.  A new tensor tries the digits again."""
+    n, nocc = 300, 40
+    system = _system(n, 1100, nocc)
+    seen = []
+    for k in range(1, 20):
+        with rijk.FockBuilder(0) as fb:
+            _set(fb, system, n)
+            fb.dm_to_f_transform_ri(system[2], system[3], 1)
+            fb.selftest_alloc_refuse(k, 3)  # the staged orbitals, the one request without another way, go through
+            seen.append(_build(fb, system, nocc))
+            fb.selftest_alloc_refuse(0, 0)
+            if "syrk_f64" in seen[-1]:
+                assert "xform_f64" in seen[-1]
+                assert "syrk_f64" in _build(fb, system, nocc)  # not asked for again with this tensor
+                _set(fb, system, n)
+                assert {"xform_i8", "syrk_i8"} <= _build(fb, system, nocc)
+            elif "xform_i8" in seen[-1]:  # no such request any more
+                break
+    # the orbitals, X, its digits and their exponents (the partial sums of the small build are large enough)
+    assert sum("syrk_f64" in s for s in seen) >= 4 and "xform_i8" in seen[-1]
