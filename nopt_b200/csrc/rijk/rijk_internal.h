@@ -280,8 +280,8 @@ int syrk_i8(rijk_ctx* ctx, const double* XT, long npad, long nt, long kdim, int 
             const uint32_t* tops, double* Kpart, cudaStream_t s);
 
 // ---- k_xform_i8.cu: the FP64 half-transform from int8 digits on tcgen05
-// The digits of the present B, made on the first call; false when there is no room for them (the caller
-// then takes the DMMA kernel).  drop_bdig gives their memory back, for_good: until B changes.  forget_bdig: a new B of nq
+// The digits of the present B, made on the first call; false when there is no room for them or the build is being
+// recorded into a CUDA graph (the caller then takes the DMMA kernel).  drop_bdig gives their memory back, for_good: until B changes.  forget_bdig: a new B of nq
 // aux functions and nt tile rows is to come; the memory stays only where the new digits fit it exactly (the next
 // geometry of a molecule).
 bool bdig_prepare(rijk_ctx* ctx);
