@@ -516,10 +516,12 @@ RIJK_API int rijk_create(rijk_ctx** out, int device) {
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = device;
   uint64_t keep = kPoolKeep;
-  if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess ||
-      cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-    rijk_destroy(ctx);
-    return RIJK_ERR_CUDA;
+  // a device or driver mode without memory pools: scratch from cudaMalloc
+  if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->pool = nullptr;
+  } else {
+    cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
   cudaEventCreate(&ctx->ev0);
   cudaEventCreate(&ctx->ev1);

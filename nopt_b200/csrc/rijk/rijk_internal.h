@@ -76,7 +76,7 @@ struct rijk_ctx {
   int sms = 148;
   // Scratch of single calls (set-up, derivatives, MO tensors), allocated and freed in stream order.  The pool
   // keeps at most kPoolKeep bytes between calls and gives everything back in rijk_destroy, or before a
-  // device allocation of the context fails.
+  // device allocation of the context fails.  Null where the device has no pools.
   cudaMemPool_t pool = nullptr;
 
   long n = 0, naux = 0, npad = 0, nt = 0, ntile = 0;
