@@ -375,8 +375,9 @@ int rijk_mo_ints_aaag(rijk_ctx* ctx, double* MO_INTS, const double* MO_VEC, long
 int rijk_soscf_hess_ints(rijk_ctx* ctx, double* aa_J, double* aa_K, const double* MO_VEC, long n_c, long n_a,
                          long n_mo);
 
-/* Aux functions per chunk of rijk_grad's Y^Q stage (0, the default: all of them at once); the
- * derivatives do not depend on it beyond rounding. */
+/* Aux functions per chunk of rijk_grad's Y^Q, and at most of its Gamma^Q (0, the default: all of them at
+ * once, or as many as find room).  A chunk bounds the scratch of dE/d(P|Q) to it; dE/d(P|mu nu) takes 2 n_c^2
+ * naux doubles whatever the chunk.  The derivatives do not depend on it. */
 int rijk_set_grad_chunk(rijk_ctx* ctx, long q_per_chunk);
 
 /* Adjoint of the Fock build (no reference counterpart; the reference differentiates by finite

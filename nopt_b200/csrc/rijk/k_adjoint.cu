@@ -28,9 +28,10 @@
 // Z and u by one GEMM with M (the pairs i >= j packed, u as one more row), the first index of C^T Z C by one
 // GEMM, and the second by one GEMM per orbital row mu, whose epilogue writes the packed pair rows.  Those rows
 // leave in blocks: the copy of one block to the host runs while the next is formed, so the device never holds
-// the whole derivative.  Behind the copies, which take longest, dE/d(P|Q) over chunks
-// of aux functions: T^Q = Y^Q C (k_gemm_f64), the packed Gamma tiles (k_gamma_f64), their rows of G by one GEMM
-// with B, and at the end M^T G M; the blocks' GEMMs take the high-priority stream beside it.
+// the whole derivative.  Behind the copies, which take longest (or with each chunk of Y, where those are smaller than
+// all aux functions), dE/d(P|Q) over chunks of aux functions: T^Q = Y^Q C (k_gemm_f64), the packed Gamma tiles
+// (k_gamma_f64), their rows of G by one GEMM with B, and at the end M^T G M; the blocks' GEMMs take the
+// high-priority stream beside it.
 // (H2O)8 cc-pVDZ, 151 MB out: 18.7 ms a call with Gamma for both derivatives and the copies at the end, 7.8 to 9.1 now
 // (the copies' speed differs between hosts); (H2O)16, 126 and 59 to 71.
 #include <algorithm>
@@ -316,17 +317,22 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
   const long np = nocc * (nocc + 1) / 2, ldp = round_up(np + 1, 2), ldP = round_up(naux, 2);
   const double* MOp = static_cast<const double*>(ctx->MOp.p);
   const double* pM = static_cast<const double*>(ctx->M.p);  // row-major [Q][P], ld nauxp
-  const long qc = ctx->grad_qchunk > 0 ? std::min(ctx->grad_qchunk, naux) : naux;
+  long qc = ctx->grad_qchunk > 0 ? std::min(ctx->grad_qchunk, naux) : naux;
   const size_t b_pairs = static_cast<size_t>(np + 1) * ldP * sizeof(double);
   // blocks of orbital rows of dE/d(P|mu nu), about 64 MB each and at least one row
   const long blk = std::max<long>(n * naux, (64L << 20) / 8);
-  const long qy = dEdPQ ? naux : qc;  // aux functions whose Y stays: all of them where G needs it again
-  // aux functions per chunk of T and Gamma, in whole tiles of G's rows: 1 GiB, less if that cannot be had (asking
-  // for the free memory first took 7 ms a call)
+  while ((rc = ensure_tmp(ctx, Y, static_cast<size_t>(qc) * noccp * nocc * sizeof(double), "grad Y"))) {
+    if (qc == 1 || ctx->fail_alloc_after == 0) return chk(rc);
+    qc = (qc + 1) / 2;
+  }
+  // aux functions per chunk of T and Gamma, in whole tiles of G's rows and no more than Y's: 1 GiB, less if that cannot
+  // be had (asking for the free memory first took 7 ms a call)
   const long per_q = te + npad * noccp;
   long gq = std::max<long>(1, std::min<long>(naux, (1L << 30) / (8 * per_q)));
   if (gq < naux && gq >= 64) gq -= gq % 64;
-  if ((rc = chk(ensure_tmp(ctx, Y, static_cast<size_t>(qy) * noccp * nocc * sizeof(double), "grad Y")))) return rc;
+  gq = std::min(gq, qc);
+  // G's chunks follow Y's, or all of them the first copies out where Y is there for every aux function
+  const bool behind = dEdPQ && dEdI3 && qc == naux;
   if (dEdPQ && ((rc = chk(ensure_tmp(ctx, Ct, static_cast<size_t>(npad) * noccp * sizeof(double), "grad Ct"))) ||
                 (rc = chk(ensure_tmp(ctx, Gm, static_cast<size_t>(naux) * naux * sizeof(double), "grad G"))) ||
                 (rc = chk(ensure_tmp(ctx, T1, static_cast<size_t>(naux) * naux * sizeof(double), "grad T1")))))
@@ -342,54 +348,42 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
                 (rc = chk(ensure_tmp(ctx, out[1], blk * sizeof(double), "grad dI3 block")))))
     return rc;
   double* pY = static_cast<double*>(Y.p);
-  for (long q0 = 0; q0 < naux; q0 += qc) {
-    const long nq = std::min(qc, naux - q0);
-    // Y^Q[i][j] = sum_nu X^Q_{i nu} C_{j nu} (= C B^Q C^T), every Q of the chunk in one product: rows (Q, i)
-    // of X^T's columns are contiguous
-    GemmF64Args g;
-    g.M = nq * noccp, g.N = nocc, g.K = npad;
-    g.A = static_cast<const double*>(ctx->XT.p) + q0 * noccp, g.lda = kdim, g.a_kmajor = false;
-    g.B = MOp, g.ldb = npad, g.b_kmajor = true;
-    double* y = pY + (dEdPQ ? q0 * noccp * nocc : 0);
-    g.C = y, g.ldc = nocc;
-    gemm_f64(g, 1, s);
-    if (!dEdI3) continue;
-    dim3 grid(static_cast<unsigned>((ldp + 255) / 256), static_cast<unsigned>(std::min<long>(nq, 1024)));
-    k_pack_pairs<<<grid, 256, 0, s>>>(y, static_cast<const double*>(ctx->w.p), q0, nq, nocc, noccp, np, ldp,
-                                      static_cast<double*>(Yp.p));
+  const size_t gsmem = (2 * G_ASTAGE + 2 * 64 * LDK) * sizeof(double);
+  if (dEdPQ) {
+    ensure_smem_limit(reinterpret_cast<const void*>(k_gamma_f64), gsmem);
+    k_transpose_mo<<<grid_of(noccp * npad), 256, 0, s>>>(MOp, noccp, npad, static_cast<double*>(Ct.p));
   }
-  tm.mark(2);
-  // dE/d(P|Q) = -M^T G M, queued on the build's stream
-  auto queue_dpq = [&]() {
-    const double* pB = static_cast<const double*>(ctx->B.p);
+  // rows q0 .. q0 + nq of G, from Y^q0 .. at y
+  auto g_rows = [&](long q0, long nq, const double* y) {
     double* pGam = static_cast<double*>(Gam.p);
     double* pT = pGam + gq * te;
-    double* pG = static_cast<double*>(Gm.p);
-    k_transpose_mo<<<grid_of(noccp * npad), 256, 0, s>>>(MOp, noccp, npad, static_cast<double*>(Ct.p));
-    const size_t gsmem = (2 * G_ASTAGE + 2 * 64 * LDK) * sizeof(double);
-    ensure_smem_limit(reinterpret_cast<const void*>(k_gamma_f64), gsmem);
-    for (long q0 = 0; q0 < naux; q0 += gq) {
-      const long nq = std::min(gq, naux - q0);
+    for (long g0 = 0; g0 < nq; g0 += gq) {
+      const long ng = std::min(gq, nq - g0);
       {  // T^Q transposed, Tt[(Q, i)][mu] = sum_j Y^Q[i][j] C_{j mu}, one GEMM for the chunk
         GemmF64Args g;
-        g.M = nq * noccp, g.N = npad, g.K = nocc;
-        g.A = pY + q0 * noccp * nocc, g.lda = nocc, g.a_kmajor = true;
+        g.M = ng * noccp, g.N = npad, g.K = nocc;
+        g.A = y + g0 * noccp * nocc, g.lda = nocc, g.a_kmajor = true;
         g.B = MOp, g.ldb = npad, g.b_kmajor = false;
         g.C = pT, g.ldc = npad;
         gemm_f64(g, 1, s);
       }
-      k_gamma_f64<<<dim3(static_cast<unsigned>(ntile), static_cast<unsigned>(nq)), G_THREADS, gsmem, s>>>(
-          pT, static_cast<const double*>(Ct.p), pD, static_cast<const double*>(ctx->w.p) + q0, n, npad, noccp, te, pGam);
-      {  // rows q0.. of G_QR = 1/2 sum_{mu nu} Gamma^Q B^R over the full squares
+      k_gamma_f64<<<dim3(static_cast<unsigned>(ntile), static_cast<unsigned>(ng)), G_THREADS, gsmem, s>>>(
+          pT, static_cast<const double*>(Ct.p), pD, static_cast<const double*>(ctx->w.p) + q0 + g0, n, npad, noccp, te,
+          pGam);
+      {  // G_QR = 1/2 sum_{mu nu} Gamma^Q B^R over the full squares
         GemmF64Args g;
-        g.M = nq, g.N = naux, g.K = te;
+        g.M = ng, g.N = naux, g.K = te;
         g.A = pGam, g.lda = te, g.a_kmajor = true;
-        g.B = pB, g.ldb = te, g.b_kmajor = true;
-        g.C = pG + q0 * naux, g.ldc = naux;
+        g.B = static_cast<const double*>(ctx->B.p), g.ldb = te, g.b_kmajor = true;
+        g.C = static_cast<double*>(Gm.p) + (q0 + g0) * naux, g.ldc = naux;
         gemm_f64(g, 1, s);
       }
       tm.mark(5);
     }
+  };
+  // dE/d(P|Q) = -M^T G M
+  auto queue_dpq = [&]() {
+    double* pG = static_cast<double*>(Gm.p);
     // T1[Q][P'] = sum_R G[Q][R] M[R][P'];  out[P][P'] = -sum_Q M[Q][P] T1[Q][P']
     GemmF64Args g;
     g.M = naux, g.N = naux, g.K = naux;
@@ -406,6 +400,25 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
     gemm_f64(h, 1, s);
     tm.mark(6);
   };
+  for (long q0 = 0; q0 < naux; q0 += qc) {
+    const long nq = std::min(qc, naux - q0);
+    // Y^Q[i][j] = sum_nu X^Q_{i nu} C_{j nu} (= C B^Q C^T), every Q of the chunk in one product: rows (Q, i)
+    // of X^T's columns are contiguous
+    GemmF64Args g;
+    g.M = nq * noccp, g.N = nocc, g.K = npad;
+    g.A = static_cast<const double*>(ctx->XT.p) + q0 * noccp, g.lda = kdim, g.a_kmajor = false;
+    g.B = MOp, g.ldb = npad, g.b_kmajor = true;
+    g.C = pY, g.ldc = nocc;
+    gemm_f64(g, 1, s);
+    if (dEdI3) {
+      dim3 grid(static_cast<unsigned>((ldp + 255) / 256), static_cast<unsigned>(std::min<long>(nq, 1024)));
+      k_pack_pairs<<<grid, 256, 0, s>>>(pY, static_cast<const double*>(ctx->w.p), q0, nq, nocc, noccp, np, ldp,
+                                        static_cast<double*>(Yp.p));
+    }
+    tm.mark(2);
+    if (dEdPQ && !behind) g_rows(q0, nq, pY);
+  }
+  if (dEdPQ && !behind) queue_dpq();
   if (dEdI3) {
     // Z[p][P] = sum_Q Y[Q][p] M_QP, the last row u_P = sum_Q w_Q M_QP
     double* pZ = static_cast<double*>(Z.p);
@@ -458,8 +471,9 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
       h.mu0 = m0, h.n_ao = n, h.D = pD, h.u = pu;
       gemm_f64(h, m1 - m0, sb);
       cudaEventRecord(ctx->ev_blk[slot], sb);
-      if (m0 == 0 && dEdPQ) {  // before the first copy, which pageable memory makes the host wait for
+      if (m0 == 0 && behind) {  // before the first copy, which pageable memory makes the host wait for
         tm.mark(4);
+        g_rows(0, naux, pY);
         queue_dpq();
       }
       if (prev0 >= 0) rc = copy_out(prev0, prev1, slot ^ 1);
@@ -470,7 +484,6 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
     tm.mark(4);
     if (!rc) rc = copy_out(prev0, prev1, slot ^ 1);
   }
-  if (dEdPQ && !dEdI3) queue_dpq();
   if (dEdPQ && !rc)
     rc = cuda_check(ctx, cudaMemcpyAsync(dEdPQ, Gm.p, static_cast<size_t>(naux) * naux * sizeof(double),
                                          cudaMemcpyDeviceToHost, s), "D2H dPQ");

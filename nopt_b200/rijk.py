@@ -377,7 +377,7 @@ class FockBuilder:
         return out, J, K
 
     def set_grad_chunk(self, q_per_chunk):
-        """Aux functions per chunk of grad's Gamma stage (0: automatic, from free HBM)."""
+        """Aux functions per chunk of grad's Y^Q, and at most of its Gamma^Q (0: all at once, or as many as find room)."""
         self._check(lib().rijk_set_grad_chunk(self._h, int(q_per_chunk)))
 
     def grad(self, MO, n_c, H, e_nuc, want_3c=False, want_metric=False, out3=None, outV=None):
