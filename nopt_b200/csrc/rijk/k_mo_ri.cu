@@ -338,14 +338,31 @@ RIJK_API int rijk_soscf_hess_ints(rijk_ctx* ctx, double* aa_J, double* aa_K, con
   // of 96 rows.  Whole calls at C10H22 cc-pVDZ (n = 250, n_aux = 1206), pairs against diagonals: 0.74 against 2.18 ms at
   // n_a = 6, 0.80, 2.21 at 10, 1.59, 2.44 at 18, 1.95, 2.49 at 22, and even at the line, 2.50, 2.52 at 26.
   const long te = ctx->ntile * TILE2, T = n_a * (n_a + 1) / 2;
-  const bool pairs_first = T * (naux + 2 * n_mo) < 2 * n_mo * naux && T * te <= 96 * npad * naux;
-  const long nd = pairs_first ? T : naux;  // tensors whose diagonals are formed, by half-transforms of batches of rows
+  bool pairs_first = T * (naux + 2 * n_mo) < 2 * n_mo * naux && T * te <= 96 * npad * naux;
+  // 96 rows a batch, or all of them while their half-transform is no larger than 256 MB
+  const long all = round_up(n_mo, 16);
+  long nd = 0, batch = 0;  // tensors whose diagonals are formed, by half-transforms of batches of rows
+  double *Yp = nullptr, *Jtu = nullptr, *Rpp = nullptr, *XT = nullptr;
+  auto scratch = [&](Scratch& sd, long rows) {
+    int r = 0;
+    nd = pairs_first ? T : naux;
+    batch = rows > 0 ? rows : npad * nd * all <= (32L << 20) ? all : 96;
+    if (pairs_first) Yp = sd.get(ctx, static_cast<size_t>(T) * naux, "packed (t u|Q)", &r);
+    if (pairs_first && !r) Jtu = sd.get(ctx, static_cast<size_t>(T) * te, "J^{tu}", &r);
+    if (!r) Rpp = sd.get(ctx, static_cast<size_t>(n_mo) * nd, "(pp| diagonals", &r);
+    if (!r) XT = sd.get(ctx, static_cast<size_t>(npad) * nd * std::min(batch, all), "batch half-transform", &r);
+    return r;
+  };
+  Scratch first, second;
+  const std::string keep = ctx->last_error;
+  if ((rc = scratch(first, 0)) == RIJK_ERR_ALLOC) {  // the diagonals in batches take the least
+    for (DeviceBuf& b : first.bufs) release(b);
+    pairs_first = false;
+    if (!(rc = scratch(second, 96))) ctx->last_error = keep;
+  }
+  if (rc) return rc;
   const double* tens = static_cast<const double*>(ctx->B.p);
   if (pairs_first) {
-    double* Yp = sc.get(ctx, static_cast<size_t>(T) * naux, "packed (t u|Q)", &rc);
-    if (rc) return rc;
-    double* Jtu = sc.get(ctx, static_cast<size_t>(T) * te, "J^{tu}", &rc);
-    if (rc) return rc;
     k_pack_tu<<<grid_of(T * naux), 256, 0, ctx->stream>>>(ap.Yt, n_a, naux, Yp);
     GemmF64Args g;
     g.M = T, g.N = te, g.K = naux;
@@ -355,23 +372,13 @@ RIJK_API int rijk_soscf_hess_ints(rijk_ctx* ctx, double* aa_J, double* aa_K, con
     gemm_f64(g, 1, ctx->stream);
     tens = Jtu;
   }
-  double* Rpp = sc.get(ctx, static_cast<size_t>(n_mo) * nd, "(pp| diagonals", &rc);
-  if (rc) return rc;
-  // 96 rows a batch, or all of them while their half-transform is no larger than 256 MB
-  const long all = round_up(n_mo, 16);
-  const long batch = npad * nd * all <= (32L << 20) ? all : 96;
-  {
-    Scratch sb;
-    double* XT = sb.get(ctx, static_cast<size_t>(npad) * nd * std::min(batch, all), "batch half-transform", &rc);
-    if (rc) return rc;
-    for (long p0 = 0; p0 < n_mo; p0 += batch) {
-      const long nr = std::min(batch, n_mo - p0), pb = round_up(nr, 16);
-      const double* rows = ap.rows_all + p0 * npad;
-      launch_xform_f64(tens, rows, nd, ctx->nt, pb, XT, ctx->stream);
-      k_diag_pair<<<grid_of(nd * pb * 8), 256, 0, ctx->stream>>>(XT, rows, nr, pb, nd, npad, Rpp + p0 * nd);
-    }
-    // p0 + pb <= round_up(n_mo, 16): the last batch's padding rows are the zero rows of rows_all
+  for (long p0 = 0; p0 < n_mo; p0 += batch) {
+    const long nr = std::min(batch, n_mo - p0), pb = round_up(nr, 16);
+    const double* rows = ap.rows_all + p0 * npad;
+    launch_xform_f64(tens, rows, nd, ctx->nt, pb, XT, ctx->stream);
+    k_diag_pair<<<grid_of(nd * pb * 8), 256, 0, ctx->stream>>>(XT, rows, nr, pb, nd, npad, Rpp + p0 * nd);
   }
+  // p0 + pb <= round_up(n_mo, 16): the last batch's padding rows are the zero rows of rows_all
   if (pairs_first) {
     k_expand_tu<<<grid_of(n_mo * n_a * n_a), 256, 0, ctx->stream>>>(Rpp, n_mo, n_a, dJ);
   } else {
