@@ -54,8 +54,8 @@ static cudaError_t device_malloc(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, bool
 }
 
 // Memory for the empty buffer b, if need be what the context can spare: the blocks its scratch pool keeps, then the
-// digits of B.  A scratch buffer is free again after its call, so the digits may come back with the next build.
-static int acquire(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what, bool pooled) {
+// digits of B.  Scratch of a single call is free again after it, so the digits may come back with the next build.
+static int acquire(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what, bool pooled, bool scratch) {
   cudaError_t e = device_malloc(ctx, b, bytes, pooled);
   if (e == cudaErrorMemoryAllocation && ctx->pool) {
     cudaGetLastError();
@@ -65,7 +65,7 @@ static int acquire(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what, 
   }
   if (e == cudaErrorMemoryAllocation && ctx->Bdig.p && &b != &ctx->Bdig) {
     cudaGetLastError();
-    drop_bdig(ctx, !pooled);
+    drop_bdig(ctx, !scratch);
     e = device_malloc(ctx, b, bytes, pooled);
   }
   if (e != cudaSuccess) {
@@ -77,7 +77,7 @@ static int acquire(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what, 
   return RIJK_OK;
 }
 
-int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
+static int ensure_kept(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what, bool pooled) {
   if (b.bytes >= bytes && b.p) return RIJK_OK;
   if (bytes > 0 && ctx->fail_alloc_after >= 0) {  // rijk_selftest_alloc_failure
     if (ctx->fail_alloc_after == 0) return set_err(ctx, RIJK_ERR_ALLOC, "%s: out of device memory (injected)", what);
@@ -89,10 +89,27 @@ int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
     if (ctx->j_stream) cudaStreamSynchronize(ctx->j_stream);
     cudaFree(b.p);
   }
-  b.p = nullptr;
-  b.bytes = 0;
+  b = DeviceBuf();
   if (bytes == 0) return RIJK_OK;
-  return acquire(ctx, b, bytes, what, false);
+  return acquire(ctx, b, bytes, what, pooled, false);
+}
+
+int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
+  return ensure_kept(ctx, b, bytes, what, false);
+}
+
+// From the pool where the buffer is small: the set-up has left its scratch there, and a block of that costs
+// next to nothing, where a cudaMalloc maps new memory.  The first build of a new context after rijk_set_basis, FP64:
+// 1.18 -> 0.19 ms at (H2O)2 cc-pVDZ, 1.38 -> 0.35 at (H2O)6, 4.9 -> 4.2 at (H2O)16, whose larger buffers stay apart so that
+// the pool can be trimmed.
+constexpr size_t kPoolBuild = 64ul << 20;
+int ensure_build(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
+  if (!ctx->pool || bytes > kPoolBuild) return ensure(ctx, b, bytes, what);
+  if (b.bytes >= bytes && b.p) return RIJK_OK;
+  const int rc = ensure_kept(ctx, b, bytes, what, true);
+  b.pool = nullptr;  // freed by cudaFree, whatever becomes of the stream
+  // the block is the context's once the work before the allocation has ended: the other streams use it, too
+  return rc ? rc : cuda_check(ctx, cudaStreamSynchronize(ctx->stream), what);
 }
 
 // The largest single scratch buffer is a 2 GiB block of raw integrals (rows_per_chunk), beside a few
@@ -110,7 +127,7 @@ int ensure_tmp(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
   }
   release(b);
   if (bytes == 0) return RIJK_OK;
-  return acquire(ctx, b, bytes, what, true);
+  return acquire(ctx, b, bytes, what, true, true);
 }
 
 cudaError_t ensure_smem_limit(const void* fn, size_t bytes) {
@@ -270,9 +287,9 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   int rc;
   int launches = 0;
   const int nsJ = coulomb_nsplit(tile_elems, naux, precision == RIJK_PREC_MIXED ? 8 : 2);
-  if ((rc = ensure(ctx, ctx->Dt, tile_elems * (sizeof(double) + sizeof(float)), "Dt")) ||
-      (rc = ensure(ctx, ctx->w, (1 + coulomb_w_mixed_chunks(ntile)) * naux * sizeof(double), "w")) ||  // w, partials
-      (rc = ensure(ctx, ctx->Jpart, static_cast<size_t>(nsJ) * tile_elems * sizeof(double), "Jpart")))
+  if ((rc = ensure_build(ctx, ctx->Dt, tile_elems * (sizeof(double) + sizeof(float)), "Dt")) ||
+      (rc = ensure_build(ctx, ctx->w, (1 + coulomb_w_mixed_chunks(ntile)) * naux * sizeof(double), "w")) ||  // w, partials
+      (rc = ensure_build(ctx, ctx->Jpart, static_cast<size_t>(nsJ) * tile_elems * sizeof(double), "Jpart")))
     return rc;
   if (precision == RIJK_PREC_MIXED && (rc = mixed_prepare(ctx))) return rc;
   // the FP64 exchange's buffers, before anything is queued: growing one drains the streams
@@ -284,9 +301,9 @@ int fock_device_impl(rijk_ctx* ctx, const double* dD, const double* dMO, long no
   bool i8x = false, i8k = tc;
   if (nocc > 0 && precision != RIJK_PREC_MIXED) {
     auto buffers = [&]() {
-      int r = ensure(ctx, ctx->MOp, noccp * npad * sizeof(double), "MOp");
-      if (!r) r = ensure(ctx, ctx->XT, static_cast<size_t>(npad) * kdim * sizeof(double), "XT");
-      return r ? r : ensure(ctx, ctx->Kpart, static_cast<size_t>(nsK) * tile_elems * sizeof(double), "Kpart");
+      int r = ensure_build(ctx, ctx->MOp, noccp * npad * sizeof(double), "MOp");
+      if (!r) r = ensure_build(ctx, ctx->XT, static_cast<size_t>(npad) * kdim * sizeof(double), "XT");
+      return r ? r : ensure_build(ctx, ctx->Kpart, static_cast<size_t>(nsK) * tile_elems * sizeof(double), "Kpart");
     };
     // The int8 tensor cores for large exchanges.  Without room for the digits of B the half-transform stays on DMMA,
     // without room for those of X, about 0.9 times its bytes, all of the exchange.
@@ -925,9 +942,9 @@ RIJK_API int rijk_fock(rijk_ctx* ctx, const double* D, const double* MO, long no
   cudaSetDevice(ctx->device);
   const long n = ctx->n;
   const size_t nn = static_cast<size_t>(n) * n * sizeof(double);
-  if ((rc = ensure(ctx, ctx->stageD, nn, "stage D")) || (rc = ensure(ctx, ctx->stageJ, nn, "stage J")) ||
-      (rc = ensure(ctx, ctx->stageK, nn, "stage K")) ||
-      (rc = ensure(ctx, ctx->stageMO, std::max<size_t>(1, nocc * n * sizeof(double)), "stage MO")))
+  if ((rc = ensure_build(ctx, ctx->stageD, nn, "stage D")) || (rc = ensure_build(ctx, ctx->stageJ, nn, "stage J")) ||
+      (rc = ensure_build(ctx, ctx->stageK, nn, "stage K")) ||
+      (rc = ensure_build(ctx, ctx->stageMO, std::max<size_t>(1, nocc * n * sizeof(double)), "stage MO")))
     return rc;
   cudaStream_t s = ctx->stream, c = ctx->copy_stream;
   // D on the build's stream; the orbitals on the copy stream (the Coulomb passes do not need

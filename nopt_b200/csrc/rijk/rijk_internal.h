@@ -150,6 +150,8 @@ void prof_mark(rijk_ctx* ctx, const char* name);
 int set_err(rijk_ctx* ctx, int code, const char* fmt, ...);
 int cuda_check(rijk_ctx* ctx, cudaError_t e, const char* what);
 int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);
+// The same for a build's own buffers, which the context keeps, too.
+int ensure_build(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);
 // Scratch that one call needs: from the context's pool, in the order of ctx->stream (a buffer that another
 // stream uses is released only once that stream has been waited for).
 int ensure_tmp(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);
