@@ -562,16 +562,6 @@ static size_t bdig_bytes(long nq, long nt) {
   return static_cast<size_t>(nq) * (nb * (nb + 1) / 2) * kSuper;
 }
 
-// Whether the context's stream is being recorded into a CUDA graph.
-static bool recording(rijk_ctx* ctx) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return st != cudaStreamCaptureStatusNone;
-}
-
 bool bdig_prepare(rijk_ctx* ctx) {
   // A recorded build reads B itself: digits formed in it would not be there before its replay, and digits formed
   // before it would be those of an earlier tensor in a replay after the next set-up.

@@ -41,6 +41,7 @@ int cuda_check(rijk_ctx* ctx, cudaError_t e, const char* what) {
     cudaGetLastError();
     return set_err(ctx, RIJK_ERR_ALLOC, "%s: out of device memory", what);
   }
+  cudaGetLastError();  // reported here, not once more by the next call's launch check
   return set_err(ctx, RIJK_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
@@ -77,6 +78,15 @@ static int acquire(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what, 
   return RIJK_OK;
 }
 
+bool recording(rijk_ctx* ctx) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 static int ensure_kept(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what, bool pooled) {
   if (b.bytes >= bytes && b.p) return RIJK_OK;
   if (bytes > 0 && ctx->fail_alloc_after >= 0) {  // rijk_selftest_alloc_failure
@@ -104,12 +114,14 @@ int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
 // the pool can be trimmed.
 constexpr size_t kPoolBuild = 64ul << 20;
 int ensure_build(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
-  if (!ctx->pool || bytes > kPoolBuild) return ensure(ctx, b, bytes, what);
   if (b.bytes >= bytes && b.p) return RIJK_OK;
-  const int rc = ensure_kept(ctx, b, bytes, what, true);
-  b.pool = nullptr;  // freed by cudaFree, whatever becomes of the stream
+  // (in a recording, a block of the pool would be the graph's; cudaMalloc is refused there)
+  if (!ctx->pool || bytes > kPoolBuild || recording(ctx)) return ensure(ctx, b, bytes, what);
+  int rc = ensure_kept(ctx, b, bytes, what, true);
   // the block is the context's once the work before the allocation has ended: the other streams use it, too
-  return rc ? rc : cuda_check(ctx, cudaStreamSynchronize(ctx->stream), what);
+  if (!rc && (rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), what))) release(b);
+  b.pool = nullptr;  // freed by cudaFree, whatever becomes of the stream
+  return rc;
 }
 
 // The largest single scratch buffer is a 2 GiB block of raw integrals (rows_per_chunk), beside a few

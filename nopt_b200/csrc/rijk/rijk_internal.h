@@ -152,6 +152,8 @@ int cuda_check(rijk_ctx* ctx, cudaError_t e, const char* what);
 int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);
 // The same for a build's own buffers, which the context keeps, too.
 int ensure_build(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);
+// Whether the context's stream is being recorded into a CUDA graph.
+bool recording(rijk_ctx* ctx);
 // Scratch that one call needs: from the context's pool, in the order of ctx->stream (a buffer that another
 // stream uses is released only once that stream has been waited for).
 int ensure_tmp(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what);

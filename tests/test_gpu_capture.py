@@ -73,3 +73,40 @@ def test_recorded_builds_and_the_digits_of_b(precision):
         graph.replay()
         check(first)
         del graph
+
+
+@pytest.mark.parametrize("nocc", [NOCC, 2])
+def test_a_recorded_first_build_is_refused(nocc):
+    """A recording cannot allocate.  A build that would have to is refused, and leaves nothing behind: the next ordinary
+    build takes its buffers and is right."""
+    import torch
+    s = _system(1)
+    D = s[3][:nocc].T @ s[3][:nocc]
+    stream = torch.cuda.Stream()
+    with rijk.FockBuilder(0) as fb:
+        fb.set_stream(stream.cuda_stream)
+        fb.set_metric(s[0])
+        fb.set_3c(s[1], N)
+        want = fb.dm_to_f_transform_ri(D, s[3], nocc)
+    with rijk.FockBuilder(0) as fb:
+        fb.set_stream(stream.cuda_stream)
+        fb.set_metric(s[0])
+        fb.set_3c(s[1], N)
+        dD = torch.from_numpy(np.ascontiguousarray(D)).cuda()
+        dC = torch.from_numpy(np.ascontiguousarray(s[3][:nocc])).cuda()
+        dJ, dK = torch.empty_like(dD), torch.empty_like(dD)
+        torch.cuda.synchronize()
+        refused = False
+        try:
+            with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=stream):
+                try:
+                    fb.fock_device(dD.data_ptr(), dC.data_ptr(), nocc, dJ.data_ptr(), dK.data_ptr())
+                except rijk.RijkError as e:
+                    refused = e.code == rijk.ERR_CUDA
+        except RuntimeError:  # torch on the recording's end
+            pass
+        assert refused
+        torch.cuda.synchronize()
+        fb.fock_device(dD.data_ptr(), dC.data_ptr(), nocc, dJ.data_ptr(), dK.data_ptr())
+        fb.sync()
+        assert all(np.array_equal(a.cpu().numpy(), b) for a, b in zip((dJ, dK), want))
