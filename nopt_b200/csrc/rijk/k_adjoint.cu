@@ -28,12 +28,13 @@
 // Z and u by one GEMM with M (the pairs i >= j packed, u as one more row), the first index of C^T Z C by one
 // GEMM, and the second by one GEMM per orbital row mu, whose epilogue writes the packed pair rows.  Those rows
 // leave in blocks: the copy of one block to the host runs while the next is formed, so the device never holds
-// the whole derivative.  Behind the copies, which take longest (or with each chunk of Y, where those are smaller than
-// all aux functions), dE/d(P|Q) over chunks of aux functions: T^Q = Y^Q C (k_gemm_f64), the packed Gamma tiles
+// the whole derivative.  Behind the copies, which take longest (or with each chunk of Y, where Y of all aux functions
+// does not fit or nothing is copied), dE/d(P|Q) over chunks of aux functions: T^Q = Y^Q C (k_gemm_f64), the packed Gamma tiles
 // (k_gamma_f64), their rows of G by one GEMM with B, and at the end M^T G M; the blocks' GEMMs take the
 // high-priority stream beside it.
-// (H2O)8 cc-pVDZ, 151 MB out: 18.7 ms a call with Gamma for both derivatives and the copies at the end, 7.8 to 9.1 now
-// (the copies' speed differs between hosts); (H2O)16, 126 and 59 to 71.
+// (H2O)8 cc-pVDZ, 151 MB out: 15.5 to 18.7 ms a call with Gamma for both derivatives and the copies at the end, 7.6 to 8.0
+// now (medians of 30 calls in three runs, output arrays reused; with new arrays, whose pages the copies
+// touch first, 38.5 to 39.1 and 29.2 to 30.2); (H2O)16, 126 and 59 to 71.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -321,18 +322,21 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
   const size_t b_pairs = static_cast<size_t>(np + 1) * ldP * sizeof(double);
   // blocks of orbital rows of dE/d(P|mu nu), about 64 MB each and at least one row
   const long blk = std::max<long>(n * naux, (64L << 20) / 8);
-  while ((rc = ensure_tmp(ctx, Y, static_cast<size_t>(qc) * noccp * nocc * sizeof(double), "grad Y"))) {
-    if (qc == 1 || ctx->fail_alloc_after == 0) return chk(rc);
-    qc = (qc + 1) / 2;
+  // With both derivatives wanted Y stays for all aux functions while that fits, beside Z, which does whatever the chunk:
+  // G then follows the first copies out instead of Y's chunks (C40H82 in chunks of 1200: 1.4 against 2.7 s).
+  long qy = dEdPQ && dEdI3 ? naux : qc;
+  while ((rc = ensure_tmp(ctx, Y, static_cast<size_t>(qy) * noccp * nocc * sizeof(double), "grad Y"))) {
+    if (qy == 1 || ctx->fail_alloc_after == 0) return chk(rc);
+    qy = qy > qc ? qc : (qy + 1) / 2;
   }
-  // aux functions per chunk of T and Gamma, in whole tiles of G's rows and no more than Y's: 1 GiB, less if that cannot
+  qc = std::min(qc, qy);
+  const bool behind = dEdPQ && dEdI3 && qy == naux;
+  // aux functions per chunk of T and Gamma, in whole tiles of G's rows and no more than the chunk: 1 GiB, less if that cannot
   // be had (asking for the free memory first took 7 ms a call)
   const long per_q = te + npad * noccp;
   long gq = std::max<long>(1, std::min<long>(naux, (1L << 30) / (8 * per_q)));
   if (gq < naux && gq >= 64) gq -= gq % 64;
   gq = std::min(gq, qc);
-  // G's chunks follow Y's, or all of them the first copies out where Y is there for every aux function
-  const bool behind = dEdPQ && dEdI3 && qc == naux;
   if (dEdPQ && ((rc = chk(ensure_tmp(ctx, Ct, static_cast<size_t>(npad) * noccp * sizeof(double), "grad Ct"))) ||
                 (rc = chk(ensure_tmp(ctx, Gm, static_cast<size_t>(naux) * naux * sizeof(double), "grad G"))) ||
                 (rc = chk(ensure_tmp(ctx, T1, static_cast<size_t>(naux) * naux * sizeof(double), "grad T1")))))
@@ -400,8 +404,8 @@ RIJK_API int rijk_grad(rijk_ctx* ctx, const double* MO, long nocc, const double*
     gemm_f64(h, 1, s);
     tm.mark(6);
   };
-  for (long q0 = 0; q0 < naux; q0 += qc) {
-    const long nq = std::min(qc, naux - q0);
+  for (long q0 = 0; q0 < naux; q0 += qy) {
+    const long nq = std::min(qy, naux - q0);
     // Y^Q[i][j] = sum_nu X^Q_{i nu} C_{j nu} (= C B^Q C^T), every Q of the chunk in one product: rows (Q, i)
     // of X^T's columns are contiguous
     GemmF64Args g;
