@@ -13,12 +13,14 @@
 // largest of B^Q.  So that this means as much to every function, whatever the sizes of the functions, the digits are
 // those of 2^-(e_mu + e_nu) B^Q_{mu nu}, with e_mu such that every row's largest element over all Q is about 1
 // (k_balance, from the magnitudes the metric contraction keeps).  The factors are exact: those of the summed index go into
-// the digits of C, those of the row nu into X.  The rounding of K_{mu nu} against sqrt(K_mu,mu K_nu,nu) is then the same for
-// any scaling of the functions (C12H26, emulated: 3.8e-16 at the most, 1.4e-15 with FP64 FMAs; without the scales
-// 3.7e-10 when the functions' sizes spread over 2^12).  An element far below that, of functions far apart, keeps fewer
-// digits of its own than FP64 FMAs would leave it (1.2e-13 in the median there, against 1.5e-15).
-// Where the rows' largest elements lie within a factor of 16, e = 0 serves as well (6.4e-16 at that factor; of
-// normalised functions in double- and triple-zeta bases they lie within 4 to 10) and saves a pass over B.
+// the digits of C, those of the row nu into X.  The error of K_{mu nu} against sqrt(K_mu,mu K_nu,nu) is then the same for
+// any scaling of the functions by powers of two: at the most 1.6e-15 for C12H26 cc-pVDZ (1.2e-15 on DMMA, 2.2e-5 without
+// the scales when the functions' sizes spread over 2^20), 3e-16 for C24H50 (2.7e-14, 3.7e-6).  An element far below
+// that size, of functions far apart, keeps fewer digits of its own than DMMA would leave it (5e-13 in the median for
+// C24H50, against 8e-15).
+// Where the rows' largest elements lie within a factor of 11, e = 0 serves as well (1.1e-15 for C12H26; 2.6e-15 at a
+// factor of 16) and saves a pass over B: those of normalised functions in double- and triple-zeta bases lie
+// within 3 to 10.
 //
 // k_xform_i8: persistent, one CTA per SM, over items (Q, 128 rows nu, batch of at most 64 orbitals), the batches of
 // one (Q, rows) next to each other so that the later ones find B's digits in L2.  Warp 0 copies stages of
@@ -101,7 +103,7 @@ __global__ void __launch_bounds__(256) k_spread(const float* __restrict__ e, lon
       a = fminf(a, lo[w]);
       b = fmaxf(b, hi[w]);
     }
-    *how = b - a > 2.0f ? kScaled : have_tops ? kPlain : kPlainNoTops;
+    *how = b - a > 1.75f ? kScaled : have_tops ? kPlain : kPlainNoTops;
   }
 }
 

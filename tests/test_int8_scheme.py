@@ -49,14 +49,14 @@ def products(a, b):
 
 
 def row_scales(B):
-    """k_balance, k_spread: exponents e with max_{Q, nu} 2^-(e_mu + e_nu) |B| about 1; none if that holds to a factor 16."""
+    """k_balance, k_spread: exponents e with max_{Q, nu} 2^-(e_mu + e_nu) |B| about 1; none if that holds to a factor 11 (2^(2 x 1.75))."""
     with np.errstate(divide="ignore"):
         L = np.log2(np.max(np.abs(B), axis=0))
     e = np.zeros(len(L))
     for step in range(8):
         m = np.max(L - e[None, :], axis=1)
         e = np.where(np.isfinite(m), 0.5 * (e + m), e)
-        if step == 0 and np.ptp(e) <= 2.0:
+        if step == 0 and np.ptp(e) <= 1.75:
             return np.zeros(len(L), int)
     return np.rint(e).astype(int)
 
