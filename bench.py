@@ -357,9 +357,9 @@ def grad_report(fb, si, MOc, nocc, fp64_peak, reps=3):
     noccp = (nocc + 15) // 16 * 16
     te = st["ntile"] * 4096
     pairs = nocc * (nocc + 1) // 2 + 1  # packed (i, j), and the row of w
-    flops = {"y_t": 2.0 * noccp * nocc * npad * naux, "gamma": 2.0 * pairs * naux * naux + 2.0 * n * nocc * nocc * naux,
-             "d3c_M_gamma": 1.0 * n * (n + 1) * nocc * naux,
-             "g_gamma_B": 2.0 * noccp * nocc * npad * naux + 2.0 * te * noccp * naux + 2.0 * te * naux * naux,
+    flops = {"y": 2.0 * noccp * nocc * npad * naux, "z_and_ctz": 2.0 * pairs * naux * naux + 2.0 * n * nocc * nocc * naux,
+             "d3c_blocks": 1.0 * n * (n + 1) * nocc * naux,
+             "t_gamma_g": 2.0 * noccp * nocc * npad * naux + 2.0 * te * noccp * naux + 2.0 * te * naux * naux,
              "dV_MtGM": 4.0 * naux ** 3}
     stages = {}
     for k, ms in st["grad_stages"].items():
@@ -373,13 +373,13 @@ def grad_report(fb, si, MOc, nocc, fp64_peak, reps=3):
             "stages": stages, "top_stage": top,
             "flops": sum(flops.values()), "fp64_peak_tflops": fp64_peak,
             "what": "rijk_grad through the C ABI: E, dE/dC, dE/d(P|mu nu) (packed) and dE/d(P|Q) to host memory; "
-                    "device_ms = its stages (events; d3c_M_gamma includes its blocks' copies to the host), wall_ms includes "
+                    "device_ms = its stages (events; d3c_blocks includes its blocks' copies to the host), wall_ms includes "
                     "every copy (%.2f GB, into pageable arrays reused between calls)"
                     % ((n * (n + 1) // 2 * naux + naux * naux) * 8 / 1e9)}
 
 
 def c40h82_grad(seed, dev, fp64_peak, chunk=1200):
-    """The C40H82 cc-pVDZ adjoint case: mixed -> FP64 SCF, then rijk_grad with Y^Q in aux chunks."""
+    """The C40H82 cc-pVDZ adjoint case: mixed -> FP64 SCF, then rijk_grad with Y^Q and Gamma^Q in aux chunks."""
     from nopt_b200 import rijk
     si, _, _ = build_system("c40h82_dz", seed, ri_integrals=False)
     with rijk.FockBuilder(dev.index) as fb:

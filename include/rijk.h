@@ -66,12 +66,13 @@ extern "C" {
                              power-of-two scales, 34 exact s32 digit products, FP64 scaling and sums
                              (the Ozaki splitting scheme); the half-transform so only while the
                              digits of B (0.9 to 1.1 times its bytes) find room in device memory.
-                             The digits are fixed-point numbers, scaled so that multiplying a basis
-                             function by a power of two does not matter: the error of K_mn is below
-                             that of FP64 FMAs against sqrt(K_mm K_nn) (4e-16 and 1.4e-15 at the
-                             most for C12H26 cc-pVDZ), but not against each K_mn of its own.  Elements
-                             far below that size, of functions far apart, keep fewer digits of their
-                             own than FMAs leave them: 1.2e-13 in the median there, against 1.5e-15 */
+                             The digits are fixed-point numbers, scaled so that multiplying basis
+                             functions by powers of two does not matter.  The error of K_mn is that of
+                             FP64 FMAs or less against sqrt(K_mm K_nn) (at the most 1.1e-15 and
+                             1.2e-15 for C12H26 cc-pVDZ, 2e-16 and 2.7e-14 for C24H50), but not
+                             against K_mn itself.  Elements far below that size, of functions far
+                             apart, keep fewer digits of their own than FMAs leave them: 5e-14 in the
+                             median for C12H26 against 1e-15, 7e-13 for C24H50 against 8e-15        */
 #define RIJK_PREC_MIXED 1 /* exchange half-transform and K on tcgen05 tensor cores with split-BF16
                              (3-term) operands and FP32 accumulation; Coulomb in FP64          */
 #define RIJK_PREC_FP64_TC 2 /* RIJK_PREC_FP64 with K = X^T X from int8 digits at every size       */
@@ -83,9 +84,9 @@ typedef struct {
   double ms_setup_3c;     /* last rijk_set_3c, device time (metric contraction included)   */
   double ms_last_fock;    /* last Fock build, device time                                   */
   double ms_coulomb;      /* from its start until J is complete (the w and J passes)        */
-  double ms_exchange;     /* from then until its end.  FP64 and FP64_TC builds run the
-                             Coulomb pair beside the exchange, so there the exchange
-                             starts before J is complete; mixed builds run them in turn    */
+  double ms_exchange;     /* from then until its end.  The Coulomb pair runs beside the
+                             exchange (unless profiling is on), so the exchange starts
+                             before J is complete                                          */
   double flops_last_fock; /* algorithmic FLOPs of the last build                            */
   double bytes_last_fock; /* algorithmic HBM bytes of the last build                        */
   long n, naux, npad, ntile;
@@ -108,8 +109,8 @@ typedef struct {
 
 int rijk_create(rijk_ctx** ctx, int device);
 int rijk_destroy(rijk_ctx* ctx);
-/* Run on the caller's CUDA stream (a cudaStream_t) instead of the context's own.  An FP64 or FP64_TC
- * build also runs its Coulomb passes on a second stream the context owns: that stream waits on the
+/* Run on the caller's CUDA stream (a cudaStream_t) instead of the context's own.  A build of any
+ * precision also runs its Coulomb passes on a second stream the context owns: that stream waits on the
  * caller's stream in the build, and the caller's stream waits on it before the build's
  * end, so work queued after the build on the caller's stream sees J and K. */
 int rijk_set_stream(rijk_ctx* ctx, void* stream);
@@ -187,7 +188,10 @@ int rijk_load(rijk_ctx* ctx, const char* path);
 /* Drop-in for DM_to_F_transform_RI(J, K, DM, MO, n_c, n_ao): host pointers, synchronous. */
 int rijk_fock(rijk_ctx* ctx, const double* DM, const double* MO, long n_c, double* J, double* K, int precision);
 
-/* Same on device pointers, asynchronous on the context's stream. */
+/* Same on device pointers, asynchronous on the context's stream.  After a build of the same sizes and
+ * precision it can be recorded into a CUDA graph.  A recorded FP64 build reads B itself, not its digits, so it
+ * may be replayed after a set-up of the same sizes; its half-transform then runs on the FP64 units.  A recorded
+ * mixed build belongs to the tensor it was recorded with. */
 int rijk_fock_device(rijk_ctx* ctx, const double* dDM, const double* dMO, long n_c, double* dJ, double* dK,
                      int precision);
 
@@ -377,7 +381,8 @@ int rijk_soscf_hess_ints(rijk_ctx* ctx, double* aa_J, double* aa_K, const double
 
 /* Aux functions per chunk of rijk_grad's Y^Q, and at most of its Gamma^Q (0, the default: all of them at
  * once, or as many as find room).  A chunk bounds the scratch of dE/d(P|Q) to it; dE/d(P|mu nu) takes 2 n_c^2
- * naux doubles whatever the chunk.  The derivatives do not depend on it. */
+ * naux doubles whatever the chunk, and Y^Q of every aux function is kept beside them while there is room, n_c^2 naux
+ * more.  The derivatives do not depend on it. */
 int rijk_set_grad_chunk(rijk_ctx* ctx, long q_per_chunk);
 
 /* Adjoint of the Fock build (no reference counterpart; the reference differentiates by finite

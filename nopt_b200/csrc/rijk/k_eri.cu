@@ -534,8 +534,9 @@ int eri_tile(long npair, long nket, int wide, int nf, int fixed) {
 
 // Launches every class of one output block.  pairs_dev holds PairLists::pairs on the device.  The classes are
 // independent, and many are too small or end too raggedly to fill the GPU alone: they run on three streams.
-// With the shared tiles, s s sums in registers, long pairs first and the streams, all of (P|Q) and (mu nu|P) took
-// 4.0 instead of 9.4 ms at (H2O)8 cc-pVTZ/cc-pVTZ-JKFIT and 0.13 instead of 0.225 s at (H2O)32.
+// All of (P|Q) and (mu nu|P): 6.5 ms at (H2O)8 cc-pVTZ/cc-pVTZ-JKFIT and 0.234 s at (H2O)32 (31.8 ms and 1.02 s with
+// k_eri alone, on one stream).  Without the shared tiles, s s sums in registers, long pairs first and the streams an earlier
+// form of k_eri_thread, not bound to k_eri's order of operations, took 9.4 instead of 4.0 ms and 0.225 instead of 0.13 s.
 int launch_classes(rijk_ctx* ctx, const EriLaunch& base, const PairLists& pl, const int2* pairs_dev,
                    const KetLists& kl, const int* kets_dev, int* launches) {
   int maxsm = 0;

@@ -32,7 +32,7 @@ _dp = ctypes.POINTER(ctypes.c_double)
 _vp = ctypes.c_void_p
 
 
-GRAD_STAGES = ("fock_energy_dEdC", "x_recompute", "y_t", "gamma", "d3c_M_gamma", "g_gamma_B", "dV_MtGM")
+GRAD_STAGES = ("fock_energy_dEdC", "unused", "y", "z_and_ctz", "d3c_blocks", "t_gamma_g", "dV_MtGM")  # rijk.h: ms_grad_stage
 
 
 class Stats(ctypes.Structure):
