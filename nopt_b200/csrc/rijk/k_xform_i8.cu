@@ -72,7 +72,8 @@ __global__ void __launch_bounds__(256) k_element_max(const double* __restrict__ 
   atomicMax(top + 2 * e + 1, my);
 }
 
-// log2 of a magnitude; nothing to balance where it is zero or not finite
+// log2 of a magnitude; nothing to balance where it is zero or not finite.  A row of nothing else has e = NaN, which the
+// maxima below pass over.
 __device__ __forceinline__ float log2_magnitude(uint32_t top) {
   if (top == 0 || top >= 0x7ff00000u) return -INFINITY;
   return static_cast<float>(static_cast<int>(top >> 20) - 1023) + __log2f(__uint_as_float(0x3f800000u | ((top & 0xfffffu) << 3)));
@@ -124,18 +125,21 @@ __global__ void __launch_bounds__(256) k_balance(const uint32_t* __restrict__ to
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) e1[mu] = m == -INFINITY ? e0[mu] : 0.5f * (e0[mu] + m);
+  if ((threadIdx.x & 31) == 0) e1[mu] = m == -INFINITY ? NAN : 0.5f * (e0[mu] + m);
 }
 constexpr int kBalanceSteps = 8;  // even: the result is where the first step read
 
-// The scales as powers of two, down = 2^-e for B and up = 2^e for C and X.
-__global__ void k_balance_scales(const float* __restrict__ e, long n, long npad2, const int* how,
-                                 double* __restrict__ down, double* __restrict__ up) {
+// The scales as powers of two, down = 2^-e for B and up = 2^e for C and X; e0: the result, e1: any step's.  A function
+// without any element has up = 0: its coefficients, whatever their size against the others', must not set the
+// exponents of C.
+__global__ void k_balance_scales(const float* __restrict__ e0, const float* __restrict__ e1, long n, long npad2,
+                                 const int* how, double* __restrict__ down, double* __restrict__ up) {
   const long mu = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (mu >= npad2) return;
-  const int x = mu < n && *how == kScaled ? static_cast<int>(rintf(fminf(fmaxf(e[mu], -600.f), 600.f))) : 0;
+  const bool none = mu < n && isnan(e1[mu]);
+  const int x = mu < n && !none && *how == kScaled ? static_cast<int>(rintf(fminf(fmaxf(e0[mu], -600.f), 600.f))) : 0;
   down[mu] = pow2i(-x);
-  up[mu] = pow2i(x);
+  up[mu] = none ? 0.0 : pow2i(x);
 }
 
 // top[Q] = the largest magnitude of the scaled B^Q
@@ -606,7 +610,7 @@ bool bdig_prepare(rijk_ctx* ctx) {
   k_spread<<<1, 256, 0, s>>>(sc.e1, ctx->n, ctx->have_btop, sc.how);
   for (int i = 1; i < kBalanceSteps; ++i)
     k_balance<<<rows, 256, 0, s>>>(top, ctx->n, sc.how, i & 1 ? sc.e1 : sc.e0, i & 1 ? sc.e0 : sc.e1);
-  k_balance_scales<<<static_cast<unsigned>(nb), 128, 0, s>>>(sc.e0, ctx->n, npad2, sc.how, sc.down, sc.up);
+  k_balance_scales<<<static_cast<unsigned>(nb), 128, 0, s>>>(sc.e0, sc.e1, ctx->n, npad2, sc.how, sc.down, sc.up);
   cudaMemsetAsync(sc.top, 0, ctx->nq * sizeof(uint32_t), s);
   k_bmax<<<dim3(static_cast<unsigned>(std::min<long>(ctx->ntile, 8)), q), 256, 0, s>>>(B, ctx->ntile, sc.how, sc.down, sc.top);
   k_exponents<<<static_cast<unsigned>((ctx->nq + 255) / 256), 256, 0, s>>>(top + te, sc.top, sc.how, ctx->nq, sc.ex, sc.scale);

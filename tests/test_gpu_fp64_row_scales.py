@@ -46,20 +46,25 @@ def test_k_keeps_its_accuracy_under_row_scales(system, spread, precision):
     assert np.max(np.abs(J - Jr)) <= 1e-11 * np.max(np.abs(Jr))
 
 
-def test_rows_that_couple_to_nothing(system):
-    """Functions without any integral, and one that couples only off the diagonal, between ordinary ones."""
+@pytest.mark.parametrize("exponent", [0, -40, 40])
+def test_rows_that_couple_to_nothing(system, exponent):
+    """Functions without any integral, and one that couples only off the diagonal, between ordinary ones, whose sizes
+    are all of one order or spread: the coefficients of the former are then of another order than all others."""
     V, I3, MO, _ = system
     rows, cols = np.tril_indices(N)
+    s = np.ldexp(1.0, np.where(np.arange(N) % 3, exponent, exponent // 2))
     I3 = I3.copy()
     for dead in (0, 77, N - 1):
         I3[(rows == dead) | (cols == dead)] = 0.0
     I3[(rows == 130) & (cols == 130)] = 0.0
     I3[(rows == 130) ^ (cols == 130)] *= 2.0 ** -30
-    D = O.gen_hf_dm(MO, N, NOCC)
-    Kr = O.dm_to_f_transform_ri(O.unpack_3c(I3, N), O.s05_calc(V)[0], D, MO, NOCC, N)[1]
+    Kr = O.dm_to_f_transform_ri(O.unpack_3c(I3, N), O.s05_calc(V)[0], O.gen_hf_dm(MO, N, NOCC), MO, NOCC, N)[1]
+    C = MO / s
+    for dead in (0, 77, N - 1):
+        C[:, dead] = MO[:, dead]
     with rijk.FockBuilder(0) as fb:
         fb.set_metric(V)
-        fb.set_3c(I3, N)
-        K = fb.dm_to_f_transform_ri(D, MO, NOCC)[1]
+        fb.set_3c(I3 * (s[rows] * s[cols])[:, None], N)
+        K = fb.dm_to_f_transform_ri(O.gen_hf_dm(C, N, NOCC), C, NOCC)[1] / np.outer(s, s)
     d = np.sqrt(np.abs(np.diag(Kr)))
     assert np.all(np.abs(K - Kr) <= 1e-11 * np.outer(d, d))

@@ -54,8 +54,7 @@ def row_scales(B):
         L = np.log2(np.max(np.abs(B), axis=0))
     e = np.zeros(len(L))
     for step in range(8):
-        m = np.max(L - e[None, :], axis=1)
-        e = np.where(np.isfinite(m), 0.5 * (e + m), e)
+        e = 0.5 * (e + np.max(L - e[None, :], axis=1))
         if step == 0 and np.ptp(e) <= 1.75:
             return np.zeros(len(L), int)
     return np.rint(e).astype(int)
