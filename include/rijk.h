@@ -72,7 +72,10 @@ extern "C" {
                              1.2e-15 for C12H26 cc-pVDZ, 2e-16 and 2.7e-14 for C24H50), but not
                              against K_mn itself.  Elements far below that size, of functions far
                              apart, keep fewer digits of their own than FMAs leave them: 5e-14 in the
-                             median for C12H26 against 1e-15, 7e-13 for C24H50 against 8e-15        */
+                             median for C12H26 against 1e-15, 7e-13 for C24H50 against 8e-15.  An
+                             orbital's coefficients are rounded at 2^-55 of its largest one (in those
+                             scales): where every orbital is smaller than that by many orders, K_mm
+                             is, too, and keeps fewer digits by as much                            */
 #define RIJK_PREC_MIXED 1 /* exchange half-transform and K on tcgen05 tensor cores with split-BF16
                              (3-term) operands and FP32 accumulation; Coulomb in FP64          */
 #define RIJK_PREC_FP64_TC 2 /* RIJK_PREC_FP64 with K = X^T X from int8 digits at every size       */
