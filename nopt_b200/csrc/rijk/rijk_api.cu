@@ -108,15 +108,16 @@ int ensure(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
   return ensure_kept(ctx, b, bytes, what, false);
 }
 
-// From the pool where the buffer is small: the set-up has left its scratch there, and a block of that costs
+// From the pool where the buffer is of ordinary size: the set-up has left its scratch there, and a block of that costs
 // next to nothing, where a cudaMalloc maps new memory.  The first build of a new context after rijk_set_basis, FP64:
-// 1.18 -> 0.19 ms at (H2O)2 cc-pVDZ, 1.38 -> 0.35 at (H2O)6, 4.9 -> 4.2 at (H2O)16, whose larger buffers stay apart so that
-// the pool can be trimmed.
-constexpr size_t kPoolBuild = 64ul << 20;
+// 1.18 -> 0.19 ms at (H2O)2 cc-pVDZ, 1.38 -> 0.34 at (H2O)6, 4.9 -> 4.0 to 4.5 at (H2O)16, whose larger buffers stay apart so that
+// the pool can be trimmed.  Below 1 MB the driver packs buffers into pages it has mapped already; in the pool they lie
+// apart, and an FP64_TC build of one water in cc-pVTZ took 62.0 instead of 60.0 us.
+constexpr size_t kPoolLeast = 1ul << 20, kPoolMost = 64ul << 20;
 int ensure_build(rijk_ctx* ctx, DeviceBuf& b, size_t bytes, const char* what) {
   if (b.bytes >= bytes && b.p) return RIJK_OK;
   // (in a recording, a block of the pool would be the graph's; cudaMalloc is refused there)
-  if (!ctx->pool || bytes > kPoolBuild || recording(ctx)) return ensure(ctx, b, bytes, what);
+  if (!ctx->pool || bytes < kPoolLeast || bytes > kPoolMost || recording(ctx)) return ensure(ctx, b, bytes, what);
   int rc = ensure_kept(ctx, b, bytes, what, true);
   // the block is the context's once the work before the allocation has ended: the other streams use it, too
   if (!rc && (rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), what))) release(b);
