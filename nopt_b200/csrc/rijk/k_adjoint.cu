@@ -32,8 +32,8 @@
 // does not fit or nothing is copied), dE/d(P|Q) over chunks of aux functions: T^Q = Y^Q C (k_gemm_f64), the packed Gamma tiles
 // (k_gamma_f64), their rows of G by one GEMM with B, and at the end M^T G M; the blocks' GEMMs take the
 // high-priority stream beside it.
-// (H2O)8 cc-pVDZ, 151 MB out: 15.5 to 18.7 ms a call with Gamma for both derivatives and the copies at the end, 7.6 to 8.0
-// now (medians of 30 calls in three runs, output arrays reused; with new arrays, whose pages the copies
+// (H2O)8 cc-pVDZ, 151 MB out: 15.5 to 18.7 ms a call with Gamma for both derivatives and the copies at the end, 7.6 to 8.5
+// now (medians of 20 to 30 calls in many runs, output arrays reused; with new arrays, whose pages the copies
 // touch first, 38.5 to 39.1 and 29.2 to 30.2); (H2O)16, 126 and 59 to 71.
 #include <algorithm>
 #include <cmath>
